@@ -734,7 +734,7 @@ void DeviceContext::DeregisterBuffer(int id) {
 void DeviceContext::RunCopy(DType dtype, const void* sendbuf, void* recvbuf, size_t n, double scale, cudaStream_t stream) {
   if (sendbuf == recvbuf && scale == 1.0) return;
   CopyParams cp{sendbuf, recvbuf, n, static_cast<int32_t>(dtype), static_cast<int32_t>(dtype), scale};
-  CUDACHECK(LaunchCopyKernel(cp, kCopyDefaultBlocks, stream));
+  CUDACHECK(LaunchCopyKernel(cp, stream));
   ++kernel_launches_;
 }
 

@@ -107,7 +107,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
 
   if (m.ws == 1) {
     CopyParams cp{sendbufs[0], recvbufs[0], n, static_cast<int32_t>(dtype), static_cast<int32_t>(dtype), scale};
-    if (!(sendbufs[0] == recvbufs[0] && scale == 1.0)) CUDACHECK(LaunchCopyKernel(cp, kCopyDefaultBlocks, stream));
+    if (!(sendbufs[0] == recvbufs[0] && scale == 1.0)) CUDACHECK(LaunchCopyKernel(cp, stream));
     m.last_channels = 0;
     if (!async) CUDACHECK(cudaStreamSynchronize(stream));
     return;
@@ -282,7 +282,7 @@ void EmuWorld::ReduceScatterOrAllGather(bool all_gather, DType dtype, const std:
   m.last_status = 0;
   if (m.ws == 1) {
     CopyParams cp{sendbufs[0], recvbufs[0], block_elems, static_cast<int32_t>(dtype), static_cast<int32_t>(dtype), all_gather ? 1.0 : scale};
-    CUDACHECK(LaunchCopyKernel(cp, kCopyDefaultBlocks, stream));
+    CUDACHECK(LaunchCopyKernel(cp, stream));
     if (!async) CUDACHECK(cudaStreamSynchronize(stream));
     return;
   }

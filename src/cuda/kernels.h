@@ -19,8 +19,7 @@ cudaError_t LaunchExecKernel(const ExecParams& p, const ExecParams* emu, int emu
 int ExecKernelThreadsFor(int channels);
 int ExecKernelMaxCoResidentBlocks(int device, int threads = 0);
 
-// ---- world_size == 1, and local staging: out = cast(in * scale) ----
-// Uses bulk asynchronous copies (TMA, non-tensor form) through shared memory.
+// ---- world_size == 1: out = cast(in * scale) ----
 struct CopyParams {
   const void* in;
   void* out;
@@ -29,12 +28,7 @@ struct CopyParams {
   int32_t dtype_out;
   double scale;
 };
-// Eight CTAs per SM of a B200 (one resident at a time, the rest queued): the
-// hardware scheduler then overlaps the tail of one launch with the head of
-// the next, which a one-CTA-per-SM persistent grid cannot (measured: 6.38 TB/s
-// read+write against 5.81 TB/s).
-constexpr int kCopyDefaultBlocks = 148 * 8;
-cudaError_t LaunchCopyKernel(const CopyParams& p, int blocks, cudaStream_t stream);
+cudaError_t LaunchCopyKernel(const CopyParams& p, cudaStream_t stream);
 
 // ---- two-shot allreduce: in the NVSwitch (multimem) or by direct peer loads/stores ----
 struct NvlsParams {

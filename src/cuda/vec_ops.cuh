@@ -48,6 +48,17 @@ __device__ __forceinline__ void St16(void* p, uint4 v) {
   asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+// 32 bytes from / to a 32-byte boundary in one access (sm_100).
+__device__ __forceinline__ void Ld32(const void* p, uint4* lo, uint4* hi) {
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(lo->x), "=r"(lo->y), "=r"(lo->z), "=r"(lo->w), "=r"(hi->x), "=r"(hi->y), "=r"(hi->z), "=r"(hi->w) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void St32(void* p, uint4 lo, uint4 hi) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y),
+               "r"(hi.z), "r"(hi.w)
+               : "memory");
+}
+
 template <typename X> struct VecIO;
 
 template <> struct VecIO<float> {
