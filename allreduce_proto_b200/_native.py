@@ -8,6 +8,7 @@ Every C call returns one of the library's error codes, which
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 from pathlib import Path
 
@@ -48,6 +49,7 @@ class StatusReport(C.Structure):
 
 
 _lib = None
+_fast = None
 
 
 def _declare(lib) -> None:
@@ -123,6 +125,24 @@ def lib():
     _lib = C.CDLL(str(LIB_PATH), mode=C.RTLD_GLOBAL)
     _declare(_lib)
     return _lib
+
+
+def fast():
+    """The extension module of the collectives' call path (src/python/fastcall.cpp), built with the library."""
+    global _fast
+    if _fast is None:
+        lib()
+        path = LIB_DIR / "_fastcall.so"
+        if not path.exists():
+            from . import build as _build
+            _build.build()
+        import torch  # noqa: F401 - the extension links against the libraries torch loads
+        spec = importlib.util.spec_from_file_location("allreduce_proto_b200._fastcall", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_error(IbcommError)
+        _fast = mod
+    return _fast
 
 
 def check(code: int) -> None:

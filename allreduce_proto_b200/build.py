@@ -6,6 +6,8 @@ objects for ``sm_100a`` only) into
 * ``allreduce_proto_b200/_lib/libibcomm_cuda.so`` — host transport, CPU
   schedules, device arena, kernels and the C API the Python package loads
 * ``allreduce_proto_b200/_lib/libibcomm.so`` — host-only variant
+* ``allreduce_proto_b200/_lib/_fastcall.so`` — the Python extension of the
+  collectives' call path (built against the installed torch)
 * ``build/bin/`` — ``ibcomm_run``, ``allreduce_tester``, ``allreduce``,
   ``allreduce_cuda``, ``sendrecv``, ``unittest``, ``bench_sweep``
 
@@ -17,10 +19,12 @@ when a source or any header is newer than the object.
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -128,6 +132,25 @@ def _compile(src: str, variant: str, hdr_mtime: float) -> Path:
     return obj
 
 
+def _build_fastcall(lib_cuda: Path, hdr_mtime: float) -> Path | None:
+    """The Python extension (src/python/fastcall.cpp).  It reads tensors through torch's own headers, so it is
+    rebuilt when the installed torch changes; None when there is no torch to build it for."""
+    spec = importlib.util.find_spec("torch")
+    if spec is None or not spec.submodule_search_locations:
+        return None
+    torch_dir = Path(spec.submodule_search_locations[0])
+    src, out = ROOT / "src" / "python" / "fastcall.cpp", LIB_DIR / "_fastcall.so"
+    if _stale(out, hdr_mtime, src, torch_dir / "version.py"):
+        cuda_inc = Path(_nvcc()).resolve().parent.parent / "include"
+        tmp = out.with_suffix(".tmp.so")
+        _run(["g++", *CXXFLAGS, "-Wno-unused-parameter", "-shared", src, "-o", tmp, f"-I{sysconfig.get_paths()['include']}",
+              "-isystem", torch_dir / "include", "-isystem", torch_dir / "include" / "torch" / "csrc" / "api" / "include",
+              f"-I{cuda_inc}", f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{LIB_DIR}",
+              "-libcomm_cuda", "-Wl,-rpath,$ORIGIN"])
+        os.replace(tmp, out)
+    return out
+
+
 def build(verbose: bool = False, jobs: int | None = None, host_only: bool = False) -> dict:
     """Builds every target that is out of date.  Returns the output paths.
 
@@ -177,6 +200,7 @@ def build(verbose: bool = False, jobs: int | None = None, host_only: bool = Fals
         _run([_nvcc(), *NVCC_ARCH, "-shared", "-o", lib_cuda, *cuda_objs, "-Xcompiler", "-pthread", "-lrt", "-ldl",
               "-cudart", "static"])
     out["libibcomm_cuda"] = lib_cuda if cuda_srcs else None
+    out["_fastcall"] = _build_fastcall(lib_cuda, hdr) if cuda_srcs else None
 
     for name, s, needs_cuda in programs:
         exe = BIN_DIR / name

@@ -1,14 +1,12 @@
 """Functional entry points over a process-wide default communicator."""
 from __future__ import annotations
 
-import ctypes as C
 from typing import Optional
 
 import torch
 
 from .. import _native
-from .._native import check
-from ..parallel.communicator import Communicator, _ptr, dtype_code
+from ..parallel.communicator import Communicator
 
 _default: Optional[Communicator] = None
 
@@ -50,7 +48,5 @@ def copy_scale(src: torch.Tensor, dst: Optional[torch.Tensor] = None, scale: flo
     world-size-1 path of the allreduce)."""
     if dst is None:
         dst = torch.empty_like(src, dtype=out_dtype or src.dtype)
-    s = torch.cuda.current_stream(src.device)
-    check(_native.lib().ibcomm_copy_scale(_ptr(src), _ptr(dst), src.numel(), dtype_code(src.dtype), dtype_code(dst.dtype),
-                                          float(scale), C.c_void_p(s.cuda_stream)))
+    _native.fast().copy_scale(src, dst, scale)
     return dst

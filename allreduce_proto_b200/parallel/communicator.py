@@ -263,22 +263,19 @@ class Communicator:
         fp32 data in 16 bits (sums are accumulated in fp32)."""
         if recvbuf is None:
             recvbuf = sendbuf
+        if sendbuf.is_cuda:
+            _native.fast().allreduce(self._h.value, sendbuf, recvbuf, ALGO_CODES[algo], scale,
+                                     -1 if wire is None else dtype_code(wire), None if stream is None else stream.cuda_stream,
+                                     2 if sync else 3)
+            return recvbuf
         if sendbuf.dtype != recvbuf.dtype or sendbuf.numel() != recvbuf.numel():
             raise IbcommError(_native.INVALID_ARGUMENT, "sendbuf and recvbuf must match in dtype and size")
-        d = dtype_code(sendbuf.dtype)
-        lib = _native.lib()
-        if not sendbuf.is_cuda:
-            if recvbuf.is_cuda:
-                raise IbcommError(_native.INVALID_ARGUMENT, "sendbuf and recvbuf must live on the same kind of device")
-            a = ALGO_CODES["ring" if algo == "auto" else algo]
-            check(lib.ibcomm_allreduce_host(self._h, a, d, _ptr(sendbuf), _ptr(recvbuf), sendbuf.numel()))
-            if scale != 1.0:
-                recvbuf.mul_(scale)
-            return recvbuf
-        w = dtype_code(wire) if wire is not None else d
-        s = stream if stream is not None else torch.cuda.current_stream(sendbuf.device)
-        check(lib.ibcomm_allreduce_cuda(self._h, ALGO_CODES[algo], d, _ptr(sendbuf), _ptr(recvbuf), sendbuf.numel(),
-                                        float(scale), w, C.c_void_p(s.cuda_stream), 2 | (0 if sync else 1)))
+        if recvbuf.is_cuda:
+            raise IbcommError(_native.INVALID_ARGUMENT, "sendbuf and recvbuf must live on the same kind of device")
+        a = ALGO_CODES["ring" if algo == "auto" else algo]
+        check(_native.lib().ibcomm_allreduce_host(self._h, a, dtype_code(sendbuf.dtype), _ptr(sendbuf), _ptr(recvbuf), sendbuf.numel()))
+        if scale != 1.0:
+            recvbuf.mul_(scale)
         return recvbuf
 
     def reduce_scatter(self, sendbuf: torch.Tensor, recvbuf: torch.Tensor, *, algo: str = "auto", scale: float = 1.0,

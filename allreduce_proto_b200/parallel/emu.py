@@ -10,7 +10,7 @@ import torch
 
 from .. import _native
 from .._native import ALGO_CODES, check
-from .communicator import _ptr, dtype_code
+from .communicator import dtype_code
 
 
 class EmuWorld:
@@ -36,32 +36,20 @@ class EmuWorld:
         """``recvbufs[r]`` = scale * sum over r of ``sendbufs[r]`` for every emulated rank."""
         if recvbufs is None:
             recvbufs = sendbufs
-        n = sendbufs[0].numel()
-        d = dtype_code(sendbufs[0].dtype)
-        w = dtype_code(wire) if wire is not None else d
-        ins = (C.c_void_p * self.num_ranks)(*[_ptr(t) for t in sendbufs])
-        outs = (C.c_void_p * self.num_ranks)(*[_ptr(t) for t in recvbufs])
-        s = stream if stream is not None else torch.cuda.current_stream()
-        check(_native.lib().ibcomm_emu_allreduce(self._h, ALGO_CODES[algo], d, ins, outs, n, float(scale), w, channels,
-                                                 C.c_void_p(s.cuda_stream), 0 if sync else 1))
+        _native.fast().emu_allreduce(self._h.value, self.num_ranks, sendbufs, recvbufs, ALGO_CODES[algo], scale,
+                                     -1 if wire is None else dtype_code(wire), channels,
+                                     None if stream is None else stream.cuda_stream, 0 if sync else 1)
         return recvbufs
 
     def reduce_scatter(self, sendbufs: Sequence[torch.Tensor], recvbufs: Sequence[torch.Tensor], *, scale: float = 1.0,
                        channels: int = 0):
         """``recvbufs[r]`` = scale * sum over ranks q of block r of ``sendbufs[q]`` (direct algorithm)."""
-        return self._rsag(0, sendbufs, recvbufs, recvbufs[0].numel(), scale, channels)
+        _native.fast().emu_rsag(self._h.value, self.num_ranks, 0, sendbufs, recvbufs, scale, channels)
+        return recvbufs
 
     def all_gather(self, sendbufs: Sequence[torch.Tensor], recvbufs: Sequence[torch.Tensor], *, channels: int = 0):
         """Block q of every ``recvbufs[r]`` = ``sendbufs[q]`` (direct algorithm)."""
-        return self._rsag(1, sendbufs, recvbufs, sendbufs[0].numel(), 1.0, channels)
-
-    def _rsag(self, all_gather, sendbufs, recvbufs, block, scale, channels):
-        d = dtype_code(sendbufs[0].dtype)
-        ins = (C.c_void_p * self.num_ranks)(*[_ptr(t) for t in sendbufs])
-        outs = (C.c_void_p * self.num_ranks)(*[_ptr(t) for t in recvbufs])
-        s = torch.cuda.current_stream()
-        check(_native.lib().ibcomm_emu_rsag(self._h, all_gather, d, ins, outs, block, float(scale), channels,
-                                            C.c_void_p(s.cuda_stream), 0))
+        _native.fast().emu_rsag(self._h.value, self.num_ranks, 1, sendbufs, recvbufs, 1.0, channels)
         return recvbufs
 
     def set_timeout_ms(self, ms: int) -> None:

@@ -458,14 +458,15 @@ void DeviceContext::OrderAfterPrevious(cudaStream_t stream) {
   // the caller switches streams.  Inside a stream capture the graph's own
   // edges order the collectives; the caller keeps them on one stream.
   // No event is recorded per call (it would put a bubble between
-  // back-to-back kernels); the rare switch of streams waits on the host.
-  if (IsCapturing(stream)) return;
-  if (have_last_ && last_stream_ != stream) CUDACHECK(cudaStreamSynchronize(last_stream_));
+  // back-to-back kernels); the rare switch of streams waits on the host.  A
+  // call on the stream of the one before needs neither the wait nor the query.
+  if (!have_last_ || last_stream_ == stream || IsCapturing(stream)) return;
+  CUDACHECK(cudaStreamSynchronize(last_stream_));
 }
 
 void DeviceContext::MarkIssued(cudaStream_t stream) {
   ++calls_;
-  if (IsCapturing(stream)) return;
+  if ((have_last_ && last_stream_ == stream) || IsCapturing(stream)) return;
   last_stream_ = stream;
   have_last_ = true;
 }
