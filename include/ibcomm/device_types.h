@@ -195,6 +195,10 @@ IBCOMM_HD inline void WindowPart(uint64_t full_nvec, uint64_t nvec, int s, int w
 struct PeerTable {
   unsigned char* arena[kMaxRanks];  // every rank's arena as mapped here
   unsigned char* mc_arena;          // multicast alias of the arenas, or null
+  // 1: every rank of the collective runs on this GPU, so its flags and fences
+  // need the scope of the GPU, not of the system.
+  int32_t one_gpu;
+  int32_t pad_;
 };
 
 struct ExecParams {

@@ -747,7 +747,7 @@ void DeviceContext::RunProgram(Algo algo, DType dtype, DType wire, const void* s
   ExecParams p = MakeExecParams(rr_, cp, dtype, wire, sendbuf, recvbuf, n, scale,
                                 static_cast<uint64_t>(comm_->timeout_ms()) * 1000000ull, trace, cap);
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
-  CUDACHECK(LaunchExecKernel(p, nullptr, 1, channels, stream));
+  CUDACHECK(LaunchExecKernel(&p, 1, channels, stream));
   ++kernel_launches_;
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
 }
@@ -757,7 +757,7 @@ void DeviceContext::RunOneShot(DType dtype, const void* sendbuf, void* recvbuf, 
   OneShotParams p = MakeOneShotParams(rr_, dtype, sendbuf, recvbuf, n, scale,
                                       static_cast<uint64_t>(comm_->timeout_ms()) * 1000000ull);
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
-  CUDACHECK(LaunchOneShotKernel(p, nullptr, 1, channels, stream));
+  CUDACHECK(LaunchOneShotKernel(&p, 1, channels, stream));
   ++kernel_launches_;
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
 }
@@ -919,7 +919,7 @@ bool DeviceContext::RunStaged(bool multimem, DType dtype, DType wire, const void
     pending_trace_.back().roles = p.trace_roles;
   }
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
-  CUDACHECK(LaunchStagedKernel(p, nullptr, 1, split ? 2 * ctas : ctas, stream));
+  CUDACHECK(LaunchStagedKernel(&p, 1, split ? 2 * ctas : ctas, stream));
   ++kernel_launches_;
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
   staged_channels_ = ctas;
@@ -1043,7 +1043,7 @@ void DeviceContext::RunTwoShot(bool multimem, DType dtype, DType wire, const voi
     }
   }
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
-  CUDACHECK(LaunchNvlsKernel(p, nullptr, 1, channels, stream));
+  CUDACHECK(LaunchNvlsKernel(&p, 1, channels, stream));
   ++kernel_launches_;
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
 }
@@ -1244,7 +1244,7 @@ void DeviceContext::ReduceScatterOrAllGather(int mode, DType dtype, const void* 
   }
   OrderAfterPrevious(stream);
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
-  CUDACHECK(LaunchRsAgKernel(p, nullptr, 1, channels, stream));
+  CUDACHECK(LaunchRsAgKernel(&p, 1, channels, stream));
   ++kernel_launches_;
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);
   MarkIssued(stream);

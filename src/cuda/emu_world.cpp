@@ -18,8 +18,6 @@ struct EmuWorld::Impl {
   std::vector<StatusBlock> status;
   std::vector<RankResources> ranks;
   ProgramCache cache;
-  void* d_params = nullptr;  // parameter blocks of one launch
-  size_t d_params_bytes = 0;
   int timeout_ms = env::kDefaultTimeoutMs;
   int max_blocks = 0;
   int last_channels = 0;
@@ -29,15 +27,6 @@ struct EmuWorld::Impl {
   int staged_max_blocks = 0;
   uint32_t last_status = 0;
   DeviceStatus last_report{};
-
-  void* Params(size_t bytes) {
-    if (bytes > d_params_bytes) {
-      if (d_params != nullptr) CUDACHECK(cudaFree(d_params));
-      CUDACHECK(cudaMalloc(&d_params, bytes));
-      d_params_bytes = bytes;
-    }
-    return d_params;
-  }
 };
 
 EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(num_ranks), impl_(new Impl()) {
@@ -61,6 +50,7 @@ EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(nu
     rr.layout = m.layout;
     for (int q = 0; q < num_ranks; ++q) rr.peers.arena[q] = m.arenas + static_cast<size_t>(q) * m.layout.total_bytes;
     rr.peers.mc_arena = nullptr;
+    rr.peers.one_gpu = 1;
     rr.d_status = m.status[static_cast<size_t>(r)].d_status;
     rr.h_doorbell = m.status[static_cast<size_t>(r)].h_doorbell;
     rr.d_doorbell = m.status[static_cast<size_t>(r)].d_doorbell;
@@ -76,7 +66,6 @@ EmuWorld::~EmuWorld() {
   m.cache.Clear();
   for (StatusBlock& s : m.status) s.Destroy();
   if (m.arenas != nullptr) cudaFree(m.arenas);
-  if (m.d_params != nullptr) cudaFree(m.d_params);
   (void)cudaGetLastError();
 }
 
@@ -169,9 +158,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.doorbell = rr.d_doorbell;
       if (r == m.silent_rank) p.len_elements = 0;  // takes no part: no window, no flag
     }
-    void* d = m.Params(ps.size() * sizeof(StagedParams));
-    CUDACHECK(cudaMemcpyAsync(d, ps.data(), ps.size() * sizeof(StagedParams), cudaMemcpyHostToDevice, stream));
-    CUDACHECK(LaunchStagedKernel(ps[0], static_cast<const StagedParams*>(d), m.ws, split ? 2 * ch : ch, stream));
+    CUDACHECK(LaunchStagedKernel(ps.data(), m.ws, split ? 2 * ch : ch, stream));
     m.last_channels = ch;
   } else if (algo == Algo::kDirect) {
     // The two-shot kernel with peer loads and stores.  All ranks' buffers live
@@ -219,9 +206,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.window_elems = staged ? TwoShotWindowElems(n, (half - 4096) / esize, esize, m.ws, ch) : std::max<uint64_t>(1, n);
       p.tail_in_off = half - 4096;  // the ragged end of a staged message lives past every window
     }
-    void* d = m.Params(ps.size() * sizeof(NvlsParams));
-    CUDACHECK(cudaMemcpyAsync(d, ps.data(), ps.size() * sizeof(NvlsParams), cudaMemcpyHostToDevice, stream));
-    CUDACHECK(LaunchNvlsKernel(ps[0], static_cast<const NvlsParams*>(d), m.ws, ch, stream));
+    CUDACHECK(LaunchNvlsKernel(ps.data(), m.ws, ch, stream));
     m.last_channels = ch;
   } else if (algo == Algo::kOneShot) {
     if (bytes > m.layout.oneshot_slot_bytes)
@@ -233,9 +218,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
                                      recvbufs[static_cast<size_t>(r)], n, scale, timeout_ns));
     int ch = channels > 0 ? channels : ChooseChannels(Algo::kOneShot, bytes, m.ws, kMaxChannels);
     ch = std::min(ch, cap);
-    void* d = m.Params(ps.size() * sizeof(OneShotParams));
-    CUDACHECK(cudaMemcpyAsync(d, ps.data(), ps.size() * sizeof(OneShotParams), cudaMemcpyHostToDevice, stream));
-    CUDACHECK(LaunchOneShotKernel(ps[0], static_cast<const OneShotParams*>(d), m.ws, ch, stream));
+    CUDACHECK(LaunchOneShotKernel(ps.data(), m.ws, ch, stream));
     m.last_channels = ch;
   } else {
     // Validation (length, chunk size) happens while the first program is cut.
@@ -249,9 +232,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
     }
     int ch = channels > 0 ? channels : ChooseChannels(algo, bytes, m.ws, kMaxChannels);
     ch = std::min(ch, cap);
-    void* d = m.Params(ps.size() * sizeof(ExecParams));
-    CUDACHECK(cudaMemcpyAsync(d, ps.data(), ps.size() * sizeof(ExecParams), cudaMemcpyHostToDevice, stream));
-    CUDACHECK(LaunchExecKernel(ps[0], static_cast<const ExecParams*>(d), m.ws, ch, stream));
+    CUDACHECK(LaunchExecKernel(ps.data(), m.ws, ch, stream));
     m.last_channels = ch;
   }
   if (async) return;
@@ -333,9 +314,7 @@ void EmuWorld::ReduceScatterOrAllGather(bool all_gather, DType dtype, const std:
       p.window_elems = block_elems;
     }
   }
-  void* d = m.Params(ps.size() * sizeof(RsAgParams));
-  CUDACHECK(cudaMemcpyAsync(d, ps.data(), ps.size() * sizeof(RsAgParams), cudaMemcpyHostToDevice, stream));
-  CUDACHECK(LaunchRsAgKernel(ps[0], static_cast<const RsAgParams*>(d), m.ws, ch, stream));
+  CUDACHECK(LaunchRsAgKernel(ps.data(), m.ws, ch, stream));
   m.last_channels = ch;
   if (async) return;
   CUDACHECK(cudaStreamSynchronize(stream));

@@ -19,9 +19,9 @@
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda
 // (ibcomm/allreduce_cuda_impl.h:24-33, 103-299, 470-707).
 //
-// With `emu` non-null the grid is (channels, ranks): blockIdx.y selects the
-// rank whose parameters to use, so that several ranks that share one GPU run
-// as ONE cooperative launch (CTAs that wait on each other are co-resident).
+// The grid is (channels, ranks): blockIdx.y selects the rank whose parameters
+// to use, so that several ranks that share one GPU run as ONE cooperative
+// launch (CTAs that wait on each other are co-resident).
 #include <cooperative_groups.h>
 
 #include <cstdlib>
@@ -238,7 +238,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, RoleSync* sync) {
   // Entry barrier per channel: every peer's channel `ch` has started this
   // call, hence finished the previous one, so staging slots are free.
   if (threadIdx.x < p.world_size && threadIdx.x != p.rank) {
-    StReleaseSys(&Ctl(p.peers, threadIdx.x)->bar[ch][p.rank], base | 1u);
+    StReleasePeers(&Ctl(p.peers, threadIdx.x)->bar[ch][p.rank], base | 1u, p.peers.one_gpu != 0);
     if (!WaitGE(&me->bar[ch][threadIdx.x], base | 1u, w, kWaitBarrier, threadIdx.x, -1)) *stop = 1;
   }
   __syncthreads();
@@ -319,7 +319,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, RoleSync* sync) {
         if (!all) break;
         const Op op = p.ops[oi];
         if (op.post_out != 0) {
-          FenceSys();
+          FencePeers(p.peers.one_gpu != 0);
           StRelaxedSys(&Ctl(p.peers, op.peer_out)->inflag[ch][p.rank], base | op.post_out);
         }
         if (op.post_credit != 0) StRelaxedSys(&Ctl(p.peers, op.peer_in)->credit[ch][p.rank], base | op.post_credit);
@@ -331,13 +331,12 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, RoleSync* sync) {
 
 template <typename T, typename W>
 __global__ void __launch_bounds__(kExecThreads, 1)
-ExecKernel(const __grid_constant__ ExecParams p0, const ExecParams* __restrict__ emu) {
+ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all) {
   __shared__ ExecParams p;
   __shared__ RoleSync s_sync;
   __shared__ uint64_t s_seq;
   {
-    const uint32_t* src = (emu != nullptr) ? reinterpret_cast<const uint32_t*>(emu + blockIdx.y)
-                                           : reinterpret_cast<const uint32_t*>(&p0);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
     for (unsigned i = threadIdx.x; i < sizeof(ExecParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
     if (threadIdx.x == 0) RoleSyncInit(&s_sync);
   }
@@ -357,31 +356,22 @@ static int ExecThreads() {
 }
 
 template <typename T, typename W>
-static cudaError_t Launch(const ExecParams& p, const ExecParams* emu, int emu_ranks, int channels, cudaStream_t stream) {
-  dim3 grid(static_cast<unsigned>(channels), static_cast<unsigned>(emu != nullptr ? emu_ranks : 1));
+static cudaError_t Launch(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
   // Beyond one CTA per SM, two smaller CTAs share an SM: while one waits for a
   // flag, the other streams.
-  const int kThreads = ExecKernelThreadsFor(channels);
-  if (emu != nullptr) {
-    // Ranks sharing one GPU wait on each other inside this launch: it must be
-    // cooperative so the runtime refuses a grid that cannot be co-resident.
-    void* args[] = {const_cast<ExecParams*>(&p), &emu};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(dev::ExecKernel<T, W>), grid, dim3(kThreads), args, 0, stream);
-  }
-  dev::ExecKernel<T, W><<<grid, kThreads, 0, stream>>>(p, nullptr);
-  return cudaGetLastError();
+  return LaunchRanks(dev::ExecKernel<T, W>, ranks, n, channels, ExecKernelThreadsFor(channels), 0, stream);
 }
 
-cudaError_t LaunchExecKernel(const ExecParams& p, const ExecParams* emu, int emu_ranks, int channels, cudaStream_t stream) {
-  const DType t = static_cast<DType>(p.dtype), w = static_cast<DType>(p.wire);
-  if (t == DType::kFloat32 && w == DType::kFloat32) return Launch<float, float>(p, emu, emu_ranks, channels, stream);
-  if (t == DType::kFloat32 && w == DType::kBFloat16) return Launch<float, __nv_bfloat16>(p, emu, emu_ranks, channels, stream);
-  if (t == DType::kFloat32 && w == DType::kFloat16) return Launch<float, __half>(p, emu, emu_ranks, channels, stream);
-  if (t == DType::kFloat64 && w == t) return Launch<double, double>(p, emu, emu_ranks, channels, stream);
-  if (t == DType::kInt32 && w == t) return Launch<int, int>(p, emu, emu_ranks, channels, stream);
-  if (t == DType::kInt64 && w == t) return Launch<long long, long long>(p, emu, emu_ranks, channels, stream);
-  if (t == DType::kFloat16 && w == t) return Launch<__half, __half>(p, emu, emu_ranks, channels, stream);
-  if (t == DType::kBFloat16 && w == t) return Launch<__nv_bfloat16, __nv_bfloat16>(p, emu, emu_ranks, channels, stream);
+cudaError_t LaunchExecKernel(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
+  const DType t = static_cast<DType>(ranks->dtype), w = static_cast<DType>(ranks->wire);
+  if (t == DType::kFloat32 && w == DType::kFloat32) return Launch<float, float>(ranks, n, channels, stream);
+  if (t == DType::kFloat32 && w == DType::kBFloat16) return Launch<float, __nv_bfloat16>(ranks, n, channels, stream);
+  if (t == DType::kFloat32 && w == DType::kFloat16) return Launch<float, __half>(ranks, n, channels, stream);
+  if (t == DType::kFloat64 && w == t) return Launch<double, double>(ranks, n, channels, stream);
+  if (t == DType::kInt32 && w == t) return Launch<int, int>(ranks, n, channels, stream);
+  if (t == DType::kInt64 && w == t) return Launch<long long, long long>(ranks, n, channels, stream);
+  if (t == DType::kFloat16 && w == t) return Launch<__half, __half>(ranks, n, channels, stream);
+  if (t == DType::kBFloat16 && w == t) return Launch<__nv_bfloat16, __nv_bfloat16>(ranks, n, channels, stream);
   return cudaErrorInvalidValue;
 }
 

@@ -29,6 +29,21 @@ __device__ __forceinline__ void StRelaxedSys(uint64_t* p, uint64_t v) {
   asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ void FenceSys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
+// The same with the scope the ranks of a collective need (PeerTable::one_gpu).
+__device__ __forceinline__ uint64_t LdAcquirePeers(const uint64_t* p, bool one_gpu) {
+  if (!one_gpu) return LdAcquireSys(p);
+  uint64_t v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void StReleasePeers(uint64_t* p, uint64_t v, bool one_gpu) {
+  if (!one_gpu) StReleaseSys(p, v);
+  else asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void FencePeers(bool one_gpu) {
+  if (!one_gpu) FenceSys();
+  else asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
 __device__ __forceinline__ uint64_t GlobalTimerNs() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -102,12 +117,13 @@ __device__ inline void BroadcastAbort(const WaitCtx& w) {
 // call was aborted elsewhere; the failure has then been reported.
 __device__ inline bool WaitGE(const uint64_t* flag, uint64_t target, const WaitCtx& w, uint32_t kind, int peer,
                               int op_index) {
-  uint64_t v = LdAcquireSys(flag);
+  const bool one_gpu = w.peers->one_gpu != 0;
+  uint64_t v = LdAcquirePeers(flag, one_gpu);
   if (v >= target) return true;
   const uint64_t t0 = GlobalTimerNs();
   const uint64_t* abort_word = &Ctl(*w.peers, w.rank)->abort_seq;
   for (uint32_t spin = 1;; ++spin) {
-    v = LdAcquireSys(flag);
+    v = LdAcquirePeers(flag, one_gpu);
     if (v >= target) return true;
     if ((spin & 31u) == 0u) {
       if (LdRelaxedSys(abort_word) == w.seq) {

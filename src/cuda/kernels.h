@@ -8,10 +8,34 @@
 
 namespace ibcomm {
 
+// The parameter blocks of one launch, by value: block `blockIdx.y` belongs to
+// the rank those CTAs work for.  A rank with a GPU of its own fills one, ranks
+// that share a GPU one each.  By value, because a copy into device memory
+// ahead of the launch costs the host 2 us and the stream another 2-4 us
+// between two kernels, and the size costs nothing (an empty kernel: 2.3 us
+// per launch with 64 bytes of parameters as with 3500).
+template <typename P>
+struct RankBlocks {
+  P rank[kMaxRanks];
+};
+// grid = (blocks, ranks).  With several ranks the launch is cooperative: their
+// CTAs wait on each other, so the runtime has to refuse a grid that is not
+// co-resident.
+template <typename P>
+cudaError_t LaunchRanks(void (*kernel)(RankBlocks<P>), const P* ranks, int n, int blocks, int threads, size_t smem, cudaStream_t stream) {
+  static_assert(sizeof(RankBlocks<P>) <= 4096, "kernel parameters");
+  if (n < 1 || n > kMaxRanks) return cudaErrorInvalidValue;
+  RankBlocks<P> all;
+  for (int r = 0; r < n; ++r) all.rank[r] = ranks[r];
+  void* args[] = {&all};
+  const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(n));
+  if (n > 1) return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, dim3(static_cast<unsigned>(threads)), args, smem, stream);
+  return cudaLaunchKernel(reinterpret_cast<const void*>(kernel), grid, dim3(static_cast<unsigned>(threads)), args, smem, stream);
+}
+
 // ---- op-program executor (ring, Rabenseifner) ----
-// `emu` == nullptr: one rank, grid = channels.  Otherwise `emu` points to
-// `emu_ranks` parameter blocks in device memory and the launch is cooperative.
-cudaError_t LaunchExecKernel(const ExecParams& p, const ExecParams* emu, int emu_ranks, int channels, cudaStream_t stream);
+// Here and below: `ranks` points to `n` parameter blocks, one per rank on this GPU.
+cudaError_t LaunchExecKernel(const ExecParams* ranks, int n, int channels, cudaStream_t stream);
 // CTA size the executor uses for a grid of `channels` CTAs, and the largest
 // grid of CTAs of `threads` threads (0 = the full-size CTA) that is co-resident
 // on `device` (0 on error).  CTA b of a rank waits for CTA b of the other
@@ -64,7 +88,7 @@ struct NvlsParams {
   DeviceStatus* status;
   uint32_t* doorbell;
 };
-cudaError_t LaunchNvlsKernel(const NvlsParams& p, const NvlsParams* emu, int emu_ranks, int blocks, cudaStream_t stream);
+cudaError_t LaunchNvlsKernel(const NvlsParams* ranks, int n, int blocks, cudaStream_t stream);
 // Largest co-resident grid of the two-shot kernels (they share CTA size and register budget).
 int TwoShotKernelMaxCoResidentBlocks(int device);
 
@@ -121,7 +145,7 @@ struct StagedParams {
   int32_t load_groups, reduce_groups, store_groups;
   int32_t posters;  // split mode: a poster warp per reducer group fences and publishes behind the data warps
 };
-cudaError_t LaunchStagedKernel(const StagedParams& p, const StagedParams* emu, int emu_ranks, int blocks, cudaStream_t stream);
+cudaError_t LaunchStagedKernel(const StagedParams* ranks, int n, int blocks, cudaStream_t stream);
 // Largest grid of the staged kernel that is co-resident on `device` (0 on error).
 int StagedKernelMaxCoResidentBlocks(int device);
 
@@ -152,7 +176,7 @@ struct RsAgParams {
   DeviceStatus* status;
   uint32_t* doorbell;
 };
-cudaError_t LaunchRsAgKernel(const RsAgParams& p, const RsAgParams* emu, int emu_ranks, int blocks, cudaStream_t stream);
+cudaError_t LaunchRsAgKernel(const RsAgParams* ranks, int n, int blocks, cudaStream_t stream);
 
 // ---- one-shot allreduce for small messages (push to every peer, sum locally) ----
 struct OneShotParams {
@@ -171,7 +195,7 @@ struct OneShotParams {
   DeviceStatus* status;
   uint32_t* doorbell;
 };
-cudaError_t LaunchOneShotKernel(const OneShotParams& p, const OneShotParams* emu, int emu_ranks, int blocks, cudaStream_t stream);
+cudaError_t LaunchOneShotKernel(const OneShotParams* ranks, int n, int blocks, cudaStream_t stream);
 
 // ---- two-sided device messaging through the peer's mailbox ----
 struct P2pParams {

@@ -168,12 +168,12 @@ __device__ void TwoShotBody(const NvlsParams& p, uint64_t seq, int& s_stop) {
 }
 
 template <typename T, int U, bool kMultimem, int kR>
-__global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_constant__ NvlsParams p0, const NvlsParams* __restrict__ emu) {
+__global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_constant__ RankBlocks<NvlsParams> all) {
   __shared__ NvlsParams p;
   __shared__ int s_stop;
   __shared__ uint64_t s_seq;
   {
-    const uint32_t* src = (emu != nullptr) ? reinterpret_cast<const uint32_t*>(emu + blockIdx.y) : reinterpret_cast<const uint32_t*>(&p0);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
     for (unsigned i = threadIdx.x; i < sizeof(NvlsParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
     if (threadIdx.x == 0) s_stop = 0;
   }
@@ -186,34 +186,28 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_const
 }  // namespace dev
 
 template <typename T, int U, bool kMultimem, int kR>
-static cudaError_t LaunchNvlsU(const NvlsParams& p, const NvlsParams* emu, int emu_ranks, int blocks, int threads, cudaStream_t stream) {
-  dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(emu != nullptr ? emu_ranks : 1));
-  if (emu != nullptr) {
-    void* args[] = {const_cast<NvlsParams*>(&p), &emu};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(dev::NvlsKernel<T, U, kMultimem, kR>), grid, dim3(threads), args, 0, stream);
-  }
-  dev::NvlsKernel<T, U, kMultimem, kR><<<grid, threads, 0, stream>>>(p, nullptr);
-  return cudaGetLastError();
+static cudaError_t LaunchNvlsU(const NvlsParams* ranks, int n, int blocks, int threads, cudaStream_t stream) {
+  return LaunchRanks(dev::NvlsKernel<T, U, kMultimem, kR>, ranks, n, blocks, threads, 0, stream);
 }
 
 template <typename T>
-static cudaError_t LaunchNvlsTyped(const NvlsParams& p, const NvlsParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
+static cudaError_t LaunchNvlsTyped(const NvlsParams* ranks, int n, int blocks, cudaStream_t stream) {
   // Tuning knobs for experiments: loads in flight per thread and CTA size.
   const int unroll = Tunable("IBCOMM_NVLS_UNROLL", 4);
   const int threads_env = Tunable("IBCOMM_NVLS_THREADS", dev::kNvlsThreads);
   const int threads = (threads_env >= 64 && threads_env <= dev::kNvlsThreads && threads_env % 32 == 0) ? threads_env : dev::kNvlsThreads;
-  if (!p.use_multimem) {
+  if (!ranks->use_multimem) {
     // Direct variant: compiled per world-size class (loads in flight per rank).
-    switch (dev::RankClass(p.world_size)) {
-      case 2: return LaunchNvlsU<T, 4, false, 2>(p, emu, emu_ranks, blocks, threads, stream);
-      case 4: return LaunchNvlsU<T, 4, false, 4>(p, emu, emu_ranks, blocks, threads, stream);
-      default: return LaunchNvlsU<T, 4, false, kMaxRanks>(p, emu, emu_ranks, blocks, threads, stream);
+    switch (dev::RankClass(ranks->world_size)) {
+      case 2: return LaunchNvlsU<T, 4, false, 2>(ranks, n, blocks, threads, stream);
+      case 4: return LaunchNvlsU<T, 4, false, 4>(ranks, n, blocks, threads, stream);
+      default: return LaunchNvlsU<T, 4, false, kMaxRanks>(ranks, n, blocks, threads, stream);
     }
   }
   if constexpr (dev::HasMultimem<T>::value) {
-    if (unroll == 8) return LaunchNvlsU<T, 8, true, kMaxRanks>(p, emu, emu_ranks, blocks, threads, stream);
-    if (unroll == 2) return LaunchNvlsU<T, 2, true, kMaxRanks>(p, emu, emu_ranks, blocks, threads, stream);
-    return LaunchNvlsU<T, 4, true, kMaxRanks>(p, emu, emu_ranks, blocks, threads, stream);
+    if (unroll == 8) return LaunchNvlsU<T, 8, true, kMaxRanks>(ranks, n, blocks, threads, stream);
+    if (unroll == 2) return LaunchNvlsU<T, 2, true, kMaxRanks>(ranks, n, blocks, threads, stream);
+    return LaunchNvlsU<T, 4, true, kMaxRanks>(ranks, n, blocks, threads, stream);
   } else {
     return cudaErrorInvalidValue;
   }
@@ -226,16 +220,16 @@ int TwoShotKernelMaxCoResidentBlocks(int device) {
   return per_sm * sms;
 }
 
-cudaError_t LaunchNvlsKernel(const NvlsParams& p, const NvlsParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  const DType t = static_cast<DType>(p.dtype);
-  if (p.use_multimem && !(t == DType::kFloat32 || t == DType::kFloat16 || t == DType::kBFloat16)) return cudaErrorInvalidValue;
+cudaError_t LaunchNvlsKernel(const NvlsParams* ranks, int n, int blocks, cudaStream_t stream) {
+  const DType t = static_cast<DType>(ranks->dtype);
+  if (ranks->use_multimem && !(t == DType::kFloat32 || t == DType::kFloat16 || t == DType::kBFloat16)) return cudaErrorInvalidValue;
   switch (t) {
-    case DType::kFloat32: return LaunchNvlsTyped<float>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat16: return LaunchNvlsTyped<__half>(p, emu, emu_ranks, blocks, stream);
-    case DType::kBFloat16: return LaunchNvlsTyped<__nv_bfloat16>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat64: return LaunchNvlsTyped<double>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt32: return LaunchNvlsTyped<int>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt64: return LaunchNvlsTyped<long long>(p, emu, emu_ranks, blocks, stream);
+    case DType::kFloat32: return LaunchNvlsTyped<float>(ranks, n, blocks, stream);
+    case DType::kFloat16: return LaunchNvlsTyped<__half>(ranks, n, blocks, stream);
+    case DType::kBFloat16: return LaunchNvlsTyped<__nv_bfloat16>(ranks, n, blocks, stream);
+    case DType::kFloat64: return LaunchNvlsTyped<double>(ranks, n, blocks, stream);
+    case DType::kInt32: return LaunchNvlsTyped<int>(ranks, n, blocks, stream);
+    case DType::kInt64: return LaunchNvlsTyped<long long>(ranks, n, blocks, stream);
   }
   return cudaErrorInvalidValue;
 }

@@ -86,7 +86,7 @@ __device__ void OneShotBody(const OneShotParams& p, uint64_t seq, int& s_stop) {
   // (2) tell them, (3) wait for theirs.
   if (threadIdx.x < ws && static_cast<int>(threadIdx.x) != me) {
     const int q = threadIdx.x;
-    StReleaseSys(&Ctl(p.peers, q)->oneshot_flag[parity][cta][me], seq);  // release: the pushes above come first
+    StReleasePeers(&Ctl(p.peers, q)->oneshot_flag[parity][cta][me], seq, p.peers.one_gpu != 0);  // release: the pushes above come first
     if (!WaitGE(&Ctl(p.peers, me)->oneshot_flag[parity][cta][q], seq, w, kWaitOneShot, q, -1)) s_stop = 1;
   }
   __syncthreads();
@@ -118,12 +118,12 @@ __device__ void OneShotBody(const OneShotParams& p, uint64_t seq, int& s_stop) {
 
 template <typename T>
 __global__ void __launch_bounds__(kOneShotThreads, 1)
-OneShotKernel(const __grid_constant__ OneShotParams p0, const OneShotParams* __restrict__ emu) {
+OneShotKernel(const __grid_constant__ RankBlocks<OneShotParams> all) {
   __shared__ OneShotParams p;
   __shared__ int s_stop;
   __shared__ uint64_t s_seq;
   {
-    const uint32_t* src = (emu != nullptr) ? reinterpret_cast<const uint32_t*>(emu + blockIdx.y) : reinterpret_cast<const uint32_t*>(&p0);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
     for (unsigned i = threadIdx.x; i < sizeof(OneShotParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
     if (threadIdx.x == 0) s_stop = 0;
   }
@@ -136,24 +136,18 @@ OneShotKernel(const __grid_constant__ OneShotParams p0, const OneShotParams* __r
 }  // namespace dev
 
 template <typename T>
-static cudaError_t LaunchOneShotTyped(const OneShotParams& p, const OneShotParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(emu != nullptr ? emu_ranks : 1));
-  if (emu != nullptr) {
-    void* args[] = {const_cast<OneShotParams*>(&p), &emu};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(dev::OneShotKernel<T>), grid, dim3(dev::kOneShotThreads), args, 0, stream);
-  }
-  dev::OneShotKernel<T><<<grid, dev::kOneShotThreads, 0, stream>>>(p, nullptr);
-  return cudaGetLastError();
+static cudaError_t LaunchOneShotTyped(const OneShotParams* ranks, int n, int blocks, cudaStream_t stream) {
+  return LaunchRanks(dev::OneShotKernel<T>, ranks, n, blocks, dev::kOneShotThreads, 0, stream);
 }
 
-cudaError_t LaunchOneShotKernel(const OneShotParams& p, const OneShotParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  switch (static_cast<DType>(p.dtype)) {
-    case DType::kFloat32: return LaunchOneShotTyped<float>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat64: return LaunchOneShotTyped<double>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt32: return LaunchOneShotTyped<int>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt64: return LaunchOneShotTyped<long long>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat16: return LaunchOneShotTyped<__half>(p, emu, emu_ranks, blocks, stream);
-    case DType::kBFloat16: return LaunchOneShotTyped<__nv_bfloat16>(p, emu, emu_ranks, blocks, stream);
+cudaError_t LaunchOneShotKernel(const OneShotParams* ranks, int n, int blocks, cudaStream_t stream) {
+  switch (static_cast<DType>(ranks->dtype)) {
+    case DType::kFloat32: return LaunchOneShotTyped<float>(ranks, n, blocks, stream);
+    case DType::kFloat64: return LaunchOneShotTyped<double>(ranks, n, blocks, stream);
+    case DType::kInt32: return LaunchOneShotTyped<int>(ranks, n, blocks, stream);
+    case DType::kInt64: return LaunchOneShotTyped<long long>(ranks, n, blocks, stream);
+    case DType::kFloat16: return LaunchOneShotTyped<__half>(ranks, n, blocks, stream);
+    case DType::kBFloat16: return LaunchOneShotTyped<__nv_bfloat16>(ranks, n, blocks, stream);
   }
   return cudaErrorInvalidValue;
 }

@@ -186,12 +186,12 @@ __device__ void RsAgBody(const RsAgParams& p, uint64_t seq, int& s_stop) {
 }
 
 template <typename T, bool kMultimem, bool kVec, int kR>
-__global__ void __launch_bounds__(kNvlsThreads, 1) RsAgKernel(const __grid_constant__ RsAgParams p0, const RsAgParams* __restrict__ emu) {
+__global__ void __launch_bounds__(kNvlsThreads, 1) RsAgKernel(const __grid_constant__ RankBlocks<RsAgParams> all) {
   __shared__ RsAgParams p;
   __shared__ int s_stop;
   __shared__ uint64_t s_seq;
   {
-    const uint32_t* src = (emu != nullptr) ? reinterpret_cast<const uint32_t*>(emu + blockIdx.y) : reinterpret_cast<const uint32_t*>(&p0);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
     for (unsigned i = threadIdx.x; i < sizeof(RsAgParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
     if (threadIdx.x == 0) s_stop = 0;
   }
@@ -204,46 +204,38 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) RsAgKernel(const __grid_const
 }  // namespace dev
 
 template <typename T, bool kMultimem, bool kVec, int kR>
-static cudaError_t LaunchRsAgU(const RsAgParams& p, const RsAgParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(emu != nullptr ? emu_ranks : 1));
-  if (emu != nullptr) {
-    // Emulated ranks wait on each other inside this launch: cooperative, so
-    // the runtime refuses a grid that cannot be co-resident.
-    void* args[] = {const_cast<RsAgParams*>(&p), &emu};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(dev::RsAgKernel<T, kMultimem, kVec, kR>), grid, dim3(dev::kNvlsThreads), args, 0, stream);
-  }
-  dev::RsAgKernel<T, kMultimem, kVec, kR><<<grid, dev::kNvlsThreads, 0, stream>>>(p, nullptr);
-  return cudaGetLastError();
+static cudaError_t LaunchRsAgU(const RsAgParams* ranks, int n, int blocks, cudaStream_t stream) {
+  return LaunchRanks(dev::RsAgKernel<T, kMultimem, kVec, kR>, ranks, n, blocks, dev::kNvlsThreads, 0, stream);
 }
 
 template <typename T>
-static cudaError_t LaunchRsAgTyped(const RsAgParams& p, const RsAgParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  const bool vec = (p.block_elems * sizeof(T)) % 16 == 0;
-  if (p.use_multimem) {
+static cudaError_t LaunchRsAgTyped(const RsAgParams* ranks, int n, int blocks, cudaStream_t stream) {
+  const bool vec = (ranks->block_elems * sizeof(T)) % 16 == 0;
+  if (ranks->use_multimem) {
     if constexpr (dev::HasMultimem<T>::value) {
       if (!vec) return cudaErrorInvalidValue;
-      return LaunchRsAgU<T, true, true, kMaxRanks>(p, emu, emu_ranks, blocks, stream);
+      return LaunchRsAgU<T, true, true, kMaxRanks>(ranks, n, blocks, stream);
     } else {
       return cudaErrorInvalidValue;
     }
   }
-  if (!vec) return LaunchRsAgU<T, false, false, kMaxRanks>(p, emu, emu_ranks, blocks, stream);
+  if (!vec) return LaunchRsAgU<T, false, false, kMaxRanks>(ranks, n, blocks, stream);
   // Peer loads: compiled per world-size class (loads in flight per rank).
-  switch (dev::RankClass(p.world_size)) {
-    case 2: return LaunchRsAgU<T, false, true, 2>(p, emu, emu_ranks, blocks, stream);
-    case 4: return LaunchRsAgU<T, false, true, 4>(p, emu, emu_ranks, blocks, stream);
-    default: return LaunchRsAgU<T, false, true, kMaxRanks>(p, emu, emu_ranks, blocks, stream);
+  switch (dev::RankClass(ranks->world_size)) {
+    case 2: return LaunchRsAgU<T, false, true, 2>(ranks, n, blocks, stream);
+    case 4: return LaunchRsAgU<T, false, true, 4>(ranks, n, blocks, stream);
+    default: return LaunchRsAgU<T, false, true, kMaxRanks>(ranks, n, blocks, stream);
   }
 }
 
-cudaError_t LaunchRsAgKernel(const RsAgParams& p, const RsAgParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  switch (static_cast<DType>(p.dtype)) {
-    case DType::kFloat32: return LaunchRsAgTyped<float>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat16: return LaunchRsAgTyped<__half>(p, emu, emu_ranks, blocks, stream);
-    case DType::kBFloat16: return LaunchRsAgTyped<__nv_bfloat16>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat64: return LaunchRsAgTyped<double>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt32: return LaunchRsAgTyped<int>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt64: return LaunchRsAgTyped<long long>(p, emu, emu_ranks, blocks, stream);
+cudaError_t LaunchRsAgKernel(const RsAgParams* ranks, int n, int blocks, cudaStream_t stream) {
+  switch (static_cast<DType>(ranks->dtype)) {
+    case DType::kFloat32: return LaunchRsAgTyped<float>(ranks, n, blocks, stream);
+    case DType::kFloat16: return LaunchRsAgTyped<__half>(ranks, n, blocks, stream);
+    case DType::kBFloat16: return LaunchRsAgTyped<__nv_bfloat16>(ranks, n, blocks, stream);
+    case DType::kFloat64: return LaunchRsAgTyped<double>(ranks, n, blocks, stream);
+    case DType::kInt32: return LaunchRsAgTyped<int>(ranks, n, blocks, stream);
+    case DType::kInt64: return LaunchRsAgTyped<long long>(ranks, n, blocks, stream);
   }
   return cudaErrorInvalidValue;
 }

@@ -136,7 +136,8 @@ __device__ __forceinline__ bool RoleWait(RoleCtx& c, int row, uint64_t flag_wind
 // included).  Everything the group wrote before is ordered ahead of the flag.
 __device__ __forceinline__ void RolePost(RoleCtx& c, int row, uint64_t flag_window, int groups, uint64_t value) {
   GroupSync(c.bar_id, c.nthr);
-  if (c.tid < c.w.world_size) StReleaseSys(FlagRow(Ctl(*c.w.peers, c.tid), row, c.cta, c.ncta, flag_window, groups) + c.w.rank, value);
+  if (c.tid < c.w.world_size)
+    StReleasePeers(FlagRow(Ctl(*c.w.peers, c.tid), row, c.cta, c.ncta, flag_window, groups) + c.w.rank, value, c.w.peers->one_gpu != 0);
 }
 
 // ---- copies in registers (with the conversion between buffer and wire type) ----
@@ -270,7 +271,7 @@ __device__ inline bool BulkCopyPieces(BulkRing& ring, unsigned char* const* dst,
 
 template <typename T, typename W, bool kMultimem, int kR>
 __global__ void __launch_bounds__(kStagedThreads, 1)
-StagedKernel(const __grid_constant__ StagedParams p0, const StagedParams* __restrict__ emu) {
+StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   static_assert(sizeof(W) <= sizeof(T), "the wire type is never wider than the buffer type");
   using AW = typename Acc<W>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));                // elements per wire vector
@@ -283,7 +284,7 @@ StagedKernel(const __grid_constant__ StagedParams p0, const StagedParams* __rest
   __shared__ uint64_t s_full[kBulkMaxRings][kBulkMaxDepth];
   __shared__ RoleSync s_sync;  // reducing blocks in split mode: done[g] = windows whose stores group g has issued
   {
-    const uint32_t* src = (emu != nullptr) ? reinterpret_cast<const uint32_t*>(emu + blockIdx.y) : reinterpret_cast<const uint32_t*>(&p0);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
     for (unsigned i = threadIdx.x; i < sizeof(StagedParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
     if (threadIdx.x == 0) {
       s_stop = 0;
@@ -553,7 +554,7 @@ StagedKernel(const __grid_constant__ StagedParams p0, const StagedParams* __rest
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
       __syncwarp();  // lane 0's acquire is ordered before the other lanes' releases
-      if (lane < ws) StReleaseSys(FlagRow(Ctl(p.peers, lane), kRowReduced, cta, ncta, k, RG) + me, base | (k + 1));
+      if (lane < ws) StReleasePeers(FlagRow(Ctl(p.peers, lane), kRowReduced, cta, ncta, k, RG) + me, base | (k + 1), p.peers.one_gpu != 0);
       if (trace != nullptr && lane == 0 && k < static_cast<uint64_t>(p.trace_capacity)) trace[k].t_done = GlobalTimerNs();
     }
   }
@@ -563,48 +564,42 @@ StagedKernel(const __grid_constant__ StagedParams p0, const StagedParams* __rest
 }  // namespace dev
 
 template <typename T, typename W, bool kMultimem, int kR>
-static cudaError_t LaunchStagedOne(const StagedParams& p, const StagedParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
+static cudaError_t LaunchStagedOne(const StagedParams* ranks, int n, int blocks, cudaStream_t stream) {
   auto kernel = dev::StagedKernel<T, W, kMultimem, kR>;
   // Per (function, device); cheap, so made on every launch.
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dev::kStagedSmemBytes));
   if (e != cudaSuccess) return e;
-  dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(emu != nullptr ? emu_ranks : 1));
-  if (emu != nullptr) {
-    void* args[] = {const_cast<StagedParams*>(&p), &emu};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), grid, dim3(dev::kStagedThreads), args, dev::kStagedSmemBytes, stream);
-  }
-  kernel<<<grid, dev::kStagedThreads, dev::kStagedSmemBytes, stream>>>(p, nullptr);
-  return cudaGetLastError();
+  return LaunchRanks(kernel, ranks, n, blocks, dev::kStagedThreads, dev::kStagedSmemBytes, stream);
 }
 
 template <typename T, typename W>
-static cudaError_t LaunchStagedTyped(const StagedParams& p, const StagedParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  if (p.use_multimem) {
+static cudaError_t LaunchStagedTyped(const StagedParams* ranks, int n, int blocks, cudaStream_t stream) {
+  if (ranks->use_multimem) {
     if constexpr (dev::HasMultimem<W>::value) {
-      return LaunchStagedOne<T, W, true, kMaxRanks>(p, emu, emu_ranks, blocks, stream);
+      return LaunchStagedOne<T, W, true, kMaxRanks>(ranks, n, blocks, stream);
     } else {
       return cudaErrorInvalidValue;
     }
   }
-  switch (dev::RankClass(p.world_size)) {
-    case 2: return LaunchStagedOne<T, W, false, 2>(p, emu, emu_ranks, blocks, stream);
-    case 4: return LaunchStagedOne<T, W, false, 4>(p, emu, emu_ranks, blocks, stream);
-    default: return LaunchStagedOne<T, W, false, kMaxRanks>(p, emu, emu_ranks, blocks, stream);
+  switch (dev::RankClass(ranks->world_size)) {
+    case 2: return LaunchStagedOne<T, W, false, 2>(ranks, n, blocks, stream);
+    case 4: return LaunchStagedOne<T, W, false, 4>(ranks, n, blocks, stream);
+    default: return LaunchStagedOne<T, W, false, kMaxRanks>(ranks, n, blocks, stream);
   }
 }
 
-cudaError_t LaunchStagedKernel(const StagedParams& p, const StagedParams* emu, int emu_ranks, int blocks, cudaStream_t stream) {
-  const DType t = static_cast<DType>(p.dtype), w = static_cast<DType>(p.wire);
-  if (t == DType::kFloat32 && w == DType::kBFloat16) return LaunchStagedTyped<float, __nv_bfloat16>(p, emu, emu_ranks, blocks, stream);
-  if (t == DType::kFloat32 && w == DType::kFloat16) return LaunchStagedTyped<float, __half>(p, emu, emu_ranks, blocks, stream);
+cudaError_t LaunchStagedKernel(const StagedParams* ranks, int n, int blocks, cudaStream_t stream) {
+  const DType t = static_cast<DType>(ranks->dtype), w = static_cast<DType>(ranks->wire);
+  if (t == DType::kFloat32 && w == DType::kBFloat16) return LaunchStagedTyped<float, __nv_bfloat16>(ranks, n, blocks, stream);
+  if (t == DType::kFloat32 && w == DType::kFloat16) return LaunchStagedTyped<float, __half>(ranks, n, blocks, stream);
   if (t != w) return cudaErrorInvalidValue;
   switch (t) {
-    case DType::kFloat32: return LaunchStagedTyped<float, float>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat16: return LaunchStagedTyped<__half, __half>(p, emu, emu_ranks, blocks, stream);
-    case DType::kBFloat16: return LaunchStagedTyped<__nv_bfloat16, __nv_bfloat16>(p, emu, emu_ranks, blocks, stream);
-    case DType::kFloat64: return LaunchStagedTyped<double, double>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt32: return LaunchStagedTyped<int, int>(p, emu, emu_ranks, blocks, stream);
-    case DType::kInt64: return LaunchStagedTyped<long long, long long>(p, emu, emu_ranks, blocks, stream);
+    case DType::kFloat32: return LaunchStagedTyped<float, float>(ranks, n, blocks, stream);
+    case DType::kFloat16: return LaunchStagedTyped<__half, __half>(ranks, n, blocks, stream);
+    case DType::kBFloat16: return LaunchStagedTyped<__nv_bfloat16, __nv_bfloat16>(ranks, n, blocks, stream);
+    case DType::kFloat64: return LaunchStagedTyped<double, double>(ranks, n, blocks, stream);
+    case DType::kInt32: return LaunchStagedTyped<int, int>(ranks, n, blocks, stream);
+    case DType::kInt64: return LaunchStagedTyped<long long, long long>(ranks, n, blocks, stream);
   }
   return cudaErrorInvalidValue;
 }

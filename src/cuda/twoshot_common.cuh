@@ -136,7 +136,7 @@ __device__ inline bool CrossRankBarrier(const PeerTable& peers, const WaitCtx& w
   if (threadIdx.x < w.world_size && static_cast<int>(threadIdx.x) != w.rank) {
     // The release store orders everything this CTA wrote before the barrier
     // (observed by this thread through __syncthreads) ahead of the flag.
-    StReleaseSys(&Ctl(peers, threadIdx.x)->bar[cta][w.rank], val);
+    StReleasePeers(&Ctl(peers, threadIdx.x)->bar[cta][w.rank], val, peers.one_gpu != 0);
     if (!WaitGE(&Ctl(peers, w.rank)->bar[cta][threadIdx.x], val, w, kWaitBarrier, threadIdx.x, static_cast<int>(phase)))
       *s_stop = 1;
   }
