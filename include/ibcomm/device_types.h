@@ -129,6 +129,11 @@ struct Op {
   // Staging offsets and the split among channels are relative to the cell, so
   // an element keeps its channel and its place in a slot in every op.
   uint64_t cell_begin;
+  // An op that reads recvbuf: number of leading ops of the program that have
+  // to be finished first (the last of them stored into the op's cell); 0 when
+  // nothing has.  Loads may run ahead of the program otherwise.
+  uint32_t wait_local;
+  uint32_t pad2_;
 };
 
 // Geometry of the staging area a program runs in.

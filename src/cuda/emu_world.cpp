@@ -20,6 +20,7 @@ struct EmuWorld::Impl {
   ProgramCache cache;
   int timeout_ms = env::kDefaultTimeoutMs;
   int max_blocks = 0;
+  int exec_max_blocks = 0;  // executor CTAs of the smaller size (two per SM)
   int last_channels = 0;
   int silent_rank = -1;
   int bad_program_rank = -1;
@@ -55,7 +56,8 @@ EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(nu
     rr.h_doorbell = m.status[static_cast<size_t>(r)].h_doorbell;
     rr.d_doorbell = m.status[static_cast<size_t>(r)].d_doorbell;
   }
-  m.max_blocks = ExecKernelMaxCoResidentBlocks(m.device, 0);
+  m.max_blocks = TwoShotKernelMaxCoResidentBlocks(m.device);
+  m.exec_max_blocks = ExecKernelMaxCoResidentBlocks(m.device, 256);
   m.staged_max_blocks = StagedKernelMaxCoResidentBlocks(m.device);
   CUDACHECK(cudaDeviceSynchronize());
 }
@@ -230,8 +232,12 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       if (r == m.silent_rank) ps.back().num_ops = 0;
       if (r == m.bad_program_rank) ps.back().len_elements = 1;
     }
-    int ch = channels > 0 ? channels : ChooseChannels(algo, bytes, m.ws, kMaxChannels);
-    ch = std::min(ch, cap);
+    // A channel for every 4 KiB of a transfer: the flags of ranks on one GPU are
+    // cheap, and more channels shorten every step of the program.  One CTA per
+    // SM at most (two smaller ones per SM are no faster).
+    const uint64_t slot = m.cache.Get(algo, 0, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false).prog.stage.slot_bytes;
+    int ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(slot / 4096, static_cast<uint64_t>(kMaxChannels)));
+    ch = std::max(1, std::min(ch, channels > 0 ? m.exec_max_blocks / m.ws : cap));
     CUDACHECK(LaunchExecKernel(ps.data(), m.ws, ch, stream));
     m.last_channels = ch;
   }

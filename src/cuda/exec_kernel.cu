@@ -8,14 +8,28 @@
 // then publishes the data flag to the receiver and returns the credit to the
 // sender.  No host round trip and no separate reduce, cast or scale kernel.
 //
-// The CTA is warp-specialised so that the synchronisation of one op overlaps
-// the data of its neighbours: one thread (the "waiter") runs ahead through
-// the program and waits for the flags of the coming ops; the data warps
-// stream op after op without a CTA-wide barrier, in two groups that take the
-// ops in turn; another thread (the "poster") follows behind, and once the
-// warps of an op's group have had their stores acknowledged it publishes the
-// op's flags.  The parties hand over through counters in shared memory (ops
-// ready; per data warp, ops done).
+// The CTA is warp-specialised so that neither the synchronisation of an op nor
+// the latency of its loads stops the stream of the next one:
+//   waiter  (a warp)    looks at the peers' data flags and slot credits and runs
+//                       ahead through the program as far as they allow;
+//   loader  (a warp)    fills a ring of shared-memory stages with bulk copies
+//                       (`cp.async.bulk`, this GPU's memory only) of the ops'
+//                       sources, several stages and hence several ops ahead: what
+//                       lies in sendbuf is fetched before the op's flag is there;
+//   data warps          take stage after stage in order: read, add, scale, cast,
+//                       store; no barrier among them;
+//   poster  (a warp)    follows behind, fences the stores of finished ops and
+//                       publishes their flags, one fence for all ops that are done.
+// They hand over through counters and mbarriers in shared memory.
+//
+// A rank's rate is bound by the bytes its CTAs have in flight: with loads into
+// registers (two groups of warps taking the ops in turn, 14 KiB each) a CTA
+// moved 10-15 GB/s whether the data came from L2 or from HBM; the ring keeps
+// 100 KiB (fp32) ahead of the data warps across op boundaries.  Per op, what is
+// left in series (flags, plan, fence) takes about 1.2 us, and a hand-over
+// between two ranks on one GPU about 3 us.  Ranks sharing a B200, before and
+// after: Rabenseifner 5 x 64 MiB 908 -> 430 us, ring 8 x 32 MiB 258 -> 192 us,
+// ring 7 x 4 MB 96 -> 70 us, ring 8 x 4 KiB 52 -> 46 us.
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda
 // (ibcomm/allreduce_cuda_impl.h:24-33, 103-299, 470-707).
 //
@@ -24,12 +38,14 @@
 // launch (CTAs that wait on each other are co-resident).
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "flags.cuh"
 #include "ibcomm/communicator.h"
 #include "ibcomm/tunables.h"
 #include "kernels.h"
+#include "tma_stage.cuh"
 #include "vec_ops.cuh"
 #include "warp_roles.cuh"
 
@@ -40,161 +56,198 @@ template <typename T, typename W>
 struct ExecTraits {
   using A = typename Acc<T>::type;
   static constexpr int kMinBytes = sizeof(T) < sizeof(W) ? sizeof(T) : sizeof(W);
-  static constexpr int P = 16 / kMinBytes;                       // elements per pack
-  static constexpr int U = 64 / (P * static_cast<int>(sizeof(T))) > 0 ? 64 / (P * static_cast<int>(sizeof(T))) : 1;
+  static constexpr int P = 16 / kMinBytes;               // elements per pack
+  static constexpr int VT = P / VecIO<T>::kN;            // 16-byte vectors per pack in the user type
+  static constexpr int VW = P / VecIO<W>::kN;            // ... in the wire type
+  static constexpr int U = VT > 1 ? 2 : 4;               // packs per thread and stage
 };
 
-// Vector path of one op: packs of P elements, U packs in flight per thread,
-// all loads of an iteration issued before any use.  The op's shape (which
-// sources, which destinations) is uniform over the CTA, so the branches below
-// are predicates on registers, not divergence.
+constexpr int kExecServiceWarps = 3;  // waiter, loader, poster
+constexpr int kExecMaxStages = 10;
+// A stage holds U packs per data thread from each of two sources: 128 bytes per
+// data thread for every pair of types.  Half of that leaves a warp waiting for
+// its own shared-memory reads (5 ranks x 64 MiB Rabenseifner 496 us against 430).
+constexpr int kExecStageBytesPerThread = 128;
+
+enum ExecTileFlags : uint32_t {
+  kTileFromStaging = 1,  // source a is in the wire type
+  kTileAdd = 2,          // source b is present
+  kTileScale = 4,
+  kTileRoundWire = 8,
+  kTileLastOfOp = 16,
+  kTileElements = 32,  // nothing in the stage: elements [lo, hi) of the op's cell, one by one
+  kTileExit = 64,      // the program is over
+};
+// What the data warps do with one stage.
+struct ExecTile {
+  uint4* local;   // recvbuf, or null
+  uint4* remote;  // the next rank's staging slot, or null
+  uint32_t packs;
+  uint32_t flags;
+  uint32_t op;
+  uint32_t pad_;
+  uint64_t lo, hi;
+};
+
+// One op of this channel, worked out by a lane of the loader's warp.
+struct ExecPlan {
+  const unsigned char* src_a;  // address of the first pack (for staging: in the wire type)
+  const unsigned char* src_b;
+  unsigned char* local;
+  unsigned char* remote;
+  uint64_t packs;      // whole packs
+  uint64_t rest, hi;   // elements [rest, hi) of the cell go one by one
+  uint32_t flags;      // ExecTileFlags of every stage of the op
+  uint32_t wait_local;
+};
+
+struct ExecShared {
+  RoleSync role;  // ready: ops whose flags have arrived; done[w]: ops whose stores data warp w has issued
+  ExecTile tile[kExecMaxStages];
+  ExecPlan plan[32];
+  uint64_t full[kExecMaxStages];   // the stage's copies have landed and its op may store
+  uint64_t empty[kExecMaxStages];  // every data warp has read the stage
+};
+
+// Waits for a phase of one of the ring's mbarriers.  The party that completes
+// it is in this CTA and itself bounded, so the limit is a safety net.
+__device__ __forceinline__ bool RingWait(uint64_t* bar, uint32_t parity, RoleSync* sync, uint64_t timeout_ns) {
+  if (MbarTryWait(bar, parity)) return true;
+  const uint64_t t0 = GlobalTimerNs();
+  for (;;) {
+    if (MbarTryWait(bar, parity)) return true;
+    if (GlobalTimerNs() - t0 > 3 * timeout_ns) {
+      *reinterpret_cast<volatile int*>(&sync->stop) = 1;
+      return false;
+    }
+  }
+}
+
+// One stage: packs of P elements, U of them per thread.
 template <typename T, typename W>
-__device__ __forceinline__ void VecLoop(const uint4* __restrict__ a_base, bool a_is_stage, const uint4* __restrict__ b_base,
-                                        uint4* l_base, uint4* r_base, uint64_t npacks, bool do_scale, double scale, bool round_wire,
-                                        unsigned tid, unsigned nthr) {
+__device__ __forceinline__ void RunTile(const ExecTile& t, const uint4* stage, uint32_t b_off, double scale, uint64_t* empty, unsigned tid,
+                                        unsigned nthr, int lane) {
   using Tr = ExecTraits<T, W>;
   using A = typename Tr::A;
-  constexpr int P = Tr::P;
-  constexpr int U = Tr::U;
-  constexpr int VT = P / VecIO<T>::kN;  // 16-byte vectors per pack in the user type
-  constexpr int VW = P / VecIO<W>::kN;  // ... in the wire type
-  const int va = a_is_stage ? VW : VT;
-  const uint64_t stride = nthr;
-  for (uint64_t i = tid; i < npacks; i += stride * U) {
-    uint4 qa[U][VT];
-    uint4 qb[U][VT];
+  constexpr int P = Tr::P, U = Tr::U, VT = Tr::VT, VW = Tr::VW;
+  const bool from_staging = (t.flags & kTileFromStaging) != 0, add = (t.flags & kTileAdd) != 0;
+  uint4 qa[U][VT], qb[U][VT];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * stride;
-      if (idx < npacks) {
-        if (a_is_stage) {
+  for (int u = 0; u < U; ++u) {
+    const unsigned i = tid + static_cast<unsigned>(u) * nthr;
+    if (i < t.packs) {
+      if (from_staging) {
 #pragma unroll
-          for (int v = 0; v < VW; ++v) qa[u][v] = Ld16Strong(a_base + idx * VW + v);
-        } else {
+        for (int v = 0; v < VW; ++v) qa[u][v] = stage[i * VW + v];
+      } else {
 #pragma unroll
-          for (int v = 0; v < VT; ++v) qa[u][v] = Ld16(a_base + idx * VT + v);
-        }
-        if (b_base != nullptr) {
-#pragma unroll
-          for (int v = 0; v < VT; ++v) qb[u][v] = Ld16(b_base + idx * VT + v);
-        }
+        for (int v = 0; v < VT; ++v) qa[u][v] = stage[i * VT + v];
       }
-    }
+      if (add) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * stride;
-      if (idx < npacks) {
-        A acc[P];
-        if (a_is_stage) {
-#pragma unroll
-          for (int v = 0; v < VW; ++v) VecIO<W>::Load(qa[u][v], acc + v * VecIO<W>::kN);
-        } else {
-#pragma unroll
-          for (int v = 0; v < VT; ++v) VecIO<T>::Load(qa[u][v], acc + v * VecIO<T>::kN);
-        }
-        if (b_base != nullptr) {
-#pragma unroll
-          for (int v = 0; v < VT; ++v) VecIO<T>::Add(qb[u][v], acc + v * VecIO<T>::kN);
-        }
-        if (do_scale) {
-#pragma unroll
-          for (int e = 0; e < P; ++e) acc[e] = ScaleAcc<A>(acc[e], scale);
-        }
-        uint4 wq[VW];
-        if (r_base != nullptr || round_wire) {
-#pragma unroll
-          for (int v = 0; v < VW; ++v) wq[v] = VecIO<W>::Store(acc + v * VecIO<W>::kN);
-        }
-        if (r_base != nullptr) {
-#pragma unroll
-          for (int v = 0; v < VW; ++v) St16(r_base + idx * VW + v, wq[v]);
-        }
-        if (l_base != nullptr) {
-          if (round_wire && sizeof(W) != sizeof(T)) {
-#pragma unroll
-            for (int v = 0; v < VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
-          }
-#pragma unroll
-          for (int v = 0; v < VT; ++v) St16(l_base + idx * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN));
-        }
+        for (int v = 0; v < VT; ++v) qb[u][v] = stage[b_off + i * VT + v];
       }
     }
   }
-  (void)va;
+  // The stage is free for the loader once every warp has read it.
+  __syncwarp();
+  if (lane == 0) MbarArrive(empty);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const unsigned i = tid + static_cast<unsigned>(u) * nthr;
+    if (i < t.packs) {
+      A acc[P];
+      if (from_staging) {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) VecIO<W>::Load(qa[u][v], acc + v * VecIO<W>::kN);
+      } else {
+#pragma unroll
+        for (int v = 0; v < VT; ++v) VecIO<T>::Load(qa[u][v], acc + v * VecIO<T>::kN);
+      }
+      if (add) {
+#pragma unroll
+        for (int v = 0; v < VT; ++v) VecIO<T>::Add(qb[u][v], acc + v * VecIO<T>::kN);
+      }
+      if (t.flags & kTileScale) {
+#pragma unroll
+        for (int e = 0; e < P; ++e) acc[e] = ScaleAcc<A>(acc[e], scale);
+      }
+      uint4 wq[VW];
+      if (t.remote != nullptr || (t.flags & kTileRoundWire)) {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) wq[v] = VecIO<W>::Store(acc + v * VecIO<W>::kN);
+      }
+      if (t.remote != nullptr) {
+#pragma unroll
+        for (int v = 0; v < VW; ++v) St16(t.remote + i * VW + v, wq[v]);
+      }
+      if (t.local != nullptr) {
+        if ((t.flags & kTileRoundWire) && sizeof(W) != sizeof(T)) {
+#pragma unroll
+          for (int v = 0; v < VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
+        }
+#pragma unroll
+        for (int v = 0; v < VT; ++v) St16(t.local + i * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN));
+      }
+    }
+  }
 }
+
+// Where an op's data lies.
+template <typename T, typename W>
+struct OpBuffers {
+  const T* sendbuf;
+  T* recvbuf;
+  const W* stage_in;
+  W* stage_out;
+  __device__ OpBuffers(const Op& op, const ExecParams& p)
+      : sendbuf(static_cast<const T*>(p.sendbuf)), recvbuf(static_cast<T*>(p.recvbuf)), stage_in(nullptr), stage_out(nullptr) {
+    const StageLayout& st = p.stage;
+    if (op.src_a == kSrcStage)
+      stage_in = reinterpret_cast<const W*>(p.peers.arena[p.rank] + st.offset +
+                                            (static_cast<uint64_t>(op.region_in) * st.slots + op.slot_in) * st.slot_bytes);
+    if (op.flags & kOpStoreRemote)
+      stage_out = reinterpret_cast<W*>(p.peers.arena[op.peer_out] + st.offset +
+                                       (static_cast<uint64_t>(op.region_out) * st.slots + op.slot_out) * st.slot_bytes);
+  }
+};
 
 // Element-at-a-time path for chunks that do not start on a 16-byte boundary
-// and for the few elements after the last whole pack.
+// and for the few elements after the last whole pack; kU loads of each source
+// in flight per thread.
 template <typename T, typename W>
-__device__ void ScalarLoop(const Op& op, const T* sendbuf, T* recvbuf, const W* stage_in, W* stage_out, uint64_t lo,
-                           uint64_t hi, double scale, unsigned tid, unsigned nthr) {
+__device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint64_t hi, unsigned tid, unsigned nthr) {
   using A = typename Acc<T>::type;
-  for (uint64_t k = lo + tid; k < hi; k += nthr) {
-    const uint64_t g = op.cell_begin + k;
-    A v;
-    if (op.src_a == kSrcStage) v = ToAcc<A, W>(LdScalarStrong<W>(stage_in + k));
-    else if (op.src_a == kSrcSend) v = ToAcc<A, T>(sendbuf[g]);
-    else v = ToAcc<A, T>(recvbuf[g]);
-    if (op.src_b == kSrcSend) v += ToAcc<A, T>(sendbuf[g]);
-    else if (op.src_b == kSrcRecv) v += ToAcc<A, T>(recvbuf[g]);
-    if (op.flags & kOpScale) v = ScaleAcc<A>(v, scale);
-    if ((op.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) v = ToAcc<A, W>(FromAcc<W, A>(v));
-    if (op.flags & kOpStoreLocal) recvbuf[g] = FromAcc<T, A>(v);
-    if (op.flags & kOpStoreRemote) stage_out[k] = FromAcc<W, A>(v);
+  constexpr int kU = 8;
+  const OpBuffers<T, W> buf(op, p);
+  const T* b_src = op.src_b == kSrcSend ? buf.sendbuf : (op.src_b == kSrcRecv ? buf.recvbuf : nullptr);
+  for (uint64_t k0 = lo + tid; k0 < hi; k0 += static_cast<uint64_t>(nthr) * kU) {
+    A a[kU];
+    T b[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t k = k0 + static_cast<uint64_t>(u) * nthr;
+      if (k < hi) {
+        if (op.src_a == kSrcStage) a[u] = ToAcc<A, W>(LdScalarStrong<W>(buf.stage_in + k));
+        else a[u] = ToAcc<A, T>((op.src_a == kSrcSend ? buf.sendbuf : buf.recvbuf)[op.cell_begin + k]);
+        if (b_src != nullptr) b[u] = b_src[op.cell_begin + k];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t k = k0 + static_cast<uint64_t>(u) * nthr;
+      if (k < hi) {
+        A v = a[u];
+        if (b_src != nullptr) v += ToAcc<A, T>(b[u]);
+        if (op.flags & kOpScale) v = ScaleAcc<A>(v, p.scale);
+        if ((op.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) v = ToAcc<A, W>(FromAcc<W, A>(v));
+        if (op.flags & kOpStoreLocal) buf.recvbuf[op.cell_begin + k] = FromAcc<T, A>(v);
+        if (op.flags & kOpStoreRemote) buf.stage_out[k] = FromAcc<W, A>(v);
+      }
+    }
   }
 }
 
-template <typename T, typename W>
-__device__ void RunOpData(const Op& op, const ExecParams& p, int ch, int nch, unsigned tid, unsigned nthr) {
-  using Tr = ExecTraits<T, W>;
-  uint64_t lo, hi;
-  ChannelSlice(op.elem_begin - op.cell_begin, op.elem_count, p.stage.slot_bytes / sizeof(W), nch, ch, &lo, &hi);
-  if (lo >= hi) return;
-  const T* sendbuf = static_cast<const T*>(p.sendbuf);
-  T* recvbuf = static_cast<T*>(p.recvbuf);
-  const StageLayout& st = p.stage;
-  const W* stage_in = nullptr;
-  W* stage_out = nullptr;
-  if (op.src_a == kSrcStage)
-    stage_in = reinterpret_cast<const W*>(p.peers.arena[p.rank] + st.offset +
-                                          (static_cast<uint64_t>(op.region_in) * st.slots + op.slot_in) * st.slot_bytes);
-  if (op.flags & kOpStoreRemote)
-    stage_out = reinterpret_cast<W*>(p.peers.arena[op.peer_out] + st.offset +
-                                     (static_cast<uint64_t>(op.region_out) * st.slots + op.slot_out) * st.slot_bytes);
-  const uint64_t g0 = op.cell_begin + lo;
-  const bool uses_send = op.src_a == kSrcSend || op.src_b == kSrcSend;
-  const bool uses_recv = op.src_a == kSrcRecv || op.src_b == kSrcRecv || (op.flags & kOpStoreLocal);
-  bool aligned = true;
-  if (uses_send) aligned &= (reinterpret_cast<uintptr_t>(sendbuf + g0) & 15u) == 0;
-  if (uses_recv) aligned &= (reinterpret_cast<uintptr_t>(recvbuf + g0) & 15u) == 0;
-  // The place inside a staging slot follows the cell, not the user buffer: a
-  // range that starts in the middle of a cell (Rabenseifner pieces, 16-bit
-  // wire) can be 16-byte aligned on the user side and not in the slot.
-  if (stage_in != nullptr) aligned &= (reinterpret_cast<uintptr_t>(stage_in + lo) & 15u) == 0;
-  if (stage_out != nullptr) aligned &= (reinterpret_cast<uintptr_t>(stage_out + lo) & 15u) == 0;
-  if (!aligned) {
-    ScalarLoop<T, W>(op, sendbuf, recvbuf, stage_in, stage_out, lo, hi, p.scale, tid, nthr);
-    return;
-  }
-  const uint64_t npacks = (hi - lo) / Tr::P;
-  {
-    const bool a_is_stage = op.src_a == kSrcStage;
-    const uint4* a_base = a_is_stage ? reinterpret_cast<const uint4*>(stage_in + lo)
-                          : (op.src_a == kSrcSend) ? reinterpret_cast<const uint4*>(sendbuf + g0)
-                                                   : reinterpret_cast<const uint4*>(recvbuf + g0);
-    const uint4* b_base = (op.src_b == kSrcSend)   ? reinterpret_cast<const uint4*>(sendbuf + g0)
-                          : (op.src_b == kSrcRecv) ? reinterpret_cast<const uint4*>(recvbuf + g0)
-                                                   : nullptr;
-    uint4* l_base = (op.flags & kOpStoreLocal) ? reinterpret_cast<uint4*>(recvbuf + g0) : nullptr;
-    uint4* r_base = (op.flags & kOpStoreRemote) ? reinterpret_cast<uint4*>(stage_out + lo) : nullptr;
-    VecLoop<T, W>(a_base, a_is_stage, b_base, l_base, r_base, npacks, (op.flags & kOpScale) != 0, p.scale,
-                  (op.flags & kOpRoundWire) != 0, tid, nthr);
-  }
-  const uint64_t done = lo + npacks * Tr::P;
-  if (done < hi) ScalarLoop<T, W>(op, sendbuf, recvbuf, stage_in, stage_out, done, hi, p.scale, tid, nthr);
-}
-
-// Body of the executor for one CTA; returns when the program is done or a wait gave up.
 // Self-check of an op before any of its addresses is formed: the message
 // range, the place inside the staging slot and the slot, region and peer
 // indices.  A failing op is reported (status "bad program") and the call
@@ -214,14 +267,261 @@ __device__ __forceinline__ bool OpInBounds(const Op& op, const ExecParams& p) {
     return false;
   if ((op.wait_in != 0 || op.post_credit != 0) && (op.peer_in < 0 || op.peer_in >= p.world_size)) return false;
   if ((op.wait_credit != 0 || op.post_out != 0) && (op.peer_out < 0 || op.peer_out >= p.world_size)) return false;
-  return true;
+  return op.wait_local < static_cast<uint32_t>(p.num_ops);
 }
 
-// Body of the executor for one CTA: warps [0, data_warps) move data, lane 0 of
-// the next warp is the waiter, lane 0 of the last warp the poster.
+// Position in the ring of stages.
+struct RingPos {
+  uint32_t s = 0, parity = 0, stages;
+  __device__ explicit RingPos(int n) : stages(static_cast<uint32_t>(n)) {}
+  __device__ void Next() {
+    if (++s == stages) s = 0, parity ^= 1u;
+  }
+};
+
+// The loader: turns the program into stages, in order, ahead of the data warps.
+// The lanes work out 32 ops at a time (an op is a 64-byte load and a division,
+// 1.5 us one after the other); lane 0 then only issues copies.  Returns after it
+// has handed out the exit stage (or could not, because the data warps gave up).
 template <typename T, typename W>
-__device__ void ExecBody(const ExecParams& p, uint64_t seq, RoleSync* sync) {
+__device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* smem, int stages, int ch, int nch, int data_warps, int lane) {
+  using Tr = ExecTraits<T, W>;
+  const unsigned nthr = static_cast<unsigned>(data_warps) * 32u;
+  const uint32_t tile_packs = nthr * Tr::U;
+  const uint32_t half_bytes = tile_packs * Tr::VT * 16u;  // source a, then source b
+  RingPos pos(stages);
+  bool first_round = true;
+  uint32_t s = 0;  // stage claimed last (lane 0)
+  auto next_stage = [&]() -> bool {
+    s = pos.s;
+    // The phase before the one the loader is about to fill: read by every data warp.
+    const bool ok = first_round || RingWait(&sh->empty[s], pos.parity ^ 1u, &sh->role, p.timeout_ns);
+    pos.Next();
+    if (pos.s == 0) first_round = false;
+    return ok;
+  };
+  // Hands out the exit stage; `fresh`: in a stage of its own, else in the claimed one
+  // (copies into it complete before its phase does).
+  auto leave = [&](bool fresh) {
+    if (lane == 0 && (!fresh || next_stage())) {
+      sh->tile[s].flags = kTileExit;
+      MbarArrive(&sh->full[s]);
+    }
+  };
+  unsigned ready = 0;  // ops known to have their flags; what they may read is visible to the copy engine
+  for (int first = 0; first < p.num_ops; first += 32) {
+    const int in_batch = p.num_ops - first < 32 ? p.num_ops - first : 32;
+    bool in_bounds = true;
+    if (lane < in_batch) {
+      const Op op = p.ops[first + lane];
+      in_bounds = OpInBounds<W>(op, p);
+      if (in_bounds) {
+        uint64_t lo, hi;
+        ChannelSlice(op.elem_begin - op.cell_begin, op.elem_count, p.stage.slot_bytes / sizeof(W), nch, ch, &lo, &hi);
+        const OpBuffers<T, W> buf(op, p);
+        const uint64_t g0 = op.cell_begin + lo;
+        const bool uses_send = op.src_a == kSrcSend || op.src_b == kSrcSend;
+        const bool uses_recv = op.src_a == kSrcRecv || op.src_b == kSrcRecv || (op.flags & kOpStoreLocal);
+        uintptr_t bits = 0;
+        if (uses_send) bits |= reinterpret_cast<uintptr_t>(buf.sendbuf + g0);
+        if (uses_recv) bits |= reinterpret_cast<uintptr_t>(buf.recvbuf + g0);
+        // The place inside a staging slot follows the cell, not the user buffer: a
+        // range that starts in the middle of a cell (Rabenseifner pieces, 16-bit
+        // wire) can be 16-byte aligned on the user side and not in the slot.
+        if (buf.stage_in != nullptr) bits |= reinterpret_cast<uintptr_t>(buf.stage_in + lo);
+        if (buf.stage_out != nullptr) bits |= reinterpret_cast<uintptr_t>(buf.stage_out + lo);
+        auto source = [&](uint8_t src) -> const unsigned char* {
+          if (src == kSrcStage) return reinterpret_cast<const unsigned char*>(buf.stage_in + lo);
+          if (src == kSrcNone) return nullptr;
+          return reinterpret_cast<const unsigned char*>((src == kSrcSend ? buf.sendbuf : buf.recvbuf) + g0);
+        };
+        ExecPlan& pl = sh->plan[lane];
+        pl.src_a = source(op.src_a);
+        pl.src_b = source(op.src_b);
+        pl.local = (op.flags & kOpStoreLocal) ? reinterpret_cast<unsigned char*>(buf.recvbuf + g0) : nullptr;
+        pl.remote = buf.stage_out != nullptr ? reinterpret_cast<unsigned char*>(buf.stage_out + lo) : nullptr;
+        pl.packs = lo < hi && (bits & 15u) == 0 ? (hi - lo) / Tr::P : 0;
+        pl.rest = lo + pl.packs * Tr::P;
+        pl.hi = hi;
+        pl.flags = (op.src_a == kSrcStage ? kTileFromStaging : 0u) | (op.src_b != kSrcNone ? kTileAdd : 0u) |
+                   ((op.flags & kOpScale) ? kTileScale : 0u) | ((op.flags & kOpRoundWire) ? kTileRoundWire : 0u);
+        pl.wait_local = op.wait_local;
+      }
+    }
+    // A bad op is reported by the waiter, which checks it as well; the ops before it still run.
+    const unsigned bad = __ballot_sync(0xffffffffu, !in_bounds);
+    const int good = bad != 0 ? __ffs(static_cast<int>(bad)) - 1 : in_batch;
+    __syncwarp();
+    for (int k = 0; k < good; ++k) {
+      const unsigned oi = static_cast<unsigned>(first + k);
+      const uint32_t wait_local = sh->plan[k].wait_local;
+      // recvbuf is read only after the data warps' stores of the ops before have
+      // landed: the fence orders their stores (observed through `done`) ahead of
+      // what the copy engine reads.
+      if (wait_local != 0) {
+        bool ok = true;
+        if (lane < data_warps) ok = SpinShared(&sh->role.done[lane], wait_local, &sh->role, p.timeout_ns);
+        if (!__all_sync(0xffffffffu, ok)) return leave(true);
+        __syncwarp();  // what the other lanes acquired is ordered before lane 0's fences
+        if (lane == 0) {
+          FencePeers(true);
+          FenceProxyAsyncAll();
+        }
+      }
+      int alive = 1;
+      if (lane == 0) {
+        const ExecPlan pl = sh->plan[k];
+        // The flags of op `oi` have arrived: one look may cover several ops, and
+        // one proxy fence what all of them read from staging (written by
+        // ordinary stores of the peers that the waiter's acquire made visible).
+        auto get_ready = [&]() -> bool {
+          if (ready > oi) return true;
+          if (!SpinShared(&sh->role.ready, oi + 1u, &sh->role, p.timeout_ns)) return false;
+          ready = LdAcquireShared(&sh->role.ready);
+          FenceProxyAsyncAll();
+          return true;
+        };
+        const bool a_staged = (pl.flags & kTileFromStaging) != 0;
+        const uint64_t a_step = static_cast<uint64_t>(a_staged ? Tr::VW : Tr::VT) * 16u;
+        for (uint64_t j = 0; j < pl.packs; j += tile_packs) {
+          if (!next_stage()) {
+            alive = -1;
+            break;
+          }
+          const uint32_t n = pl.packs - j < tile_packs ? static_cast<uint32_t>(pl.packs - j) : tile_packs;
+          unsigned char* dst = smem + static_cast<size_t>(s) * 2 * half_bytes;
+          ExecTile& t = sh->tile[s];
+          t.local = pl.local != nullptr ? reinterpret_cast<uint4*>(pl.local + j * Tr::VT * 16u) : nullptr;
+          t.remote = pl.remote != nullptr ? reinterpret_cast<uint4*>(pl.remote + j * Tr::VW * 16u) : nullptr;
+          t.packs = n;
+          t.op = oi;
+          t.flags = pl.flags | (j + n >= pl.packs && pl.rest >= pl.hi ? kTileLastOfOp : 0u);
+          // What does not depend on a peer first, then the op's flags, then the staging slot.
+          const uint32_t user_bytes = n * Tr::VT * 16u, a_bytes = n * static_cast<uint32_t>(a_step);
+          if (pl.src_b != nullptr) {
+            MbarExpectTxOnly(&sh->full[s], user_bytes);
+            BulkLoad(dst + half_bytes, pl.src_b + j * Tr::VT * 16u, user_bytes, &sh->full[s]);
+          }
+          if (!a_staged) {
+            MbarExpectTxOnly(&sh->full[s], a_bytes);
+            BulkLoad(dst, pl.src_a + j * a_step, a_bytes, &sh->full[s]);
+          }
+          if (!get_ready()) {
+            alive = 0;
+            break;
+          }
+          if (a_staged) {
+            MbarExpectTxOnly(&sh->full[s], a_bytes);
+            BulkLoad(dst, pl.src_a + j * a_step, a_bytes, &sh->full[s]);
+          }
+          MbarArrive(&sh->full[s]);
+        }
+        // Elements outside whole packs, or an op without elements for this channel (which still has to be reported done).
+        if (alive > 0 && (pl.rest < pl.hi || pl.packs == 0)) {
+          if (!next_stage()) {
+            alive = -1;
+          } else if (!get_ready()) {
+            alive = 0;
+          } else {
+            ExecTile& t = sh->tile[s];
+            t.flags = kTileElements | kTileLastOfOp;
+            t.op = oi;
+            t.lo = pl.rest;
+            t.hi = pl.hi;
+            MbarArrive(&sh->full[s]);
+          }
+        }
+      }
+      alive = __shfl_sync(0xffffffffu, alive, 0);
+      if (alive < 0) return;
+      if (alive == 0) return leave(false);
+    }
+    if (good < in_batch) break;
+    __syncwarp();  // lane 0 is done with the plans of this batch
+  }
+  leave(true);
+}
+
+// The waiter: a warp that looks at all of this channel's flags at once (lane q:
+// data from rank q, lane 8 + q: credit from rank q) and releases every op whose
+// flags are there.  Lane k holds op first + k.
+template <typename W>
+__device__ void WaiterBody(const ExecParams& p, const WaitCtx& w, RoleSync* sync, uint64_t base, int ch, int lane, DeviceTraceRec* trace) {
+  static_assert(kMaxRanks == 8, "one lane per flag");
+  ControlPage* const me = Ctl(p.peers, p.rank);
+  const uint64_t* const my_flag = lane < 8 ? &me->inflag[ch][lane] : &me->credit[ch][lane & 7];
+  const bool watches = lane < 16 && (lane & 7) < p.world_size;
+  const bool one_gpu = p.peers.one_gpu != 0;
+  const uint64_t* const abort_word = &me->abort_seq;
+  uint64_t seen = 0;
+  for (int first = 0; first < p.num_ops; first += 32) {
+    const int mine = first + lane;
+    uint64_t need_data = 0, need_credit = 0;
+    int from = 0, to = 0;
+    bool bad = false;
+    uint64_t elem_begin = 0, elem_count = 0;
+    if (mine < p.num_ops) {
+      const Op op = p.ops[mine];
+      bad = !OpInBounds<W>(op, p);
+      elem_begin = op.elem_begin;
+      elem_count = op.elem_count;
+      if (!bad && op.wait_in != 0) need_data = base | op.wait_in, from = op.peer_in;
+      if (!bad && op.wait_credit != 0) need_credit = base | op.wait_credit, to = op.peer_out;
+    }
+    const int in_batch = p.num_ops - first < 32 ? p.num_ops - first : 32;
+    int released = 0;
+    uint64_t t0 = GlobalTimerNs();
+    for (uint32_t spin = 0; released < in_batch; ++spin) {
+      if (watches) seen = LdAcquirePeers(my_flag, one_gpu);
+      const uint64_t data = __shfl_sync(0xffffffffu, seen, from), credit = __shfl_sync(0xffffffffu, seen, 8 + to);
+      const bool go = !bad && (need_data == 0 || data >= need_data) && (need_credit == 0 || credit >= need_credit);
+      const unsigned blocked = ~__ballot_sync(0xffffffffu, go || lane < released);
+      const int upto = blocked == 0 ? 32 : __ffs(static_cast<int>(blocked)) - 1;
+      const int now = upto < in_batch ? upto : in_batch;
+      if (now > released) {
+        if (trace != nullptr && lane >= released && lane < now && mine < p.trace_capacity) trace[mine].t_wait_done = GlobalTimerNs();
+        released = now;
+        __syncwarp();  // what every lane acquired is ordered before the release
+        if (lane == 0) StReleaseShared(&sync->ready, static_cast<unsigned>(first + released));
+        t0 = GlobalTimerNs();
+        continue;
+      }
+      if (*reinterpret_cast<volatile int*>(&sync->stop) != 0) return;
+      int give_up = 0;
+      if (lane == released) {
+        if (bad) {
+          ReportFailure(w, kStatusBadProgram, 0, -1, mine, elem_begin, elem_count);
+          BroadcastAbort(w);
+          give_up = 1;
+        } else if ((spin & 31u) == 31u) {
+          const bool on_data = need_data != 0 && data < need_data;
+          const uint32_t kind = on_data ? kWaitData : kWaitCredit;
+          if (LdRelaxedSys(abort_word) == w.seq) {
+            ReportFailure(w, kStatusPeerAbort, kind, on_data ? from : to, mine, on_data ? need_data : need_credit, on_data ? data : credit);
+            give_up = 1;
+          } else if (GlobalTimerNs() - t0 > p.timeout_ns) {
+            ReportFailure(w, kStatusWaitTimeout, kind, on_data ? from : to, mine, on_data ? need_data : need_credit, on_data ? data : credit);
+            BroadcastAbort(w);
+            give_up = 1;
+          }
+        }
+      }
+      if (__any_sync(0xffffffffu, give_up)) {
+        if (lane == 0) *reinterpret_cast<volatile int*>(&sync->stop) = 1;
+        return;
+      }
+      if (spin > 4096u) __nanosleep(100);
+    }
+  }
+}
+
+// Body of the executor for one CTA: warps [0, data_warps) move data, then the
+// waiter's, the loader's and the poster's warp.
+template <typename T, typename W>
+__device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsigned char* smem, int stages) {
+  using Tr = ExecTraits<T, W>;
   const int ch = blockIdx.x, nch = gridDim.x;
+  RoleSync* const sync = &sh->role;
   WaitCtx w;
   w.peers = &p.peers;
   w.status = p.status;
@@ -245,85 +545,70 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, RoleSync* sync) {
   if (*stop) return;
 
   DeviceTraceRec* trace = (p.trace != nullptr && p.trace_capacity > 0) ? p.trace + static_cast<size_t>(ch) * p.trace_capacity : nullptr;
-  const int warps = static_cast<int>(blockDim.x) / 32;
-  const int data_warps = warps - 2;
+  const int data_warps = static_cast<int>(blockDim.x) / 32 - kExecServiceWarps;
   const int warp = static_cast<int>(threadIdx.x) / 32, lane = static_cast<int>(threadIdx.x) % 32;
+  const unsigned nthr = static_cast<unsigned>(data_warps) * 32u;
+  const uint32_t half_vecs = nthr * Tr::U * Tr::VT;
 
   if (warp < data_warps) {
-    // Two groups of data warps (even and odd warps) take the ops in turn.
-    // After its stores a group waits until they are acknowledged over NVLink
-    // (the release below) before the poster may publish the op; meanwhile the
-    // other group loads and stores the next op, so the link does not idle
-    // during the hand-over.  Consecutive ops are independent of each other
-    // (different chains of the ring, different pieces of a halving step) with
-    // one exception, handled by the barrier below.
-    const int group = warp & 1;
-    const unsigned all_threads = static_cast<unsigned>(data_warps) * 32u;
-    const unsigned nthr = static_cast<unsigned>((data_warps + 1 - group) / 2) * 32u;
-    const unsigned gtid = static_cast<unsigned>(warp >> 1) * 32u + static_cast<unsigned>(lane);
-    bool alive = true;
-    for (int oi = 0; oi < p.num_ops; ++oi) {
-      const Op op = p.ops[oi];
-      // No barrier separates consecutive ops, and an element need not map to
-      // the same thread in two ops that cover different ranges.  An op that
-      // reads recvbuf (Rabenseifner's running partial sums, written by earlier
-      // ops) therefore first waits until every data warp, of both groups, has
-      // finished the ops before it.  Every data warp walks the whole program
-      // and meets these barriers, also after the call was stopped.
-      // Overwrites need no such barrier: a range is overwritten only by data
-      // that a peer derived from this rank's own transfer of the range, which
-      // the poster published after all warps of the op's group had read it.
-      if (op.src_a == kSrcRecv || op.src_b == kSrcRecv) asm volatile("bar.sync 1, %0;" ::"r"(all_threads) : "memory");
-      if ((oi & 1) != group || !alive) continue;
-      int go = 1;
-      if (lane == 0) go = SpinShared(&sync->ready, static_cast<unsigned>(oi) + 1u, sync, p.timeout_ns) ? 1 : 0;
-      go = __shfl_sync(0xffffffffu, go, 0);
-      if (!go) {
-        alive = false;
-        continue;
+    for (RingPos pos(stages);; pos.Next()) {
+      const uint32_t s = pos.s;
+      if (!RingWait(&sh->full[s], pos.parity, sync, p.timeout_ns)) break;
+      const ExecTile t = sh->tile[s];
+      if (t.flags & kTileExit) break;
+      if (t.flags & kTileElements) {
+        __syncwarp();
+        if (lane == 0) MbarArrive(&sh->empty[s]);
+        RunElements<T, W>(p.ops[t.op], p, t.lo, t.hi, threadIdx.x, nthr);
+      } else {
+        RunTile<T, W>(t, reinterpret_cast<const uint4*>(smem) + static_cast<size_t>(s) * 2 * half_vecs, half_vecs, p.scale, &sh->empty[s],
+                      threadIdx.x, nthr, lane);
       }
-      RunOpData<T, W>(op, p, ch, nch, gtid, nthr);
-      __syncwarp();
-      if (lane == 0) StReleaseShared(&sync->done[warp], static_cast<unsigned>(oi) + 1u);
+      if (t.flags & kTileLastOfOp) {
+        __syncwarp();
+        if (lane == 0) StReleaseShared(&sync->done[warp], t.op + 1u);
+      }
     }
   } else if (warp == data_warps) {
-    if (lane == 0) {
-      // Waiter: bounds check, then the op's data flag and slot credit.
-      for (int oi = 0; oi < p.num_ops && *stop == 0; ++oi) {
-        const Op op = p.ops[oi];
-        bool ok = OpInBounds<W>(op, p);
-        if (!ok) {
-          ReportFailure(w, kStatusBadProgram, 0, -1, oi, op.elem_begin, op.elem_count);
-          BroadcastAbort(w);
-        }
-        if (ok && op.wait_in != 0) ok = WaitGE(&me->inflag[ch][op.peer_in], base | op.wait_in, w, kWaitData, op.peer_in, oi);
-        if (ok && op.wait_credit != 0)
-          ok = WaitGE(&me->credit[ch][op.peer_out], base | op.wait_credit, w, kWaitCredit, op.peer_out, oi);
-        if (!ok) {
-          *stop = 1;
-          break;
-        }
-        if (trace != nullptr && oi < p.trace_capacity) trace[oi].t_wait_done = GlobalTimerNs();
-        StReleaseShared(&sync->ready, static_cast<unsigned>(oi) + 1u);
-      }
-    }
+    WaiterBody<W>(p, w, sync, base, ch, lane, trace);
+  } else if (warp == data_warps + 1) {
+    LoaderBody<T, W>(p, sh, smem, stages, ch, nch, data_warps, lane);
   } else {
-    if (lane == 0) {
-      // Poster: when all data warps have issued the op's stores, make them
-      // visible system-wide and publish the op's flags.
-      for (int oi = 0; oi < p.num_ops; ++oi) {
-        // The warps of the group that ran op oi.
-        bool all = true;
-        for (int wi = oi & 1; wi < data_warps && all; wi += 2)
-          all = SpinShared(&sync->done[wi], static_cast<unsigned>(oi) + 1u, sync, p.timeout_ns);
-        if (!all) break;
-        const Op op = p.ops[oi];
-        if (op.post_out != 0) {
-          FencePeers(p.peers.one_gpu != 0);
-          StRelaxedSys(&Ctl(p.peers, op.peer_out)->inflag[ch][p.rank], base | op.post_out);
+    // Poster: when every data warp has issued an op's stores, make them visible
+    // to the peers and publish the op's flags.  Lane k holds op first + k.
+    for (int first = 0; first < p.num_ops; first += 32) {
+      const int mine = first + lane;
+      uint32_t post_out = 0, post_credit = 0;
+      int peers = 0;
+      if (mine < p.num_ops) {
+        const Op op = p.ops[mine];
+        post_out = op.post_out;
+        post_credit = op.post_credit;
+        peers = (static_cast<uint8_t>(op.peer_in) << 8) | static_cast<uint8_t>(op.peer_out);
+      }
+      const int end = first + 32 < p.num_ops ? first + 32 : p.num_ops;
+      int posted = first;
+      while (posted < end) {
+        bool ok = true;
+        if (lane < data_warps) ok = SpinShared(&sync->done[lane], static_cast<unsigned>(posted) + 1u, sync, p.timeout_ns);
+        if (!__all_sync(0xffffffffu, ok)) return;
+        // How far the slowest data warp is by now.
+        unsigned upto = lane < data_warps ? LdAcquireShared(&sync->done[lane]) : 0xffffffffu;
+        upto = __reduce_min_sync(0xffffffffu, upto);
+        const int until = static_cast<int>(upto) < end ? static_cast<int>(upto) : end;
+        const bool publishes = __any_sync(0xffffffffu, mine >= posted && mine < until && post_out != 0);
+        __syncwarp();  // what the other lanes acquired is ordered before lane 0's fence
+        if (publishes && lane == 0) FencePeers(p.peers.one_gpu != 0);
+        for (; posted < until; ++posted) {
+          const int k = posted - first;
+          const uint32_t out = __shfl_sync(0xffffffffu, post_out, k), credit = __shfl_sync(0xffffffffu, post_credit, k);
+          const int who = __shfl_sync(0xffffffffu, peers, k);
+          if (lane == 0) {
+            if (out != 0) StRelaxedSys(&Ctl(p.peers, who & 0xff)->inflag[ch][p.rank], base | out);
+            if (credit != 0) StRelaxedSys(&Ctl(p.peers, who >> 8)->credit[ch][p.rank], base | credit);
+            if (trace != nullptr && posted < p.trace_capacity) trace[posted].t_done = GlobalTimerNs();
+          }
         }
-        if (op.post_credit != 0) StRelaxedSys(&Ctl(p.peers, op.peer_in)->credit[ch][p.rank], base | op.post_credit);
-        if (trace != nullptr && oi < p.trace_capacity) trace[oi].t_done = GlobalTimerNs();
       }
     }
   }
@@ -331,20 +616,28 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, RoleSync* sync) {
 
 template <typename T, typename W>
 __global__ void __launch_bounds__(kExecThreads, 1)
-ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all) {
+ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all, int stages) {
   __shared__ ExecParams p;
-  __shared__ RoleSync s_sync;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ ExecShared s_exec;
   __shared__ uint64_t s_seq;
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
     for (unsigned i = threadIdx.x; i < sizeof(ExecParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
-    if (threadIdx.x == 0) RoleSyncInit(&s_sync);
+    if (threadIdx.x == 0) {
+      RoleSyncInit(&s_exec.role);
+      for (int i = 0; i < kExecMaxStages; ++i) {
+        MbarInit(&s_exec.full[i], 1);
+        MbarInit(&s_exec.empty[i], blockDim.x / 32 - kExecServiceWarps);
+      }
+      MbarInitFence();
+    }
   }
   __syncthreads();
   if (p.world_size <= 1) return;
   const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
   // num_ops <= 0: this rank sits the call out (test hook), but still counts it.
-  if (p.num_ops > 0) ExecBody<T, W>(p, seq, &s_sync);
+  if (p.num_ops > 0) ExecBody<T, W>(p, seq, &s_exec, smem, stages);
   EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
@@ -352,14 +645,29 @@ ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all) {
 
 static int ExecThreads() {
   const int v = Tunable("IBCOMM_EXEC_THREADS", 0);
-  return (v >= 64 && v <= kExecThreads && v % 32 == 0) ? v : kExecThreads;
+  return (v >= 128 && v <= kExecThreads && v % 32 == 0) ? v : kExecThreads;
+}
+
+// Stages of the ring: what fits into an SM's shared memory, or into half of it
+// for the smaller CTAs, of which two share an SM.
+static int ExecStages(int threads) {
+  const int stage = (threads - 32 * dev::kExecServiceWarps) * dev::kExecStageBytesPerThread;
+  const int room = (threads > 256 ? 208 : 104) << 10;
+  return std::min(dev::kExecMaxStages, std::max(2, room / stage));
+}
+static size_t ExecSmemBytes(int threads) {
+  return static_cast<size_t>(ExecStages(threads)) * static_cast<size_t>((threads - 32 * dev::kExecServiceWarps) * dev::kExecStageBytesPerThread);
 }
 
 template <typename T, typename W>
 static cudaError_t Launch(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
   // Beyond one CTA per SM, two smaller CTAs share an SM: while one waits for a
   // flag, the other streams.
-  return LaunchRanks(dev::ExecKernel<T, W>, ranks, n, channels, ExecKernelThreadsFor(channels), 0, stream);
+  const int threads = ExecKernelThreadsFor(channels * n);
+  const size_t smem = ExecSmemBytes(threads);
+  const cudaError_t e = AllowSharedMemory(dev::ExecKernel<T, W>, smem);
+  if (e != cudaSuccess) return e;
+  return LaunchRanks(dev::ExecKernel<T, W>, ranks, n, channels, threads, smem, stream, ExecStages(threads));
 }
 
 cudaError_t LaunchExecKernel(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
@@ -375,12 +683,14 @@ cudaError_t LaunchExecKernel(const ExecParams* ranks, int n, int channels, cudaS
   return cudaErrorInvalidValue;
 }
 
-int ExecKernelThreadsFor(int channels) { return (channels > 148 && ExecThreads() > 256) ? 256 : ExecThreads(); }
+int ExecKernelThreadsFor(int ctas) { return (ctas > 148 && ExecThreads() > 256) ? 256 : ExecThreads(); }
 
 int ExecKernelMaxCoResidentBlocks(int device, int threads) {
   int per_sm = 0, sms = 0;
   if (threads <= 0) threads = kExecThreads;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::ExecKernel<float, float>, threads, 0) != cudaSuccess) return 0;
+  const size_t smem = ExecSmemBytes(threads);
+  if (AllowSharedMemory(dev::ExecKernel<float, float>, smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::ExecKernel<float, float>, threads, smem) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
   return per_sm * sms;
 }

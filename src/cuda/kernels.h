@@ -21,26 +21,33 @@ struct RankBlocks {
 // grid = (blocks, ranks).  With several ranks the launch is cooperative: their
 // CTAs wait on each other, so the runtime has to refuse a grid that is not
 // co-resident.
-template <typename P>
-cudaError_t LaunchRanks(void (*kernel)(RankBlocks<P>), const P* ranks, int n, int blocks, int threads, size_t smem, cudaStream_t stream) {
-  static_assert(sizeof(RankBlocks<P>) <= 4096, "kernel parameters");
+template <typename P, typename... Rest>
+cudaError_t LaunchRanks(void (*kernel)(RankBlocks<P>, Rest...), const P* ranks, int n, int blocks, int threads, size_t smem,
+                        cudaStream_t stream, Rest... rest) {
+  static_assert(sizeof(RankBlocks<P>) <= 4000, "kernel parameters");
   if (n < 1 || n > kMaxRanks) return cudaErrorInvalidValue;
   RankBlocks<P> all;
   for (int r = 0; r < n; ++r) all.rank[r] = ranks[r];
-  void* args[] = {&all};
+  void* args[] = {&all, &rest...};
   const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(n));
   if (n > 1) return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, dim3(static_cast<unsigned>(threads)), args, smem, stream);
   return cudaLaunchKernel(reinterpret_cast<const void*>(kernel), grid, dim3(static_cast<unsigned>(threads)), args, smem, stream);
+}
+// Opts `kernel` in to `bytes` of dynamic shared memory (beyond 48 KiB it has to
+// be): a property of the (function, device) pair, cheap, so set at every launch.
+template <typename Kernel>
+cudaError_t AllowSharedMemory(Kernel* kernel, size_t bytes) {
+  return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
 // ---- op-program executor (ring, Rabenseifner) ----
 // Here and below: `ranks` points to `n` parameter blocks, one per rank on this GPU.
 cudaError_t LaunchExecKernel(const ExecParams* ranks, int n, int channels, cudaStream_t stream);
-// CTA size the executor uses for a grid of `channels` CTAs, and the largest
+// CTA size the executor uses for a grid of `ctas` CTAs, and the largest
 // grid of CTAs of `threads` threads (0 = the full-size CTA) that is co-resident
 // on `device` (0 on error).  CTA b of a rank waits for CTA b of the other
 // ranks, so a collective never launches more CTAs than fit at once.
-int ExecKernelThreadsFor(int channels);
+int ExecKernelThreadsFor(int ctas);
 int ExecKernelMaxCoResidentBlocks(int device, int threads = 0);
 
 // ---- world_size == 1: out = cast(in * scale) ----

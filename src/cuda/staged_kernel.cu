@@ -566,8 +566,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
 template <typename T, typename W, bool kMultimem, int kR>
 static cudaError_t LaunchStagedOne(const StagedParams* ranks, int n, int blocks, cudaStream_t stream) {
   auto kernel = dev::StagedKernel<T, W, kMultimem, kR>;
-  // Per (function, device); cheap, so made on every launch.
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dev::kStagedSmemBytes));
+  const cudaError_t e = AllowSharedMemory(kernel, dev::kStagedSmemBytes);
   if (e != cudaSuccess) return e;
   return LaunchRanks(kernel, ranks, n, blocks, dev::kStagedThreads, dev::kStagedSmemBytes, stream);
 }
@@ -607,7 +606,7 @@ cudaError_t LaunchStagedKernel(const StagedParams* ranks, int n, int blocks, cud
 int StagedKernelMaxCoResidentBlocks(int device) {
   int per_sm = 0, sms = 0;
   auto kernel = dev::StagedKernel<float, float, false, kMaxRanks>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dev::kStagedSmemBytes)) != cudaSuccess) return 0;
+  if (AllowSharedMemory(kernel, dev::kStagedSmemBytes) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, dev::kStagedThreads, dev::kStagedSmemBytes) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
   return per_sm * sms;

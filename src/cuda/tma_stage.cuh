@@ -22,19 +22,27 @@ __device__ __forceinline__ void MbarInitFence() { asm volatile("fence.mbarrier_i
 __device__ __forceinline__ void MbarExpectTx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void MbarExpectTxOnly(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void MbarArrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemAddr(bar)) : "memory");
+}
+__device__ __forceinline__ bool MbarTryWait(uint64_t* bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(SmemAddr(bar)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 // Bounded wait on a phase; false when the limit ran out.
 __device__ __forceinline__ bool MbarWait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t spin = 0; spin < kMbarSpinLimit; ++spin) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(SmemAddr(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
+  for (uint32_t spin = 0; spin < kMbarSpinLimit; ++spin)
+    if (MbarTryWait(bar, parity)) return true;
   return false;
 }
 // global -> shared; completion is counted in bytes on `bar`.

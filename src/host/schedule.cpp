@@ -2,6 +2,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <unordered_map>
 
 #include "ibcomm/tunables.h"
 
@@ -151,8 +152,11 @@ void BuildRing(Builder* bld) {
   // flag travels, the CTA moves the others' data.  A group of g chains keeps
   // up to g transfers ahead of the downstream rank's receives, so it needs
   // g + 1 staging slots (with g slots every rank would wait for a credit that
-  // its neighbour can only return after the same wait).
-  const size_t group = std::max<size_t>(1, std::min<size_t>(positions, bld->slots > 1 ? bld->slots - 1 : 1));
+  // its neighbour can only return after the same wait).  With s slots an op
+  // needs its neighbour's op s - g before it: with g + 1 the ranks go op by op,
+  // each waiting for the other's hand-over (4 us on one GPU), so half the
+  // slots are left to run ahead into.
+  const size_t group = std::max<size_t>(1, std::min<size_t>(positions, bld->slots / 2));
   for (size_t i0 = 0; i0 < positions; i0 += group) {
     const size_t i1 = std::min(positions, i0 + group);
     for (size_t i = i0; i < i1; ++i) {
@@ -320,6 +324,16 @@ Program BuildProgram(const ProgramRequest& req) {
     default:
       IBCOMM_FAIL(INVALID_ARGUMENT, "No op program exists for algorithm '%s'.\n", AlgoName(req.algo));
   }
+  // A cell is stored and read as a whole or in parts, never across cells.
+  std::unordered_map<uint64_t, uint32_t> stored;  // cell -> 1 + the last op that stored into it
+  for (size_t i = 0; i < bld.prog.ops.size(); ++i) {
+    Op& op = bld.prog.ops[i];
+    if (op.src_a == kSrcRecv || op.src_b == kSrcRecv) {
+      const auto it = stored.find(op.cell_begin);
+      if (it != stored.end()) op.wait_local = it->second;
+    }
+    if (op.flags & kOpStoreLocal) stored[op.cell_begin] = static_cast<uint32_t>(i + 1);
+  }
   return bld.prog;
 }
 
@@ -398,6 +412,8 @@ std::string ValidateProgram(const Program& prog, uint64_t len_elements, size_t w
       why = "peer_out is not a rank";
     } else if ((op.wait_in != 0 || op.post_credit != 0) && (op.peer_in < 0 || op.peer_in >= world_size)) {
       why = "peer_in is not a rank";
+    } else if (op.wait_local > i) {
+      why = "waits for an op that comes later";
     }
     if (why != nullptr) return "op " + std::to_string(i) + ": " + why + ": " + DescribeOp(op);
   }
