@@ -219,6 +219,8 @@ struct ExecParams {
   const Op* ops;
   int32_t num_ops;
   int32_t trace_capacity;  // records per channel, 0 = tracing off
+  int32_t stream_recv;     // no op reads recvbuf: its stores need not stay in L2
+  int32_t pad_;
   StageLayout stage;
   uint64_t timeout_ns;   // limit of every wait
   DeviceStatus* status;  // device memory, fetched by the host after a failure

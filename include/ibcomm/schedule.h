@@ -12,8 +12,9 @@
 // rank ^ (1 << s), nearest first, the lower rank giving away the front part;
 // recursive doubling in mirror order; every rank-block moves as its pipeline
 // chunks.  World sizes that are not a power of two are folded first: ranks
-// below 2 * (ws - 2^k) pair up, swap halves and add, the even rank hands its
-// half over and sits out, and gets the result back at the end.
+// below 2 * (ws - 2^k) pair up, the even rank gives its message away and sits
+// out, and gets the result back at the end, one half from its partner and one
+// from the rank its partner exchanges halves with.
 #pragma once
 
 #include <string>
@@ -43,6 +44,7 @@ struct ProgramRequest {
 struct Program {
   std::vector<Op> ops;
   StageLayout stage{};
+  bool reads_recv = false;    // some op has recvbuf as a source
   std::vector<int> in_peers;  // region index -> source rank, for this rank
   // Transfers per peer over the whole program, for tests and credit audits.
   uint32_t sent_to[kMaxRanks] = {0};

@@ -226,7 +226,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
     // Validation (length, chunk size) happens while the first program is cut.
     std::vector<ExecParams> ps;
     for (int r = 0; r < m.ws; ++r) {
-      const CachedProgram& cp = m.cache.Get(algo, r, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false);
+      const CachedProgram& cp = m.cache.Get(algo, r, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false, m.ws);
       ps.push_back(MakeExecParams(m.ranks[static_cast<size_t>(r)], cp, dtype, wire, sendbufs[static_cast<size_t>(r)],
                                   recvbufs[static_cast<size_t>(r)], n, scale, timeout_ns, nullptr, 0));
       if (r == m.silent_rank) ps.back().num_ops = 0;
@@ -235,7 +235,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
     // A channel for every 4 KiB of a transfer: the flags of ranks on one GPU are
     // cheap, and more channels shorten every step of the program.  One CTA per
     // SM at most (two smaller ones per SM are no faster).
-    const uint64_t slot = m.cache.Get(algo, 0, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false).prog.stage.slot_bytes;
+    const uint64_t slot = ps.back().stage.slot_bytes;
     int ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(slot / 4096, static_cast<uint64_t>(kMaxChannels)));
     ch = std::max(1, std::min(ch, channels > 0 ? m.exec_max_blocks / m.ws : cap));
     CUDACHECK(LaunchExecKernel(ps.data(), m.ws, ch, stream));

@@ -143,7 +143,7 @@ void ProgramCache::NoteSynchronized() {
 }
 
 const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size_t len_elements, DType dtype, DType wire,
-                                       const ArenaLayout& layout, bool apply_scale, cudaStream_t stream, bool capturing) {
+                                       const ArenaLayout& layout, bool apply_scale, cudaStream_t stream, bool capturing, int ranks_on_gpu) {
   const size_t esize = DTypeSize(dtype), wsize = DTypeSize(wire);
   // Read at the point of use, like the reference: a bad value fails the call.
   const long long env_chunk = env::ReadChunkSize();
@@ -152,12 +152,20 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   // region and, since one collective runs at a time, in the pool in front of
   // it as well (the two are adjacent in the arena).
   const uint64_t stage_off = layout.pool_offset;
-  const uint64_t stage_bytes = ring ? layout.pool_bytes : layout.pool_bytes + layout.work_bytes;
+  // The ranks that share a GPU share its L2 too: a ring whose slots fit into it
+  // together keeps its transfers there (a byte is written to staging and read
+  // back 1.75 times).  Halving and doubling read recvbuf back as well, which
+  // does not fit, and get large pieces instead.
+  const uint64_t stage_bytes = ring ? std::min<uint64_t>(layout.pool_bytes, kSharedGpuStageBytes / static_cast<uint64_t>(ranks_on_gpu > 1 ? ranks_on_gpu : 1))
+                                    : layout.pool_bytes + layout.work_bytes;
   // Knobs that shape the program are part of the key: the ring's chunks per
   // rank and the number of pieces Rabenseifner cuts the message into.
   const size_t ring_cpr = ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size)) : 0;
-  int raben_div = Tunable("IBCOMM_RABEN_PIECES", 8);
-  if (raben_div < 1 || raben_div > 1024) raben_div = 8;
+  // Ranks on one GPU: four pieces of up to 8 MiB (a hand-over costs what 100 KiB
+  // per channel cost; 5 ranks, 4 / 16 MiB: 75 / 134 us with eight, 64 / 122 with four).
+  int raben_div = Tunable("IBCOMM_RABEN_PIECES", 0);
+  if (raben_div < 1 || raben_div > 1024)
+    raben_div = ranks_on_gpu > 1 ? static_cast<int>(std::min<size_t>(1024, std::max<size_t>(4, util::ceilDiv(len_elements * esize, size_t(8) << 20)))) : 8;
   Key key{static_cast<int>(algo), rank, world_size, len_elements, static_cast<int>(dtype), static_cast<int>(wire),
           env_chunk, apply_scale, stage_off, stage_bytes, ring ? static_cast<int>(ring_cpr) : raben_div};
   auto it = cache_.find(key);
@@ -245,6 +253,7 @@ ExecParams MakeExecParams(const RankResources& rr, const CachedProgram& cp, DTyp
   p.num_ops = static_cast<int32_t>(cp.prog.ops.size());
   p.trace_capacity = trace_capacity;
   p.stage = cp.prog.stage;
+  p.stream_recv = cp.prog.reads_recv ? 0 : 1;
   p.timeout_ns = timeout_ns;
   p.status = rr.d_status;
   p.doorbell = rr.d_doorbell;

@@ -27,7 +27,9 @@
 // moved 10-15 GB/s whether the data came from L2 or from HBM; the ring keeps
 // 100 KiB (fp32) ahead of the data warps across op boundaries.  Per op, what is
 // left in series (flags, plan, fence) takes about 1.2 us, and a hand-over
-// between two ranks on one GPU about 3 us.  Ranks sharing a B200, before and
+// between two ranks on one GPU about 3 us.  User data that is touched once goes
+// through L2 as evict-first, so that the staging slots of ranks sharing a GPU
+// stay there (ring 8 x 256 MiB 1.40 -> 1.23 ms).  Ranks sharing a B200, before and
 // after: Rabenseifner 5 x 64 MiB 908 -> 430 us, ring 8 x 32 MiB 258 -> 192 us,
 // ring 7 x 4 MB 96 -> 70 us, ring 8 x 4 KiB 52 -> 46 us.
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda
@@ -125,7 +127,7 @@ __device__ __forceinline__ bool RingWait(uint64_t* bar, uint32_t parity, RoleSyn
 
 // One stage: packs of P elements, U of them per thread.
 template <typename T, typename W>
-__device__ __forceinline__ void RunTile(const ExecTile& t, const uint4* stage, uint32_t b_off, double scale, uint64_t* empty, unsigned tid,
+__device__ __forceinline__ void RunTile(const ExecTile& t, const uint4* stage, uint32_t b_off, double scale, uint64_t* empty, uint64_t local_policy, unsigned tid,
                                         unsigned nthr, int lane) {
   using Tr = ExecTraits<T, W>;
   using A = typename Tr::A;
@@ -187,7 +189,7 @@ __device__ __forceinline__ void RunTile(const ExecTile& t, const uint4* stage, u
           for (int v = 0; v < VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
         }
 #pragma unroll
-        for (int v = 0; v < VT; ++v) St16(t.local + i * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN));
+        for (int v = 0; v < VT; ++v) St16Hint(t.local + i * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), local_policy);
       }
     }
   }
@@ -289,6 +291,8 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
   const unsigned nthr = static_cast<unsigned>(data_warps) * 32u;
   const uint32_t tile_packs = nthr * Tr::U;
   const uint32_t half_bytes = tile_packs * Tr::VT * 16u;  // source a, then source b
+  // sendbuf is read once; what is read back from recvbuf may be needed again.
+  const uint64_t user_policy = p.stream_recv != 0 ? PolicyEvictFirst() : PolicyNormal();
   RingPos pos(stages);
   bool first_round = true;
   uint32_t s = 0;  // stage claimed last (lane 0)
@@ -400,11 +404,11 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           const uint32_t user_bytes = n * Tr::VT * 16u, a_bytes = n * static_cast<uint32_t>(a_step);
           if (pl.src_b != nullptr) {
             MbarExpectTxOnly(&sh->full[s], user_bytes);
-            BulkLoad(dst + half_bytes, pl.src_b + j * Tr::VT * 16u, user_bytes, &sh->full[s]);
+            BulkLoadHint(dst + half_bytes, pl.src_b + j * Tr::VT * 16u, user_bytes, &sh->full[s], user_policy);
           }
           if (!a_staged) {
             MbarExpectTxOnly(&sh->full[s], a_bytes);
-            BulkLoad(dst, pl.src_a + j * a_step, a_bytes, &sh->full[s]);
+            BulkLoadHint(dst, pl.src_a + j * a_step, a_bytes, &sh->full[s], user_policy);
           }
           if (!get_ready()) {
             alive = 0;
@@ -551,6 +555,8 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
   const uint32_t half_vecs = nthr * Tr::U * Tr::VT;
 
   if (warp < data_warps) {
+    // A result nobody reads back should leave L2 before the staging slots do.
+    const uint64_t local_policy = p.stream_recv != 0 ? PolicyEvictFirst() : PolicyNormal();
     for (RingPos pos(stages);; pos.Next()) {
       const uint32_t s = pos.s;
       if (!RingWait(&sh->full[s], pos.parity, sync, p.timeout_ns)) break;
@@ -561,7 +567,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
         if (lane == 0) MbarArrive(&sh->empty[s]);
         RunElements<T, W>(p.ops[t.op], p, t.lo, t.hi, threadIdx.x, nthr);
       } else {
-        RunTile<T, W>(t, reinterpret_cast<const uint4*>(smem) + static_cast<size_t>(s) * 2 * half_vecs, half_vecs, p.scale, &sh->empty[s],
+        RunTile<T, W>(t, reinterpret_cast<const uint4*>(smem) + static_cast<size_t>(s) * 2 * half_vecs, half_vecs, p.scale, &sh->empty[s], local_policy,
                       threadIdx.x, nthr, lane);
       }
       if (t.flags & kTileLastOfOp) {

@@ -51,6 +51,12 @@ __device__ __forceinline__ void BulkLoad(void* smem_dst, const void* gmem_src, u
                "l"(gmem_src), "r"(bytes), "r"(SmemAddr(bar))
                : "memory");
 }
+// The same with a cache policy for L2.
+__device__ __forceinline__ void BulkLoadHint(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar, uint64_t policy) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(SmemAddr(smem_dst)),
+               "l"(gmem_src), "r"(bytes), "r"(SmemAddr(bar)), "l"(policy)
+               : "memory");
+}
 // shared -> global, as part of the thread's current bulk group.
 __device__ __forceinline__ void BulkStore(void* gmem_dst, const void* smem_src, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(SmemAddr(smem_src)), "r"(bytes)

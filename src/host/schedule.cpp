@@ -191,22 +191,17 @@ void BuildRabenseifner(Builder* bld) {
   auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
   std::vector<int> all(static_cast<size_t>(C));
   for (int i = 0; i < C; ++i) all[static_cast<size_t>(i)] = i;
-  const std::vector<int> front(all.begin(), all.begin() + C / 2), back(all.begin() + C / 2, all.end());
   const std::vector<int> none;
 
   int vrank;
   OpSrc partial = kSrcSend;  // where my running partial sum lives
   if (r < 2 * extra) {
-    const bool even = (r & 1) == 0;
-    const int partner = even ? r + 1 : r - 1;
-    const std::vector<int>& keep = even ? front : back;
-    const std::vector<int>& give = even ? back : front;
-    bld->Exchange(partner, give, kSrcSend, keep, kSrcSend, false);
-    if (even) {
-      bld->Exchange(partner, keep, kSrcRecv, none, kSrcNone, false);
+    // The even rank gives its whole message away and sits out until the end.
+    if ((r & 1) == 0) {
+      bld->Exchange(r + 1, all, kSrcSend, none, kSrcNone, false);
       vrank = -1;
     } else {
-      bld->Exchange(partner, none, kSrcRecv, give, kSrcNone, false);
+      bld->Exchange(r - 1, none, kSrcNone, all, kSrcSend, false);
       vrank = r / 2;
       partial = kSrcRecv;
     }
@@ -241,15 +236,25 @@ void BuildRabenseifner(Builder* bld) {
       } else {
         rb = b - w; re = b;
       }
-      bld->Exchange(real_rank(vpeer), ChunksOfBlocks(blocks, b, e), kSrcRecv, ChunksOfBlocks(blocks, rb, re), kSrcNone, false);
+      const std::vector<int> mine = ChunksOfBlocks(blocks, b, e);
+      bld->Exchange(real_rank(vpeer), mine, kSrcRecv, ChunksOfBlocks(blocks, rb, re), kSrcNone, false);
+      if (s == exp - 1) {
+        // The halves of the last exchange are all a folded rank needs: it gets
+        // one from its partner and one from the partner's partner, its own first.
+        for (int v : {vrank, vpeer})
+          if (v < extra) bld->Exchange(2 * v, mine, kSrcRecv, none, kSrcNone, false);
+      }
       b = std::min(b, rb);
       e = std::max(e, re);
     }
-  }
-
-  if (r < 2 * extra) {
-    if ((r & 1) == 0) bld->Exchange(r + 1, none, kSrcRecv, all, kSrcNone, false);
-    else bld->Exchange(r - 1, all, kSrcRecv, none, kSrcNone, false);
+  } else {
+    const std::vector<std::vector<int>> blocks = GetRankToChunk(static_cast<size_t>(C), static_cast<size_t>(p));
+    const int v = r / 2;
+    // What rank `v` of the halving owns before the last exchange: the half of the
+    // message on its side of the first halving step.
+    auto half = [&](int who) { return (who & 1) == 0 ? ChunksOfBlocks(blocks, p - p / 2, p) : ChunksOfBlocks(blocks, 0, p - p / 2); };
+    bld->Exchange(real_rank(v), none, kSrcNone, half(v), kSrcNone, false);
+    bld->Exchange(real_rank(v ^ 1), none, kSrcNone, half(v ^ 1), kSrcNone, false);
   }
 }
 
@@ -270,6 +275,8 @@ std::vector<int> InPeers(Algo algo, int rank, int world_size) {
   int vrank;
   if (rank < 2 * extra) {
     peers.push_back((rank & 1) == 0 ? rank + 1 : rank - 1);
+    // A folded rank gets half of the result from its partner's last exchange partner.
+    if ((rank & 1) == 0) peers.push_back(real_rank((rank / 2) ^ 1));
     vrank = (rank & 1) == 0 ? -1 : rank / 2;
   } else {
     vrank = rank - extra;
@@ -329,6 +336,7 @@ Program BuildProgram(const ProgramRequest& req) {
   for (size_t i = 0; i < bld.prog.ops.size(); ++i) {
     Op& op = bld.prog.ops[i];
     if (op.src_a == kSrcRecv || op.src_b == kSrcRecv) {
+      bld.prog.reads_recv = true;
       const auto it = stored.find(op.cell_begin);
       if (it != stored.end()) op.wait_local = it->second;
     }
