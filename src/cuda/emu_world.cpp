@@ -30,6 +30,51 @@ struct EmuWorld::Impl {
   DeviceStatus last_report{};
 };
 
+namespace {
+
+// How the pipelined staged kernel runs when its ranks share a GPU.
+struct StagedShape {
+  bool split;    // copy roles in blocks of their own
+  int buffers;   // windows of each kind
+  int blocks;    // reducing blocks per rank (and copying blocks when split)
+  uint64_t window_bytes;
+  int load_groups, reduce_groups, store_groups;
+};
+
+// `bytes`: of a rank's message in the wire type; `resident`: blocks of the kernel
+// the GPU holds at once.  Measured on a B200 (the knobs override each choice):
+//  * The windows of all ranks share one L2, and what falls out of it is written
+//    to HBM and read back: 72 MiB of them in four buffers of each kind (4 ranks
+//    x 64 MiB: 205 us; 24 MiB 440, all of the pool 248), or 40 MiB in three
+//    with a 16-bit wire (8 x 25 MiB of fp32: 182 us against 257).
+//  * A pass of a role over a window is a chain of flag and memory round trips;
+//    with several windows two groups per role overlap them.
+//  * A message of one window has nothing to overlap, and from 1 MiB on is faster
+//    when every block does every role in turn (4 ranks x 4 MiB: 25 against 30 us).
+//  * A block per 16 KiB: with one per 128 KiB a 0.5 MiB message on 5 ranks takes
+//    27 us, with one per 16 KiB 21.
+StagedShape StagedShapeOnOneGpu(uint64_t bytes, bool narrow_wire, int ws, uint64_t staging_bytes, int resident, int channels) {
+  StagedShape s;
+  s.buffers = std::max(3, std::min(Tunable("IBCOMM_STAGED_BUFFERS", narrow_wire ? 3 : 4), kStagedMaxBuffers));
+  const uint64_t l2_bytes = static_cast<uint64_t>(narrow_wire ? 40 : 72) << 20;
+  const uint64_t kinds = static_cast<uint64_t>(2 * s.buffers);
+  const uint64_t room = staging_bytes / kinds / 4096 * 4096;
+  const bool one_window = bytes <= room && bytes * 2 * static_cast<uint64_t>(ws) <= l2_bytes;
+  s.window_bytes = one_window ? room : std::min(room, l2_bytes / (kinds * static_cast<uint64_t>(ws)) / 4096 * 4096);
+  const int per_rank = std::max(1, resident / ws);
+  s.split = Tunable("IBCOMM_STAGED_SPLIT", one_window && bytes >= (1u << 20) ? 0 : 1) != 0 && per_rank >= 2;
+  const int most = std::min(128, s.split ? per_rank / 2 : per_rank);
+  s.blocks = std::max(1, std::min(channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(bytes / (16u << 10), 128)), most));
+  const int copy_groups = one_window ? 1 : 2;
+  auto groups = [](const char* knob, int dflt) { return std::max(1, std::min(Tunable(knob, dflt), 4)); };
+  s.load_groups = groups("IBCOMM_STAGED_LOAD_GROUPS", copy_groups);
+  s.reduce_groups = groups("IBCOMM_STAGED_REDUCE_GROUPS", 2);
+  s.store_groups = groups("IBCOMM_STAGED_STORE_GROUPS", copy_groups);
+  return s;
+}
+
+}  // namespace
+
 EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(num_ranks), impl_(new Impl()) {
   if (num_ranks < 1 || num_ranks > kMaxRanks)
     IBCOMM_FAIL(NOT_SUPPORTED, "EmuWorld supports 1..%d ranks (got %d).\n", kMaxRanks, num_ranks);
@@ -116,16 +161,11 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
   const size_t wsize = DTypeSize(wire);
   if (algo == Algo::kDirect && (wire != dtype || m.direct_staging == 2)) {
     // The pipelined staged kernel (what ordinary buffers and 16-bit wires get on several GPUs).
-    // Copy roles in blocks of their own: twice the blocks, all of them co-resident with every rank's.
-    const bool split = Tunable("IBCOMM_STAGED_SPLIT", 1) != 0 && m.staged_max_blocks / m.ws >= 2;
-    int buffers = Tunable("IBCOMM_STAGED_BUFFERS", 3);
-    buffers = std::max(3, std::min(buffers, kStagedMaxBuffers));
-    const uint64_t quarter = (m.layout.pool_bytes + m.layout.work_bytes) / static_cast<uint64_t>(2 * buffers) / 4096 * 4096;
-    if (!all_aligned || (n * wsize) % 16 != 0 || quarter < 4096)
+    const StagedShape sh = StagedShapeOnOneGpu(n * wsize, wire != dtype, m.ws, m.layout.pool_bytes + m.layout.work_bytes,
+                                               m.staged_max_blocks, channels);
+    if (!all_aligned || (n * wsize) % 16 != 0 || sh.window_bytes < 4096)
       IBCOMM_FAIL(NOT_SUPPORTED, "The pipelined staged two-shot needs 16-byte aligned buffers of whole 16-byte wire vectors.\n");
-    int ch = channels > 0 ? channels : ChooseChannels(Algo::kDirect, n * wsize, m.ws, kMaxChannels);
-    ch = std::max(1, std::min(std::min(ch, 128), std::max(1, m.staged_max_blocks / m.ws)));
-    if (split) ch = std::max(1, std::min(ch, m.staged_max_blocks / m.ws / 2));
+    const int ch = sh.blocks;
     std::vector<StagedParams> ps(static_cast<size_t>(m.ws));
     for (int r = 0; r < m.ws; ++r) {
       StagedParams& p = ps[static_cast<size_t>(r)];
@@ -142,25 +182,25 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.recvbuf = recvbufs[static_cast<size_t>(r)];
       p.len_elements = n;
       p.scale = scale;
-      p.window_elems = TwoShotWindowElems(n, quarter / wsize, wsize, m.ws, ch);
-      p.buffers = buffers;
-      p.split_ctas = split ? 1 : 0;
-      p.load_groups = std::max(1, std::min(Tunable("IBCOMM_STAGED_LOAD_GROUPS", 1), 4));
-      p.reduce_groups = std::max(1, std::min(Tunable("IBCOMM_STAGED_REDUCE_GROUPS", 2), 4));
-      p.store_groups = std::max(1, std::min(Tunable("IBCOMM_STAGED_STORE_GROUPS", 1), 4));
+      p.window_elems = TwoShotWindowElems(n, sh.window_bytes / wsize, wsize, m.ws, ch);
+      p.buffers = sh.buffers;
+      p.split_ctas = sh.split ? 1 : 0;
+      p.load_groups = sh.load_groups;
+      p.reduce_groups = sh.reduce_groups;
+      p.store_groups = sh.store_groups;
       p.posters = Tunable("IBCOMM_STAGED_POSTERS", 0) != 0 ? 1 : 0;
       for (int q = 0; q < m.ws; ++q) p.stage[q] = rr.peers.arena[q];
       p.mc_stage = nullptr;
-      for (int j = 0; j < buffers; ++j) {
-        p.in_off[j] = m.layout.pool_offset + static_cast<uint64_t>(j) * quarter;
-        p.out_off[j] = m.layout.pool_offset + static_cast<uint64_t>(buffers + j) * quarter;
+      for (int j = 0; j < sh.buffers; ++j) {
+        p.in_off[j] = m.layout.pool_offset + static_cast<uint64_t>(j) * sh.window_bytes;
+        p.out_off[j] = m.layout.pool_offset + static_cast<uint64_t>(sh.buffers + j) * sh.window_bytes;
       }
       p.timeout_ns = timeout_ns;
       p.status = rr.d_status;
       p.doorbell = rr.d_doorbell;
       if (r == m.silent_rank) p.len_elements = 0;  // takes no part: no window, no flag
     }
-    CUDACHECK(LaunchStagedKernel(ps.data(), m.ws, split ? 2 * ch : ch, stream));
+    CUDACHECK(LaunchStagedKernel(ps.data(), m.ws, sh.split ? 2 * ch : ch, stream));
     m.last_channels = ch;
   } else if (algo == Algo::kDirect) {
     // The two-shot kernel with peer loads and stores.  All ranks' buffers live

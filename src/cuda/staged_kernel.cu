@@ -37,6 +37,10 @@
 //     reducer groups optional poster warps that fence and publish behind the
 //     data warps (both off by default: within a few percent on 2 B200).
 //
+// With peer loads and stores in the buffers' own type a rank's own shard skips
+// the pool: nobody else needs it there, so its reducers take it from sendbuf and
+// put the result into recvbuf (1 / world_size of the copying saved).
+//
 // When the wire type equals the buffer type the copies are bulk asynchronous
 // copies (TMA, `cp.async.bulk`, global -> shared -> global, no multicast, this
 // GPU's memory only) driven by one thread per copy group through a ring of
@@ -116,18 +120,32 @@ struct RoleCtx {
   uint32_t round;
 };
 
-// Waits until every rank's word for `flag_window` in `row` (a role with
-// `groups` groups) has reached `value`.  All threads of the group call it and
-// get the same answer: false when the call is over (a wait ran out here or
-// elsewhere).
-__device__ __forceinline__ bool RoleWait(RoleCtx& c, int row, uint64_t flag_window, int groups, uint64_t value, uint32_t kind, int window) {
-  uint64_t* words = FlagRow(Ctl(*c.w.peers, c.w.rank), row, c.cta, c.ncta, flag_window, groups);
+// What a role waits for: every rank's word for window `flag_window` in `row` (a
+// role with `groups` groups) has reached `value`.
+struct RoleNeed {
+  int row;
+  uint64_t flag_window;
+  int groups;
+  uint64_t value;
+  uint32_t kind;
+};
+
+// Waits for `need`, and at the same time for `also` where there is one (watched
+// by the group's second warp: one look at memory instead of two in a row).  All
+// threads of the group call it and get the same answer: false when the call is
+// over (a wait ran out here or elsewhere).
+__device__ __forceinline__ bool RoleWait(RoleCtx& c, const RoleNeed& need, int window, const RoleNeed* also = nullptr) {
   const int slot = static_cast<int>(c.round & 1u);
   ++c.round;
-  bool mine = true;
-  if (c.tid < c.w.world_size) mine = WaitGE(words + c.tid, value, c.w, kind, c.tid, window);
-  if (!mine) *c.stop = 1;
-  if (!mine || (c.tid == 0 && *c.stop != 0)) c.role_stop[c.slot][slot] = 1;
+  const RoleNeed* mine = c.tid < c.w.world_size ? &need : (also != nullptr && c.tid >= 32 && c.tid - 32 < c.w.world_size ? also : nullptr);
+  bool ok = true;
+  if (mine != nullptr) {
+    const int q = c.tid & 31;
+    const uint64_t* words = FlagRow(Ctl(*c.w.peers, c.w.rank), mine->row, c.cta, c.ncta, mine->flag_window, mine->groups);
+    ok = WaitGE(words + q, mine->value, c.w, mine->kind, q, window);
+  }
+  if (!ok) *c.stop = 1;
+  if (!ok || (c.tid == 0 && *c.stop != 0)) c.role_stop[c.slot][slot] = 1;
   GroupSync(c.bar_id, c.nthr);
   return c.role_stop[c.slot][slot] == 0;
 }
@@ -143,7 +161,7 @@ __device__ __forceinline__ void RolePost(RoleCtx& c, int row, uint64_t flag_wind
 // ---- copies in registers (with the conversion between buffer and wire type) ----
 // Wire vectors [b, e) of a window; `user` and `wire` point at the window's first element.
 template <typename T, typename W>
-__device__ __forceinline__ void CastIn(uint4* wire, const uint4* user, uint64_t b, uint64_t e, int tid, int nthr) {
+__device__ __forceinline__ void CastIn(uint4* wire, const uint4* user, uint64_t b, uint64_t e, uint64_t policy, int tid, int nthr) {
   using A = typename Acc<T>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
@@ -155,7 +173,7 @@ __device__ __forceinline__ void CastIn(uint4* wire, const uint4* user, uint64_t 
       const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
       if (idx < e) {
 #pragma unroll
-        for (int v = 0; v < VT; ++v) q[u][v] = Ld16(user + idx * VT + v);
+        for (int v = 0; v < VT; ++v) q[u][v] = Ld16Hint(user + idx * VT + v, policy);
       }
     }
 #pragma unroll
@@ -176,7 +194,7 @@ __device__ __forceinline__ void CastIn(uint4* wire, const uint4* user, uint64_t 
 }
 
 template <typename T, typename W>
-__device__ __forceinline__ void CastOut(uint4* user, const uint4* wire, uint64_t b, uint64_t e, int tid, int nthr) {
+__device__ __forceinline__ void CastOut(uint4* user, const uint4* wire, uint64_t b, uint64_t e, uint64_t policy, int tid, int nthr) {
   using A = typename Acc<T>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
@@ -193,12 +211,12 @@ __device__ __forceinline__ void CastOut(uint4* user, const uint4* wire, uint64_t
       const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
       if (idx < e) {
         if constexpr (sizeof(T) == sizeof(W)) {
-          St16(user + idx, q[u]);
+          St16Hint(user + idx, q[u], policy);
         } else {
           A acc[P];
           VecIO<W>::Load(q[u], acc);
 #pragma unroll
-          for (int v = 0; v < VT; ++v) St16(user + idx * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN));
+          for (int v = 0; v < VT; ++v) St16Hint(user + idx * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), policy);
         }
       }
     }
@@ -221,7 +239,7 @@ struct BulkRing {
 // two B200 under the reducers' traffic: half the stages for loads and half for
 // stores in flight, and a lane per stage, each with its own load-store chain.)
 __device__ inline bool BulkCopyPieces(BulkRing& ring, unsigned char* const* dst, const unsigned char* const* src,
-                                      const uint64_t* bytes, int npieces) {
+                                      const uint64_t* bytes, int npieces, uint64_t load_policy, uint64_t store_policy) {
   const uint32_t chunk = ring.chunk, depth = ring.depth;
   uint32_t total = 0;
   for (int s = 0; s < npieces; ++s) total += static_cast<uint32_t>((bytes[s] + chunk - 1) / chunk);
@@ -237,7 +255,7 @@ __device__ inline bool BulkCopyPieces(BulkRing& ring, unsigned char* const* dst,
     const uint32_t n = left < chunk ? static_cast<uint32_t>(left) : chunk;
     const uint32_t stage = (ring.count + ld) % depth;
     MbarExpectTx(&ring.full[stage], n);
-    BulkLoad(ring.smem + static_cast<size_t>(stage) * chunk, src[ls] + loff, n, &ring.full[stage]);
+    BulkLoadHint(ring.smem + static_cast<size_t>(stage) * chunk, src[ls] + loff, n, &ring.full[stage], load_policy);
     loff += n;
     ++ld;
   };
@@ -256,7 +274,7 @@ __device__ inline bool BulkCopyPieces(BulkRing& ring, unsigned char* const* dst,
     }
     const uint64_t left = bytes[ss] - soff;
     const uint32_t n = left < chunk ? static_cast<uint32_t>(left) : chunk;
-    BulkStore(dst[ss] + soff, ring.smem + static_cast<size_t>(stage) * chunk, n);
+    BulkStoreHint(dst[ss] + soff, ring.smem + static_cast<size_t>(stage) * chunk, n, store_policy);
     BulkCommit();
     soff += n;
     // All stores but this one have read their stage: the previous chunk's
@@ -282,6 +300,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   __shared__ int s_stop;
   __shared__ int s_role_stop[3 * kStagedMaxGroups][2];
   __shared__ uint64_t s_full[kBulkMaxRings][kBulkMaxDepth];
+  __shared__ uint64_t s_part[kMaxRanks][2];  // this block's part of every shard of a full window, in vectors
   __shared__ RoleSync s_sync;  // reducing blocks in split mode: done[g] = windows whose stores group g has issued
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
@@ -289,9 +308,10 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
     if (threadIdx.x == 0) {
       s_stop = 0;
       RoleSyncInit(&s_sync);
-      for (int r = 0; r < 3 * kStagedMaxGroups; ++r) s_role_stop[r][0] = s_role_stop[r][1] = 0;
-      for (int r = 0; r < kBulkMaxRings; ++r)
-        for (int s = 0; s < kBulkMaxDepth; ++s) MbarInit(&s_full[r][s], 1);
+    }
+    if (threadIdx.x < 3 * kStagedMaxGroups) s_role_stop[threadIdx.x][0] = s_role_stop[threadIdx.x][1] = 0;
+    if (threadIdx.x < kBulkMaxRings * kBulkMaxDepth) {
+      MbarInit(&s_full[threadIdx.x / kBulkMaxDepth][threadIdx.x % kBulkMaxDepth], 1);
       MbarInitFence();
     }
   }
@@ -328,6 +348,17 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   const int LG = split ? clamp_groups(p.load_groups) : 1;
   const int SG = split ? clamp_groups(p.store_groups) : 1;
   const int RG = split ? clamp_groups(p.reduce_groups) : 2;
+
+  if (static_cast<int>(threadIdx.x) < ws) WindowPart(full_nv, full_nv, static_cast<int>(threadIdx.x), ws, cta, ncta, &s_part[threadIdx.x][0], &s_part[threadIdx.x][1]);
+  __syncthreads();
+  // Shard s of a window of `nv` vectors (the last one is short).
+  auto part = [&](int shard, uint64_t nv, uint64_t* b, uint64_t* e) {
+    *b = s_part[shard][0] < nv ? s_part[shard][0] : nv;
+    *e = s_part[shard][1] < nv ? s_part[shard][1] : nv;
+  };
+  // Peer loads and stores of the buffers' own type: this rank's shard need not
+  // pass through its pool, its reducers read sendbuf and write recvbuf.
+  constexpr bool kOwnInPlace = !kMultimem && sizeof(T) == sizeof(W);
 
   constexpr int kWarps = kStagedThreads / 32;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -393,6 +424,8 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   const int ring_index = role == 0 ? group : LG + group;
   BulkRing ring{smem + static_cast<size_t>(ring_index) * ring_bytes, s_full[ring_index % kBulkMaxRings], ring_chunk, ring_depth, 0};
   const bool mover = !tma || gtid == 0;
+  // The user's buffers are touched once and should leave L2 before the windows do.
+  const uint64_t once = PolicyEvictFirst(), keep = PolicyNormal();
   if (role == 0) {
     // ------------------------------------------------------------ loader
     for (uint64_t k = static_cast<uint64_t>(group); k < windows; k += static_cast<uint64_t>(LG)) {
@@ -400,8 +433,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       const uint64_t v0 = k * full_nv;
       const uint64_t nv = total_nv - v0 < full_nv ? total_nv - v0 : full_nv;
       // The input buffer is free once every rank has reduced the window that used it before.
-      if (k >= kStagedBuffers &&
-          !RoleWait(c, kRowReduced, k - kStagedBuffers, RG, base | (k - kStagedBuffers + 1), kWaitBarrier, static_cast<int>(k)))
+      if (k >= kStagedBuffers && !RoleWait(c, {kRowReduced, k - kStagedBuffers, RG, base | (k - kStagedBuffers + 1), kWaitBarrier}, static_cast<int>(k)))
         break;
       if (role_w != 0 && gtid == 0) trace[role_w + k].t_wait_done = GlobalTimerNs();
       unsigned char* win = p.stage[me] + p.in_off[j];
@@ -412,13 +444,13 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         uint64_t bytes[kMaxRanks];
         for (int s = 0; s < ws; ++s) {
           uint64_t b, e;
-          WindowPart(full_nv, nv, s, ws, cta, ncta, &b, &e);
+          part(s, nv, &b, &e);
           dst[s] = win + b * 16;
           src[s] = user + b * 16;
-          bytes[s] = (e - b) * 16;
+          bytes[s] = kOwnInPlace && s == me ? 0 : (e - b) * 16;
         }
         FenceProxyAsyncAll();
-        if (!BulkCopyPieces(ring, dst, src, bytes, ws)) {
+        if (!BulkCopyPieces(ring, dst, src, bytes, ws, once, keep)) {
           // Reported here; the group leaves together at its next wait.
           ReportFailure(c.w, kStatusWaitTimeout, kWaitData, me, static_cast<int>(k), 0, 0);
           BroadcastAbort(c.w);
@@ -428,8 +460,9 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       } else if (!tma) {
         for (int s = 0; s < ws; ++s) {
           uint64_t b, e;
-          WindowPart(full_nv, nv, s, ws, cta, ncta, &b, &e);
-          CastIn<T, W>(reinterpret_cast<uint4*>(win), reinterpret_cast<const uint4*>(user), b, e, c.tid, c.nthr);
+          part(s, nv, &b, &e);
+          if (kOwnInPlace && s == me) continue;
+          CastIn<T, W>(reinterpret_cast<uint4*>(win), reinterpret_cast<const uint4*>(user), b, e, once, c.tid, c.nthr);
         }
       }
       RolePost(c, kRowInReady, k, LG, base | (k + 1));
@@ -441,7 +474,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       const int j = static_cast<int>(k % kStagedBuffers);
       const uint64_t v0 = k * full_nv;
       const uint64_t nv = total_nv - v0 < full_nv ? total_nv - v0 : full_nv;
-      if (!RoleWait(c, kRowReduced, k, RG, base | (k + 1), kWaitBarrier, static_cast<int>(k))) break;
+      if (!RoleWait(c, {kRowReduced, k, RG, base | (k + 1), kWaitBarrier}, static_cast<int>(k))) break;
       if (role_w != 0 && gtid == 0) trace[2 * role_w + k].t_wait_done = GlobalTimerNs();
       const unsigned char* win = p.stage[me] + p.out_off[j];
       unsigned char* user = static_cast<unsigned char*>(p.recvbuf) + v0 * 16 * VT;
@@ -451,15 +484,15 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         uint64_t bytes[kMaxRanks];
         for (int s = 0; s < ws; ++s) {
           uint64_t b, e;
-          WindowPart(full_nv, nv, s, ws, cta, ncta, &b, &e);
+          part(s, nv, &b, &e);
           dst[s] = user + b * 16;
           src[s] = win + b * 16;
-          bytes[s] = (e - b) * 16;
+          bytes[s] = kOwnInPlace && s == me ? 0 : (e - b) * 16;
         }
         // The window was written by ordinary stores of the peers (made
         // visible by the flags just acquired); the copy engine reads it.
         FenceProxyAsyncAll();
-        if (!BulkCopyPieces(ring, dst, src, bytes, ws)) {
+        if (!BulkCopyPieces(ring, dst, src, bytes, ws, keep, once)) {
           // Reported here; the group leaves together at its next wait.
           ReportFailure(c.w, kStatusWaitTimeout, kWaitData, me, static_cast<int>(k), 0, 0);
           BroadcastAbort(c.w);
@@ -469,8 +502,9 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       } else if (!tma) {
         for (int s = 0; s < ws; ++s) {
           uint64_t b, e;
-          WindowPart(full_nv, nv, s, ws, cta, ncta, &b, &e);
-          CastOut<T, W>(reinterpret_cast<uint4*>(user), reinterpret_cast<const uint4*>(win), b, e, c.tid, c.nthr);
+          part(s, nv, &b, &e);
+          if (kOwnInPlace && s == me) continue;
+          CastOut<T, W>(reinterpret_cast<uint4*>(user), reinterpret_cast<const uint4*>(win), b, e, once, c.tid, c.nthr);
         }
       }
       RolePost(c, kRowOutFree, k, SG, base | (k + 1));
@@ -487,14 +521,13 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       const uint64_t nv = total_nv - v0 < full_nv ? total_nv - v0 : full_nv;
       // Every rank's input window k is filled (which also says that every rank
       // runs this call, hence is done with whatever used the pool before) ...
-      if (!RoleWait(c, kRowInReady, k, LG, base | (k + 1), kWaitData, static_cast<int>(k))) break;
       // ... and every rank has emptied the output buffer this window reuses.
-      if (k >= kStagedBuffers &&
-          !RoleWait(c, kRowOutFree, k - kStagedBuffers, SG, base | (k - kStagedBuffers + 1), kWaitCredit, static_cast<int>(k)))
-        break;
+      const RoleNeed filled = {kRowInReady, k, LG, base | (k + 1), kWaitData};
+      const RoleNeed emptied = {kRowOutFree, k - kStagedBuffers, SG, base | (k - kStagedBuffers + 1), kWaitCredit};
+      if (!RoleWait(c, filled, static_cast<int>(k), k >= kStagedBuffers ? &emptied : nullptr)) break;
       if (trace != nullptr && c.tid == 0 && k < static_cast<uint64_t>(p.trace_capacity)) trace[k].t_wait_done = GlobalTimerNs();
       uint64_t b, e;
-      WindowPart(full_nv, nv, me, ws, cta, ncta, &b, &e);
+      part(me, nv, &b, &e);
       if constexpr (kMultimem) {
         constexpr int kU = 4;
         const unsigned char* mi = p.mc_stage + p.in_off[j];
@@ -522,13 +555,26 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
           }
         }
       } else {
-        unsigned char* const* arenas = p.stage;
-        const uint64_t out_off = p.out_off[j];
-        PeerReduceGroup<W, kR>(arenas, ws, p.in_off[j], b, e, do_scale, p.scale,
+        // Where rank q's vectors come from and where they go to, this rank's own in place.
+        unsigned char* from[kR];
+        unsigned char* to[kR];
+#pragma unroll
+        for (int q = 0; q < kR; ++q) {
+          from[q] = to[q] = nullptr;
+          if (q < ws) {
+            from[q] = p.stage[q] + p.in_off[j];
+            to[q] = p.stage[q] + p.out_off[j];
+            if (kOwnInPlace && q == me) {
+              from[q] = static_cast<unsigned char*>(const_cast<void*>(p.sendbuf)) + v0 * 16;
+              to[q] = static_cast<unsigned char*>(p.recvbuf) + v0 * 16;
+            }
+          }
+        }
+        PeerReduceGroup<W, kR>(from, ws, 0, b, e, do_scale, p.scale,
                                [&](uint64_t idx, uint4 r) {
 #pragma unroll
-                                 for (int q = 0; q < kMaxRanks; ++q)
-                                   if (q < ws) St16(arenas[q] + out_off + idx * 16, r);
+                                 for (int q = 0; q < kR; ++q)
+                                   if (q < ws) St16(to[q] + idx * 16, r);
                                },
                                static_cast<unsigned>(c.tid), static_cast<unsigned>(reduce_threads));
       }

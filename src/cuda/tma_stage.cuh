@@ -62,6 +62,11 @@ __device__ __forceinline__ void BulkStore(void* gmem_dst, const void* smem_src, 
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(SmemAddr(smem_src)), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void BulkStoreHint(void* gmem_dst, const void* smem_src, uint32_t bytes, uint64_t policy) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(gmem_dst), "r"(SmemAddr(smem_src)), "r"(bytes),
+               "l"(policy)
+               : "memory");
+}
 __device__ __forceinline__ void BulkCommit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Waits until at most N of the thread's bulk groups still READ shared memory.
 template <int N>
