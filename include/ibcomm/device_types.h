@@ -168,10 +168,15 @@ IBCOMM_HD inline void ChannelSlice(uint64_t first, uint64_t count, uint64_t slot
 }
 
 // ---- how the two-shot kernels split a staging window among ranks and CTAs ----
-// [*b, *e) = part `part` of `parts` of the range [lo, hi).
+// [*b, *e) = part `part` of `parts` of the range [lo, hi).  Parts of 16 or more
+// times kPartAlign start on multiples of it from `lo` (512 bytes when the unit
+// is a 16-byte vector), so that a warp's accesses cover whole cache lines; the
+// last part is up to a sixteenth shorter than the others for it.
+constexpr uint64_t kPartAlign = 32;
 IBCOMM_HD inline void SubRange(uint64_t lo, uint64_t hi, int part, int parts, uint64_t* b, uint64_t* e) {
   const uint64_t len = hi - lo;
-  const uint64_t per = (len + static_cast<uint64_t>(parts) - 1) / static_cast<uint64_t>(parts);
+  uint64_t per = (len + static_cast<uint64_t>(parts) - 1) / static_cast<uint64_t>(parts);
+  if (per >= 16 * kPartAlign) per = (per + kPartAlign - 1) / kPartAlign * kPartAlign;
   uint64_t x = lo + per * static_cast<uint64_t>(part);
   if (x > hi) x = hi;
   uint64_t y = x + per;

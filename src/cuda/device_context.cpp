@@ -1202,7 +1202,7 @@ void DeviceContext::ReduceScatterOrAllGather(int mode, DType dtype, const void* 
   const size_t remote_bytes = block_bytes * static_cast<size_t>(ws_);
   const bool vec = block_bytes % 16 == 0;
   unsigned char* mapped[kMaxRanks];
-  bool zero_copy = vec && FindPeerMapped(remote, remote_bytes, mapped);
+  bool zero_copy = FindPeerMapped(remote, remote_bytes, mapped);
   for (int q = 0; q < ws_ && zero_copy; ++q)
     if ((reinterpret_cast<uintptr_t>(mapped[q]) & 15u) != 0) zero_copy = false;  // the same decision on every rank
   const SymmetricAlloc* sym = FindSymmetric(remote, remote_bytes);
@@ -1240,7 +1240,6 @@ void DeviceContext::ReduceScatterOrAllGather(int mode, DType dtype, const void* 
     // Equal windows, each a whole number of units per channel.
     const uint64_t cap = p.sub_stride_bytes / esize;
     p.window_elems = TwoShotWindowElems(block_elems, cap, esize, 1, channels);
-    if (!vec) p.window_elems = std::min<uint64_t>(std::max<uint64_t>(p.window_elems, 1), cap);
   }
   OrderAfterPrevious(stream);
   IBCOMM_TRACE(*tracer_, kTraceIssueReduKernel);

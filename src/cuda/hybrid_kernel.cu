@@ -95,11 +95,11 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) HybridKernel(const __grid_con
     } else {
       const int ws = p.world_size;
       unsigned char* const* outs = p.peer_out;
-      PeerReduce<T, kR>(p.peer_in, ws, 0, b, e, do_scale, p.scale, [&](uint64_t idx, uint4 r) {
+      PeerReduceGroup<T, kR>(p.peer_in, ws, 0, b, e, do_scale, p.scale, [&](uint64_t idx, uint4 r) {
 #pragma unroll
         for (int q = 0; q < kMaxRanks; ++q)
           if (q < ws) St16(outs[q] + idx * 16, r);
-      });
+      }, threadIdx.x, blockDim.x);
     }
     // The ragged end (< 16 bytes): summed by every rank itself, written after
     // the barrier (in place, the peers are still reading this rank's input).

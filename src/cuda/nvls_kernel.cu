@@ -35,7 +35,7 @@ namespace dev {
 
 // Body of the two-shot kernel for one CTA; returns early when a barrier gave up.
 template <typename T, int U, bool kMultimem, int kR>
-__device__ void TwoShotBody(const NvlsParams& p, uint64_t seq, int& s_stop) {
+__device__ void TwoShotBody(const NvlsParams& p, uint64_t seq, int& s_stop, unsigned char* smem) {
   using A = typename Acc<T>::type;
   constexpr int kVecElems = 16 / static_cast<int>(sizeof(T));
   const int cta = blockIdx.x, ncta = gridDim.x;
@@ -120,9 +120,9 @@ __device__ void TwoShotBody(const NvlsParams& p, uint64_t seq, int& s_stop) {
         // bits are the same.  The result goes to every rank's output window.
         const int ws = p.world_size;
         unsigned char* const* outs = p.peer_out;
-        PeerReduce<T, kR>(p.peer_in, ws, win_bytes_off, b, e, do_scale, p.scale, [&](uint64_t idx, uint4 r) {
+        PeerReduce<T, kR>(smem, p.peer_in, ws, win_bytes_off, b, e, do_scale, p.scale, [&](uint64_t idx, uint4 r) {
 #pragma unroll
-          for (int q = 0; q < kMaxRanks; ++q)
+          for (int q = 0; q < kR; ++q)
             if (q < ws) St16(outs[q] + wout_bytes_off + idx * 16, r);
         });
       }
@@ -169,6 +169,7 @@ __device__ void TwoShotBody(const NvlsParams& p, uint64_t seq, int& s_stop) {
 
 template <typename T, int U, bool kMultimem, int kR>
 __global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_constant__ RankBlocks<NvlsParams> all) {
+  extern __shared__ __align__(128) unsigned char smem[];
   __shared__ NvlsParams p;
   __shared__ int s_stop;
   __shared__ uint64_t s_seq;
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_const
   }
   __syncthreads();
   const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
-  TwoShotBody<T, U, kMultimem, kR>(p, seq, s_stop);
+  TwoShotBody<T, U, kMultimem, kR>(p, seq, s_stop, smem);
   EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
@@ -187,7 +188,12 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_const
 
 template <typename T, int U, bool kMultimem, int kR>
 static cudaError_t LaunchNvlsU(const NvlsParams* ranks, int n, int blocks, int threads, cudaStream_t stream) {
-  return LaunchRanks(dev::NvlsKernel<T, U, kMultimem, kR>, ranks, n, blocks, threads, 0, stream);
+  const size_t smem = kMultimem ? 0 : dev::kReduceSmemPerThread * static_cast<size_t>(threads);
+  if (smem != 0) {
+    const cudaError_t e = AllowSharedMemory(dev::NvlsKernel<T, U, kMultimem, kR>, smem);
+    if (e != cudaSuccess) return e;
+  }
+  return LaunchRanks(dev::NvlsKernel<T, U, kMultimem, kR>, ranks, n, blocks, threads, smem, stream);
 }
 
 template <typename T>
@@ -215,7 +221,10 @@ static cudaError_t LaunchNvlsTyped(const NvlsParams* ranks, int n, int blocks, c
 
 int TwoShotKernelMaxCoResidentBlocks(int device) {
   int per_sm = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::NvlsKernel<float, 4, false, kMaxRanks>, dev::kNvlsThreads, 0) != cudaSuccess) return 0;
+  const auto kernel = dev::NvlsKernel<float, 4, false, kMaxRanks>;
+  const size_t smem = dev::kReduceSmemPerThread * dev::kNvlsThreads;
+  if (AllowSharedMemory(kernel, smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, dev::kNvlsThreads, smem) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
   return per_sm * sms;
 }

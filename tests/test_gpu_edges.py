@@ -33,3 +33,32 @@ def test_copy_scale_quanta_heads_and_tails(types, offsets):
         ar.ops.copy_scale(x, y, scale=scale)
         assert torch.equal(y, (x.double() * scale).to(types[1])), n
         assert torch.all(guard[:offsets[1]] == 7) and torch.all(guard[offsets[1] + n:] == 7), n
+
+
+@pytest.mark.parametrize("staged", [0, 1])
+@pytest.mark.parametrize("offset", [0, 1, 3])
+@pytest.mark.parametrize("ws", [2, 3, 8])
+def test_reduce_scatter_and_all_gather_ragged_blocks(ws, offset, staged):
+    # Blocks that start off the 16-byte boundary of the remote side (every rank's head differs), shorter than a unit,
+    # a unit and a bit, and long enough for parts on cache lines; buffers that miss the boundary alike.
+    world = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+    world.set_direct_staging(staged)
+    for dtype in (torch.float32, torch.bfloat16, torch.float64):
+        for m in (1, 2, 5, 9, 1023, 70001):
+            full = [values(m * ws, dtype, 10 * m + r, offset) for r in range(ws)]
+            want = torch.stack([t.double() for t in full]).sum(0) * 0.5
+            guard = [torch.full((m + offset + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+            shards = [g[offset:offset + m] for g in guard]
+            world.reduce_scatter(full, shards, scale=0.5)
+            tol = 1e-5 if dtype == torch.float32 else (2e-2 if dtype == torch.bfloat16 else 1e-12)
+            for r in range(ws):
+                torch.testing.assert_close(shards[r].double(), want[r * m:(r + 1) * m], rtol=tol, atol=tol)
+                assert torch.all(guard[r][:offset] == 7) and torch.all(guard[r][offset + m:] == 7)
+            guard = [torch.full((m * ws + offset + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+            gathered = [g[offset:offset + m * ws] for g in guard]
+            world.all_gather(shards, gathered)
+            whole = torch.cat(shards)
+            for r in range(ws):
+                assert torch.equal(gathered[r], whole)
+                assert torch.all(guard[r][:offset] == 7) and torch.all(guard[r][offset + m * ws:] == 7)
+    world.close()
