@@ -54,17 +54,14 @@ struct ControlPage {
   uint64_t bcast_credit[kP2pCtas][kMaxRanks];
   // Set (to the call sequence) by any rank that gave up; polled by waiters.
   uint64_t abort_seq;
-  // Written only by this rank's own kernels: the number of collectives it has
-  // completed, and how many CTAs of the running one have finished.  Every
-  // collective kernel takes its sequence number from here (call_seq + 1) and
-  // the last CTA to finish publishes it, so a kernel's parameters carry
-  // nothing that changes from call to call and a captured CUDA graph of
-  // collectives can be replayed.  All ranks issue the same collectives in the
-  // same order, so their counters agree.
-  uint64_t call_seq;
-  uint32_t done_ctas;
-  uint32_t pad32_;
-  uint64_t pad_[5];
+  // Written only by this rank's own kernels: (collectives it has begun << 16) |
+  // CTAs of the running one that have taken their sequence number.  Every
+  // collective kernel takes its number from here (BeginCollective, flags.cuh),
+  // so a kernel's parameters carry nothing that changes from call to call and a
+  // captured CUDA graph of collectives can be replayed.  All ranks issue the
+  // same collectives in the same order, so their counters agree.
+  uint64_t call_word;
+  uint64_t pad_[6];
   // One-shot allreduce flags: [parity][cta][source].
   uint64_t oneshot_flag[2][kMaxChannels][kMaxRanks];
 };

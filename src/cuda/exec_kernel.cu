@@ -623,13 +623,11 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
 template <typename T, typename W>
 __global__ void __launch_bounds__(kExecThreads, 1)
 ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all, int stages) {
-  __shared__ ExecParams p;
+  const ExecParams& p = all.rank[blockIdx.y];
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ ExecShared s_exec;
   __shared__ uint64_t s_seq;
   {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
-    for (unsigned i = threadIdx.x; i < sizeof(ExecParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
     if (threadIdx.x == 0) {
       RoleSyncInit(&s_exec.role);
       for (int i = 0; i < kExecMaxStages; ++i) {
@@ -639,12 +637,10 @@ ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all, int stages) {
       MbarInitFence();
     }
   }
-  __syncthreads();
   if (p.world_size <= 1) return;
-  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
+  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq, gridDim.x);
   // num_ops <= 0: this rank sits the call out (test hook), but still counts it.
   if (p.num_ops > 0) ExecBody<T, W>(p, seq, &s_exec, smem, stages);
-  EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
 }  // namespace dev

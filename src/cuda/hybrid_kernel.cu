@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) HybridKernel(const __grid_con
   if (threadIdx.x == 0) s_stop = 0;
   __syncthreads();
   const NvlsParams& p = h.base;
-  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
+  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq, gridDim.x);
 
   const int bar_index = blockIdx.x;  // one barrier slot per CTA of the grid, whatever its role
   const bool switch_role = static_cast<int>(blockIdx.x) < h.nvls_ctas;
@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) HybridKernel(const __grid_con
     alive = CrossRankBarrier(p.peers, w, bar_index, 2, &s_stop);
     if (alive && has_tail) reinterpret_cast<T*>(p.local_out)[tail0 + threadIdx.x] = FromAcc<T, A>(tail_acc);
   }
-  EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
 }  // namespace dev

@@ -170,18 +170,12 @@ __device__ void TwoShotBody(const NvlsParams& p, uint64_t seq, int& s_stop, unsi
 template <typename T, int U, bool kMultimem, int kR>
 __global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_constant__ RankBlocks<NvlsParams> all) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ NvlsParams p;
+  const NvlsParams& p = all.rank[blockIdx.y];
   __shared__ int s_stop;
   __shared__ uint64_t s_seq;
-  {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
-    for (unsigned i = threadIdx.x; i < sizeof(NvlsParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
-    if (threadIdx.x == 0) s_stop = 0;
-  }
-  __syncthreads();
-  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
+  if (threadIdx.x == 0) s_stop = 0;
+  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq, gridDim.x);
   TwoShotBody<T, U, kMultimem, kR>(p, seq, s_stop, smem);
-  EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
 }  // namespace dev

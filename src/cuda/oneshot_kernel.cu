@@ -59,29 +59,37 @@ __device__ void OneShotBody(const OneShotParams& p, uint64_t seq, int& s_stop) {
     return reinterpret_cast<T*>(p.peers.arena[owner_rank] + p.slot_offset +
                                 (static_cast<uint64_t>(parity) * static_cast<uint64_t>(ws) + static_cast<uint64_t>(src_rank)) * p.slot_bytes);
   };
-  const bool aligned = ((reinterpret_cast<uintptr_t>(sendbuf) | reinterpret_cast<uintptr_t>(recvbuf)) & 15u) == 0;
-  const uint64_t nfull = aligned ? (hi - lo) / kVecElems : 0;  // whole vectors handled by the vector path
+  // Slots are 16-byte aligned and so is `lo`; a user buffer may be only
+  // element-aligned, then its side of a vector goes element by element.
+  const unsigned char* const mine = reinterpret_cast<const unsigned char*>(sendbuf + lo);
+  unsigned char* const out = reinterpret_cast<unsigned char*>(recvbuf + lo);
+  const bool send_aligned = (reinterpret_cast<uintptr_t>(mine) & 15u) == 0, recv_aligned = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  const uint64_t nfull = (hi - lo) / kVecElems;
+  const uint64_t ragged = lo + nfull * kVecElems;
 
-  // (1) push my slice to every peer.
-  for (int k = 1; k < ws; ++k) {
-    const int q = (me + k) % ws;  // start with a different peer on every rank
-    T* dst = slot(q, me);
-    constexpr int kU = 4;  // vectors in flight per thread
-    for (uint64_t i = threadIdx.x; i < nfull; i += static_cast<uint64_t>(blockDim.x) * kU) {
-      uint4 v[kU];
+  // (1) push my slice to every peer: read once, stored ws - 1 times, starting
+  // with a different peer on every rank.
+  constexpr int kU = 4;  // vectors in flight per thread
+  for (uint64_t i = threadIdx.x; i < nfull; i += static_cast<uint64_t>(blockDim.x) * kU) {
+    uint4 v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t idx = i + static_cast<uint64_t>(u) * blockDim.x;
+      if (idx < nfull) v[u] = LdUser16<T>(mine + idx * 16, send_aligned);
+    }
+    for (int k = 1; k < ws; ++k) {
+      const int q = me + k < ws ? me + k : me + k - ws;
+      uint4* const dst = reinterpret_cast<uint4*>(slot(q, me) + lo);
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
         const uint64_t idx = i + static_cast<uint64_t>(u) * blockDim.x;
-        if (idx < nfull) v[u] = Ld16(reinterpret_cast<const uint4*>(sendbuf + lo) + idx);
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const uint64_t idx = i + static_cast<uint64_t>(u) * blockDim.x;
-        if (idx < nfull) St16(reinterpret_cast<uint4*>(dst + lo) + idx, v[u]);
+        if (idx < nfull) St16(dst + idx, v[u]);
       }
     }
-    for (uint64_t i = lo + nfull * kVecElems + threadIdx.x; i < hi; i += blockDim.x) dst[i] = sendbuf[i];
   }
+  for (uint64_t i = ragged + threadIdx.x; i < hi; i += blockDim.x)
+    for (int q = 0; q < ws; ++q)
+      if (q != me) slot(q, me)[i] = sendbuf[i];
   __syncthreads();
   // (2) tell them, (3) wait for theirs.
   if (threadIdx.x < ws && static_cast<int>(threadIdx.x) != me) {
@@ -91,24 +99,25 @@ __device__ void OneShotBody(const OneShotParams& p, uint64_t seq, int& s_stop) {
   }
   __syncthreads();
   if (s_stop) return;
-  // (4) sum in rank order.
+  // (4) sum in rank order, every rank's vector in flight.
   const bool do_scale = p.scale != 1.0;
   for (uint64_t i = threadIdx.x; i < nfull; i += blockDim.x) {
-    A acc[kVecElems];
+    uint4 v[kMaxRanks];
 #pragma unroll
-    for (int e = 0; e < kVecElems; ++e) acc[e] = A(0);
-    for (int q = 0; q < ws; ++q) {
-      const uint4 v = (q == me) ? Ld16(reinterpret_cast<const uint4*>(sendbuf + lo) + i)
-                                : Ld16Strong(reinterpret_cast<const uint4*>(slot(me, q) + lo) + i);
-      VecIO<T>::Add(v, acc);
-    }
+    for (int q = 0; q < kMaxRanks; ++q)
+      if (q < ws) v[q] = (q == me) ? LdUser16<T>(mine + i * 16, send_aligned) : Ld16Strong(reinterpret_cast<const uint4*>(slot(me, q) + lo) + i);
+    A acc[kVecElems];
+    VecIO<T>::Load(v[0], acc);
+#pragma unroll
+    for (int q = 1; q < kMaxRanks; ++q)
+      if (q < ws) VecIO<T>::Add(v[q], acc);
     if (do_scale) {
 #pragma unroll
       for (int e = 0; e < kVecElems; ++e) acc[e] = ScaleAcc<A>(acc[e], p.scale);
     }
-    St16(reinterpret_cast<uint4*>(recvbuf + lo) + i, VecIO<T>::Store(acc));
+    StUser16<T>(out + i * 16, VecIO<T>::Store(acc), recv_aligned);
   }
-  for (uint64_t i = lo + nfull * kVecElems + threadIdx.x; i < hi; i += blockDim.x) {
+  for (uint64_t i = ragged + threadIdx.x; i < hi; i += blockDim.x) {
     A acc = A(0);
     for (int q = 0; q < ws; ++q) acc += (q == me) ? ToAcc<A, T>(sendbuf[i]) : ToAcc<A, T>(LdScalarStrong<T>(slot(me, q) + i));
     if (do_scale) acc = ScaleAcc<A>(acc, p.scale);
@@ -119,18 +128,12 @@ __device__ void OneShotBody(const OneShotParams& p, uint64_t seq, int& s_stop) {
 template <typename T>
 __global__ void __launch_bounds__(kOneShotThreads, 1)
 OneShotKernel(const __grid_constant__ RankBlocks<OneShotParams> all) {
-  __shared__ OneShotParams p;
+  const OneShotParams& p = all.rank[blockIdx.y];
   __shared__ int s_stop;
   __shared__ uint64_t s_seq;
-  {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
-    for (unsigned i = threadIdx.x; i < sizeof(OneShotParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
-    if (threadIdx.x == 0) s_stop = 0;
-  }
-  __syncthreads();
-  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
+  if (threadIdx.x == 0) s_stop = 0;
+  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq, gridDim.x);
   OneShotBody<T>(p, seq, s_stop);
-  EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
 }  // namespace dev

@@ -37,38 +37,6 @@
 namespace ibcomm {
 namespace dev {
 
-template <int kBytes> struct UIntOf;
-template <> struct UIntOf<2> { using type = unsigned short; };
-template <> struct UIntOf<4> { using type = unsigned int; };
-template <> struct UIntOf<8> { using type = unsigned long long; };
-
-// 16 bytes from / to a user buffer that may be only element-aligned.
-template <typename T>
-__device__ __forceinline__ uint4 LdUser16(const unsigned char* p, bool aligned) {
-  if (aligned) return Ld16(p);
-  using U = typename UIntOf<sizeof(T)>::type;
-  constexpr int kN = 16 / static_cast<int>(sizeof(T));
-  union { uint4 v; U e[kN]; } u;
-  const U* s = reinterpret_cast<const U*>(p);
-#pragma unroll
-  for (int k = 0; k < kN; ++k) u.e[k] = s[k];
-  return u.v;
-}
-template <typename T>
-__device__ __forceinline__ void StUser16(unsigned char* p, uint4 v, bool aligned) {
-  if (aligned) {
-    St16(p, v);
-    return;
-  }
-  using U = typename UIntOf<sizeof(T)>::type;
-  constexpr int kN = 16 / static_cast<int>(sizeof(T));
-  union { uint4 v; U e[kN]; } u;
-  u.v = v;
-  U* d = reinterpret_cast<U*>(p);
-#pragma unroll
-  for (int k = 0; k < kN; ++k) d[k] = u.e[k];
-}
-
 template <typename T, bool kMultimem, int kR>
 __device__ void RsAgBody(const RsAgParams& p, uint64_t seq, int& s_stop, unsigned char* smem) {
   using A = typename Acc<T>::type;
@@ -214,18 +182,12 @@ __device__ void RsAgBody(const RsAgParams& p, uint64_t seq, int& s_stop, unsigne
 template <typename T, bool kMultimem, int kR>
 __global__ void __launch_bounds__(kNvlsThreads, 1) RsAgKernel(const __grid_constant__ RankBlocks<RsAgParams> all) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ RsAgParams p;
+  const RsAgParams& p = all.rank[blockIdx.y];
   __shared__ int s_stop;
   __shared__ uint64_t s_seq;
-  {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
-    for (unsigned i = threadIdx.x; i < sizeof(RsAgParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
-    if (threadIdx.x == 0) s_stop = 0;
-  }
-  __syncthreads();
-  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
+  if (threadIdx.x == 0) s_stop = 0;
+  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq, gridDim.x);
   RsAgBody<T, kMultimem, kR>(p, seq, s_stop, smem);
-  EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
 }  // namespace dev

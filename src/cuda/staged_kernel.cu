@@ -295,7 +295,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   constexpr int P = 16 / static_cast<int>(sizeof(W));                // elements per wire vector
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;           // user vectors per wire vector
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ StagedParams p;
+  const StagedParams& p = all.rank[blockIdx.y];
   __shared__ uint64_t s_seq;
   __shared__ int s_stop;
   __shared__ int s_role_stop[3 * kStagedMaxGroups][2];
@@ -303,8 +303,6 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   __shared__ uint64_t s_part[kMaxRanks][2];  // this block's part of every shard of a full window, in vectors
   __shared__ RoleSync s_sync;  // reducing blocks in split mode: done[g] = windows whose stores group g has issued
   {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&all.rank[blockIdx.y]);
-    for (unsigned i = threadIdx.x; i < sizeof(StagedParams) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(&p)[i] = src[i];
     if (threadIdx.x == 0) {
       s_stop = 0;
       RoleSyncInit(&s_sync);
@@ -315,8 +313,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       MbarInitFence();
     }
   }
-  __syncthreads();
-  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq);
+  const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq, gridDim.x);
 
   // Roles share a block, or - `split_ctas` - live in blocks of their own:
   // blocks [0, n) reduce with all 16 warps, blocks [n, 2n) copy (block n + b
@@ -604,7 +601,6 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       if (trace != nullptr && lane == 0 && k < static_cast<uint64_t>(p.trace_capacity)) trace[k].t_done = GlobalTimerNs();
     }
   }
-  EndCollective(p.peers, p.rank, seq, gridDim.x);
 }
 
 }  // namespace dev

@@ -79,6 +79,38 @@ __device__ __forceinline__ void St32(void* p, uint4 lo, uint4 hi) {
                : "memory");
 }
 
+template <int kBytes> struct UIntOf;
+template <> struct UIntOf<2> { using type = unsigned short; };
+template <> struct UIntOf<4> { using type = unsigned int; };
+template <> struct UIntOf<8> { using type = unsigned long long; };
+
+// 16 bytes from / to a user buffer that may be only element-aligned.
+template <typename T>
+__device__ __forceinline__ uint4 LdUser16(const unsigned char* p, bool aligned) {
+  if (aligned) return Ld16(p);
+  using U = typename UIntOf<sizeof(T)>::type;
+  constexpr int kN = 16 / static_cast<int>(sizeof(T));
+  union { uint4 v; U e[kN]; } u;
+  const U* s = reinterpret_cast<const U*>(p);
+#pragma unroll
+  for (int k = 0; k < kN; ++k) u.e[k] = s[k];
+  return u.v;
+}
+template <typename T>
+__device__ __forceinline__ void StUser16(unsigned char* p, uint4 v, bool aligned) {
+  if (aligned) {
+    St16(p, v);
+    return;
+  }
+  using U = typename UIntOf<sizeof(T)>::type;
+  constexpr int kN = 16 / static_cast<int>(sizeof(T));
+  union { uint4 v; U e[kN]; } u;
+  u.v = v;
+  U* d = reinterpret_cast<U*>(p);
+#pragma unroll
+  for (int k = 0; k < kN; ++k) d[k] = u.e[k];
+}
+
 template <typename X> struct VecIO;
 
 template <> struct VecIO<float> {
