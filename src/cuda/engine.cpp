@@ -160,7 +160,7 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
                                     : layout.pool_bytes + layout.work_bytes;
   // Knobs that shape the program are part of the key: the ring's chunks per
   // rank and the number of pieces Rabenseifner cuts the message into.
-  const size_t ring_cpr = ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size)) : 0;
+  const size_t ring_cpr = ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size), ranks_on_gpu > 1) : 0;
   // Ranks on one GPU: four pieces of up to 8 MiB (a hand-over costs what 100 KiB
   // per channel cost; 5 ranks, 4 / 16 MiB: 75 / 134 us with eight, 64 / 122 with four).
   int raben_div = Tunable("IBCOMM_RABEN_PIECES", 0);

@@ -84,11 +84,13 @@ enum ExecTileFlags : uint32_t {
 struct ExecTile {
   uint4* local;   // recvbuf, or null
   uint4* remote;  // the next rank's staging slot, or null
-  uint32_t packs;
+  uint32_t packs;  // the one with only `tail` elements included
   uint32_t flags;
   uint32_t op;
-  uint32_t pad_;
+  uint32_t tail;  // elements of the last pack, 0 = it is whole
   uint64_t lo, hi;
+  const unsigned char* tail_a;  // where the last pack lies in the user's buffers
+  const unsigned char* tail_b;
 };
 
 // One op of this channel, worked out by a lane of the loader's warp.
@@ -97,10 +99,12 @@ struct ExecPlan {
   const unsigned char* src_b;
   unsigned char* local;
   unsigned char* remote;
-  uint64_t packs;      // whole packs
-  uint64_t rest, hi;   // elements [rest, hi) of the cell go one by one
+  uint64_t packs;      // packs, the last one with only `tail` elements unless `tail` is 0
+  uint64_t lo, hi;     // elements [lo, hi) of the cell go one by one (nothing is in packs then)
   uint32_t flags;      // ExecTileFlags of every stage of the op
   uint32_t wait_local;
+  uint32_t tail;
+  uint32_t pad_;
 };
 
 struct ExecShared {
@@ -125,19 +129,60 @@ __device__ __forceinline__ bool RingWait(uint64_t* bar, uint32_t parity, RoleSyn
   }
 }
 
-// One stage: packs of P elements, U of them per thread.
+// The last pack of a message that ends inside it: `staged` is its place in the
+// stage when source a comes from staging; the user's buffers are accessed up to
+// the message's end.  A slot's pack is written whole: it lies in this channel's
+// part of the slot, and nobody reads past the message's end either.
 template <typename T, typename W>
-__device__ __forceinline__ void RunTile(const ExecTile& t, const uint4* stage, uint32_t b_off, double scale, uint64_t* empty, uint64_t local_policy, unsigned tid,
+__device__ __noinline__ void RunTailPack(const ExecTile* t, const uint4* staged, double scale) {
+  using Tr = ExecTraits<T, W>;
+  using A = typename Tr::A;
+  constexpr int P = Tr::P;
+  const int n = static_cast<int>(t->tail);
+  A acc[P];
+#pragma unroll
+  for (int v = 0; v < Tr::VW; ++v)
+    if (t->flags & kTileFromStaging) VecIO<W>::Load(staged[v], acc + v * VecIO<W>::kN);
+#pragma unroll
+  for (int e = 0; e < P; ++e) {
+    if (!(t->flags & kTileFromStaging)) acc[e] = e < n ? ToAcc<A, T>(reinterpret_cast<const T*>(t->tail_a)[e]) : A(0);
+    if ((t->flags & kTileAdd) && e < n) acc[e] += ToAcc<A, T>(reinterpret_cast<const T*>(t->tail_b)[e]);
+    if (t->flags & kTileScale) acc[e] = ScaleAcc<A>(acc[e], scale);
+  }
+  uint4 wq[Tr::VW];
+#pragma unroll
+  for (int v = 0; v < Tr::VW; ++v) wq[v] = VecIO<W>::Store(acc + v * VecIO<W>::kN);
+  const uint32_t at = t->packs - 1;
+  if (t->remote != nullptr) {
+#pragma unroll
+    for (int v = 0; v < Tr::VW; ++v) St16(t->remote + at * Tr::VW + v, wq[v]);
+  }
+  if (t->local != nullptr) {
+    if ((t->flags & kTileRoundWire) && sizeof(W) != sizeof(T)) {
+#pragma unroll
+      for (int v = 0; v < Tr::VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
+    }
+    T* const out = reinterpret_cast<T*>(t->local + at * Tr::VT);
+#pragma unroll
+    for (int e = 0; e < P; ++e)
+      if (e < n) out[e] = FromAcc<T, A>(acc[e]);
+  }
+}
+
+// One stage: packs of P elements, U of them per thread.  `tile` is `t` in shared memory.
+template <typename T, typename W>
+__device__ __forceinline__ void RunTile(const ExecTile& t, const ExecTile* tile, const uint4* stage, uint32_t b_off, double scale, uint64_t* empty, uint64_t local_policy, unsigned tid,
                                         unsigned nthr, int lane) {
   using Tr = ExecTraits<T, W>;
   using A = typename Tr::A;
   constexpr int P = Tr::P, U = Tr::U, VT = Tr::VT, VW = Tr::VW;
   const bool from_staging = (t.flags & kTileFromStaging) != 0, add = (t.flags & kTileAdd) != 0;
+  const uint32_t whole = t.packs - (t.tail != 0 ? 1u : 0u);
   uint4 qa[U][VT], qb[U][VT];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const unsigned i = tid + static_cast<unsigned>(u) * nthr;
-    if (i < t.packs) {
+    if (i < whole) {
       if (from_staging) {
 #pragma unroll
         for (int v = 0; v < VW; ++v) qa[u][v] = stage[i * VW + v];
@@ -152,12 +197,14 @@ __device__ __forceinline__ void RunTile(const ExecTile& t, const uint4* stage, u
     }
   }
   // The stage is free for the loader once every warp has read it.
-  __syncwarp();
-  if (lane == 0) MbarArrive(empty);
+  if (t.tail == 0) {
+    __syncwarp();
+    if (lane == 0) MbarArrive(empty);
+  }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const unsigned i = tid + static_cast<unsigned>(u) * nthr;
-    if (i < t.packs) {
+    if (i < whole) {
       A acc[P];
       if (from_staging) {
 #pragma unroll
@@ -192,6 +239,11 @@ __device__ __forceinline__ void RunTile(const ExecTile& t, const uint4* stage, u
         for (int v = 0; v < VT; ++v) St16Hint(t.local + i * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), local_policy);
       }
     }
+  }
+  if (t.tail != 0) {
+    if (whole % nthr == tid) RunTailPack<T, W>(tile, stage + whole * VW, scale);
+    __syncwarp();
+    if (lane == 0) MbarArrive(empty);
   }
 }
 
@@ -344,8 +396,10 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
         pl.src_b = source(op.src_b);
         pl.local = (op.flags & kOpStoreLocal) ? reinterpret_cast<unsigned char*>(buf.recvbuf + g0) : nullptr;
         pl.remote = buf.stage_out != nullptr ? reinterpret_cast<unsigned char*>(buf.stage_out + lo) : nullptr;
-        pl.packs = lo < hi && (bits & 15u) == 0 ? (hi - lo) / Tr::P : 0;
-        pl.rest = lo + pl.packs * Tr::P;
+        const bool in_packs = lo < hi && (bits & 15u) == 0;
+        pl.packs = in_packs ? (hi - lo + Tr::P - 1) / Tr::P : 0;
+        pl.tail = in_packs ? static_cast<uint32_t>((hi - lo) % Tr::P) : 0;
+        pl.lo = in_packs ? hi : lo;
         pl.hi = hi;
         pl.flags = (op.src_a == kSrcStage ? kTileFromStaging : 0u) | (op.src_b != kSrcNone ? kTileAdd : 0u) |
                    ((op.flags & kOpScale) ? kTileScale : 0u) | ((op.flags & kOpRoundWire) ? kTileRoundWire : 0u);
@@ -399,16 +453,24 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           t.remote = pl.remote != nullptr ? reinterpret_cast<uint4*>(pl.remote + j * Tr::VW * 16u) : nullptr;
           t.packs = n;
           t.op = oi;
-          t.flags = pl.flags | (j + n >= pl.packs && pl.rest >= pl.hi ? kTileLastOfOp : 0u);
+          const bool last = j + n >= pl.packs;
+          t.flags = pl.flags | (last ? kTileLastOfOp : 0u);
+          t.tail = last ? pl.tail : 0;
+          const uint32_t whole = n - (t.tail != 0 ? 1u : 0u);
+          if (t.tail != 0) {
+            t.tail_a = pl.src_a + (j + whole) * Tr::VT * 16u;
+            t.tail_b = pl.src_b + (j + whole) * Tr::VT * 16u;
+          }
           // What does not depend on a peer first, then the op's flags, then the staging slot.
-          const uint32_t user_bytes = n * Tr::VT * 16u, a_bytes = n * static_cast<uint32_t>(a_step);
-          if (pl.src_b != nullptr) {
+          // The user's buffers end where the message ends; a slot holds whole packs.
+          const uint32_t user_bytes = whole * Tr::VT * 16u, a_bytes = n * static_cast<uint32_t>(a_step);
+          if (pl.src_b != nullptr && whole != 0) {
             MbarExpectTxOnly(&sh->full[s], user_bytes);
             BulkLoadHint(dst + half_bytes, pl.src_b + j * Tr::VT * 16u, user_bytes, &sh->full[s], user_policy);
           }
-          if (!a_staged) {
-            MbarExpectTxOnly(&sh->full[s], a_bytes);
-            BulkLoadHint(dst, pl.src_a + j * a_step, a_bytes, &sh->full[s], user_policy);
+          if (!a_staged && whole != 0) {
+            MbarExpectTxOnly(&sh->full[s], user_bytes);
+            BulkLoadHint(dst, pl.src_a + j * a_step, user_bytes, &sh->full[s], user_policy);
           }
           if (!get_ready()) {
             alive = 0;
@@ -420,8 +482,8 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           }
           MbarArrive(&sh->full[s]);
         }
-        // Elements outside whole packs, or an op without elements for this channel (which still has to be reported done).
-        if (alive > 0 && (pl.rest < pl.hi || pl.packs == 0)) {
+        // A range that is not on 16-byte boundaries, or an op without elements for this channel (which still has to be reported done).
+        if (alive > 0 && pl.packs == 0) {
           if (!next_stage()) {
             alive = -1;
           } else if (!get_ready()) {
@@ -430,7 +492,7 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
             ExecTile& t = sh->tile[s];
             t.flags = kTileElements | kTileLastOfOp;
             t.op = oi;
-            t.lo = pl.rest;
+            t.lo = pl.lo;
             t.hi = pl.hi;
             MbarArrive(&sh->full[s]);
           }
@@ -567,7 +629,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
         if (lane == 0) MbarArrive(&sh->empty[s]);
         RunElements<T, W>(p.ops[t.op], p, t.lo, t.hi, threadIdx.x, nthr);
       } else {
-        RunTile<T, W>(t, reinterpret_cast<const uint4*>(smem) + static_cast<size_t>(s) * 2 * half_vecs, half_vecs, p.scale, &sh->empty[s], local_policy,
+        RunTile<T, W>(t, &sh->tile[s], reinterpret_cast<const uint4*>(smem) + static_cast<size_t>(s) * 2 * half_vecs, half_vecs, p.scale, &sh->empty[s], local_policy,
                       threadIdx.x, nthr, lane);
       }
       if (t.flags & kTileLastOfOp) {

@@ -181,6 +181,17 @@ void BuildRing(Builder* bld) {
   }
 }
 
+// Block that rank `v` of `p` (a power of two) is left with after the halving.
+int OwnedBlock(int v, int p) {
+  int b = 0, e = p;
+  for (int s = 1; s < p; s <<= 1) {
+    const int mid = e - (e - b) / 2;
+    if (v < (v ^ s)) b = mid;
+    else e = mid;
+  }
+  return b;
+}
+
 void BuildRabenseifner(Builder* bld) {
   const ProgramRequest& q = bld->req;
   const int ws = q.world_size, r = q.rank;
@@ -189,72 +200,61 @@ void BuildRabenseifner(Builder* bld) {
   const int exp = util::GetExpOfTwo(static_cast<uint64_t>(p));
   const int C = static_cast<int>(q.ranges.size());
   auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
-  std::vector<int> all(static_cast<size_t>(C));
-  for (int i = 0; i < C; ++i) all[static_cast<size_t>(i)] = i;
   const std::vector<int> none;
+  const std::vector<std::vector<int>> blocks = GetRankToChunk(static_cast<size_t>(C), static_cast<size_t>(p));
 
-  int vrank;
-  OpSrc partial = kSrcSend;  // where my running partial sum lives
-  if (r < 2 * extra) {
-    // The even rank gives its whole message away and sits out until the end.
-    if ((r & 1) == 0) {
-      bld->Exchange(r + 1, all, kSrcSend, none, kSrcNone, false);
-      vrank = -1;
-    } else {
-      bld->Exchange(r - 1, none, kSrcNone, all, kSrcSend, false);
-      vrank = r / 2;
-      partial = kSrcRecv;
+  if (r < 2 * extra && (r & 1) == 0) {
+    // An extra rank hands every block of its message to the rank that will own
+    // it and gets the results back from there.  Piece by piece over the owners,
+    // so that all of them have something to work on.
+    std::vector<std::vector<Range>> pieces;
+    size_t most = 0;
+    for (int v = 0; v < p; ++v) {
+      pieces.push_back(bld->Pieces(blocks[static_cast<size_t>(OwnedBlock(v, p))]));
+      most = std::max(most, pieces.back().size());
     }
-  } else {
-    vrank = r - extra;
+    for (size_t i = 0; i < most; ++i)
+      for (int v = 0; v < p; ++v)
+        if (i < pieces[static_cast<size_t>(v)].size()) bld->Send(pieces[static_cast<size_t>(v)][i], kSrcSend, real_rank(v));
+    for (size_t i = 0; i < most; ++i)
+      for (int v = 0; v < p; ++v)
+        if (i < pieces[static_cast<size_t>(v)].size()) bld->Recv(pieces[static_cast<size_t>(v)][i], real_rank(v), kSrcNone, true, false, -1);
+    return;
   }
-
-  if (vrank >= 0) {
-    const std::vector<std::vector<int>> blocks = GetRankToChunk(static_cast<size_t>(C), static_cast<size_t>(p));
-    int b = 0, e = p;
-    for (int s = 0; s < exp; ++s) {
-      const int vpeer = vrank ^ (1 << s);
-      const int mid = e - (e - b) / 2;
-      int sb, se, kb, ke;
-      if (vrank < vpeer) {
-        sb = b; se = mid; kb = mid; ke = e;
-      } else {
-        kb = b; ke = mid; sb = mid; se = e;
-      }
-      bld->Exchange(real_rank(vpeer), ChunksOfBlocks(blocks, sb, se), partial, ChunksOfBlocks(blocks, kb, ke), partial,
-                    s == exp - 1);
-      partial = kSrcRecv;
-      b = kb;
-      e = ke;
+  const int vrank = r < 2 * extra ? r / 2 : r - extra;
+  OpSrc partial = kSrcSend;  // where my running partial sum lives
+  int b = 0, e = p;
+  for (int s = 0; s < exp; ++s) {
+    const int vpeer = vrank ^ (1 << s);
+    const int mid = e - (e - b) / 2;
+    int sb, se, kb, ke;
+    if (vrank < vpeer) {
+      sb = b; se = mid; kb = mid; ke = e;
+    } else {
+      kb = b; ke = mid; sb = mid; se = e;
     }
-    for (int s = 0; s < exp; ++s) {
-      const int vpeer = vrank ^ (1 << (exp - 1 - s));
-      const int w = e - b;
-      int rb, re;
-      if (vrank > vpeer) {
-        rb = e; re = e + w;
-      } else {
-        rb = b - w; re = b;
-      }
-      const std::vector<int> mine = ChunksOfBlocks(blocks, b, e);
-      bld->Exchange(real_rank(vpeer), mine, kSrcRecv, ChunksOfBlocks(blocks, rb, re), kSrcNone, false);
-      if (s == exp - 1) {
-        // The halves of the last exchange are all a folded rank needs: it gets
-        // one from its partner and one from the partner's partner, its own first.
-        for (int v : {vrank, vpeer})
-          if (v < extra) bld->Exchange(2 * v, mine, kSrcRecv, none, kSrcNone, false);
-      }
-      b = std::min(b, rb);
-      e = std::max(e, re);
+    bld->Exchange(real_rank(vpeer), ChunksOfBlocks(blocks, sb, se), partial, ChunksOfBlocks(blocks, kb, ke), partial,
+                  s == exp - 1 && extra == 0);
+    partial = kSrcRecv;
+    b = kb;
+    e = ke;
+  }
+  // What the extra ranks contribute to my block arrived while the halving ran.
+  const std::vector<int> own = ChunksOfBlocks(blocks, b, e);
+  for (int x = 0; x < extra; ++x) bld->Exchange(2 * x, none, kSrcNone, own, kSrcRecv, x == extra - 1);
+  for (int x = 0; x < extra; ++x) bld->Exchange(2 * x, own, kSrcRecv, none, kSrcNone, false);
+  for (int s = 0; s < exp; ++s) {
+    const int vpeer = vrank ^ (1 << (exp - 1 - s));
+    const int w = e - b;
+    int rb, re;
+    if (vrank > vpeer) {
+      rb = e; re = e + w;
+    } else {
+      rb = b - w; re = b;
     }
-  } else {
-    const std::vector<std::vector<int>> blocks = GetRankToChunk(static_cast<size_t>(C), static_cast<size_t>(p));
-    const int v = r / 2;
-    // What rank `v` of the halving owns before the last exchange: the half of the
-    // message on its side of the first halving step.
-    auto half = [&](int who) { return (who & 1) == 0 ? ChunksOfBlocks(blocks, p - p / 2, p) : ChunksOfBlocks(blocks, 0, p - p / 2); };
-    bld->Exchange(real_rank(v), none, kSrcNone, half(v), kSrcNone, false);
-    bld->Exchange(real_rank(v ^ 1), none, kSrcNone, half(v ^ 1), kSrcNone, false);
+    bld->Exchange(real_rank(vpeer), ChunksOfBlocks(blocks, b, e), kSrcRecv, ChunksOfBlocks(blocks, rb, re), kSrcNone, false);
+    b = std::min(b, rb);
+    e = std::max(e, re);
   }
 }
 
@@ -267,22 +267,19 @@ std::vector<int> InPeers(Algo algo, int rank, int world_size) {
     peers.push_back(Mod(rank - 1, world_size));
     return peers;
   }
-  // Rabenseifner: fold partner first, then the halving partners by step.
+  // Rabenseifner: the halving partners by step, then the extra ranks; an extra
+  // rank hears from every rank of the halving.
   const int p = static_cast<int>(util::FloorPow2(static_cast<uint64_t>(world_size)));
   const int extra = world_size - p;
   const int exp = util::GetExpOfTwo(static_cast<uint64_t>(p));
   auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
-  int vrank;
-  if (rank < 2 * extra) {
-    peers.push_back((rank & 1) == 0 ? rank + 1 : rank - 1);
-    // A folded rank gets half of the result from its partner's last exchange partner.
-    if ((rank & 1) == 0) peers.push_back(real_rank((rank / 2) ^ 1));
-    vrank = (rank & 1) == 0 ? -1 : rank / 2;
-  } else {
-    vrank = rank - extra;
+  if (rank < 2 * extra && (rank & 1) == 0) {
+    for (int v = 0; v < p; ++v) peers.push_back(real_rank(v));
+    return peers;
   }
-  if (vrank >= 0)
-    for (int s = 0; s < exp; ++s) peers.push_back(real_rank(vrank ^ (1 << s)));
+  const int vrank = rank < 2 * extra ? rank / 2 : rank - extra;
+  for (int s = 0; s < exp; ++s) peers.push_back(real_rank(vrank ^ (1 << s)));
+  for (int x = 0; x < extra; ++x) peers.push_back(2 * x);
   return peers;
 }
 
@@ -378,10 +375,10 @@ std::vector<Range> SplitForDevice(size_t len_elements, size_t elem_bytes, size_t
   return out;
 }
 
-size_t RingChunksPerRank(size_t len_elements, size_t elem_bytes, size_t world_size) {
-  const int positions = Tunable("IBCOMM_RING_POSITIONS", 4);
+size_t RingChunksPerRank(size_t len_elements, size_t elem_bytes, size_t world_size, bool one_gpu) {
+  const int positions = Tunable("IBCOMM_RING_POSITIONS", one_gpu ? 2 : 4);
   size_t cpr = positions >= 1 && positions <= 64 ? static_cast<size_t>(positions) : 4;
-  const int min_env = Tunable("IBCOMM_RING_MIN_CHUNK", 16384);
+  const int min_env = Tunable("IBCOMM_RING_MIN_CHUNK", one_gpu ? 65536 : 16384);
   const size_t min_chunk = min_env > 0 ? static_cast<size_t>(min_env) : 1;
   const size_t bytes = len_elements * elem_bytes;
   while (cpr > 1 && bytes / (cpr * world_size) < min_chunk) --cpr;
