@@ -34,9 +34,10 @@ namespace {
 
 // How the pipelined staged kernel runs when its ranks share a GPU.
 struct StagedShape {
-  bool split;    // copy roles in blocks of their own
-  int buffers;   // windows of each kind
-  int blocks;    // reducing blocks per rank (and copying blocks when split)
+  bool split;      // copy roles in blocks of their own
+  int buffers;     // windows of each kind
+  int blocks;      // reducing blocks per rank (and copying blocks when split)
+  int copy_warps;  // unsplit: warps of the loader and of the storer
   uint64_t window_bytes;
   int load_groups, reduce_groups, store_groups;
 };
@@ -44,32 +45,34 @@ struct StagedShape {
 // `bytes`: of a rank's message in the wire type; `resident`: blocks of the kernel
 // the GPU holds at once.  Measured on a B200 (the knobs override each choice):
 //  * The windows of all ranks share one L2, and what falls out of it is written
-//    to HBM and read back: 72 MiB of them in four buffers of each kind (4 ranks
-//    x 64 MiB: 205 us; 24 MiB 440, all of the pool 248), or 40 MiB in three
-//    with a 16-bit wire (8 x 25 MiB of fp32: 182 us against 257).
-//  * A pass of a role over a window is a chain of flag and memory round trips;
-//    with several windows two groups per role overlap them.
-//  * A message of one window has nothing to overlap, and from 1 MiB on is faster
-//    when every block does every role in turn (4 ranks x 4 MiB: 25 against 30 us).
+//    to HBM and read back, while short windows pay a chain of flags for little:
+//    72 MiB in three buffers of each kind (4 ranks x 64 MiB: 170 us; 56 MiB 172,
+//    96 MiB 182, all of the pool 248).
+//  * No fence here waits for a link, so the copy roles need no blocks of their
+//    own, and copies by the threads, with their loads rounds deep, beat the copy
+//    engine's (8 x 25 MiB of fp32, bf16 wire: 156 us against 240 split; 4 x 64
+//    MiB: 170 against 200 with bulk copies).
+//  * Five warps load, five store, six reduce; a message of one window has its
+//    roles one after the other and does with four (4 x 4 MiB 19 us against 21).
 //  * A block per 16 KiB: with one per 128 KiB a 0.5 MiB message on 5 ranks takes
 //    27 us, with one per 16 KiB 21.
-StagedShape StagedShapeOnOneGpu(uint64_t bytes, bool narrow_wire, int ws, uint64_t staging_bytes, int resident, int channels) {
+StagedShape StagedShapeOnOneGpu(uint64_t bytes, int ws, uint64_t staging_bytes, int resident, int channels) {
   StagedShape s;
-  s.buffers = std::max(3, std::min(Tunable("IBCOMM_STAGED_BUFFERS", narrow_wire ? 3 : 4), kStagedMaxBuffers));
-  const uint64_t l2_bytes = static_cast<uint64_t>(narrow_wire ? 40 : 72) << 20;
+  s.buffers = std::max(3, std::min(Tunable("IBCOMM_STAGED_BUFFERS", 3), kStagedMaxBuffers));
+  constexpr uint64_t kL2Bytes = 72ull << 20;
   const uint64_t kinds = static_cast<uint64_t>(2 * s.buffers);
   const uint64_t room = staging_bytes / kinds / 4096 * 4096;
-  const bool one_window = bytes <= room && bytes * 2 * static_cast<uint64_t>(ws) <= l2_bytes;
-  s.window_bytes = one_window ? room : std::min(room, l2_bytes / (kinds * static_cast<uint64_t>(ws)) / 4096 * 4096);
+  const bool one_window = bytes <= room && bytes * 2 * static_cast<uint64_t>(ws) <= kL2Bytes;
+  s.window_bytes = one_window ? room : std::min(room, kL2Bytes / (kinds * static_cast<uint64_t>(ws)) / 4096 * 4096);
   const int per_rank = std::max(1, resident / ws);
-  s.split = Tunable("IBCOMM_STAGED_SPLIT", one_window && bytes >= (1u << 20) ? 0 : 1) != 0 && per_rank >= 2;
+  s.split = Tunable("IBCOMM_STAGED_SPLIT", 0) != 0 && per_rank >= 2;
   const int most = std::min(128, s.split ? per_rank / 2 : per_rank);
   s.blocks = std::max(1, std::min(channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(bytes / (16u << 10), 128)), most));
-  const int copy_groups = one_window ? 1 : 2;
+  s.copy_warps = one_window ? 4 : 5;
   auto groups = [](const char* knob, int dflt) { return std::max(1, std::min(Tunable(knob, dflt), 4)); };
-  s.load_groups = groups("IBCOMM_STAGED_LOAD_GROUPS", copy_groups);
+  s.load_groups = groups("IBCOMM_STAGED_LOAD_GROUPS", 1);
   s.reduce_groups = groups("IBCOMM_STAGED_REDUCE_GROUPS", 2);
-  s.store_groups = groups("IBCOMM_STAGED_STORE_GROUPS", copy_groups);
+  s.store_groups = groups("IBCOMM_STAGED_STORE_GROUPS", 1);
   return s;
 }
 
@@ -174,7 +177,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
   const size_t wsize = DTypeSize(wire);
   if (algo == Algo::kDirect && (wire != dtype || m.direct_staging == 2)) {
     // The pipelined staged kernel (what ordinary buffers and 16-bit wires get on several GPUs).
-    const StagedShape sh = StagedShapeOnOneGpu(n * wsize, wire != dtype, m.ws, m.layout.pool_bytes + m.layout.work_bytes,
+    const StagedShape sh = StagedShapeOnOneGpu(n * wsize, m.ws, m.layout.pool_bytes + m.layout.work_bytes,
                                                m.staged_max_blocks, channels);
     if (!all_aligned || (n * wsize) % 16 != 0 || sh.window_bytes < 4096)
       IBCOMM_FAIL(NOT_SUPPORTED, "The pipelined staged two-shot needs 16-byte aligned buffers of whole 16-byte wire vectors.\n");
@@ -189,7 +192,8 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.dtype = static_cast<int32_t>(dtype);
       p.wire = static_cast<int32_t>(wire);
       p.use_multimem = 0;
-      p.use_tma = (wire == dtype && Tunable("IBCOMM_STAGED_TMA", 1) != 0) ? 1 : 0;
+      p.use_tma = (wire == dtype && Tunable("IBCOMM_STAGED_TMA", 0) != 0) ? 1 : 0;
+      p.copy_warps = sh.copy_warps;
       p.peers = rr.peers;
       p.sendbuf = sendbufs[static_cast<size_t>(r)];
       p.recvbuf = recvbufs[static_cast<size_t>(r)];

@@ -150,6 +150,7 @@ struct StagedParams {
   // Split mode: groups per role (1 .. 4) that take the windows in turn.  groups x reducing blocks <= 256
   // (a group has flag rows of its own).
   int32_t load_groups, reduce_groups, store_groups;
+  int32_t copy_warps;  // unsplit, copies by the threads: warps of the loader and of the storer (0: three each)
   int32_t posters;  // split mode: a poster warp per reducer group fences and publishes behind the data warps
 };
 cudaError_t LaunchStagedKernel(const StagedParams* ranks, int n, int blocks, cudaStream_t stream);

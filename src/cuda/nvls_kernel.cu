@@ -124,7 +124,7 @@ __device__ void TwoShotBody(const NvlsParams& p, uint64_t seq, int& s_stop, unsi
 #pragma unroll
           for (int q = 0; q < kR; ++q)
             if (q < ws) St16(outs[q] + wout_bytes_off + idx * 16, r);
-        });
+        }, threadIdx.x, blockDim.x);
       }
     }
     // Ragged end (< 16 bytes): every rank sums it itself from the peers'
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) NvlsKernel(const __grid_const
 
 template <typename T, int U, bool kMultimem, int kR>
 static cudaError_t LaunchNvlsU(const NvlsParams* ranks, int n, int blocks, int threads, cudaStream_t stream) {
-  const size_t smem = kMultimem ? 0 : dev::kReduceSmemPerThread * static_cast<size_t>(threads);
+  const size_t smem = kMultimem ? 0 : dev::kRoundSmemPerThread * static_cast<size_t>(threads);
   if (smem != 0) {
     const cudaError_t e = AllowSharedMemory(dev::NvlsKernel<T, U, kMultimem, kR>, smem);
     if (e != cudaSuccess) return e;
@@ -216,7 +216,7 @@ static cudaError_t LaunchNvlsTyped(const NvlsParams* ranks, int n, int blocks, c
 int TwoShotKernelMaxCoResidentBlocks(int device) {
   int per_sm = 0, sms = 0;
   const auto kernel = dev::NvlsKernel<float, 4, false, kMaxRanks>;
-  const size_t smem = dev::kReduceSmemPerThread * dev::kNvlsThreads;
+  const size_t smem = dev::kRoundSmemPerThread * dev::kNvlsThreads;
   if (AllowSharedMemory(kernel, smem) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, dev::kNvlsThreads, smem) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;

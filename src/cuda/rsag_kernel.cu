@@ -133,7 +133,7 @@ __device__ void RsAgBody(const RsAgParams& p, uint64_t seq, int& s_stop, unsigne
         }
       } else {
         PeerReduce<T, kR>(smem, p.peer_buf, ws, off, b, ev, do_scale, p.scale,
-                          [&](uint64_t idx, uint4 r) { StUser16<T>(out + idx * 16, r, out_aligned); });
+                          [&](uint64_t idx, uint4 r) { StUser16<T>(out + idx * 16, r, out_aligned); }, threadIdx.x, blockDim.x);
         each_element([&](int64_t k) {
           A acc = A(0);
           for (int q = 0; q < ws; ++q) acc += ToAcc<A, T>(LdScalarStrong<T>(reinterpret_cast<const T*>(p.peer_buf[q] + off) + k));
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kNvlsThreads, 1) RsAgKernel(const __grid_const
 
 template <typename T, bool kMultimem, int kR>
 static cudaError_t LaunchRsAgU(const RsAgParams* ranks, int n, int blocks, cudaStream_t stream) {
-  const size_t smem = kMultimem || ranks->mode != kRsAgReduceScatter ? 0 : dev::kReduceSmemPerThread * dev::kNvlsThreads;
+  const size_t smem = kMultimem || ranks->mode != kRsAgReduceScatter ? 0 : dev::kRoundSmemPerThread * dev::kNvlsThreads;
   if (smem != 0) {
     const cudaError_t e = AllowSharedMemory(dev::RsAgKernel<T, kMultimem, kR>, smem);
     if (e != cudaSuccess) return e;

@@ -25,9 +25,9 @@
 //
 // Where the roles run:
 //   * every block runs all of them (one loader, one storer, two reducer
-//     groups: 1 + 1 + 14 warps with bulk copies, 3 + 3 + 10 with copies in
-//     registers), or
-//   * split (the default where twice the blocks are co-resident): blocks
+//     groups: 1 + 1 + 14 warps with bulk copies, 3 + 3 + 10, or as the host
+//     says, with copies by the threads), or
+//   * split (the default between GPUs, where twice the blocks are co-resident): blocks
 //     [0, n) only reduce, blocks [n, 2n) only copy, block n + b serving the
 //     same part of every window as block b.  A release at system scope waits
 //     for every store the SM has in flight; next to reducers that made a
@@ -44,8 +44,11 @@
 // When the wire type equals the buffer type the copies are bulk asynchronous
 // copies (TMA, `cp.async.bulk`, global -> shared -> global, no multicast, this
 // GPU's memory only) driven by one thread per copy group through a ring of
-// shared-memory stages; with a 16-bit wire the copy groups convert in
-// registers instead (fp32 accumulation in the reducers either way).
+// shared-memory stages; with a 16-bit wire, and between ranks on one GPU, the
+// threads of the copy groups move and convert instead (fp32 accumulation in the
+// reducers either way).  Thread copies and the reducers' peer loads keep three
+// rounds in flight (AsyncRounds, twoshot_common.cuh): B200, 4 ranks x 64 MiB 203
+// -> 170 us, 8 x 25 MiB bucket with a bf16 wire 183 -> 156 us.
 //
 // Synchronisation is per block index across ranks, with rows of the control
 // page (values (call << 32) | window + 1, growing only; group g of a role
@@ -84,14 +87,15 @@ namespace dev {
 constexpr int kStagedThreads = 512;
 // Warps per group.  With bulk copies one thread drives each copy group, so
 // the loader and the storer are one warp each and 14 warps reduce; with
-// copies in registers (16-bit wire) the split is 3 / 3 / 10.
+// copies by the threads the split is 3 / 3 / 10 unless the host says otherwise.
 constexpr int kLoadWarpsRegs = 3;
 constexpr int kStagedMaxCtas = 128;   // blocks that reduce (and, unsplit, copy too)
 constexpr int kStagedMaxGroups = 4;   // groups of one role that work on different windows at the same time
 constexpr uint32_t kBulkChunk = 8192;   // bytes per bulk copy
 constexpr int kBulkMaxDepth = 12;       // stages per ring at most (a lane and an mbarrier each)
 constexpr int kBulkMaxRings = 2 * kStagedMaxGroups;
-constexpr size_t kStagedSmemBytes = 192u << 10;
+constexpr size_t kStagedSmemBytes = 192u << 10;  // bulk-copy rings, or the threads' loads
+static_assert(kStagedSmemBytes >= kStagedThreads * kRoundSmemPerThread, "three rounds of loads per thread");
 
 enum StagedRow : int { kRowInReady = 0, kRowReduced = 1, kRowOutFree = 2 };
 
@@ -158,69 +162,52 @@ __device__ __forceinline__ void RolePost(RoleCtx& c, int row, uint64_t flag_wind
     StReleasePeers(FlagRow(Ctl(*c.w.peers, c.tid), row, c.cta, c.ncta, flag_window, groups) + c.w.rank, value, c.w.peers->one_gpu != 0);
 }
 
-// ---- copies in registers (with the conversion between buffer and wire type) ----
-// Wire vectors [b, e) of a window; `user` and `wire` point at the window's first element.
+// ---- copies by the threads (with the conversion between buffer and wire type) ----
+// This block's wire vectors of a window (vector numbers of the window), one range
+// per shard that goes through the pool; `user` and `wire` point at the window's
+// first element.  A range is a round or two, so the loads have to run over its end.
+struct CopyParts {
+  uint64_t from[kMaxRanks], to[kMaxRanks];
+  int parts;
+  __device__ __forceinline__ int count() const { return parts; }
+  __device__ __forceinline__ uint64_t begin(int q) const { return from[q]; }
+  __device__ __forceinline__ uint64_t end(int q) const { return to[q]; }
+};
+
 template <typename T, typename W>
-__device__ __forceinline__ void CastIn(uint4* wire, const uint4* user, uint64_t b, uint64_t e, uint64_t policy, int tid, int nthr) {
+__device__ __forceinline__ void CastIn(unsigned char* smem, uint4* wire, const uint4* user, const CopyParts& parts, uint64_t policy, int tid, int nthr) {
   using A = typename Acc<T>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
-  constexpr int U = VT == 1 ? 8 : 4;
-  for (uint64_t i = b + tid; i < e; i += static_cast<uint64_t>(nthr) * U) {
-    uint4 q[U][VT];
+  AsyncRounds<kRoundVecs / VT>(
+      smem, parts, static_cast<unsigned>(tid), static_cast<unsigned>(nthr),
+      [&](uint64_t vec, uint32_t slot, uint32_t stride) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
-      if (idx < e) {
+        for (int v = 0; v < VT; ++v) CpAsync16Hint(slot + static_cast<uint32_t>(v) * stride, user + vec * VT + v, policy);
+      },
+      [&](uint64_t vec, const unsigned char* slot, uint32_t stride) {
+        A acc[P];
 #pragma unroll
-        for (int v = 0; v < VT; ++v) q[u][v] = Ld16Hint(user + idx * VT + v, policy);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
-      if (idx < e) {
-        if constexpr (sizeof(T) == sizeof(W)) {
-          St16(wire + idx, q[u][0]);
-        } else {
-          A acc[P];
-#pragma unroll
-          for (int v = 0; v < VT; ++v) VecIO<T>::Load(q[u][v], acc + v * VecIO<T>::kN);
-          St16(wire + idx, VecIO<W>::Store(acc));
-        }
-      }
-    }
-  }
+        for (int v = 0; v < VT; ++v)
+          VecIO<T>::Load(*reinterpret_cast<const uint4*>(slot + static_cast<uint32_t>(v) * stride), acc + v * VecIO<T>::kN);
+        St16(wire + vec, VecIO<W>::Store(acc));
+      });
 }
 
 template <typename T, typename W>
-__device__ __forceinline__ void CastOut(uint4* user, const uint4* wire, uint64_t b, uint64_t e, uint64_t policy, int tid, int nthr) {
+__device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const uint4* wire, const CopyParts& parts, uint64_t policy, int tid, int nthr) {
   using A = typename Acc<T>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
-  constexpr int U = 8;
-  for (uint64_t i = b + tid; i < e; i += static_cast<uint64_t>(nthr) * U) {
-    uint4 q[U];
+  AsyncRounds<kRoundVecs>(
+      smem, parts, static_cast<unsigned>(tid), static_cast<unsigned>(nthr),
+      [&](uint64_t vec, uint32_t slot, uint32_t) { CpAsync16(slot, wire + vec); },
+      [&](uint64_t vec, const unsigned char* slot, uint32_t) {
+        A acc[P];
+        VecIO<W>::Load(*reinterpret_cast<const uint4*>(slot), acc);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
-      if (idx < e) q[u] = Ld16Strong(wire + idx);  // written by the peers
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
-      if (idx < e) {
-        if constexpr (sizeof(T) == sizeof(W)) {
-          St16Hint(user + idx, q[u], policy);
-        } else {
-          A acc[P];
-          VecIO<W>::Load(q[u], acc);
-#pragma unroll
-          for (int v = 0; v < VT; ++v) St16Hint(user + idx * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), policy);
-        }
-      }
-    }
-  }
+        for (int v = 0; v < VT; ++v) St16Hint(user + vec * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), policy);
+      });
 }
 
 // ---- copies by the bulk copy engine: global -> shared -> global, one thread ----
@@ -300,6 +287,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   __shared__ int s_stop;
   __shared__ int s_role_stop[3 * kStagedMaxGroups][2];
   __shared__ uint64_t s_full[kBulkMaxRings][kBulkMaxDepth];
+  __shared__ CopyParts s_copy[2];  // what the copy roles move of a full window, and of the last one
   __shared__ uint64_t s_part[kMaxRanks][2];  // this block's part of every shard of a full window, in vectors
   __shared__ RoleSync s_sync;  // reducing blocks in split mode: done[g] = windows whose stores group g has issued
   {
@@ -356,12 +344,29 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   // Peer loads and stores of the buffers' own type: this rank's shard need not
   // pass through its pool, its reducers read sendbuf and write recvbuf.
   constexpr bool kOwnInPlace = !kMultimem && sizeof(T) == sizeof(W);
+  // The parts the copy roles move.
+  auto fill_parts = [&](CopyParts* cp, uint64_t nv) {
+    cp->parts = 0;
+    cp->from[0] = cp->to[0] = 0;
+    for (int s = 0; s < ws; ++s) {
+      uint64_t b, e;
+      part(s, nv, &b, &e);
+      if ((kOwnInPlace && s == me) || b >= e) continue;
+      cp->from[cp->parts] = b;
+      cp->to[cp->parts] = e;
+      ++cp->parts;
+    }
+  };
+
+  if (!tma && threadIdx.x < 2 && windows != 0) fill_parts(&s_copy[threadIdx.x], threadIdx.x == 0 ? full_nv : total_nv - (windows - 1) * full_nv);
+  __syncthreads();
+  auto parts_of = [&](uint64_t nv) -> const CopyParts& { return s_copy[nv == full_nv ? 0 : 1]; };
 
   constexpr int kWarps = kStagedThreads / 32;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   // Warps of a copy group: one when a thread drives the copy engine, otherwise
   // 3 (unsplit) or as many as fit into half a block (split).
-  const int copy_warps = tma ? 1 : (split ? kWarps / 2 / (LG > SG ? LG : SG) : kLoadWarpsRegs);
+  const int copy_warps = tma ? 1 : (split ? kWarps / 2 / (LG > SG ? LG : SG) : (p.copy_warps >= 1 && p.copy_warps <= kWarps / 2 - 1 ? p.copy_warps : kLoadWarpsRegs));
   // role: 0 loader, 1 storer, 2 reducer, -1 none; group inside the role; thread inside the group.
   int role = -1, group = 0, gthreads = 0, gtid = 0;
   if (!split) {
@@ -455,12 +460,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         }
         FenceProxyAsyncAll();
       } else if (!tma) {
-        for (int s = 0; s < ws; ++s) {
-          uint64_t b, e;
-          part(s, nv, &b, &e);
-          if (kOwnInPlace && s == me) continue;
-          CastIn<T, W>(reinterpret_cast<uint4*>(win), reinterpret_cast<const uint4*>(user), b, e, once, c.tid, c.nthr);
-        }
+        CastIn<T, W>(smem, reinterpret_cast<uint4*>(win), reinterpret_cast<const uint4*>(user), parts_of(nv), once, c.tid, c.nthr);
       }
       RolePost(c, kRowInReady, k, LG, base | (k + 1));
       if (role_w != 0 && gtid == 0) trace[role_w + k].t_done = GlobalTimerNs();
@@ -497,12 +497,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         }
         FenceProxyAsyncAll();
       } else if (!tma) {
-        for (int s = 0; s < ws; ++s) {
-          uint64_t b, e;
-          part(s, nv, &b, &e);
-          if (kOwnInPlace && s == me) continue;
-          CastOut<T, W>(reinterpret_cast<uint4*>(user), reinterpret_cast<const uint4*>(win), b, e, once, c.tid, c.nthr);
-        }
+        CastOut<T, W>(smem, reinterpret_cast<uint4*>(user), reinterpret_cast<const uint4*>(win), parts_of(nv), once, c.tid, c.nthr);
       }
       RolePost(c, kRowOutFree, k, SG, base | (k + 1));
       if (role_w != 0 && gtid == 0) trace[2 * role_w + k].t_done = GlobalTimerNs();
@@ -567,13 +562,16 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
             }
           }
         }
-        PeerReduceGroup<W, kR>(from, ws, 0, b, e, do_scale, p.scale,
-                               [&](uint64_t idx, uint4 r) {
+        auto store = [&](uint64_t idx, uint4 r) {
 #pragma unroll
-                                 for (int q = 0; q < kR; ++q)
-                                   if (q < ws) St16(to[q] + idx * 16, r);
-                               },
-                               static_cast<unsigned>(c.tid), static_cast<unsigned>(reduce_threads));
+          for (int q = 0; q < kR; ++q)
+            if (q < ws) St16(to[q] + idx * 16, r);
+        };
+        // Beside bulk-copy rings the shared memory is theirs.
+        if (split || !tma)
+          PeerReduce<W, kR>(smem, from, ws, 0, b, e, do_scale, p.scale, store, static_cast<unsigned>(c.tid), static_cast<unsigned>(reduce_threads));
+        else
+          PeerReduceGroup<W, kR>(from, ws, 0, b, e, do_scale, p.scale, store, static_cast<unsigned>(c.tid), static_cast<unsigned>(reduce_threads));
       }
       if (role_w != 0 && c.tid == 0) trace[3 * role_w + k].t_wait_done = GlobalTimerNs();
       if (has_poster) {

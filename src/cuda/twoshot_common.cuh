@@ -113,76 +113,119 @@ __device__ __forceinline__ void PeerReduceUnits(unsigned char* const* peer, int 
   }
 }
 
-// The same by a whole CTA, with the loads of kReduceDepth rounds in flight: a
-// thread's vectors go to slots of its own in shared memory (`cp.async`, 16 bytes
-// through L2), so nothing but the thread's own wait orders them and the depth
-// costs no registers.  `smem`: kReduceSmemPerThread bytes per thread.  With one
-// round in registers a CTA waited a memory round trip per 64 KiB; B200, 8 ranks x
-// 32 MiB fp32 in place: 113 -> 102 us, 2 x 64 MiB: 76 -> 53 us (5.1 TB/s).  The
-// same depth in registers spills, whether as a second buffer or as a second CTA
-// per SM (123 us and more).
-constexpr int kReduceDepth = 3;
-constexpr size_t kReduceSmemPerThread = static_cast<size_t>(kReduceDepth) * kMaxRanks * 16;
+// ---- loads several rounds deep ----
+// With one round of loads in registers a CTA waits a memory round trip per 64
+// KiB, and more in registers spills, whether as a second buffer or as a second
+// CTA per SM (8 ranks x 16 MiB of bf16: 68 us, 123 and more when spilling).
+// Instead a thread's vectors of the coming rounds go to slots of its own in
+// shared memory (`cp.async`, 16 bytes through L2): nothing but the thread's own
+// wait orders them, and the depth costs no registers.  B200, in place: 8 ranks x
+// 32 MiB fp32 113 -> 102 us, 2 x 64 MiB 76 -> 53 us (5.1 TB/s).
+constexpr int kRoundVecs = 8;   // 16-byte vectors per thread and round
+constexpr int kRoundDepth = 3;  // rounds in flight
+constexpr size_t kRoundSmemPerThread = static_cast<size_t>(kRoundDepth) * kRoundVecs * 16;
 
 __device__ __forceinline__ void CpAsync16(uint32_t smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void CpAsync16Hint(uint32_t smem_dst, const void* src, uint64_t policy) {
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(src), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void CpAsyncCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void CpAsyncWait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <typename T, int kR, typename Store>
-__device__ __forceinline__ void PeerReduce(unsigned char* smem, unsigned char* const* peer, int ws, uint64_t off, uint64_t b, uint64_t e,
-                                           bool do_scale, double scale, Store store) {
-  using A = typename Acc<T>::type;
-  constexpr int kVecElems = 16 / static_cast<int>(sizeof(T));
-  constexpr int kU = kMaxRanks / kR;  // vectors per rank and round
-  const unsigned nthr = blockDim.x;
+// Ranges of items, walked one after the other in rounds of `step` items; a round
+// belongs to one range.
+struct OneRange {
+  uint64_t b, e;
+  __device__ __forceinline__ int count() const { return 1; }
+  __device__ __forceinline__ uint64_t begin(int) const { return b; }
+  __device__ __forceinline__ uint64_t end(int) const { return e; }
+};
+template <typename Ranges>
+struct RoundCursor {
+  int q;
+  uint64_t base, end;
+  __device__ __forceinline__ explicit RoundCursor(const Ranges& r) : q(0), base(r.begin(0)), end(r.end(0)) { Settle(r); }
+  __device__ __forceinline__ void Settle(const Ranges& r) {
+    while (base >= end && ++q < r.count()) base = r.begin(q), end = r.end(q);
+  }
+  __device__ __forceinline__ void Next(const Ranges& r, uint64_t step) {
+    base += step;
+    Settle(r);
+  }
+  __device__ __forceinline__ bool Done(const Ranges& r) const { return q >= r.count(); }
+};
+
+// Every item of `ranges` over `nthr` threads numbered `tid`, kU items per thread
+// and round, each of kRoundVecs / kU vectors: `issue(item, smem, stride)` starts
+// the loads of one item into slots `smem`, `smem + stride`, ..., `use(item, slots,
+// stride)` consumes it.  `smem`: kRoundSmemPerThread bytes for every thread of the
+// block.  The loads run over the ends of ranges.
+template <int kU, typename Ranges, typename Issue, typename Use>
+__device__ __forceinline__ void AsyncRounds(unsigned char* smem, const Ranges& ranges, unsigned tid, unsigned nthr, Issue issue, Use use) {
+  constexpr int kV = kRoundVecs / kU;
   const uint64_t step = static_cast<uint64_t>(nthr) * kU;
-  const uint32_t slot_bytes = nthr * 16u, round_bytes = slot_bytes * kU * kR;
+  const uint32_t stride = blockDim.x * 16u, round_bytes = stride * kRoundVecs;
   unsigned char* const mine = smem + threadIdx.x * 16u;
   const uint32_t mine_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(mine));
-  auto issue = [&](uint64_t i, uint32_t at) {
+  RoundCursor<Ranges> in(ranges), out = in;
+  uint32_t at = 0, ahead = 0;
+  auto start = [&]() {
+    if (!in.Done(ranges)) {
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
-      if (idx < e) {
-#pragma unroll
-        for (int q = 0; q < kR; ++q)
-          if (q < ws) CpAsync16(mine_u32 + at + static_cast<uint32_t>(u * kR + q) * slot_bytes, peer[q] + off + idx * 16);
+      for (int u = 0; u < kU; ++u) {
+        const uint64_t idx = in.base + tid + static_cast<uint64_t>(u) * nthr;
+        if (idx < in.end) issue(idx, mine_u32 + ahead + static_cast<uint32_t>(u * kV) * stride, stride);
       }
+      in.Next(ranges, step);
     }
     CpAsyncCommit();
+    ahead = ahead + round_bytes == kRoundDepth * round_bytes ? 0 : ahead + round_bytes;
   };
-  uint64_t i = b + threadIdx.x;
-  if (i >= e) return;
 #pragma unroll
-  for (int d = 0; d + 1 < kReduceDepth; ++d) issue(i + static_cast<uint64_t>(d) * step, static_cast<uint32_t>(d) * round_bytes);
-  uint32_t at = 0, ahead = (kReduceDepth - 1) * round_bytes;
-  for (; i < e; i += step) {
-    issue(i + (kReduceDepth - 1) * step, ahead);
-    CpAsyncWait<kReduceDepth - 1>();
+  for (int d = 0; d + 1 < kRoundDepth; ++d) start();
+  while (!out.Done(ranges)) {
+    start();
+    CpAsyncWait<kRoundDepth - 1>();
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      const uint64_t idx = i + static_cast<uint64_t>(u) * nthr;
-      if (idx < e) {
-        const unsigned char* from = mine + at + static_cast<uint32_t>(u * kR) * slot_bytes;
+      const uint64_t idx = out.base + tid + static_cast<uint64_t>(u) * nthr;
+      if (idx < out.end) use(idx, mine + at + static_cast<uint32_t>(u * kV) * stride, stride);
+    }
+    out.Next(ranges, step);
+    at = at + round_bytes == kRoundDepth * round_bytes ? 0 : at + round_bytes;
+  }
+  CpAsyncWait<0>();
+}
+
+// PeerReduceUnits that way, by `nthr` threads numbered `tid`.
+template <typename T, int kR, typename Store>
+__device__ __forceinline__ void PeerReduce(unsigned char* smem, unsigned char* const* peer, int ws, uint64_t off, uint64_t b, uint64_t e,
+                                           bool do_scale, double scale, Store store, unsigned tid, unsigned nthr) {
+  using A = typename Acc<T>::type;
+  constexpr int kVecElems = 16 / static_cast<int>(sizeof(T));
+  static_assert(kRoundVecs % kR == 0, "a round holds whole items");
+  AsyncRounds<kRoundVecs / kR>(
+      smem, OneRange{b, e}, tid, nthr,
+      [&](uint64_t idx, uint32_t slot, uint32_t stride) {
+#pragma unroll
+        for (int q = 0; q < kR; ++q)
+          if (q < ws) CpAsync16(slot + static_cast<uint32_t>(q) * stride, peer[q] + off + idx * 16);
+      },
+      [&](uint64_t idx, const unsigned char* slot, uint32_t stride) {
         A acc[kVecElems];
-        VecIO<T>::Load(*reinterpret_cast<const uint4*>(from), acc);
+        VecIO<T>::Load(*reinterpret_cast<const uint4*>(slot), acc);
 #pragma unroll
         for (int q = 1; q < kR; ++q)
-          if (q < ws) VecIO<T>::Add(*reinterpret_cast<const uint4*>(from + static_cast<uint32_t>(q) * slot_bytes), acc);
+          if (q < ws) VecIO<T>::Add(*reinterpret_cast<const uint4*>(slot + static_cast<uint32_t>(q) * stride), acc);
         if (do_scale) {
 #pragma unroll
           for (int k = 0; k < kVecElems; ++k) acc[k] = ScaleAcc<A>(acc[k], scale);
         }
         store(idx, VecIO<T>::Store(acc));
-      }
-    }
-    ahead = at;
-    at = at + round_bytes == kReduceDepth * round_bytes ? 0 : at + round_bytes;
-  }
-  CpAsyncWait<0>();
+      });
 }
 
 // The kernels are compiled per world-size class kR (2, 4 or 8 ranks at most)
