@@ -16,7 +16,10 @@
 // of their message to the rank that ends up owning it, which adds it to its own
 // sum, and get the results back from the owners.  Against folding an extra rank
 // into one partner first, which had that partner move 1.5 times what the others
-// move, 5 ranks x 64 MiB on one B200 take 359 us instead of 407.
+// move, 5 ranks x 64 MiB on one B200 take 359 us instead of 407.  A piece that goes
+// on to the next step's partner does so in the op that receives (and adds) it, in
+// both directions: the partial sums given away are never stored and read back (8
+// ranks x 64 MiB 634 -> 556 us, 8 x 16 MiB 157 -> 138, 5 x 64 MiB 359 -> 331).
 #pragma once
 
 #include <string>

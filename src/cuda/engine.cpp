@@ -162,10 +162,12 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   // rank and the number of pieces Rabenseifner cuts the message into.
   const size_t ring_cpr = ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size), ranks_on_gpu > 1) : 0;
   // Ranks on one GPU: four pieces of up to 8 MiB (a hand-over costs what 100 KiB
-  // per channel cost; 5 ranks, 4 / 16 MiB: 75 / 134 us with eight, 64 / 122 with four).
+  // per channel cost; 5 ranks, 4 / 16 MiB: 45 / 90 us with eight, 44 / 86 with four),
+  // two up to 2 MiB where extra ranks add transfers (3 ranks, 1 MiB: 23 against 28).
+  const bool small_with_extras = (world_size & (world_size - 1)) != 0 && len_elements * esize <= (size_t(2) << 20);
   int raben_div = Tunable("IBCOMM_RABEN_PIECES", 0);
   if (raben_div < 1 || raben_div > 1024)
-    raben_div = ranks_on_gpu > 1 ? static_cast<int>(std::min<size_t>(1024, std::max<size_t>(4, util::ceilDiv(len_elements * esize, size_t(8) << 20)))) : 8;
+    raben_div = ranks_on_gpu > 1 ? static_cast<int>(std::min<size_t>(1024, std::max<size_t>(small_with_extras ? 2 : 4, util::ceilDiv(len_elements * esize, size_t(8) << 20)))) : 8;
   Key key{static_cast<int>(algo), rank, world_size, len_elements, static_cast<int>(dtype), static_cast<int>(wire),
           env_chunk, apply_scale, stage_off, stage_bytes, ring ? static_cast<int>(ring_cpr) : raben_div};
   auto it = cache_.find(key);

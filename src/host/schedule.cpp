@@ -109,17 +109,27 @@ struct Builder {
     prog.ops.push_back(op);
   }
 
-  // One exchange step with a single partner: `sends` leave, `recvs` arrive.
-  // Sends run at most `slots` ahead of the receives so that neither side can
-  // block on credits the other side has not had a chance to return.
-  void Exchange(int peer, const std::vector<int>& send_chunks, OpSrc send_src, const std::vector<int>& recv_chunks,
-                OpSrc recv_add, bool recv_scale) {
-    const std::vector<Range> sends = Pieces(send_chunks), recvs = Pieces(recv_chunks);
-    size_t si = 0, ri = 0;
-    const size_t ahead = slots;
-    while (si < sends.size() && si < ahead) Send(sends[si++], send_src, peer);
-    while (ri < recvs.size()) {
-      Recv(recvs[ri], peer, recv_add, true, recv_scale, -1);
+  // What a step receives, in order.  The first `forward` pieces go on to
+  // `forward_to` in the same op, and are stored here as well when `keep`; the
+  // others always are.
+  struct Arrivals {
+    std::vector<Range> pieces;
+    OpSrc add = kSrcNone;
+    bool final_sum = false;
+    size_t forward = 0;
+    int forward_to = -1;
+    bool keep = true;
+  };
+  // One exchange step with a single partner: `sends` leave, of which the first
+  // `sent` already did (forwarded as they arrived), and `in` arrives.  Sends run at
+  // most `slots` ahead of the receives so that neither side can block on credits
+  // the other side has not had a chance to return.
+  void Exchange(int peer, const std::vector<Range>& sends, size_t sent, OpSrc send_src, const Arrivals& in) {
+    size_t si = sent, ri = 0;
+    while (si < sends.size() && si < slots) Send(sends[si++], send_src, peer);
+    while (ri < in.pieces.size()) {
+      const bool fwd = ri < in.forward;
+      Recv(in.pieces[ri], peer, in.add, in.keep || !fwd, in.final_sum, fwd ? in.forward_to : -1);
       ++ri;
       if (si < sends.size()) Send(sends[si++], send_src, peer);
     }
@@ -181,16 +191,46 @@ void BuildRing(Builder* bld) {
   }
 }
 
-// Block that rank `v` of `p` (a power of two) is left with after the halving.
-int OwnedBlock(int v, int p) {
-  int b = 0, e = p;
-  for (int s = 1; s < p; s <<= 1) {
-    const int mid = e - (e - b) / 2;
-    if (v < (v ^ s)) b = mid;
-    else e = mid;
+// The halving of `p` ranks (a power of two) over their `blocks`, and the order in
+// which pieces travel so that a piece can be handed on in the op that receives it.
+struct Halving {
+  const Builder& bld;
+  const std::vector<std::vector<int>>& blocks;
+  int p, exp;
+
+  // Blocks rank `v` still works on after `steps` steps.
+  std::pair<int, int> Run(int v, int steps) const {
+    int b = 0, e = p;
+    for (int s = 0; s < steps; ++s) {
+      const int mid = e - (e - b) / 2;
+      if (v < (v ^ (1 << s))) b = mid;
+      else e = mid;
+    }
+    return {b, e};
   }
-  return b;
-}
+  std::vector<Range> Pieces(std::pair<int, int> run) const { return bld.Pieces(ChunksOfBlocks(blocks, run.first, run.second)); }
+  std::vector<Range> Own(int v) const { return Pieces(Run(v, exp)); }
+
+  // What rank `v` receives in step `s`, in order: first what it gives away in
+  // step s + 1, as its partner there wants it, then what it keeps.
+  std::vector<Range> Kept(int v, int s) const {
+    if (s + 1 == exp) return Own(v);
+    std::vector<Range> out = Kept(v ^ (1 << (s + 1)), s + 1);
+    const std::vector<Range> rest = Pieces(Run(v, s + 2));
+    out.insert(out.end(), rest.begin(), rest.end());
+    return out;
+  }
+  int DoublingPartner(int v, int t) const { return v ^ (1 << (exp - 1 - t)); }
+  // What rank `v` has collected when step `t` of the doubling begins, in the order
+  // it passes it on: what came in last first, since that is handed on on arrival.
+  std::vector<Range> Collected(int v, int t) const {
+    if (t == 0) return Own(v);
+    std::vector<Range> out = Collected(DoublingPartner(v, t - 1), t - 1);
+    const std::vector<Range> before = Collected(v, t - 1);
+    out.insert(out.end(), before.begin(), before.end());
+    return out;
+  }
+};
 
 void BuildRabenseifner(Builder* bld) {
   const ProgramRequest& q = bld->req;
@@ -198,10 +238,11 @@ void BuildRabenseifner(Builder* bld) {
   const int p = static_cast<int>(util::FloorPow2(static_cast<uint64_t>(ws)));
   const int extra = ws - p;
   const int exp = util::GetExpOfTwo(static_cast<uint64_t>(p));
-  const int C = static_cast<int>(q.ranges.size());
   auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
-  const std::vector<int> none;
-  const std::vector<std::vector<int>> blocks = GetRankToChunk(static_cast<size_t>(C), static_cast<size_t>(p));
+  const std::vector<std::vector<int>> blocks = GetRankToChunk(q.ranges.size(), static_cast<size_t>(p));
+  const Halving half{*bld, blocks, p, exp};
+  const std::vector<Range> none;
+  using Arrivals = Builder::Arrivals;
 
   if (r < 2 * extra && (r & 1) == 0) {
     // An extra rank hands every block of its message to the rank that will own
@@ -210,7 +251,7 @@ void BuildRabenseifner(Builder* bld) {
     std::vector<std::vector<Range>> pieces;
     size_t most = 0;
     for (int v = 0; v < p; ++v) {
-      pieces.push_back(bld->Pieces(blocks[static_cast<size_t>(OwnedBlock(v, p))]));
+      pieces.push_back(half.Own(v));
       most = std::max(most, pieces.back().size());
     }
     for (size_t i = 0; i < most; ++i)
@@ -222,39 +263,61 @@ void BuildRabenseifner(Builder* bld) {
     return;
   }
   const int vrank = r < 2 * extra ? r / 2 : r - extra;
-  OpSrc partial = kSrcSend;  // where my running partial sum lives
-  int b = 0, e = p;
+  const size_t slots = bld->slots;
+
+  // Halving.  A partial sum that goes to the next step's partner is forwarded in
+  // the op that computes it and not stored, up to the partner's slots: those are
+  // all free until that step, so no forward waits for a credit that the partner
+  // could only return after waiting for one of ours.
+  size_t sent = 0;        // of what this step sends, forwarded during the one before
+  size_t first_sent = 0;  // of my own block, to the first partner of the doubling
+  const std::vector<Range> own = half.Own(vrank);
   for (int s = 0; s < exp; ++s) {
     const int vpeer = vrank ^ (1 << s);
-    const int mid = e - (e - b) / 2;
-    int sb, se, kb, ke;
-    if (vrank < vpeer) {
-      sb = b; se = mid; kb = mid; ke = e;
-    } else {
-      kb = b; ke = mid; sb = mid; se = e;
+    const std::vector<Range> sends = half.Kept(vpeer, s);
+    Arrivals in;
+    in.pieces = half.Kept(vrank, s);
+    in.add = s == 0 ? kSrcSend : kSrcRecv;
+    size_t next_sent = 0;
+    if (s + 1 < exp) {
+      in.forward = next_sent = std::min(half.Kept(vrank ^ (1 << (s + 1)), s + 1).size(), slots);
+      in.forward_to = real_rank(vrank ^ (1 << (s + 1)));
+      in.keep = false;
+    } else if (extra == 0) {
+      // My block is final.  Its way back leads to the same partner: behind what
+      // goes there in this step, into the slots that leaves free.
+      in.final_sum = true;
+      in.forward = first_sent = sends.size() < slots ? std::min(own.size(), slots - sends.size()) : 0;
+      in.forward_to = real_rank(vpeer);
     }
-    bld->Exchange(real_rank(vpeer), ChunksOfBlocks(blocks, sb, se), partial, ChunksOfBlocks(blocks, kb, ke), partial,
-                  s == exp - 1 && extra == 0);
-    partial = kSrcRecv;
-    b = kb;
-    e = ke;
+    bld->Exchange(real_rank(vpeer), sends, sent, s == 0 ? kSrcSend : kSrcRecv, in);
+    sent = next_sent;
   }
   // What the extra ranks contribute to my block arrived while the halving ran.
-  const std::vector<int> own = ChunksOfBlocks(blocks, b, e);
-  for (int x = 0; x < extra; ++x) bld->Exchange(2 * x, none, kSrcNone, own, kSrcRecv, x == extra - 1);
-  for (int x = 0; x < extra; ++x) bld->Exchange(2 * x, own, kSrcRecv, none, kSrcNone, false);
-  for (int s = 0; s < exp; ++s) {
-    const int vpeer = vrank ^ (1 << (exp - 1 - s));
-    const int w = e - b;
-    int rb, re;
-    if (vrank > vpeer) {
-      rb = e; re = e + w;
-    } else {
-      rb = b - w; re = b;
+  for (int x = 0; x < extra; ++x) {
+    Arrivals in;
+    in.pieces = own;
+    in.add = kSrcRecv;
+    if (x == extra - 1) {
+      in.final_sum = true;
+      in.forward = first_sent = std::min(own.size(), slots);
+      in.forward_to = real_rank(half.DoublingPartner(vrank, 0));
     }
-    bld->Exchange(real_rank(vpeer), ChunksOfBlocks(blocks, b, e), kSrcRecv, ChunksOfBlocks(blocks, rb, re), kSrcNone, false);
-    b = std::min(b, rb);
-    e = std::max(e, re);
+    bld->Exchange(2 * x, none, 0, kSrcNone, in);
+  }
+  for (int x = 0; x < extra; ++x) bld->Exchange(2 * x, own, 0, kSrcRecv, Arrivals());
+  // Doubling, with the same forwards: what arrives in a step goes on in the next.
+  sent = first_sent;
+  for (int t = 0; t < exp; ++t) {
+    const int vpeer = half.DoublingPartner(vrank, t);
+    Arrivals in;
+    in.pieces = half.Collected(vpeer, t);
+    if (t + 1 < exp) {
+      in.forward = std::min(in.pieces.size(), slots);
+      in.forward_to = real_rank(half.DoublingPartner(vrank, t + 1));
+    }
+    bld->Exchange(real_rank(vpeer), half.Collected(vrank, t), sent, kSrcRecv, in);
+    sent = in.forward;
   }
 }
 
