@@ -62,3 +62,27 @@ def test_reduce_scatter_and_all_gather_ragged_blocks(ws, offset, staged):
                 assert torch.equal(gathered[r], whole)
                 assert torch.all(guard[r][:offset] == 7) and torch.all(guard[r][offset + m * ws:] == 7)
     world.close()
+
+
+@pytest.mark.parametrize("algo", ["oneshot", "direct", "ring", "rabenseifner"])
+@pytest.mark.parametrize("ws", [2, 3, 5, 8])
+def test_allreduce_ragged_ends(ws, algo):
+    # Lengths around a vector, a round of loads per thread, a stage of the executor and a part on cache lines, all with
+    # a ragged end; slices off the boundary; 16-bit wires where there are op programs.
+    world = ar.EmuWorld(ws)
+    wires = [None, torch.bfloat16] if algo in ("ring", "rabenseifner") else [None]
+    for dtype in (torch.float32, torch.bfloat16, torch.float64):
+        for offset in (0, 1):
+            for n in (ws + 1, 129, 2047, 8 * 512 * ws + 5, 100003):
+                for wire in wires if dtype == torch.float32 else [None]:
+                    ins = [values(n, dtype, n + r, offset) for r in range(ws)]
+                    guard = [torch.full((n + offset + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+                    outs = [g[offset:offset + n] for g in guard]
+                    world.allreduce(ins, outs, algo=algo, scale=1.0 / ws, wire=wire)
+                    want = torch.stack([t.double() for t in ins]).sum(0) / ws
+                    tol = 2e-2 if dtype == torch.bfloat16 or wire is not None else (1e-5 if dtype == torch.float32 else 1e-12)
+                    for g, o in zip(guard, outs):
+                        torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
+                        assert torch.equal(o, outs[0])
+                        assert torch.all(g[:offset] == 7) and torch.all(g[offset + n:] == 7)
+    world.close()
