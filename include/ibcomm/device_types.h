@@ -103,6 +103,8 @@ enum OpFlags : uint8_t {
   // The value is final: round it through the wire type before the local store,
   // so that the owner keeps the same bits every other rank will receive.
   kOpRoundWire = 8,
+  // A later op reads what the local store leaves in recvbuf: it should stay in L2.
+  kOpReadBack = 16,
 };
 
 struct Op {
@@ -221,8 +223,6 @@ struct ExecParams {
   const Op* ops;
   int32_t num_ops;
   int32_t trace_capacity;  // records per channel, 0 = tracing off
-  int32_t stream_recv;     // no op reads recvbuf: its stores need not stay in L2
-  int32_t pad_;
   StageLayout stage;
   uint64_t timeout_ns;   // limit of every wait
   DeviceStatus* status;  // device memory, fetched by the host after a failure

@@ -49,7 +49,6 @@ struct ProgramRequest {
 struct Program {
   std::vector<Op> ops;
   StageLayout stage{};
-  bool reads_recv = false;    // some op has recvbuf as a source
   std::vector<int> in_peers;  // region index -> source rank, for this rank
   // Transfers per peer over the whole program, for tests and credit audits.
   uint32_t sent_to[kMaxRanks] = {0};

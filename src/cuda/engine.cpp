@@ -255,7 +255,6 @@ ExecParams MakeExecParams(const RankResources& rr, const CachedProgram& cp, DTyp
   p.num_ops = static_cast<int32_t>(cp.prog.ops.size());
   p.trace_capacity = trace_capacity;
   p.stage = cp.prog.stage;
-  p.stream_recv = cp.prog.reads_recv ? 0 : 1;
   p.timeout_ns = timeout_ns;
   p.status = rr.d_status;
   p.doorbell = rr.d_doorbell;

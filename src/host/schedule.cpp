@@ -396,9 +396,11 @@ Program BuildProgram(const ProgramRequest& req) {
   for (size_t i = 0; i < bld.prog.ops.size(); ++i) {
     Op& op = bld.prog.ops[i];
     if (op.src_a == kSrcRecv || op.src_b == kSrcRecv) {
-      bld.prog.reads_recv = true;
       const auto it = stored.find(op.cell_begin);
-      if (it != stored.end()) op.wait_local = it->second;
+      if (it != stored.end()) {
+        op.wait_local = it->second;
+        bld.prog.ops[it->second - 1].flags |= kOpReadBack;
+      }
     }
     if (op.flags & kOpStoreLocal) stored[op.cell_begin] = static_cast<uint32_t>(i + 1);
   }
