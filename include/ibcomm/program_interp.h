@@ -25,8 +25,9 @@ struct SimResult {
 template <typename T>
 class ProgramSimulator {
  public:
-  ProgramSimulator(Algo algo, int world_size, size_t stage_bytes, int channels, size_t piece_elems = 0)
-      : algo_(algo), ws_(world_size), stage_bytes_(stage_bytes), nch_(channels), piece_elems_(piece_elems) {}
+  ProgramSimulator(Algo algo, int world_size, size_t stage_bytes, int channels, size_t piece_elems = 0,
+                   std::vector<size_t> segments = {})
+      : algo_(algo), ws_(world_size), stage_bytes_(stage_bytes), nch_(channels), piece_elems_(piece_elems), segments_(std::move(segments)) {}
 
   // inputs[r] is rank r's send buffer; outputs[r] receives its result.
   // `in_place` makes every rank use one buffer for both.
@@ -41,6 +42,7 @@ class ProgramSimulator {
       q.world_size = ws_;
       q.ranges = ranges;
       q.piece_elems = piece_elems_;
+      q.segments = segments_;
       q.wire_elem_bytes = sizeof(T);
       q.stage_bytes = stage_bytes_;
       q.apply_scale = (scale != 1.0);
@@ -143,6 +145,7 @@ class ProgramSimulator {
   size_t stage_bytes_;
   int nch_;
   size_t piece_elems_;
+  std::vector<size_t> segments_;
   std::vector<Program> programs_;
 };
 

@@ -19,7 +19,9 @@
 // move, 5 ranks x 64 MiB on one B200 take 359 us instead of 407.  A piece that goes
 // on to the next step's partner does so in the op that receives (and adds) it, in
 // both directions: the partial sums given away are never stored and read back (8
-// ranks x 64 MiB 634 -> 556 us, 8 x 16 MiB 157 -> 138, 5 x 64 MiB 359 -> 331).
+// ranks x 64 MiB 634 -> 556 us, 8 x 16 MiB 157 -> 138, 5 x 64 MiB 359 -> 331).  The
+// algorithm can run on segments of the message one after the other; ranks on one
+// GPU do, so that what a segment puts down is picked up while it is in L2.
 #pragma once
 
 #include <string>
@@ -40,6 +42,10 @@ struct ProgramRequest {
   // length the run is cut into pieces of that length regardless of chunk
   // boundaries (fewer, larger ops).  Must be the same on every rank.
   size_t piece_elems = 0;
+  // Rabenseifner only: first chunk of every segment, where `ranges` are cells of
+  // piece_elems (SplitSegments).  The algorithm runs on one segment after the
+  // other; empty = the message as one.  The same on every rank.
+  std::vector<size_t> segments;
   size_t wire_elem_bytes = 4;     // element size in staging
   uint64_t stage_offset = 0;      // where the staging area starts in the arena
   uint64_t stage_bytes = 0;       // how large it is
@@ -79,6 +85,9 @@ Program BuildProgram(const ProgramRequest& req);
 // that a ring step moves a useful amount of data (see RingChunksPerRank).
 std::vector<Range> SplitForDevice(size_t len_elements, size_t elem_bytes, size_t world_size,
                                   int64_t env_chunk_bytes, size_t max_chunk_bytes, size_t chunks_per_rank = 4);
+// Rabenseifner in segments: the message as cells of piece_elems, *segments the first
+// one of every segment_pieces of them (the last may have fewer).
+std::vector<Range> SplitSegments(size_t len_elements, size_t piece_elems, size_t segment_pieces, std::vector<size_t>* segments);
 // Chunks per rank of the device ring when IBCOMM_CHUNKSIZE is unset: the
 // reference's 4 (knob IBCOMM_RING_POSITIONS) as long as a chunk then holds at
 // least IBCOMM_RING_MIN_CHUNK bytes (default 16 KiB), fewer (down to one)

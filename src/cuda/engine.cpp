@@ -152,22 +152,25 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   // region and, since one collective runs at a time, in the pool in front of
   // it as well (the two are adjacent in the arena).
   const uint64_t stage_off = layout.pool_offset;
-  // The ranks that share a GPU share its L2 too: a ring whose slots fit into it
-  // together keeps its transfers there (a byte is written to staging and read
-  // back 1.75 times).  Halving and doubling read recvbuf back as well, which
-  // does not fit, and get large pieces instead.
-  const uint64_t stage_bytes = ring ? std::min<uint64_t>(layout.pool_bytes, kSharedGpuStageBytes / static_cast<uint64_t>(ranks_on_gpu > 1 ? ranks_on_gpu : 1))
-                                    : layout.pool_bytes + layout.work_bytes;
+  int raben_div = Tunable("IBCOMM_RABEN_PIECES", 0);
+  const bool asked = raben_div >= 1 && raben_div <= 1024;
+  // Ranks on one GPU run Rabenseifner in segments, unless the pieces are prescribed.
+  const bool segmented = !ring && ranks_on_gpu > 1 && env_chunk <= 0 && !asked;
+  // The ranks that share a GPU share its L2 too: slots that fit into it together
+  // keep the transfers there (a ring writes a byte to staging and reads it back 1.75
+  // times).  Rabenseifner divides its area among a region per partner; with four or
+  // more of them a part of L2 leaves each two slots, and the owners wait for the
+  // extra ranks (5 ranks x 64 MiB 283 us in 128 MiB against 277 in all there is, 6
+  // ranks 417 in 96 MiB against 374; 8 ranks, three regions, 435 against 460).
+  const int regions = NumRegions(algo, world_size);
+  const uint64_t sharers = static_cast<uint64_t>(ranks_on_gpu > 1 ? ranks_on_gpu : 1);
+  uint64_t stage_bytes = ring ? std::min<uint64_t>(layout.pool_bytes, kSharedGpuStageBytes / sharers) : layout.pool_bytes + layout.work_bytes;
+  if (segmented && regions <= 3) stage_bytes = std::min<uint64_t>(stage_bytes, kSharedGpuHalvingBytes / sharers);
   // Knobs that shape the program are part of the key: the ring's chunks per
   // rank and the number of pieces Rabenseifner cuts the message into.
   const size_t ring_cpr = ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size), ranks_on_gpu > 1) : 0;
-  // Ranks on one GPU: four pieces of up to 8 MiB (a hand-over costs what 100 KiB
-  // per channel cost; 5 ranks, 4 / 16 MiB: 45 / 90 us with eight, 44 / 86 with four),
-  // two up to 2 MiB where extra ranks add transfers (3 ranks, 1 MiB: 23 against 28).
-  const bool small_with_extras = (world_size & (world_size - 1)) != 0 && len_elements * esize <= (size_t(2) << 20);
-  int raben_div = Tunable("IBCOMM_RABEN_PIECES", 0);
-  if (raben_div < 1 || raben_div > 1024)
-    raben_div = ranks_on_gpu > 1 ? static_cast<int>(std::min<size_t>(1024, std::max<size_t>(small_with_extras ? 2 : 4, util::ceilDiv(len_elements * esize, size_t(8) << 20)))) : 8;
+  if (segmented) raben_div = 0;
+  else if (!asked) raben_div = 8;
   Key key{static_cast<int>(algo), rank, world_size, len_elements, static_cast<int>(dtype), static_cast<int>(wire),
           env_chunk, apply_scale, stage_off, stage_bytes, ring ? static_cast<int>(ring_cpr) : raben_div};
   auto it = cache_.find(key);
@@ -180,7 +183,6 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
     return hit;
   }
 
-  const int regions = NumRegions(algo, world_size);
   ProgramRequest req;
   req.algo = algo;
   req.rank = rank;
@@ -200,19 +202,37 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
     req.ranges = SplitForDevice(len_elements, esize, static_cast<size_t>(world_size), env_chunk, 0);
     size_t cap = static_cast<size_t>(stage_bytes / (static_cast<uint64_t>(regions) * 2) / wsize) / 32 * 32;
     if (cap < 32) cap = 32;
-    size_t piece = env_chunk > 0 ? static_cast<size_t>(env_chunk) / esize : std::max<size_t>(util::ceilDiv(len_elements, static_cast<size_t>(raben_div)), 16384);
-    if (piece > cap) {
-      static bool warned = false;
-      if (!warned && rank == 0) {
-        warned = true;
-        IBCOMM_WARN("IBCOMM_MEMORY_POOL_PRE_ALLOC + IBCOMM_WORK_GPU_MEMORY_SIZE (%llu bytes) limit Rabenseifner's transfer "
-                    "pieces to %zu bytes instead of %zu; increase them for large messages.\n",
-                    static_cast<unsigned long long>(stage_bytes), cap * wsize, piece * wsize);
+    if (segmented) {
+      // Segments: the transfers and partial sums of one stay in L2.  24 MiB, less
+      // where more ranks share it, more where only two halve (2 ranks x 64 MiB 75 us
+      // with 32 MiB, 80 with 24; 64 MiB per rank, the message as one and in
+      // segments: 4 ranks 240 -> 182 us, 8 ranks 552 -> 435, 5 ranks 325 -> 277), and
+      // one piece per block: an op costs as much as moving 100 KiB per channel does,
+      // and a block of whole pieces leaves no slivers (5 ranks x 4 MiB 45 -> 38 us, 3
+      // x 1 MiB 23 -> 21).  Two from 4 MiB on where only two ranks halve, since each
+      // would wait for the other's only piece (2 ranks x 12 MiB 24.6 -> 22.9).
+      const size_t p = static_cast<size_t>(util::FloorPow2(static_cast<uint64_t>(world_size)));
+      const size_t bytes = len_elements * wsize;
+      const size_t most = std::min<size_t>(std::min<size_t>(size_t(p == 2 ? 32 : 24) << 20, (size_t(128) << 20) / static_cast<size_t>(ranks_on_gpu)), cap * wsize * p);
+      const size_t count = std::max<size_t>(1, util::ceilDiv(bytes, most));
+      const size_t own = p == 2 && bytes / (count * p) > (size_t(4) << 20) ? 2 : 1;
+      req.piece_elems = std::min<size_t>(cap, util::ceilDiv(util::ceilDiv(len_elements, count * p * own), size_t(32)) * 32);
+      req.ranges = SplitSegments(len_elements, req.piece_elems, p * own, &req.segments);
+    } else {
+      size_t piece = env_chunk > 0 ? static_cast<size_t>(env_chunk) / esize : std::max<size_t>(util::ceilDiv(len_elements, static_cast<size_t>(raben_div)), 16384);
+      if (piece > cap) {
+        static bool warned = false;
+        if (!warned && rank == 0) {
+          warned = true;
+          IBCOMM_WARN("IBCOMM_MEMORY_POOL_PRE_ALLOC + IBCOMM_WORK_GPU_MEMORY_SIZE (%llu bytes) limit Rabenseifner's transfer "
+                      "pieces to %zu bytes instead of %zu; increase them for large messages.\n",
+                      static_cast<unsigned long long>(stage_bytes), cap * wsize, piece * wsize);
+        }
+        piece = cap;
       }
-      piece = cap;
+      if (env_chunk <= 0 && piece >= 32) piece = util::ceilDiv(piece, size_t(32)) * 32;
+      req.piece_elems = piece;
     }
-    if (env_chunk <= 0 && piece >= 32) piece = util::ceilDiv(piece, size_t(32)) * 32;
-    req.piece_elems = piece;
   }
   req.wire_elem_bytes = wsize;
   req.stage_offset = stage_off;

@@ -21,6 +21,9 @@ namespace ibcomm {
 // (many small chunks), 64 MiB 1.23 ms, 96 MiB 1.34 ms, 512 MiB 1.87 ms (every
 // transfer goes to HBM and back).
 constexpr uint64_t kSharedGpuStageBytes = 64ull << 20;
+// The same for Rabenseifner where a rank has few partners (64 MiB per rank; in 64,
+// 96 and 128 MiB: 4 ranks 192, 181, 181 us, 8 ranks no room, 435, 437).
+constexpr uint64_t kSharedGpuHalvingBytes = 96ull << 20;
 
 // What a launch needs to know about one rank.
 struct RankResources {

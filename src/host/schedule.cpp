@@ -232,36 +232,29 @@ struct Halving {
   }
 };
 
-void BuildRabenseifner(Builder* bld) {
-  const ProgramRequest& q = bld->req;
-  const int ws = q.world_size, r = q.rank;
+// A segment of the message: chunks [first, second).
+using Segment = std::pair<size_t, size_t>;
+
+// The chunks of every rank of the halving in a segment.
+std::vector<std::vector<int>> SegmentBlocks(const Segment& segment, int p) {
+  std::vector<std::vector<int>> blocks = GetRankToChunk(segment.second - segment.first, static_cast<size_t>(p));
+  for (std::vector<int>& b : blocks)
+    for (int& c : b) c += static_cast<int>(segment.first);
+  return blocks;
+}
+
+// Halving and doubling of one segment.
+void BuildHalvingDoubling(Builder* bld, const Segment& segment) {
+  const int ws = bld->req.world_size, r = bld->req.rank;
   const int p = static_cast<int>(util::FloorPow2(static_cast<uint64_t>(ws)));
   const int extra = ws - p;
   const int exp = util::GetExpOfTwo(static_cast<uint64_t>(p));
   auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
-  const std::vector<std::vector<int>> blocks = GetRankToChunk(q.ranges.size(), static_cast<size_t>(p));
+  const std::vector<std::vector<int>> blocks = SegmentBlocks(segment, p);
   const Halving half{*bld, blocks, p, exp};
   const std::vector<Range> none;
   using Arrivals = Builder::Arrivals;
 
-  if (r < 2 * extra && (r & 1) == 0) {
-    // An extra rank hands every block of its message to the rank that will own
-    // it and gets the results back from there.  Piece by piece over the owners,
-    // so that all of them have something to work on.
-    std::vector<std::vector<Range>> pieces;
-    size_t most = 0;
-    for (int v = 0; v < p; ++v) {
-      pieces.push_back(half.Own(v));
-      most = std::max(most, pieces.back().size());
-    }
-    for (size_t i = 0; i < most; ++i)
-      for (int v = 0; v < p; ++v)
-        if (i < pieces[static_cast<size_t>(v)].size()) bld->Send(pieces[static_cast<size_t>(v)][i], kSrcSend, real_rank(v));
-    for (size_t i = 0; i < most; ++i)
-      for (int v = 0; v < p; ++v)
-        if (i < pieces[static_cast<size_t>(v)].size()) bld->Recv(pieces[static_cast<size_t>(v)][i], real_rank(v), kSrcNone, true, false, -1);
-    return;
-  }
   const int vrank = r < 2 * extra ? r / 2 : r - extra;
   const size_t slots = bld->slots;
 
@@ -319,6 +312,58 @@ void BuildRabenseifner(Builder* bld) {
     bld->Exchange(real_rank(vpeer), half.Collected(vrank, t), sent, kSrcRecv, in);
     sent = in.forward;
   }
+}
+
+// An extra rank hands every block of its message to the rank that will own it and
+// gets the results back from there.  Piece by piece over the owners, so that all of
+// them have something to work on.  It sends a segment ahead of the one it receives
+// if the owners' slots hold one: its sends then wait only for what the owners take
+// in before they return anything of the segment being received (5 ranks x 64 MiB
+// 301 -> 298 us, 6 ranks 395 -> 386).
+void BuildExtraRank(Builder* bld, const std::vector<Segment>& segments) {
+  const int ws = bld->req.world_size;
+  const int p = static_cast<int>(util::FloorPow2(static_cast<uint64_t>(ws)));
+  const int extra = ws - p;
+  auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
+  std::vector<std::vector<std::pair<Range, int>>> moves(segments.size());  // piece and owner
+  std::vector<bool> ahead(segments.size());
+  for (size_t k = 0; k < segments.size(); ++k) {
+    const std::vector<std::vector<int>> blocks = SegmentBlocks(segments[k], p);
+    const Halving half{*bld, blocks, p, util::GetExpOfTwo(static_cast<uint64_t>(p))};
+    std::vector<std::vector<Range>> pieces;
+    size_t most = 0;
+    for (int v = 0; v < p; ++v) {
+      pieces.push_back(half.Own(v));
+      most = std::max(most, pieces.back().size());
+    }
+    ahead[k] = most <= bld->slots;
+    for (size_t i = 0; i < most; ++i)
+      for (int v = 0; v < p; ++v)
+        if (i < pieces[static_cast<size_t>(v)].size()) moves[k].emplace_back(pieces[static_cast<size_t>(v)][i], real_rank(v));
+  }
+  auto send = [&](size_t k) {
+    for (const auto& m : moves[k]) bld->Send(m.first, kSrcSend, m.second);
+  };
+  send(0);
+  for (size_t k = 0; k < segments.size(); ++k) {
+    const bool next = k + 1 < segments.size();
+    if (next && ahead[k + 1]) send(k + 1);
+    for (const auto& m : moves[k]) bld->Recv(m.first, m.second, kSrcNone, true, false, -1);
+    if (next && !ahead[k + 1]) send(k + 1);
+  }
+}
+
+// Segment after segment.  No op of a segment waits for one of a later segment, so
+// what holds for one segment (all slots free when it begins) holds for each.
+void BuildRabenseifner(Builder* bld) {
+  const ProgramRequest& q = bld->req;
+  std::vector<Segment> segments;
+  for (size_t k = 0; k < q.segments.size(); ++k)
+    segments.emplace_back(q.segments[k], k + 1 < q.segments.size() ? q.segments[k + 1] : q.ranges.size());
+  if (segments.empty()) segments.emplace_back(0, q.ranges.size());
+  const int extra = q.world_size - static_cast<int>(util::FloorPow2(static_cast<uint64_t>(q.world_size)));
+  if (q.rank < 2 * extra && (q.rank & 1) == 0) return BuildExtraRank(bld, segments);
+  for (const Segment& g : segments) BuildHalvingDoubling(bld, g);
 }
 
 }  // namespace
@@ -437,6 +482,13 @@ std::vector<Range> SplitForDevice(size_t len_elements, size_t elem_bytes, size_t
       b = e;
     }
   }
+  return out;
+}
+
+std::vector<Range> SplitSegments(size_t len_elements, size_t piece_elems, size_t segment_pieces, std::vector<size_t>* segments) {
+  std::vector<Range> out;
+  for (size_t b = 0; b < len_elements; b += piece_elems) out.emplace_back(b, std::min(len_elements, b + piece_elems));
+  for (size_t c = 0; c < out.size(); c += segment_pieces) segments->push_back(c);
   return out;
 }
 

@@ -13,13 +13,15 @@ using namespace ibcomm;
 
 template <typename T>
 static bool RunCase(Algo algo, int ws, size_t n, int64_t env_chunk, size_t stage_bytes, int nch, bool in_place,
-                    double scale, size_t max_chunk_bytes = 0, size_t piece_elems = 0) {
-  std::vector<Range> ranges = SplitForDevice(n, sizeof(T), static_cast<size_t>(ws), env_chunk, max_chunk_bytes);
+                    double scale, size_t max_chunk_bytes = 0, size_t piece_elems = 0, size_t segment_pieces = 0) {
+  std::vector<size_t> segments;
+  std::vector<Range> ranges = segment_pieces == 0 ? SplitForDevice(n, sizeof(T), static_cast<size_t>(ws), env_chunk, max_chunk_bytes)
+                                                  : SplitSegments(n, piece_elems, segment_pieces, &segments);
   std::vector<std::vector<T>> in(static_cast<size_t>(ws), std::vector<T>(n)), out;
   std::mt19937 gen(static_cast<unsigned>(n * 31 + static_cast<size_t>(ws)));
   for (int r = 0; r < ws; ++r)
     for (size_t i = 0; i < n; ++i) in[static_cast<size_t>(r)][i] = static_cast<T>(static_cast<int>(gen() % 2001) - 1000);
-  ProgramSimulator<T> sim(algo, ws, stage_bytes, nch, piece_elems);
+  ProgramSimulator<T> sim(algo, ws, stage_bytes, nch, piece_elems, segments);
   SimResult res = sim.Run(ranges, in, &out, scale, in_place);
   if (!res.ok) {
     fprintf(stderr, "%s ws=%d n=%zu: %s", AlgoName(algo), ws, n, res.error.c_str());
@@ -108,6 +110,20 @@ MINI_TEST(RabenseifnerMergedPieces) {
         const size_t regions = static_cast<size_t>(NumRegions(Algo::kRabenseifner, ws));
         CHECK_TRUE(RunCase<int>(Algo::kRabenseifner, ws, 50000, 0, 2 * regions * ((piece * 4 + 127) / 128 * 128), nch, true, 1.0, 0, piece));
       }
+}
+
+MINI_TEST(RabenseifnerSegments) {
+  // One, two and many segments, the last one shorter; blocks of one piece and of
+  // several; slots for a segment ahead, and two per region.
+  for (int ws = 2; ws <= 8; ++ws) {
+    const size_t p = ws < 4 ? 2 : ws < 8 ? 4 : 8, regions = static_cast<size_t>(NumRegions(Algo::kRabenseifner, ws));
+    for (size_t piece : {size_t(256), size_t(1024)})
+      for (size_t own : {size_t(1), size_t(3)})
+        for (size_t n : {own * p * piece, 2 * own * p * piece - 5, 20003 + 4 * own * p * piece})
+          for (size_t slots : {size_t(2), 2 * own, 4 * own + 1})
+            for (int nch : {1, 3})
+              CHECK_TRUE(RunCase<int>(Algo::kRabenseifner, ws, n, 0, slots * regions * piece * 4, nch, slots == 2, 1.0, 0, piece, own * p));
+  }
 }
 
 MINI_TEST(EnvChunkSizes) {

@@ -86,3 +86,28 @@ def test_allreduce_ragged_ends(ws, algo):
                         assert torch.equal(o, outs[0])
                         assert torch.all(g[:offset] == 7) and torch.all(g[offset + n:] == 7)
     world.close()
+
+
+@pytest.mark.parametrize("in_place", [False, True])
+@pytest.mark.parametrize("ws", [2, 3, 4, 5, 6, 7, 8])
+def test_rabenseifner_segments(ws, in_place):
+    # A small staging area makes segments of a few pieces: one, an exact number of them, a last one that is shorter
+    # or lacks blocks, and many; partial sums read back from recvbuf.
+    p = 1 << (ws.bit_length() - 1)
+    regions = max(p.bit_length() - 1 + ws - p, p if ws != p else 0)
+    area = 2 * regions * 65536
+    world = ar.EmuWorld(ws, area // 2, area // 2)
+    for wire, size in ((None, 4), (torch.bfloat16, 2)):
+        piece = 65536 // size
+        for n in (p, piece * p, piece * p + 1, 2 * piece * p - 5, 5 * piece * p + piece + 3):
+            if n < 4 * ws:
+                n = 4 * ws
+            ins = [values(n, torch.float32, n + r, 0) for r in range(ws)]
+            want = torch.stack([t.double() for t in ins]).sum(0) / ws
+            outs = ins if in_place else [torch.full_like(t, 7) for t in ins]
+            world.allreduce(ins, outs, algo="rabenseifner", scale=1.0 / ws, wire=wire)
+            tol = 2e-2 if wire is not None else 1e-5
+            for o in outs:
+                torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
+                assert torch.equal(o, outs[0])
+    world.close()
