@@ -37,38 +37,35 @@ struct StagedShape {
   bool split;      // copy roles in blocks of their own
   int buffers;     // windows of each kind
   int blocks;      // reducing blocks per rank (and copying blocks when split)
-  int copy_warps;  // unsplit: warps of the loader and of the storer
   uint64_t window_bytes;
   int load_groups, reduce_groups, store_groups;
 };
 
 // `bytes`: of a rank's message in the wire type; `resident`: blocks of the kernel
 // the GPU holds at once.  Measured on a B200 (the knobs override each choice):
-//  * The windows of all ranks share one L2, and what falls out of it is written
-//    to HBM and read back, while short windows pay a chain of flags for little:
-//    72 MiB in three buffers of each kind (4 ranks x 64 MiB: 170 us; 56 MiB 172,
-//    96 MiB 182, all of the pool 248).
+//  * The windows of all ranks share one L2.  A line leaves it unwritten as soon as its
+//    reader has it (StagedParams::drop_lines), so that windows of 128 MiB together, in
+//    four buffers of each kind, hardly reach HBM: 8 ranks x 32 MiB wrote 531 MB there
+//    and took 209 us in 72 MiB, 299 MB with the lines dropped, 188 us in 128 MiB; 4
+//    ranks x 64 MiB 183 -> 164 us (without dropping 187 and more in larger windows).
 //  * No fence here waits for a link, so the copy roles need no blocks of their
 //    own, and copies by the threads, with their loads rounds deep, beat the copy
 //    engine's (8 x 25 MiB of fp32, bf16 wire: 156 us against 240 split; 4 x 64
 //    MiB: 170 against 200 with bulk copies).
-//  * Five warps load, five store, six reduce; a message of one window has its
-//    roles one after the other and does with four (4 x 4 MiB 19 us against 21).
+//  * Four warps load, four store, eight reduce: 5 ranks x 64 MiB 229 us against 239
+//    with five, 2 x 12 MiB 21 against 23 (but 8 x 64 MiB 368 against 360).
 //  * A block per 16 KiB: with one per 128 KiB a 0.5 MiB message on 5 ranks takes
 //    27 us, with one per 16 KiB 21.
 StagedShape StagedShapeOnOneGpu(uint64_t bytes, int ws, uint64_t staging_bytes, int resident, int channels) {
   StagedShape s;
-  s.buffers = std::max(3, std::min(Tunable("IBCOMM_STAGED_BUFFERS", 3), kStagedMaxBuffers));
-  constexpr uint64_t kL2Bytes = 72ull << 20;
+  s.buffers = std::max(3, std::min(Tunable("IBCOMM_STAGED_BUFFERS", 4), kStagedMaxBuffers));
+  constexpr uint64_t kWindowsBytes = 128ull << 20;
   const uint64_t kinds = static_cast<uint64_t>(2 * s.buffers);
-  const uint64_t room = staging_bytes / kinds / 4096 * 4096;
-  const bool one_window = bytes <= room && bytes * 2 * static_cast<uint64_t>(ws) <= kL2Bytes;
-  s.window_bytes = one_window ? room : std::min(room, kL2Bytes / (kinds * static_cast<uint64_t>(ws)) / 4096 * 4096);
+  s.window_bytes = std::min(staging_bytes / kinds, kWindowsBytes / (kinds * static_cast<uint64_t>(ws))) / 4096 * 4096;
   const int per_rank = std::max(1, resident / ws);
   s.split = Tunable("IBCOMM_STAGED_SPLIT", 0) != 0 && per_rank >= 2;
   const int most = std::min(128, s.split ? per_rank / 2 : per_rank);
   s.blocks = std::max(1, std::min(channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(bytes / (16u << 10), 128)), most));
-  s.copy_warps = one_window ? 4 : 5;
   auto groups = [](const char* knob, int dflt) { return std::max(1, std::min(Tunable(knob, dflt), 4)); };
   s.load_groups = groups("IBCOMM_STAGED_LOAD_GROUPS", 1);
   s.reduce_groups = groups("IBCOMM_STAGED_REDUCE_GROUPS", 2);
@@ -193,7 +190,8 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.wire = static_cast<int32_t>(wire);
       p.use_multimem = 0;
       p.use_tma = (wire == dtype && Tunable("IBCOMM_STAGED_TMA", 0) != 0) ? 1 : 0;
-      p.copy_warps = sh.copy_warps;
+      p.copy_warps = 4;
+      p.drop_lines = p.use_tma == 0 ? 1 : 0;
       p.peers = rr.peers;
       p.sendbuf = sendbufs[static_cast<size_t>(r)];
       p.recvbuf = recvbufs[static_cast<size_t>(r)];

@@ -151,6 +151,7 @@ struct StagedParams {
   // (a group has flag rows of its own).
   int32_t load_groups, reduce_groups, store_groups;
   int32_t copy_warps;  // unsplit, copies by the threads: warps of the loader and of the storer (0: three each)
+  int32_t drop_lines;  // 1: lines of the windows leave L2 unwritten once their reader has them
   int32_t posters;  // split mode: a poster warp per reducer group fences and publishes behind the data warps
 };
 cudaError_t LaunchStagedKernel(const StagedParams* ranks, int n, int blocks, cudaStream_t stream);

@@ -50,6 +50,12 @@
 // rounds in flight (AsyncRounds, twoshot_common.cuh): B200, 4 ranks x 64 MiB 203
 // -> 170 us, 8 x 25 MiB bucket with a bf16 wire 183 -> 156 us.
 //
+// A line of a window has one reader (a shard's reducer, or the storer).  Ranks on one
+// GPU have it drop the line from L2 (`drop_lines`) once its warp holds the data and
+// before the flag that frees the window, which orders the two: what is dead is not
+// written to HBM, half of the staging stores before.  One discard per lane and round;
+// as eight for every eighth lane it cost as much as it gave (8 ranks x 32 MiB 211 us).
+//
 // Synchronisation is per block index across ranks, with rows of the control
 // page (values (call << 32) | window + 1, growing only; group g of a role
 // owns the rows b + g * n, so groups publish independently):
@@ -195,7 +201,7 @@ __device__ __forceinline__ void CastIn(unsigned char* smem, uint4* wire, const u
 }
 
 template <typename T, typename W>
-__device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const uint4* wire, const CopyParts& parts, uint64_t policy, int tid, int nthr) {
+__device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const uint4* wire, const CopyParts& parts, uint64_t policy, bool drop, int tid, int nthr) {
   using A = typename Acc<T>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
@@ -207,7 +213,10 @@ __device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const 
         VecIO<W>::Load(*reinterpret_cast<const uint4*>(slot), acc);
 #pragma unroll
         for (int v = 0; v < VT; ++v) St16Hint(user + vec * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), policy);
-      });
+      },
+      Dropping([&](int, uint64_t vec) {
+        if (drop) DiscardLine(reinterpret_cast<const unsigned char*>(wire + vec));
+      }));
 }
 
 // ---- copies by the bulk copy engine: global -> shared -> global, one thread ----
@@ -497,7 +506,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         }
         FenceProxyAsyncAll();
       } else if (!tma) {
-        CastOut<T, W>(smem, reinterpret_cast<uint4*>(user), reinterpret_cast<const uint4*>(win), parts_of(nv), once, c.tid, c.nthr);
+        CastOut<T, W>(smem, reinterpret_cast<uint4*>(user), reinterpret_cast<const uint4*>(win), parts_of(nv), once, p.drop_lines != 0, c.tid, c.nthr);
       }
       RolePost(c, kRowOutFree, k, SG, base | (k + 1));
       if (role_w != 0 && gtid == 0) trace[2 * role_w + k].t_done = GlobalTimerNs();
@@ -567,9 +576,13 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
           for (int q = 0; q < kR; ++q)
             if (q < ws) St16(to[q] + idx * 16, r);
         };
+        // Vector v of an item is rank v's; this rank's own is the user's.
+        auto drop = [&](int v, uint64_t idx) {
+          if (p.drop_lines != 0 && v < ws && !(kOwnInPlace && v == me)) DiscardLine(p.stage[v] + p.in_off[j] + idx * 16);
+        };
         // Beside bulk-copy rings the shared memory is theirs.
         if (split || !tma)
-          PeerReduce<W, kR>(smem, from, ws, 0, b, e, do_scale, p.scale, store, static_cast<unsigned>(c.tid), static_cast<unsigned>(reduce_threads));
+          PeerReduce<W, kR>(smem, from, ws, 0, b, e, do_scale, p.scale, store, static_cast<unsigned>(c.tid), static_cast<unsigned>(reduce_threads), Dropping(drop));
         else
           PeerReduceGroup<W, kR>(from, ws, 0, b, e, do_scale, p.scale, store, static_cast<unsigned>(c.tid), static_cast<unsigned>(reduce_threads));
       }

@@ -158,14 +158,38 @@ struct RoundCursor {
   __device__ __forceinline__ bool Done(const Ranges& r) const { return q >= r.count(); }
 };
 
+// Drops the 128-byte line at `p` from L2 without writing it back: for lines of the
+// pool whose only reader has them.  It is a write of no particular value, so it goes
+// before the flag that frees the buffer, and takes whole lines.
+__device__ __forceinline__ void DiscardLine(const unsigned char* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 127u) == 0) asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
+}
+struct KeepLines {
+  static constexpr bool kDrops = false;
+  __device__ __forceinline__ void operator()(int, uint64_t) const {}
+};
+template <typename Fn>
+struct DropLines {
+  static constexpr bool kDrops = true;
+  Fn fn;
+  __device__ __forceinline__ void operator()(int v, uint64_t idx) const { fn(v, idx); }
+};
+template <typename Fn>
+__device__ __forceinline__ DropLines<Fn> Dropping(Fn fn) {
+  return DropLines<Fn>{fn};
+}
+
 // Every item of `ranges` over `nthr` threads numbered `tid`, kU items per thread
 // and round, each of kRoundVecs / kU vectors: `issue(item, smem, stride)` starts
 // the loads of one item into slots `smem`, `smem + stride`, ..., `use(item, slots,
 // stride)` consumes it.  `smem`: kRoundSmemPerThread bytes for every thread of the
-// block.  The loads run over the ends of ranges.
-template <int kU, typename Ranges, typename Issue, typename Use>
-__device__ __forceinline__ void AsyncRounds(unsigned char* smem, const Ranges& ranges, unsigned tid, unsigned nthr, Issue issue, Use use) {
+// block.  The loads run over the ends of ranges.  `drop(v, item)` is called for the
+// vectors v of items item .. item + 7 when the warp has them: a round is 32 lines of 8
+// vectors for a warp, one per lane.
+template <int kU, typename Ranges, typename Issue, typename Use, typename Drop = KeepLines>
+__device__ __forceinline__ void AsyncRounds(unsigned char* smem, const Ranges& ranges, unsigned tid, unsigned nthr, Issue issue, Use use, Drop drop = Drop()) {
   constexpr int kV = kRoundVecs / kU;
+  static_assert(kRoundVecs == 8, "a line per lane");
   const uint64_t step = static_cast<uint64_t>(nthr) * kU;
   const uint32_t stride = blockDim.x * 16u, round_bytes = stride * kRoundVecs;
   unsigned char* const mine = smem + threadIdx.x * 16u;
@@ -189,6 +213,12 @@ __device__ __forceinline__ void AsyncRounds(unsigned char* smem, const Ranges& r
   while (!out.Done(ranges)) {
     start();
     CpAsyncWait<kRoundDepth - 1>();
+    if constexpr (Drop::kDrops) {
+      __syncwarp();  // every lane's loads of the round have landed
+      const unsigned lane = threadIdx.x & 31u, chunk = lane / 4;
+      const uint64_t idx = out.base + (tid - lane) + static_cast<uint64_t>(chunk / kV) * nthr + (lane & 3u) * 8;
+      if (idx + 8 <= out.end) drop(static_cast<int>(chunk % kV), idx);
+    }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const uint64_t idx = out.base + tid + static_cast<uint64_t>(u) * nthr;
@@ -201,9 +231,9 @@ __device__ __forceinline__ void AsyncRounds(unsigned char* smem, const Ranges& r
 }
 
 // PeerReduceUnits that way, by `nthr` threads numbered `tid`.
-template <typename T, int kR, typename Store>
+template <typename T, int kR, typename Store, typename Drop = KeepLines>
 __device__ __forceinline__ void PeerReduce(unsigned char* smem, unsigned char* const* peer, int ws, uint64_t off, uint64_t b, uint64_t e,
-                                           bool do_scale, double scale, Store store, unsigned tid, unsigned nthr) {
+                                           bool do_scale, double scale, Store store, unsigned tid, unsigned nthr, Drop drop = Drop()) {
   using A = typename Acc<T>::type;
   constexpr int kVecElems = 16 / static_cast<int>(sizeof(T));
   static_assert(kRoundVecs % kR == 0, "a round holds whole items");
@@ -225,7 +255,8 @@ __device__ __forceinline__ void PeerReduce(unsigned char* smem, unsigned char* c
           for (int k = 0; k < kVecElems; ++k) acc[k] = ScaleAcc<A>(acc[k], scale);
         }
         store(idx, VecIO<T>::Store(acc));
-      });
+      },
+      drop);
 }
 
 // The kernels are compiled per world-size class kR (2, 4 or 8 ranks at most)

@@ -111,3 +111,24 @@ def test_rabenseifner_segments(ws, in_place):
                 torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
                 assert torch.equal(o, outs[0])
     world.close()
+
+
+@pytest.mark.parametrize("wire", [None, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("ws", [2, 3, 5, 8])
+def test_staged_windows_reused(ws, wire):
+    # Windows that are reused many times while their lines are dropped as they are read: parts that end inside a
+    # 128-byte line, parts of whole lines, a short last window; a second call on the same windows.
+    world = ar.EmuWorld(ws, 64 << 10, 64 << 10)
+    world.set_direct_staging(2)
+    for n in (8 * ws, 8 * 1237, 8 * 16384 * ws, 1000000 + 8):
+        for call in range(2):
+            ins = [values(n, torch.float32, n + r + call, 0) for r in range(ws)]
+            before = [t.clone() for t in ins]
+            outs = [torch.full_like(t, 7) for t in ins]
+            world.allreduce(ins, outs, algo="direct", scale=1.0 / ws, wire=wire)
+            want = torch.stack([t.double() for t in ins]).sum(0) / ws
+            tol = 2e-2 if wire is not None else 1e-5
+            for o, i, b in zip(outs, ins, before):
+                torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
+                assert torch.equal(i, b)
+    world.close()
