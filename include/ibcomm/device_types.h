@@ -224,6 +224,8 @@ struct ExecParams {
   int32_t num_ops;
   int32_t trace_capacity;  // records per channel, 0 = tracing off
   StageLayout stage;
+  int32_t drop_lines;    // 1: lines of a staging slot leave L2 unwritten once they are read
+  int32_t pad_;
   uint64_t timeout_ns;   // limit of every wait
   DeviceStatus* status;  // device memory, fetched by the host after a failure
   uint32_t* doorbell;    // host-mapped word a failing kernel sets non-zero

@@ -156,16 +156,19 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   const bool asked = raben_div >= 1 && raben_div <= 1024;
   // Ranks on one GPU run Rabenseifner in segments, unless the pieces are prescribed.
   const bool segmented = !ring && ranks_on_gpu > 1 && env_chunk <= 0 && !asked;
-  // The ranks that share a GPU share its L2 too: slots that fit into it together
-  // keep the transfers there (a ring writes a byte to staging and reads it back 1.75
-  // times).  Rabenseifner divides its area among a region per partner; with four or
-  // more of them a part of L2 leaves each two slots, and the owners wait for the
-  // extra ranks (5 ranks x 64 MiB 283 us in 128 MiB against 277 in all there is, 6
-  // ranks 417 in 96 MiB against 374; 8 ranks, three regions, 435 against 460).
+  // The ranks that share a GPU share its L2 too: a ring whose slots fit into it
+  // together keeps its transfers there (a byte is written to staging and read back
+  // 1.75 times).  Rabenseifner has the lines of its slots dropped from L2 as they are
+  // read, and may then take all the staging there is, where the transfers would not
+  // fit into L2 together and are of the user's type (64 MiB per rank: 5 ranks 283 ->
+  // 267 us, 8 ranks 435 -> 424, 2 ranks 75 -> 71; 8 x 4 MiB 57 -> 59, 8 x 64 MiB with
+  // a bf16 wire 346 -> 364).  Else, with few partners, a part of L2: four regions or
+  // more leave each two slots of it, and the owners wait for the extra ranks.
   const int regions = NumRegions(algo, world_size);
   const uint64_t sharers = static_cast<uint64_t>(ranks_on_gpu > 1 ? ranks_on_gpu : 1);
+  const bool drop_lines = segmented && wsize == esize && sharers * len_elements * wsize >= (48ull << 20);
   uint64_t stage_bytes = ring ? std::min<uint64_t>(layout.pool_bytes, kSharedGpuStageBytes / sharers) : layout.pool_bytes + layout.work_bytes;
-  if (segmented && regions <= 3) stage_bytes = std::min<uint64_t>(stage_bytes, kSharedGpuHalvingBytes / sharers);
+  if (segmented && !drop_lines && regions <= 3) stage_bytes = std::min<uint64_t>(stage_bytes, kSharedGpuHalvingBytes / sharers);
   // Knobs that shape the program are part of the key: the ring's chunks per
   // rank and the number of pieces Rabenseifner cuts the message into.
   const size_t ring_cpr = ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size), ranks_on_gpu > 1) : 0;
@@ -240,6 +243,7 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   req.apply_scale = apply_scale;
   std::unique_ptr<CachedProgram> cp(new CachedProgram());
   cp->prog = BuildProgram(req);
+  cp->drop_lines = drop_lines;
   {
     const std::string bad = ValidateProgram(cp->prog, len_elements, wsize, world_size);
     if (!bad.empty()) IBCOMM_FAIL(INVALID_ARGUMENT, "Internal error: the %s program for %zu elements on %d ranks is out of bounds (%s).\n",
@@ -275,6 +279,7 @@ ExecParams MakeExecParams(const RankResources& rr, const CachedProgram& cp, DTyp
   p.num_ops = static_cast<int32_t>(cp.prog.ops.size());
   p.trace_capacity = trace_capacity;
   p.stage = cp.prog.stage;
+  p.drop_lines = rr.peers.one_gpu != 0 && cp.drop_lines ? 1 : 0;
   p.timeout_ns = timeout_ns;
   p.status = rr.d_status;
   p.doorbell = rr.d_doorbell;

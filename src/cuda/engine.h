@@ -49,6 +49,7 @@ struct StatusBlock {
 
 struct CachedProgram {
   Program prog;
+  bool drop_lines = false;  // ExecParams::drop_lines
   Op* d_ops = nullptr;
   int slab = -1;        // slab that holds d_ops
   bool pinned = false;  // recorded into a CUDA graph: kept for the cache's lifetime

@@ -29,7 +29,10 @@
 // left in series (flags, plan, fence) takes about 1.2 us, and a hand-over
 // between two ranks on one GPU about 3 us.  User data that is touched once goes
 // through L2 as evict-first, so that the staging slots of ranks sharing a GPU
-// stay there (ring 8 x 256 MiB 1.40 -> 1.23 ms).  Ranks sharing a B200, before and
+// stay there (ring 8 x 256 MiB 1.40 -> 1.23 ms).  A slot's line has one reader;
+// with `drop_lines` the data warps drop it from L2 when the stage's copy has landed
+// and before the credit that frees the slot, so that dead data is not written to HBM
+// (not the ring's, whose slots stay in L2: 8 x 256 MiB 1.23 -> 1.26 ms).  Ranks sharing a B200, before and
 // after: Rabenseifner 5 x 64 MiB 908 -> 430 us, ring 8 x 32 MiB 258 -> 192 us,
 // ring 7 x 4 MB 96 -> 70 us, ring 8 x 4 KiB 52 -> 46 us.
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda
@@ -92,6 +95,10 @@ struct ExecTile {
   uint64_t lo, hi;
   const unsigned char* tail_a;  // where the last pack lies in the user's buffers
   const unsigned char* tail_b;
+  // Whole lines of the staging slot that the stage came from, to be dropped from L2.
+  unsigned char* drop;
+  uint32_t drop_lines;
+  uint32_t pad_;
 };
 
 // One op of this channel, worked out by a lane of the loader's warp.
@@ -197,6 +204,7 @@ __device__ __forceinline__ void RunTile(const ExecTile& t, const ExecTile* tile,
       }
     }
   }
+  for (unsigned l = tid; l < t.drop_lines; l += nthr) DiscardLine(t.drop + static_cast<size_t>(l) * 128u);
   // The stage is free for the loader once every warp has read it.
   if (t.tail == 0) {
     __syncwarp();
@@ -442,6 +450,7 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           return true;
         };
         const bool a_staged = (pl.flags & kTileFromStaging) != 0;
+        const bool drop = p.drop_lines != 0;
         const uint64_t a_step = static_cast<uint64_t>(a_staged ? Tr::VW : Tr::VT) * 16u;
         for (uint64_t j = 0; j < pl.packs; j += tile_packs) {
           if (!next_stage()) {
@@ -458,6 +467,13 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           const bool last = j + n >= pl.packs;
           t.flags = pl.flags | (last ? kTileLastOfOp : 0u);
           t.tail = last ? pl.tail : 0;
+          t.drop_lines = 0;
+          if (drop && a_staged) {
+            const uintptr_t at = reinterpret_cast<uintptr_t>(pl.src_a + j * a_step), line = (at + 127u) & ~uintptr_t(127);
+            const uintptr_t end = at + n * a_step;
+            t.drop = reinterpret_cast<unsigned char*>(line);
+            t.drop_lines = end > line ? static_cast<uint32_t>((end - line) / 128u) : 0;
+          }
           const uint32_t whole = n - (t.tail != 0 ? 1u : 0u);
           if (t.tail != 0) {
             t.tail_a = pl.src_a + (j + whole) * Tr::VT * 16u;

@@ -215,7 +215,7 @@ __device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const 
         for (int v = 0; v < VT; ++v) St16Hint(user + vec * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), policy);
       },
       Dropping([&](int, uint64_t vec) {
-        if (drop) DiscardLine(reinterpret_cast<const unsigned char*>(wire + vec));
+        if (drop) DropLine(reinterpret_cast<const unsigned char*>(wire + vec));
       }));
 }
 
@@ -578,7 +578,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         };
         // Vector v of an item is rank v's; this rank's own is the user's.
         auto drop = [&](int v, uint64_t idx) {
-          if (p.drop_lines != 0 && v < ws && !(kOwnInPlace && v == me)) DiscardLine(p.stage[v] + p.in_off[j] + idx * 16);
+          if (p.drop_lines != 0 && v < ws && !(kOwnInPlace && v == me)) DropLine(p.stage[v] + p.in_off[j] + idx * 16);
         };
         // Beside bulk-copy rings the shared memory is theirs.
         if (split || !tma)

@@ -158,11 +158,9 @@ struct RoundCursor {
   __device__ __forceinline__ bool Done(const Ranges& r) const { return q >= r.count(); }
 };
 
-// Drops the 128-byte line at `p` from L2 without writing it back: for lines of the
-// pool whose only reader has them.  It is a write of no particular value, so it goes
-// before the flag that frees the buffer, and takes whole lines.
-__device__ __forceinline__ void DiscardLine(const unsigned char* p) {
-  if ((reinterpret_cast<uintptr_t>(p) & 127u) == 0) asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
+// Where a part may start inside a line.
+__device__ __forceinline__ void DropLine(const unsigned char* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 127u) == 0) DiscardLine(p);
 }
 struct KeepLines {
   static constexpr bool kDrops = false;

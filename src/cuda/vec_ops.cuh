@@ -60,6 +60,12 @@ __device__ __forceinline__ uint64_t PolicyNormal() {
   asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+// Drops the 128-byte line at `p` from L2 without writing it back: for lines of the
+// pool whose only reader has them.  It is a write of no particular value, so it goes
+// before the flag that frees the buffer, and takes whole lines.
+__device__ __forceinline__ void DiscardLine(const unsigned char* p) {
+  asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
+}
 __device__ __forceinline__ void St16Hint(void* p, uint4 v, uint64_t policy) {
   asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1,%2,%3,%4}, %5;" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(policy) : "memory");
 }

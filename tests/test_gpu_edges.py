@@ -132,3 +132,19 @@ def test_staged_windows_reused(ws, wire):
                 torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
                 assert torch.equal(i, b)
     world.close()
+
+
+@pytest.mark.parametrize("ws", [2, 5, 8])
+def test_rabenseifner_drops_lines(ws):
+    # Long enough for slots whose lines are dropped as they are read; a ragged end, in place as well, two calls.
+    world = ar.EmuWorld(ws)
+    n = (52 << 20) // 4 // ws + 7
+    for in_place in (False, True):
+        for call in range(2):
+            ins = [values(n, torch.float32, r + call, 0) for r in range(ws)]
+            want = torch.stack([t.double() for t in ins]).sum(0) / ws
+            outs = ins if in_place else [torch.full_like(t, 7) for t in ins]
+            world.allreduce(ins, outs, algo="rabenseifner", scale=1.0 / ws)
+            for o in outs:
+                torch.testing.assert_close(o.double(), want, rtol=1e-5, atol=1e-5)
+    world.close()
