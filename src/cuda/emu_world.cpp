@@ -44,10 +44,11 @@ struct StagedShape {
 // `bytes`: of a rank's message in the wire type; `resident`: blocks of the kernel
 // the GPU holds at once.  Measured on a B200 (the knobs override each choice):
 //  * The windows of all ranks share one L2.  A line leaves it unwritten as soon as its
-//    reader has it (StagedParams::drop_lines), so that windows of 128 MiB together, in
-//    four buffers of each kind, hardly reach HBM: 8 ranks x 32 MiB wrote 531 MB there
-//    and took 209 us in 72 MiB, 299 MB with the lines dropped, 188 us in 128 MiB; 4
-//    ranks x 64 MiB 183 -> 164 us (without dropping 187 and more in larger windows).
+//    reader has it (StagedParams::drop_lines).  8 ranks x 32 MiB, 268 MB of results:
+//    in 72 MiB 531 MB written to HBM without that and 299 MB with it, in about the
+//    same time (a chain of flags per window binds); in 128 MiB, four buffers of each
+//    kind, fewer chains, 460 MB and 188 us instead of 209.  4 ranks x 64 MiB 183 -> 164
+//    us; without dropping, larger windows take 187 and more.
 //  * No fence here waits for a link, so the copy roles need no blocks of their
 //    own, and copies by the threads, with their loads rounds deep, beat the copy
 //    engine's (8 x 25 MiB of fp32, bf16 wire: 156 us against 240 split; 4 x 64

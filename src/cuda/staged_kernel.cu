@@ -52,8 +52,8 @@
 //
 // A line of a window has one reader (a shard's reducer, or the storer).  Ranks on one
 // GPU have it drop the line from L2 (`drop_lines`) once its warp holds the data and
-// before the flag that frees the window, which orders the two: what is dead is not
-// written to HBM, half of the staging stores before.  One discard per lane and round;
+// before the flag that frees the window, which orders the two: less of what is dead
+// is written to HBM (half of the staging stores before).  One discard per lane and round;
 // as eight for every eighth lane it cost as much as it gave (8 ranks x 32 MiB 211 us).
 //
 // Synchronisation is per block index across ranks, with rows of the control
