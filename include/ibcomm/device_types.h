@@ -135,6 +135,15 @@ struct Op {
   uint32_t pad2_;
 };
 
+// Whether a finished op's flags need a fence between what the op wrote and the
+// flags: a transfer into the peer's slot always, and the credit for a slot whose
+// lines were dropped from L2.  Dropping a line is a write (of no particular
+// value): if it came after the peer's next stores into the slot, they would be
+// gone.  A slot that was only read needs none, its loads are complete.
+IBCOMM_HD inline bool FlagsNeedFence(uint32_t post_out, uint32_t post_credit, bool drop_lines) {
+  return post_out != 0 || (drop_lines && post_credit != 0);
+}
+
 // Geometry of the staging area a program runs in.
 struct StageLayout {
   uint64_t offset;       // byte offset of the area inside the arena

@@ -30,11 +30,12 @@
 // between two ranks on one GPU about 3 us.  User data that is touched once goes
 // through L2 as evict-first, so that the staging slots of ranks sharing a GPU
 // stay there (ring 8 x 256 MiB 1.40 -> 1.23 ms).  A slot's line has one reader;
-// with `drop_lines` the data warps drop it from L2 when the stage's copy has landed
-// and before the credit that frees the slot, so that dead data is not written to HBM
-// (not the ring's, whose slots stay in L2: 8 x 256 MiB 1.23 -> 1.26 ms).  Ranks sharing a B200, before and
-// after: Rabenseifner 5 x 64 MiB 908 -> 430 us, ring 8 x 32 MiB 258 -> 192 us,
-// ring 7 x 4 MB 96 -> 70 us, ring 8 x 4 KiB 52 -> 46 us.
+// with `drop_lines` the data warps drop it from L2 when the stage's copy has landed,
+// and the poster's fence orders that ahead of the credit that frees the slot, so
+// that dead data is not written to HBM (not the ring's, whose slots stay in L2: 8 x
+// 256 MiB 1.23 -> 1.26 ms).  Ranks sharing a B200, before and after:
+// Rabenseifner 5 x 64 MiB 908 -> 430 us, ring 8 x 32 MiB 258 -> 192 us, ring 7 x 4
+// MB 96 -> 70 us, ring 8 x 4 KiB 52 -> 46 us.
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda
 // (ibcomm/allreduce_cuda_impl.h:24-33, 103-299, 470-707).
 //
@@ -683,9 +684,9 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
         unsigned upto = lane < data_warps ? LdAcquireShared(&sync->done[lane]) : 0xffffffffu;
         upto = __reduce_min_sync(0xffffffffu, upto);
         const int until = static_cast<int>(upto) < end ? static_cast<int>(upto) : end;
-        const bool publishes = __any_sync(0xffffffffu, mine >= posted && mine < until && post_out != 0);
+        const bool fence = __any_sync(0xffffffffu, mine >= posted && mine < until && FlagsNeedFence(post_out, post_credit, p.drop_lines != 0));
         __syncwarp();  // what the other lanes acquired is ordered before lane 0's fence
-        if (publishes && lane == 0) FencePeers(p.peers.one_gpu != 0);
+        if (fence && lane == 0) FencePeers(p.peers.one_gpu != 0);
         for (; posted < until; ++posted) {
           const int k = posted - first;
           const uint32_t out = __shfl_sync(0xffffffffu, post_out, k), credit = __shfl_sync(0xffffffffu, post_credit, k);

@@ -126,6 +126,36 @@ MINI_TEST(RabenseifnerSegments) {
   }
 }
 
+MINI_TEST(FlagsBehindWritesNeedAFence) {
+  // Where the lines of a slot are dropped as they are read, freeing the slot comes after a
+  // write too: every op that writes what its flags hand over has a fence before them.
+  for (int ws : {2, 5, 7, 8}) {
+    const size_t p = ws < 4 ? 2 : ws < 8 ? 4 : 8, piece = 1024;
+    std::vector<size_t> segments;
+    ProgramRequest q;
+    q.algo = Algo::kRabenseifner;
+    q.world_size = ws;
+    q.ranges = SplitSegments(6 * p * piece - 5, piece, 2 * p, &segments);
+    q.segments = segments;
+    q.piece_elems = piece;
+    q.stage_bytes = 2 * static_cast<size_t>(NumRegions(q.algo, ws)) * piece * 4;
+    size_t frees_only = 0, reuses = 0;
+    for (int r = 0; r < ws; ++r) {
+      q.rank = r;
+      for (const Op& op : BuildProgram(q).ops) {
+        for (bool drop : {false, true}) {
+          const bool hands_over = op.post_out != 0 && (op.flags & kOpStoreRemote) != 0;
+          const bool frees = op.post_credit != 0 && op.src_a == kSrcStage && drop;
+          CHECK_EQ(FlagsNeedFence(op.post_out, op.post_credit, drop), hands_over || frees);
+        }
+        frees_only += op.post_out == 0 && op.post_credit != 0 ? 1 : 0;
+        reuses += op.wait_credit != 0 ? 1 : 0;
+      }
+    }
+    CHECK_TRUE(frees_only != 0 && reuses != 0);
+  }
+}
+
 MINI_TEST(EnvChunkSizes) {
   for (int64_t chunk : {4, 8, 16, 32, 64, 128})
     CHECK_TRUE(RunCase<int>(Algo::kRing, 4, 256, chunk, size_t(1) << 16, 1, false, 1.0));
