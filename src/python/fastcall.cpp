@@ -54,7 +54,7 @@ int DTypeCode(c10::ScalarType t) {
 }
 
 // The tensor behind `o`; null with an exception set when it is none, has an
-// unsupported type or is not contiguous.
+// unsupported type, is not contiguous or out of the GPU's reach.
 const at::Tensor* Tensor(PyObject* o, int* dtype) {
   if (!THPVariable_Check(o)) {
     PyErr_SetString(PyExc_TypeError, "a torch.Tensor is expected");
@@ -68,6 +68,11 @@ const at::Tensor* Tensor(PyObject* o, int* dtype) {
   const int d = DTypeCode(t.scalar_type());
   if (d < 0) {
     Raise(kNotSupported, (std::string("unsupported dtype ") + c10::toString(t.scalar_type())).c_str());
+    return nullptr;
+  }
+  // A kernel reads and writes it: memory of a GPU, or pinned host memory.
+  if (!t.is_cuda() && !t.is_pinned()) {
+    Raise(kInvalidArgument, "tensors must live on the GPU");
     return nullptr;
   }
   if (dtype != nullptr) *dtype = d;
@@ -164,6 +169,7 @@ PyObject* CopyScale(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (s == nullptr) return nullptr;
   const at::Tensor* d = Tensor(a[1], &dout);
   if (d == nullptr) return nullptr;
+  if (!s->is_cuda()) return Raise(kInvalidArgument, "src must be a CUDA tensor");
   const double scale = PyFloat_AsDouble(a[2]);
   if (PyErr_Occurred()) return nullptr;
   const void* in = s->data_ptr();
