@@ -8,10 +8,13 @@
 // the path of a collective (set-up, messaging, diagnostics) stays in ctypes.
 //
 // The functions raise the package's IbcommError and return None.  The GIL is
-// released around the library call, as ctypes does.
+// released around the library call, as ctypes does.  Tensors without storage, a
+// missing driver and the like are C++ exceptions in torch: the entry points turn
+// them into the Python exceptions torch's own methods raise.
 #include <Python.h>
 
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "ibcomm/c_api.h"
@@ -136,6 +139,7 @@ PyObject* SetError(PyObject*, PyObject* cls) {
 
 // allreduce(handle, send, recv, algo, scale, wire, stream, flags); wire < 0: the tensors' type
 PyObject* Allreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (!WantArgs(n, 8)) return nullptr;
   ibcomm_comm* c;
   if (!ToHandle(a[0], &c)) return nullptr;
@@ -159,10 +163,12 @@ PyObject* Allreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   code = ibcomm_allreduce_cuda(c, algo, d, in, out, len, scale, wire < 0 ? d : wire, stream, flags);
   Py_END_ALLOW_THREADS;
   return Done(code);
+  END_HANDLE_TH_ERRORS
 }
 
 // copy_scale(src, dst, scale)
 PyObject* CopyScale(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (!WantArgs(n, 3)) return nullptr;
   int di, dout;
   const at::Tensor* s = Tensor(a[0], &di);
@@ -181,10 +187,12 @@ PyObject* CopyScale(PyObject*, PyObject* const* a, Py_ssize_t n) {
   code = ibcomm_copy_scale(in, out, len, di, dout, scale, stream);
   Py_END_ALLOW_THREADS;
   return Done(code);
+  END_HANDLE_TH_ERRORS
 }
 
 // emu_allreduce(handle, ranks, sends, recvs, algo, scale, wire, channels, stream, async)
 PyObject* EmuAllreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (!WantArgs(n, 10)) return nullptr;
   ibcomm_emu* w;
   if (!ToHandle(a[0], &w)) return nullptr;
@@ -209,10 +217,12 @@ PyObject* EmuAllreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   code = ibcomm_emu_allreduce(w, algo, d, in, out, len, scale, wire < 0 ? d : wire, channels, stream, async);
   Py_END_ALLOW_THREADS;
   return Done(code);
+  END_HANDLE_TH_ERRORS
 }
 
 // emu_rsag(handle, ranks, all_gather, sends, recvs, scale, channels)
 PyObject* EmuRsAg(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (!WantArgs(n, 7)) return nullptr;
   ibcomm_emu* w;
   if (!ToHandle(a[0], &w)) return nullptr;
@@ -236,6 +246,7 @@ PyObject* EmuRsAg(PyObject*, PyObject* const* a, Py_ssize_t n) {
   code = ibcomm_emu_rsag(w, all_gather, d, in, out, block, scale, channels, stream, 0);
   Py_END_ALLOW_THREADS;
   return Done(code);
+  END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef kMethods[] = {

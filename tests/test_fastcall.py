@@ -33,3 +33,20 @@ def outcome(snippet):
 ])
 def test_host_tensors_are_refused(call):
     assert outcome(call) == "IbcommError [ibcomm error 1] tensors must live on the GPU"
+
+
+FAKE = """from torch._subclasses.fake_tensor import FakeTensorMode
+with FakeTensorMode():
+    t = torch.ones(8, device="cuda")
+    """
+
+
+@pytest.mark.parametrize("call", [
+    "ar.ops.copy_scale(t, t)",
+    "fast.emu_allreduce(0, 2, [t] * 2, [t] * 2, 1, 1.0, -1, 0, None, 0)",
+    "fast.emu_rsag(0, 2, 0, [t] * 2, [t] * 2, 1.0, 0)",
+    "fast.allreduce(0, t, t, 1, 1.0, -1, None, 2)",
+])
+def test_exceptions_of_torch_become_python_exceptions(call):
+    # A tensor that claims to be on the GPU and has no memory; without a driver its stream cannot be had either.
+    assert outcome(FAKE + call).split()[0] in ("RuntimeError", "AcceleratorError", "IbcommError")
