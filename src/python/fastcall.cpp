@@ -104,26 +104,38 @@ bool WantArgs(Py_ssize_t n, Py_ssize_t want) {
   return false;
 }
 
-// Pointers of a sequence of `ranks` tensors; a short sequence leaves nulls, which the library refuses.
-bool Pointers(PyObject* seq, int ranks, void** ptrs, const at::Tensor** first, int* dtype) {
-  PyObject* fast = PySequence_Fast(seq, "a sequence of tensors is expected");
-  if (fast == nullptr) return false;
-  const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast);
-  bool ok = true;
-  if (n > ranks || n == 0) {
-    PyErr_SetString(PyExc_IndexError, "one tensor per rank is expected");
-    ok = false;
+// The tensors of a sequence, one per rank.  It holds on to the sequence: one that
+// makes its items as it is read (the rows of a tensor) has them live no longer
+// than the list they were gathered in.
+struct RankTensors {
+  PyObject* list = nullptr;
+  void* ptr[ibcomm::kMaxRanks] = {};
+  const at::Tensor* first = nullptr;
+  int dtype = 0;  // of the first
+
+  RankTensors() = default;
+  RankTensors(const RankTensors&) = delete;
+  RankTensors& operator=(const RankTensors&) = delete;
+  ~RankTensors() { Py_XDECREF(list); }
+
+  // A short sequence leaves nulls, which the library refuses.
+  bool Read(PyObject* seq, int ranks) {
+    list = PySequence_Fast(seq, "a sequence of tensors is expected");
+    if (list == nullptr) return false;
+    const Py_ssize_t n = PySequence_Fast_GET_SIZE(list);
+    if (n > ranks || n == 0) {
+      PyErr_SetString(PyExc_IndexError, "one tensor per rank is expected");
+      return false;
+    }
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      const at::Tensor* t = Tensor(PySequence_Fast_GET_ITEM(list, i), i == 0 ? &dtype : nullptr);
+      if (t == nullptr) return false;
+      if (i == 0) first = t;
+      ptr[i] = t->data_ptr();
+    }
+    return true;
   }
-  for (Py_ssize_t i = 0; ok && i < n; ++i) {
-    const at::Tensor* t = Tensor(PySequence_Fast_GET_ITEM(fast, i), i == 0 ? dtype : nullptr);
-    ok = t != nullptr;
-    if (!ok) break;
-    ptrs[i] = t->data_ptr();
-    if (i == 0 && first != nullptr) *first = t;
-  }
-  Py_DECREF(fast);
-  return ok;
-}
+};
 
 PyObject* Done(int code) {
   if (code != 0) return RaiseLast(code);
@@ -197,13 +209,10 @@ PyObject* EmuAllreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   ibcomm_emu* w;
   if (!ToHandle(a[0], &w)) return nullptr;
   const int ranks = static_cast<int>(PyLong_AsLong(a[1]));
-  void* in[ibcomm::kMaxRanks] = {};
-  void* out[ibcomm::kMaxRanks] = {};
-  const at::Tensor* first = nullptr;
-  int d = 0;
+  RankTensors in, out;
   if (PyErr_Occurred()) return nullptr;
   if (ranks < 1 || ranks > ibcomm::kMaxRanks) return Raise(kNotSupported, "the number of ranks is out of range");
-  if (!Pointers(a[2], ranks, in, &first, &d) || !Pointers(a[3], ranks, out, nullptr, nullptr)) return nullptr;
+  if (!in.Read(a[2], ranks) || !out.Read(a[3], ranks)) return nullptr;
   const int algo = static_cast<int>(PyLong_AsLong(a[4]));
   const double scale = PyFloat_AsDouble(a[5]);
   const int wire = static_cast<int>(PyLong_AsLong(a[6]));
@@ -211,10 +220,10 @@ PyObject* EmuAllreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int async = static_cast<int>(PyLong_AsLong(a[9]));
   void* stream;
   if (PyErr_Occurred() || !ToStream(a[8], -1, &stream)) return nullptr;
-  const size_t len = static_cast<size_t>(first->numel());
+  const size_t len = static_cast<size_t>(in.first->numel());
   int code;
   Py_BEGIN_ALLOW_THREADS;
-  code = ibcomm_emu_allreduce(w, algo, d, in, out, len, scale, wire < 0 ? d : wire, channels, stream, async);
+  code = ibcomm_emu_allreduce(w, algo, in.dtype, in.ptr, out.ptr, len, scale, wire < 0 ? in.dtype : wire, channels, stream, async);
   Py_END_ALLOW_THREADS;
   return Done(code);
   END_HANDLE_TH_ERRORS
@@ -228,22 +237,18 @@ PyObject* EmuRsAg(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!ToHandle(a[0], &w)) return nullptr;
   const int ranks = static_cast<int>(PyLong_AsLong(a[1]));
   const int all_gather = static_cast<int>(PyLong_AsLong(a[2]));
-  void* in[ibcomm::kMaxRanks] = {};
-  void* out[ibcomm::kMaxRanks] = {};
-  const at::Tensor* first_in = nullptr;
-  const at::Tensor* first_out = nullptr;
-  int d = 0, rd = 0;
+  RankTensors in, out;
   if (PyErr_Occurred()) return nullptr;
   if (ranks < 1 || ranks > ibcomm::kMaxRanks) return Raise(kNotSupported, "the number of ranks is out of range");
-  if (!Pointers(a[3], ranks, in, &first_in, &d) || !Pointers(a[4], ranks, out, &first_out, &rd)) return nullptr;
+  if (!in.Read(a[3], ranks) || !out.Read(a[4], ranks)) return nullptr;
   const double scale = PyFloat_AsDouble(a[5]);
   const int channels = static_cast<int>(PyLong_AsLong(a[6]));
   void* stream;
   if (PyErr_Occurred() || !ToStream(Py_None, -1, &stream)) return nullptr;
-  const size_t block = static_cast<size_t>(all_gather ? first_in->numel() : first_out->numel());
+  const size_t block = static_cast<size_t>((all_gather ? in : out).first->numel());
   int code;
   Py_BEGIN_ALLOW_THREADS;
-  code = ibcomm_emu_rsag(w, all_gather, d, in, out, block, scale, channels, stream, 0);
+  code = ibcomm_emu_rsag(w, all_gather, in.dtype, in.ptr, out.ptr, block, scale, channels, stream, 0);
   Py_END_ALLOW_THREADS;
   return Done(code);
   END_HANDLE_TH_ERRORS

@@ -173,3 +173,19 @@ def test_rabenseifner_drops_lines_of_reused_slots(ws):
                 else:
                     assert torch.equal(o.double(), want)
     world.close()
+
+
+def test_ranks_as_rows_of_one_tensor():
+    # The rows are tensors made while the call reads them.
+    world = ar.EmuWorld(4)
+    x = values(4 * 4096, torch.float32, 1).view(4, 4096)
+    want = x.double().sum(0)
+    y = torch.zeros_like(x)
+    world.allreduce(x, y, algo="oneshot")
+    shards, whole = torch.zeros(4, 1024, device="cuda"), torch.zeros_like(x)
+    world.reduce_scatter(x, shards)
+    world.all_gather(shards, whole)
+    for r in range(4):
+        torch.testing.assert_close(y[r].double(), want, rtol=1e-5, atol=1e-5)
+        torch.testing.assert_close(whole[r].double(), want, rtol=1e-5, atol=1e-5)
+    world.close()
