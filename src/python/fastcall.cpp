@@ -78,9 +78,12 @@ const at::Tensor* Tensor(PyObject* o, int* dtype) {
     Raise(kInvalidArgument, "tensors must live on the GPU");
     return nullptr;
   }
-  if (dtype != nullptr) *dtype = d;
+  *dtype = d;
   return &t;
 }
+
+// Whether a kernel that runs on the GPU of `a` can be given `b` too.
+bool SameGpu(const at::Tensor& a, const at::Tensor& b) { return !a.is_cuda() || !b.is_cuda() || a.device() == b.device(); }
 
 template <typename Handle>
 bool ToHandle(PyObject* o, Handle** h) {
@@ -111,12 +114,16 @@ struct RankTensors {
   PyObject* list = nullptr;
   void* ptr[ibcomm::kMaxRanks] = {};
   const at::Tensor* first = nullptr;
-  int dtype = 0;  // of the first
+  int dtype = 0;
+  int64_t shortest = 0;  // fewest elements of one
 
   RankTensors() = default;
   RankTensors(const RankTensors&) = delete;
   RankTensors& operator=(const RankTensors&) = delete;
   ~RankTensors() { Py_XDECREF(list); }
+
+  // `elements` fit into every tensor, and `o` is of the same type on the same GPU.
+  bool Hold(int64_t elements, const RankTensors& o) const { return shortest >= elements && dtype == o.dtype && SameGpu(*first, *o.first); }
 
   // A short sequence leaves nulls, which the library refuses.
   bool Read(PyObject* seq, int ranks) {
@@ -128,9 +135,15 @@ struct RankTensors {
       return false;
     }
     for (Py_ssize_t i = 0; i < n; ++i) {
-      const at::Tensor* t = Tensor(PySequence_Fast_GET_ITEM(list, i), i == 0 ? &dtype : nullptr);
+      int d;
+      const at::Tensor* t = Tensor(PySequence_Fast_GET_ITEM(list, i), &d);
       if (t == nullptr) return false;
-      if (i == 0) first = t;
+      if (i == 0) first = t, dtype = d, shortest = t->numel();
+      if (d != dtype || !SameGpu(*first, *t)) {
+        Raise(kInvalidArgument, "the ranks' tensors must match in dtype and live on one GPU");
+        return false;
+      }
+      if (t->numel() < shortest) shortest = t->numel();
       ptr[i] = t->data_ptr();
     }
     return true;
@@ -161,6 +174,7 @@ PyObject* Allreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* r = Tensor(a[2], &rd);
   if (r == nullptr) return nullptr;
   if (d != rd || s->numel() != r->numel()) return Raise(kInvalidArgument, "sendbuf and recvbuf must match in dtype and size");
+  if (!SameGpu(*s, *r)) return Raise(kInvalidArgument, "sendbuf and recvbuf must live on the same GPU");
   const int algo = static_cast<int>(PyLong_AsLong(a[3]));
   const double scale = PyFloat_AsDouble(a[4]);
   const int wire = static_cast<int>(PyLong_AsLong(a[5]));
@@ -170,6 +184,7 @@ PyObject* Allreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const void* in = s->data_ptr();
   void* out = r->data_ptr();
   const size_t len = static_cast<size_t>(s->numel());
+  if (len != 0 && (in == nullptr || out == nullptr)) return Raise(kInvalidArgument, "tensors must have memory");
   int code;
   Py_BEGIN_ALLOW_THREADS;
   code = ibcomm_allreduce_cuda(c, algo, d, in, out, len, scale, wire < 0 ? d : wire, stream, flags);
@@ -188,11 +203,13 @@ PyObject* CopyScale(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* d = Tensor(a[1], &dout);
   if (d == nullptr) return nullptr;
   if (!s->is_cuda()) return Raise(kInvalidArgument, "src must be a CUDA tensor");
+  if (d->numel() < s->numel() || !SameGpu(*s, *d)) return Raise(kInvalidArgument, "dst must hold every element of src, on the same GPU");
   const double scale = PyFloat_AsDouble(a[2]);
   if (PyErr_Occurred()) return nullptr;
   const void* in = s->data_ptr();
   void* out = d->data_ptr();
   const size_t len = static_cast<size_t>(s->numel());
+  if (len != 0 && (in == nullptr || out == nullptr)) return Raise(kInvalidArgument, "tensors must have memory");
   void* stream = c10::cuda::getCurrentCUDAStream(s->device().index()).stream();
   int code;
   Py_BEGIN_ALLOW_THREADS;
@@ -213,6 +230,9 @@ PyObject* EmuAllreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   if (ranks < 1 || ranks > ibcomm::kMaxRanks) return Raise(kNotSupported, "the number of ranks is out of range");
   if (!in.Read(a[2], ranks) || !out.Read(a[3], ranks)) return nullptr;
+  const int64_t len = in.first->numel();
+  if (!in.Hold(len, out) || !out.Hold(len, in))
+    return Raise(kInvalidArgument, "every rank's tensors must match in dtype and hold as many elements as the first");
   const int algo = static_cast<int>(PyLong_AsLong(a[4]));
   const double scale = PyFloat_AsDouble(a[5]);
   const int wire = static_cast<int>(PyLong_AsLong(a[6]));
@@ -220,10 +240,9 @@ PyObject* EmuAllreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int async = static_cast<int>(PyLong_AsLong(a[9]));
   void* stream;
   if (PyErr_Occurred() || !ToStream(a[8], -1, &stream)) return nullptr;
-  const size_t len = static_cast<size_t>(in.first->numel());
   int code;
   Py_BEGIN_ALLOW_THREADS;
-  code = ibcomm_emu_allreduce(w, algo, in.dtype, in.ptr, out.ptr, len, scale, wire < 0 ? in.dtype : wire, channels, stream, async);
+  code = ibcomm_emu_allreduce(w, algo, in.dtype, in.ptr, out.ptr, static_cast<size_t>(len), scale, wire < 0 ? in.dtype : wire, channels, stream, async);
   Py_END_ALLOW_THREADS;
   return Done(code);
   END_HANDLE_TH_ERRORS
@@ -241,14 +260,16 @@ PyObject* EmuRsAg(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   if (ranks < 1 || ranks > ibcomm::kMaxRanks) return Raise(kNotSupported, "the number of ranks is out of range");
   if (!in.Read(a[3], ranks) || !out.Read(a[4], ranks)) return nullptr;
+  const int64_t block = (all_gather ? in : out).first->numel();
+  if (!in.Hold(all_gather ? block : block * ranks, out) || !out.Hold(all_gather ? block * ranks : block, in))
+    return Raise(kInvalidArgument, "every rank's tensors must match in dtype and hold a block, or a block per rank");
   const double scale = PyFloat_AsDouble(a[5]);
   const int channels = static_cast<int>(PyLong_AsLong(a[6]));
   void* stream;
   if (PyErr_Occurred() || !ToStream(Py_None, -1, &stream)) return nullptr;
-  const size_t block = static_cast<size_t>((all_gather ? in : out).first->numel());
   int code;
   Py_BEGIN_ALLOW_THREADS;
-  code = ibcomm_emu_rsag(w, all_gather, in.dtype, in.ptr, out.ptr, block, scale, channels, stream, 0);
+  code = ibcomm_emu_rsag(w, all_gather, in.dtype, in.ptr, out.ptr, static_cast<size_t>(block), scale, channels, stream, 0);
   Py_END_ALLOW_THREADS;
   return Done(code);
   END_HANDLE_TH_ERRORS

@@ -189,3 +189,21 @@ def test_ranks_as_rows_of_one_tensor():
         torch.testing.assert_close(y[r].double(), want, rtol=1e-5, atol=1e-5)
         torch.testing.assert_close(whole[r].double(), want, rtol=1e-5, atol=1e-5)
     world.close()
+
+
+def test_longer_and_pinned_outputs():
+    # A prefix of a longer output is written, and memory of the host that the GPU can reach.
+    x = values(1000, torch.float32, 1)
+    y = torch.full((1008,), 7.0, device="cuda")
+    ar.ops.copy_scale(x, y, scale=0.5)
+    assert torch.equal(y[:1000], x * 0.5) and torch.all(y[1000:] == 7)
+    h = torch.zeros(1000, pin_memory=True)
+    ar.ops.copy_scale(x, h, scale=0.5)
+    torch.cuda.synchronize()
+    assert torch.equal(h, (x * 0.5).cpu())
+    world = ar.EmuWorld(2)
+    ins, outs = [x, y], [torch.full((1003,), 7.0, device="cuda") for _ in range(2)]
+    world.allreduce(ins, outs, algo="oneshot")
+    for o in outs:
+        assert torch.equal(o[:1000], x + y[:1000]) and torch.all(o[1000:] == 7)
+    world.close()
