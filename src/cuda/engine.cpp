@@ -167,7 +167,7 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   const int regions = NumRegions(algo, world_size);
   const uint64_t sharers = static_cast<uint64_t>(ranks_on_gpu > 1 ? ranks_on_gpu : 1);
   const bool drop_lines = segmented && wsize == esize && sharers * len_elements * wsize >= (48ull << 20);
-  uint64_t stage_bytes = ring ? std::min<uint64_t>(layout.pool_bytes, kSharedGpuStageBytes / sharers) : layout.pool_bytes + layout.work_bytes;
+  uint64_t stage_bytes = ring ? RingStageBytes(layout.pool_bytes, ranks_on_gpu) : layout.pool_bytes + layout.work_bytes;
   if (segmented && !drop_lines && regions <= 3) stage_bytes = std::min<uint64_t>(stage_bytes, kSharedGpuHalvingBytes / sharers);
   // Knobs that shape the program are part of the key: the ring's chunks per
   // rank and the number of pieces Rabenseifner cuts the message into.

@@ -16,12 +16,8 @@
 
 namespace ibcomm {
 
-// Staging that the ranks on one GPU cycle through together, when several share
-// it.  Eight ranks x 256 MiB, ring, on a B200 (126 MB of L2): 40 MiB 1.39 ms
-// (many small chunks), 64 MiB 1.23 ms, 96 MiB 1.34 ms, 512 MiB 1.87 ms (every
-// transfer goes to HBM and back).
-constexpr uint64_t kSharedGpuStageBytes = 64ull << 20;
-// The same for Rabenseifner where a rank has few partners (64 MiB per rank; in 64,
+// Staging that Rabenseifner's ranks on one GPU cycle through together where a rank
+// has few partners (see kSharedGpuStageBytes; 64 MiB per rank; in 64,
 // 96 and 128 MiB: 4 ranks 192, 181, 181 us, 8 ranks no room, 435, 437).
 constexpr uint64_t kSharedGpuHalvingBytes = 96ull << 20;
 

@@ -492,6 +492,10 @@ std::vector<Range> SplitSegments(size_t len_elements, size_t piece_elems, size_t
   return out;
 }
 
+uint64_t RingStageBytes(uint64_t pool_bytes, int ranks_on_gpu) {
+  return ranks_on_gpu > 1 ? std::min(pool_bytes, kSharedGpuStageBytes / static_cast<uint64_t>(ranks_on_gpu)) : pool_bytes;
+}
+
 size_t RingChunksPerRank(size_t len_elements, size_t elem_bytes, size_t world_size, bool one_gpu) {
   const int positions = Tunable("IBCOMM_RING_POSITIONS", one_gpu ? 2 : 4);
   size_t cpr = positions >= 1 && positions <= 64 ? static_cast<size_t>(positions) : 4;

@@ -156,6 +156,14 @@ MINI_TEST(FlagsBehindWritesNeedAFence) {
   }
 }
 
+MINI_TEST(RingStaging) {
+  // A rank with a GPU of its own stages in its whole pool, however large; ranks on one GPU share.
+  for (uint64_t mib : {1, 64, 65, 1024}) CHECK_EQ(RingStageBytes(mib << 20, 1), mib << 20);
+  CHECK_EQ(RingStageBytes(uint64_t(64) << 20, 8), uint64_t(8) << 20);
+  CHECK_EQ(RingStageBytes(uint64_t(64) << 20, 2), uint64_t(32) << 20);
+  CHECK_EQ(RingStageBytes(uint64_t(1) << 20, 8), uint64_t(1) << 20);
+}
+
 MINI_TEST(EnvChunkSizes) {
   for (int64_t chunk : {4, 8, 16, 32, 64, 128})
     CHECK_TRUE(RunCase<int>(Algo::kRing, 4, 256, chunk, size_t(1) << 16, 1, false, 1.0));
