@@ -88,6 +88,9 @@ std::vector<Range> SplitForDevice(size_t len_elements, size_t elem_bytes, size_t
 // Rabenseifner in segments: the message as cells of piece_elems, *segments the first
 // one of every segment_pieces of them (the last may have fewer).
 std::vector<Range> SplitSegments(size_t len_elements, size_t piece_elems, size_t segment_pieces, std::vector<size_t>* segments);
+// Longest piece of Rabenseifner, in elements of the wire type, of which a region of
+// the staging holds two: a slot is whole 128-byte lines, so a piece is too.
+size_t MaxPieceElems(uint64_t stage_bytes, int regions, size_t wire_elem_bytes);
 // Staging that the ranks on one GPU cycle through together, when several share
 // it.  Eight ranks x 256 MiB, ring, on a B200 (126 MB of L2): 40 MiB 1.39 ms
 // (many small chunks), 64 MiB 1.23 ms, 96 MiB 1.34 ms, 512 MiB 1.87 ms (every

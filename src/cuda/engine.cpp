@@ -203,8 +203,7 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
     // pieces in the largest step; knob IBCOMM_RABEN_PIECES), as far as two
     // slots per partner fit.
     req.ranges = SplitForDevice(len_elements, esize, static_cast<size_t>(world_size), env_chunk, 0);
-    size_t cap = static_cast<size_t>(stage_bytes / (static_cast<uint64_t>(regions) * 2) / wsize) / 32 * 32;
-    if (cap < 32) cap = 32;
+    const size_t cap = MaxPieceElems(stage_bytes, regions, wsize);
     if (segmented) {
       // Segments: the transfers and partial sums of one stay in L2.  24 MiB, less
       // where more ranks share it, more where only two halve (2 ranks x 64 MiB 75 us

@@ -492,6 +492,12 @@ std::vector<Range> SplitSegments(size_t len_elements, size_t piece_elems, size_t
   return out;
 }
 
+size_t MaxPieceElems(uint64_t stage_bytes, int regions, size_t wire_elem_bytes) {
+  const size_t step = std::max<size_t>(32, 128 / wire_elem_bytes);
+  const size_t most = static_cast<size_t>(stage_bytes / (static_cast<uint64_t>(regions) * 2) / wire_elem_bytes) / step * step;
+  return std::max(most, step);
+}
+
 uint64_t RingStageBytes(uint64_t pool_bytes, int ranks_on_gpu) {
   return ranks_on_gpu > 1 ? std::min(pool_bytes, kSharedGpuStageBytes / static_cast<uint64_t>(ranks_on_gpu)) : pool_bytes;
 }

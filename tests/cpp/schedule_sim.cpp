@@ -164,6 +164,24 @@ MINI_TEST(RingStaging) {
   CHECK_EQ(RingStageBytes(uint64_t(1) << 20, 8), uint64_t(1) << 20);
 }
 
+MINI_TEST(LongestPieceLeavesTwoSlots) {
+  // Staging sizes that do not divide evenly among the regions, every element size on the
+  // wire: the longest piece still fits twice into each region.
+  for (int ws = 2; ws <= 8; ++ws)
+    for (size_t stage : {size_t(4096) * 2, size_t(4096) * 3, size_t(128) << 20, (size_t(96) << 20) / 7, (size_t(100) << 20) + 4096, size_t(65536) * 11})
+      for (size_t wire : {size_t(2), size_t(4), size_t(8)}) {
+        ProgramRequest q;
+        q.algo = Algo::kRabenseifner;
+        q.world_size = ws;
+        q.wire_elem_bytes = wire;
+        q.stage_bytes = stage;
+        const int regions = NumRegions(q.algo, ws);
+        q.piece_elems = MaxPieceElems(stage, regions, wire);
+        CHECK_TRUE(PlanStage(q).slots >= 2);
+        CHECK_TRUE((q.piece_elems + 64) * wire * 2 * static_cast<size_t>(regions) + 128 > stage);  // and is not much shorter than it might be
+      }
+}
+
 MINI_TEST(EnvChunkSizes) {
   for (int64_t chunk : {4, 8, 16, 32, 64, 128})
     CHECK_TRUE(RunCase<int>(Algo::kRing, 4, 256, chunk, size_t(1) << 16, 1, false, 1.0));
