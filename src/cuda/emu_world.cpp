@@ -60,6 +60,7 @@ struct StagedShape {
 StagedShape StagedShapeOnOneGpu(uint64_t bytes, int ws, uint64_t staging_bytes, int resident, int channels) {
   StagedShape s;
   s.buffers = std::max(3, std::min(Tunable("IBCOMM_STAGED_BUFFERS", 4), kStagedMaxBuffers));
+  while (s.buffers > 3 && staging_bytes / static_cast<uint64_t>(2 * s.buffers) < 4096) --s.buffers;  // a window is a page at least
   constexpr uint64_t kWindowsBytes = 128ull << 20;
   const uint64_t kinds = static_cast<uint64_t>(2 * s.buffers);
   s.window_bytes = std::min(staging_bytes / kinds, kWindowsBytes / (kinds * static_cast<uint64_t>(ws))) / 4096 * 4096;

@@ -207,3 +207,16 @@ def test_longer_and_pinned_outputs():
     for o in outs:
         assert torch.equal(o[:1000], x + y[:1000]) and torch.all(o[1000:] == 7)
     world.close()
+
+
+@pytest.mark.parametrize("pages", [6, 7, 8])
+def test_staged_in_the_smallest_staging(pages):
+    # Three windows of each kind is the least the kernel works with: six pages of staging.
+    world = ar.EmuWorld(2, (pages - 1) * 4096, 4096)
+    ins = [values(8 * 3001, torch.float32, r) for r in range(2)]
+    outs = [torch.full_like(t, 7) for t in ins]
+    world.allreduce(ins, outs, algo="direct", wire=torch.bfloat16)
+    want = ins[0].double() + ins[1].double()
+    for o in outs:
+        torch.testing.assert_close(o.double(), want, rtol=2e-2, atol=2e-2)
+    world.close()
