@@ -13,15 +13,16 @@
 // recursive doubling in mirror order; every rank-block moves as its pipeline
 // chunks.  World sizes that are not a power of two have extra ranks (0, 2, ...
 // below 2 * (ws - 2^k)) that take no part in the halving: they hand every block
-// of their message to the rank that ends up owning it, which adds it to its own
-// sum, and get the results back from the owners.  Against folding an extra rank
-// into one partner first, which had that partner move 1.5 times what the others
-// move, 5 ranks x 64 MiB on one B200 take 359 us instead of 407.  A piece that goes
-// on to the next step's partner does so in the op that receives (and adds) it, in
-// both directions: the partial sums given away are never stored and read back (8
-// ranks x 64 MiB 634 -> 556 us, 8 x 16 MiB 157 -> 138, 5 x 64 MiB 359 -> 331).  The
-// algorithm can run on segments of the message one after the other; ranks on one
-// GPU do, so that what a segment puts down is picked up while it is in L2.
+// of their message to a rank that adds it early on (a different one for every
+// block), and get the results back from the blocks' owners.  Against folding an
+// extra rank into one partner first, which had that partner move 1.5 times what
+// the others move, 5 ranks x 64 MiB on one B200 take 359 us instead of 407.  A
+// piece that goes on to the next step's partner does so in the op that receives
+// (and adds) it, in both directions: the partial sums given away are never stored
+// and read back (8 ranks x 64 MiB 634 -> 556 us, 8 x 16 MiB 157 -> 138, 5 x 64 MiB
+// 359 -> 331).  The algorithm can run on segments of the message one after the
+// other; ranks on one GPU do, so that what a segment puts down is picked up while
+// it is in L2.
 #pragma once
 
 #include <string>

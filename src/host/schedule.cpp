@@ -2,6 +2,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <functional>
 #include <unordered_map>
 
 #include "ibcomm/tunables.h"
@@ -109,31 +110,53 @@ struct Builder {
     prog.ops.push_back(op);
   }
 
+  // A piece, and the rank of the halving that ends up with it (-1: a run of several
+  // ranks' blocks).
+  struct Piece {
+    Range range;
+    int owner;
+  };
   // What a step receives, in order.  The first `forward` pieces go on to
   // `forward_to` in the same op, and are stored here as well when `keep`; the
   // others always are.
   struct Arrivals {
-    std::vector<Range> pieces;
+    std::vector<Piece> pieces;
     OpSrc add = kSrcNone;
     bool final_sum = false;
     size_t forward = 0;
     int forward_to = -1;
     bool keep = true;
   };
+  // Contributions of extra ranks that this rank adds in a step (see Joiner).
+  struct Joins {
+    std::function<int(const Piece&)> from;  // the extra rank, or -1
+    bool done;                              // they are in recvbuf already
+    int From(const Piece& g) const { return from ? from(g) : -1; }
+  };
   // One exchange step with a single partner: `sends` leave, of which the first
   // `sent` already did (forwarded as they arrived), and `in` arrives.  Sends run at
   // most `slots` ahead of the receives so that neither side can block on credits
   // the other side has not had a chance to return.
-  void Exchange(int peer, const std::vector<Range>& sends, size_t sent, OpSrc send_src, const Arrivals& in) {
+  void Exchange(int peer, const std::vector<Piece>& sends, size_t sent, OpSrc send_src, const Arrivals& in, const Joins& joins = Joins()) {
     size_t si = sent, ri = 0;
-    while (si < sends.size() && si < slots) Send(sends[si++], send_src, peer);
+    auto send = [&]() {
+      const Piece& g = sends[si++];
+      const int from = joins.From(g);
+      if (from >= 0 && !joins.done) Recv(g.range, from, send_src, false, false, peer);
+      else Send(g.range, from >= 0 ? kSrcRecv : send_src, peer);
+    };
+    while (si < sends.size() && si < slots) send();
+    for (const Piece& g : in.pieces)
+      if (joins.From(g) >= 0 && !joins.done) Recv(g.range, joins.From(g), in.add, true, false, -1);
     while (ri < in.pieces.size()) {
+      const Piece& g = in.pieces[ri];
       const bool fwd = ri < in.forward;
-      Recv(in.pieces[ri], peer, in.add, in.keep || !fwd, in.final_sum, fwd ? in.forward_to : -1);
+      const int from = joins.From(g);
+      Recv(g.range, peer, from >= 0 ? kSrcRecv : in.add, in.keep || !fwd, in.final_sum, fwd ? in.forward_to : -1);
       ++ri;
-      if (si < sends.size()) Send(sends[si++], send_src, peer);
+      if (si < sends.size()) send();
     }
-    while (si < sends.size()) Send(sends[si++], send_src, peer);
+    while (si < sends.size()) send();
   }
 };
 
@@ -194,6 +217,7 @@ void BuildRing(Builder* bld) {
 // The halving of `p` ranks (a power of two) over their `blocks`, and the order in
 // which pieces travel so that a piece can be handed on in the op that receives it.
 struct Halving {
+  using Piece = Builder::Piece;
   const Builder& bld;
   const std::vector<std::vector<int>>& blocks;
   int p, exp;
@@ -208,29 +232,51 @@ struct Halving {
     }
     return {b, e};
   }
-  std::vector<Range> Pieces(std::pair<int, int> run) const { return bld.Pieces(ChunksOfBlocks(blocks, run.first, run.second)); }
-  std::vector<Range> Own(int v) const { return Pieces(Run(v, exp)); }
+  std::vector<Piece> Pieces(int v, int steps) const {
+    const std::pair<int, int> run = Run(v, steps);
+    std::vector<Piece> out;
+    for (const Range& g : bld.Pieces(ChunksOfBlocks(blocks, run.first, run.second))) out.push_back({g, run.second - run.first == 1 ? v : -1});
+    return out;
+  }
+  std::vector<Piece> Own(int v) const { return Pieces(v, exp); }
+  size_t LongestOwn() const {
+    size_t most = 0;
+    for (int v = 0; v < p; ++v) most = std::max(most, Own(v).size());
+    return most;
+  }
 
   // What rank `v` receives in step `s`, in order: first what it gives away in
   // step s + 1, as its partner there wants it, then what it keeps.
-  std::vector<Range> Kept(int v, int s) const {
+  std::vector<Piece> Kept(int v, int s) const {
     if (s + 1 == exp) return Own(v);
-    std::vector<Range> out = Kept(v ^ (1 << (s + 1)), s + 1);
-    const std::vector<Range> rest = Pieces(Run(v, s + 2));
+    std::vector<Piece> out = Kept(v ^ (1 << (s + 1)), s + 1);
+    const std::vector<Piece> rest = Pieces(v, s + 2);
     out.insert(out.end(), rest.begin(), rest.end());
     return out;
   }
   int DoublingPartner(int v, int t) const { return v ^ (1 << (exp - 1 - t)); }
   // What rank `v` has collected when step `t` of the doubling begins, in the order
   // it passes it on: what came in last first, since that is handed on on arrival.
-  std::vector<Range> Collected(int v, int t) const {
+  std::vector<Piece> Collected(int v, int t) const {
     if (t == 0) return Own(v);
-    std::vector<Range> out = Collected(DoublingPartner(v, t - 1), t - 1);
-    const std::vector<Range> before = Collected(v, t - 1);
+    std::vector<Piece> out = Collected(DoublingPartner(v, t - 1), t - 1);
+    const std::vector<Piece> before = Collected(v, t - 1);
     out.insert(out.end(), before.begin(), before.end());
     return out;
   }
 };
+
+// The rank of the halving that adds extra rank `x`'s contribution to the block of
+// `owner`.  No sum may get longer before its last additions than where an extra rank is
+// folded into a partner first: with all of them added by the owner after the halving, one
+// by one, 7 ranks' sums of bf16 were 13 % further from the exact ones, 5 ranks' 5 %.
+//   * One extra rank: the owner adds it to the sum of two that the first step leaves.
+//     (Before that step: 5 ranks x 16 MiB 79 us against 76.5, 3 x 16 MiB 53.4 against 52.)
+//   * Two or three: before the halving, to what a rank has of its own, a different rank for
+//     every extra one.  Every rank does so for one block of each, so all have the same to
+//     do.  Against the owner after the halving: 6 ranks x 64 MiB 365 -> 353 us, 7 ranks
+//     475 -> 457; 7 x 64 MiB with a bf16 wire 408 -> 412.
+int Joiner(int owner, int x) { return owner ^ x; }
 
 // A segment of the message: chunks [first, second).
 using Segment = std::pair<size_t, size_t>;
@@ -252,11 +298,32 @@ void BuildHalvingDoubling(Builder* bld, const Segment& segment) {
   auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
   const std::vector<std::vector<int>> blocks = SegmentBlocks(segment, p);
   const Halving half{*bld, blocks, p, exp};
-  const std::vector<Range> none;
+  const std::vector<Builder::Piece> none;
+  using Piece = Builder::Piece;
   using Arrivals = Builder::Arrivals;
 
   const int vrank = r < 2 * extra ? r / 2 : r - extra;
   const size_t slots = bld->slots;
+  // Where there are extra ranks, at most four ranks halve, and every piece is of one
+  // block.  Their contributions are added before step `join_step` (see Joiner), in the op
+  // that sends a piece or ahead of those that add to what is kept.  That relies on an extra
+  // rank getting rid of all it sends; where its blocks do not fit into the slots, it waits
+  // for ranks that have got further, and they for it.  There the contributions come before
+  // all else.
+  Builder::Joins joins{};
+  int join_step = extra > 1 ? 0 : 1;
+  if (extra != 0) {
+    joins.from = [&](const Piece& g) -> int {
+      for (int x = 0; x < extra; ++x)
+        if (Joiner(g.owner, x) == vrank) return 2 * x;
+      return -1;
+    };
+    joins.done = join_step < exp && half.LongestOwn() > slots;
+    if (joins.done) join_step = 0;
+    for (int x = 0; x < extra && joins.done; ++x)
+      for (const Piece& g : half.Own(Joiner(vrank, x))) bld->Recv(g.range, 2 * x, kSrcSend, true, false, -1);
+  }
+  const bool join_last = extra != 0 && join_step == exp;
 
   // Halving.  A partial sum that goes to the next step's partner is forwarded in
   // the op that computes it and not stored, up to the partner's slots: those are
@@ -264,10 +331,10 @@ void BuildHalvingDoubling(Builder* bld, const Segment& segment) {
   // could only return after waiting for one of ours.
   size_t sent = 0;        // of what this step sends, forwarded during the one before
   size_t first_sent = 0;  // of my own block, to the first partner of the doubling
-  const std::vector<Range> own = half.Own(vrank);
+  const std::vector<Piece> own = half.Own(vrank);
   for (int s = 0; s < exp; ++s) {
     const int vpeer = vrank ^ (1 << s);
-    const std::vector<Range> sends = half.Kept(vpeer, s);
+    const std::vector<Piece> sends = half.Kept(vpeer, s);
     Arrivals in;
     in.pieces = half.Kept(vrank, s);
     in.add = s == 0 ? kSrcSend : kSrcRecv;
@@ -276,27 +343,24 @@ void BuildHalvingDoubling(Builder* bld, const Segment& segment) {
       in.forward = next_sent = std::min(half.Kept(vrank ^ (1 << (s + 1)), s + 1).size(), slots);
       in.forward_to = real_rank(vrank ^ (1 << (s + 1)));
       in.keep = false;
-    } else if (extra == 0) {
+    } else if (!join_last) {
       // My block is final.  Its way back leads to the same partner: behind what
       // goes there in this step, into the slots that leaves free.
       in.final_sum = true;
       in.forward = first_sent = sends.size() < slots ? std::min(own.size(), slots - sends.size()) : 0;
       in.forward_to = real_rank(vpeer);
     }
-    bld->Exchange(real_rank(vpeer), sends, sent, s == 0 ? kSrcSend : kSrcRecv, in);
+    bld->Exchange(real_rank(vpeer), sends, sent, s == 0 ? kSrcSend : kSrcRecv, in, s == join_step ? joins : Builder::Joins());
     sent = next_sent;
   }
-  // What the extra ranks contribute to my block arrived while the halving ran.
-  for (int x = 0; x < extra; ++x) {
+  if (join_last) {
     Arrivals in;
     in.pieces = own;
     in.add = kSrcRecv;
-    if (x == extra - 1) {
-      in.final_sum = true;
-      in.forward = first_sent = std::min(own.size(), slots);
-      in.forward_to = real_rank(half.DoublingPartner(vrank, 0));
-    }
-    bld->Exchange(2 * x, none, 0, kSrcNone, in);
+    in.final_sum = true;
+    in.forward = first_sent = std::min(own.size(), slots);
+    in.forward_to = real_rank(half.DoublingPartner(vrank, 0));
+    bld->Exchange(0, none, 0, kSrcNone, in);
   }
   for (int x = 0; x < extra; ++x) bld->Exchange(2 * x, own, 0, kSrcRecv, Arrivals());
   // Doubling, with the same forwards: what arrives in a step goes on in the next.
@@ -314,41 +378,38 @@ void BuildHalvingDoubling(Builder* bld, const Segment& segment) {
   }
 }
 
-// An extra rank hands every block of its message to the rank that will own it and
-// gets the results back from there.  Piece by piece over the owners, so that all of
-// them have something to work on.  It sends a segment ahead of the one it receives
-// if the owners' slots hold one: its sends then wait only for what the owners take
-// in before they return anything of the segment being received (5 ranks x 64 MiB
-// 301 -> 298 us, 6 ranks 395 -> 386).
+// An extra rank hands every block of its message to the rank that adds it (Joiner) and
+// gets the results back from the owners.  Piece by piece over the blocks, so that all of
+// them have something to work on.  It sends a segment ahead of the one it receives if the
+// others' slots hold one: its sends then wait only for what those take in before they
+// return anything of the segment being received (5 ranks x 64 MiB 301 -> 298 us, 6 ranks
+// 395 -> 386).
 void BuildExtraRank(Builder* bld, const std::vector<Segment>& segments) {
-  const int ws = bld->req.world_size;
+  const int ws = bld->req.world_size, x = bld->req.rank / 2;
   const int p = static_cast<int>(util::FloorPow2(static_cast<uint64_t>(ws)));
   const int extra = ws - p;
   auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
-  std::vector<std::vector<std::pair<Range, int>>> moves(segments.size());  // piece and owner
+  std::vector<std::vector<Builder::Piece>> moves(segments.size());
   std::vector<bool> ahead(segments.size());
   for (size_t k = 0; k < segments.size(); ++k) {
     const std::vector<std::vector<int>> blocks = SegmentBlocks(segments[k], p);
     const Halving half{*bld, blocks, p, util::GetExpOfTwo(static_cast<uint64_t>(p))};
-    std::vector<std::vector<Range>> pieces;
-    size_t most = 0;
-    for (int v = 0; v < p; ++v) {
-      pieces.push_back(half.Own(v));
-      most = std::max(most, pieces.back().size());
-    }
+    std::vector<std::vector<Builder::Piece>> pieces;
+    for (int v = 0; v < p; ++v) pieces.push_back(half.Own(v));
+    const size_t most = half.LongestOwn();
     ahead[k] = most <= bld->slots;
     for (size_t i = 0; i < most; ++i)
-      for (int v = 0; v < p; ++v)
-        if (i < pieces[static_cast<size_t>(v)].size()) moves[k].emplace_back(pieces[static_cast<size_t>(v)][i], real_rank(v));
+      for (const std::vector<Builder::Piece>& b : pieces)
+        if (i < b.size()) moves[k].push_back(b[i]);
   }
   auto send = [&](size_t k) {
-    for (const auto& m : moves[k]) bld->Send(m.first, kSrcSend, m.second);
+    for (const Builder::Piece& m : moves[k]) bld->Send(m.range, kSrcSend, real_rank(Joiner(m.owner, x)));
   };
   send(0);
   for (size_t k = 0; k < segments.size(); ++k) {
     const bool next = k + 1 < segments.size();
     if (next && ahead[k + 1]) send(k + 1);
-    for (const auto& m : moves[k]) bld->Recv(m.first, m.second, kSrcNone, true, false, -1);
+    for (const Builder::Piece& m : moves[k]) bld->Recv(m.range, real_rank(m.owner), kSrcNone, true, false, -1);
     if (next && !ahead[k + 1]) send(k + 1);
   }
 }

@@ -126,6 +126,45 @@ MINI_TEST(RabenseifnerSegments) {
   }
 }
 
+// A partial sum as what it costs in precision: every addition rounds a sum of so many
+// terms, and the error of a rounding grows with the sum.
+struct Rounded {
+  int terms = 1, cost = 0;
+  Rounded() = default;
+  explicit Rounded(int) {}
+  Rounded operator*(double) const { return *this; }
+};
+static Rounded operator+(const Rounded& a, const Rounded& b) {
+  Rounded s;
+  s.terms = a.terms + b.terms;
+  s.cost = a.cost + b.cost + s.terms;
+  return s;
+}
+
+MINI_TEST(RabenseifnerRoundsLikeAFold) {
+  // With extra ranks every element's sum is as good as where each extra rank is added to a
+  // partner of its own first: 2 terms there, all terms once per step of the halving.
+  for (int ws = 2; ws <= 8; ++ws) {
+    const int p = ws < 4 ? 2 : ws < 8 ? 4 : 8, exp = util::GetExpOfTwo(static_cast<uint64_t>(p));
+    const size_t n = 3001, piece = 128;
+    for (size_t slots : {size_t(2), size_t(64)})  // contributions of extra ranks before all else, and where they are needed
+      for (bool in_segments : {false, true}) {
+        std::vector<size_t> segments;
+        const std::vector<Range> ranges = in_segments ? SplitSegments(n, piece, 4 * static_cast<size_t>(p), &segments)
+                                                      : SplitForDevice(n, sizeof(Rounded), static_cast<size_t>(ws), 0, 0);
+        const size_t stage = slots * static_cast<size_t>(NumRegions(Algo::kRabenseifner, ws)) * piece * sizeof(Rounded);
+        ProgramSimulator<Rounded> sim(Algo::kRabenseifner, ws, stage, 1, piece, segments);
+        std::vector<std::vector<Rounded>> out;
+        CHECK_TRUE(sim.Run(ranges, std::vector<std::vector<Rounded>>(static_cast<size_t>(ws), std::vector<Rounded>(n)), &out, 1.0, false).ok);
+        int worst = 0, terms = 0;
+        for (const auto& o : out)
+          for (const Rounded& e : o) worst = std::max(worst, e.cost), terms = std::max(terms, std::abs(e.terms - ws));
+        CHECK_EQ(terms, 0);
+        CHECK_EQ(worst, 2 * (ws - p) + exp * ws);
+      }
+  }
+}
+
 MINI_TEST(FlagsBehindWritesNeedAFence) {
   // Where the lines of a slot are dropped as they are read, freeing the slot comes after a
   // write too: every op that writes what its flags hand over has a fence before them.
