@@ -4,8 +4,13 @@
 // slots, credits).  It is the schedule simulator used to validate programs,
 // slot/credit accounting and deadlock freedom without a GPU, and it can be
 // built with -fsanitize=thread to check the flag protocol for data races.
+//
+// Two liberties the device takes are taken to their limit here: what an op reads
+// from recvbuf is loaded as soon as Op::wait_local allows, and what a slot held is
+// gone once it has been read, before the credit that frees it.
 #pragma once
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstring>
@@ -91,7 +96,17 @@ class ProgramSimulator {
         }
         return true;
       };
+      std::vector<std::vector<T>> early(pg.ops.size());        // per op: its slice of recvbuf
+      std::vector<std::vector<size_t>> due(pg.ops.size() + 1);  // by the ops that have to be finished: the ops that may load
+      for (size_t i = 0; i < pg.ops.size(); ++i)
+        if (pg.ops[i].src_a == kSrcRecv || pg.ops[i].src_b == kSrcRecv) due[pg.ops[i].wait_local].push_back(i);
       for (size_t oi = 0; oi < pg.ops.size(); ++oi) {
+        for (size_t i : due[oi]) {
+          const Op& ahead = pg.ops[i];
+          uint64_t b, e;
+          ChannelSlice(ahead.elem_begin - ahead.cell_begin, ahead.elem_count, st.slot_bytes / sizeof(T), nch_, ch, &b, &e);
+          early[i].assign(recvbuf + ahead.cell_begin + b, recvbuf + ahead.cell_begin + e);
+        }
         const Op& op = pg.ops[oi];
         uint64_t lo, hi;
         ChannelSlice(op.elem_begin - op.cell_begin, op.elem_count, st.slot_bytes / sizeof(T), nch_, ch, &lo, &hi);
@@ -102,22 +117,24 @@ class ProgramSimulator {
         if (op.wait_credit != 0 &&
             !wait_for(me.credit[static_cast<size_t>(ch * kMaxRanks + op.peer_out)], op.wait_credit, "credit", oi))
           return;
-        const T* stage_in = nullptr;
+        T* stage_in = nullptr;
         if (op.src_a == kSrcStage)
-          stage_in = reinterpret_cast<const T*>(me.stage.data() + (static_cast<size_t>(op.region_in) * st.slots + op.slot_in) * st.slot_bytes);
+          stage_in = reinterpret_cast<T*>(me.stage.data() + (static_cast<size_t>(op.region_in) * st.slots + op.slot_in) * st.slot_bytes);
         T* stage_out = nullptr;
         if (op.flags & kOpStoreRemote)
           stage_out = reinterpret_cast<T*>(mem[static_cast<size_t>(op.peer_out)].stage.data() +
                                            (static_cast<size_t>(op.region_out) * st.slots + op.slot_out) * st.slot_bytes);
         for (uint64_t k = lo; k < hi; ++k) {
           const uint64_t g = op.cell_begin + k;
-          T v = op.src_a == kSrcStage ? stage_in[k] : (op.src_a == kSrcSend ? sendbuf[g] : recvbuf[g]);
+          T v = op.src_a == kSrcStage ? stage_in[k] : (op.src_a == kSrcSend ? sendbuf[g] : early[oi][k - lo]);
           if (op.src_b == kSrcSend) v = static_cast<T>(v + sendbuf[g]);
-          else if (op.src_b == kSrcRecv) v = static_cast<T>(v + recvbuf[g]);
+          else if (op.src_b == kSrcRecv) v = static_cast<T>(v + early[oi][k - lo]);
           if (op.flags & kOpScale) v = static_cast<T>(v * scale);
           if (op.flags & kOpStoreLocal) recvbuf[g] = v;
           if (stage_out != nullptr) stage_out[k] = v;
         }
+        if (stage_in != nullptr) std::fill(stage_in + lo, stage_in + hi, T(-99));
+        early[oi] = std::vector<T>();
         if (op.post_out != 0)
           mem[static_cast<size_t>(op.peer_out)].inflag[static_cast<size_t>(ch * kMaxRanks + r)].store(op.post_out, std::memory_order_release);
         if (op.post_credit != 0)
