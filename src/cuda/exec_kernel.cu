@@ -42,10 +42,7 @@
 // The grid is (channels, ranks): blockIdx.y selects the rank whose parameters
 // to use, so that several ranks that share one GPU run as ONE cooperative
 // launch (CTAs that wait on each other are co-resident).
-#include <cooperative_groups.h>
-
 #include <algorithm>
-#include <cstdlib>
 
 #include "flags.cuh"
 #include "ibcomm/communicator.h"

@@ -120,9 +120,7 @@ __device__ inline bool WaitGE(const uint64_t* flag, uint64_t target, const WaitC
   const uint64_t* abort_word = &Ctl(*w.peers, w.rank)->abort_seq;
   for (uint32_t spin = 1;; ++spin) {
     v = LdAcquirePeers(flag, one_gpu);
-    if (v >= target) {
-          return true;
-    }
+    if (v >= target) return true;
     if ((spin & 31u) == 0u) {
       if (LdRelaxedSys(abort_word) == w.seq) {
         ReportFailure(w, kStatusPeerAbort, kind, peer, op_index, target, v);

@@ -15,8 +15,6 @@
 // the split has to be tuned on the machine.  Zero-copy only; the element
 // types of the switch path (fp32, fp16, bf16).  The reference has no
 // counterpart (no intra-node path, README.md:66).
-#include <cooperative_groups.h>
-
 #include "flags.cuh"
 #include "ibcomm/communicator.h"
 #include "kernels.h"

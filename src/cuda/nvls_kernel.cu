@@ -19,9 +19,6 @@
 // several ranks on one GPU), moves 2*S*(ws-1)/ws per direction like the ring
 // but in two synchronisation steps instead of 2*(ws-1), and supports every
 // element type.
-#include <cooperative_groups.h>
-
-#include <cstdlib>
 
 #include "flags.cuh"
 #include "ibcomm/communicator.h"

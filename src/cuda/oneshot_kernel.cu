@@ -9,8 +9,6 @@
 // consecutive calls need no exit barrier: a peer can only reach call k+2 after
 // it consumed this rank's data of call k+1, which this rank sent after it had
 // finished reading call k.
-#include <cooperative_groups.h>
-
 #include "flags.cuh"
 #include "ibcomm/communicator.h"
 #include "kernels.h"

@@ -26,8 +26,6 @@
 // accessed element by element where it has to be.  Blocks of an odd length moved
 // one element at a time took 311 us to scatter and 278 us to gather (8 ranks x 16
 // MiB of bf16 on one B200); by units 58 and 54 us.
-#include <cooperative_groups.h>
-
 #include "flags.cuh"
 #include "ibcomm/communicator.h"
 #include "kernels.h"

@@ -57,11 +57,7 @@ __device__ __forceinline__ void BulkLoadHint(void* smem_dst, const void* gmem_sr
                "l"(gmem_src), "r"(bytes), "r"(SmemAddr(bar)), "l"(policy)
                : "memory");
 }
-// shared -> global, as part of the thread's current bulk group.
-__device__ __forceinline__ void BulkStore(void* gmem_dst, const void* smem_src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(SmemAddr(smem_src)), "r"(bytes)
-               : "memory");
-}
+// shared -> global with a cache policy for L2, as part of the thread's current bulk group.
 __device__ __forceinline__ void BulkStoreHint(void* gmem_dst, const void* smem_src, uint32_t bytes, uint64_t policy) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(gmem_dst), "r"(SmemAddr(smem_src)), "r"(bytes),
                "l"(policy)
@@ -79,7 +75,6 @@ __device__ __forceinline__ void BulkWaitAll() { asm volatile("cp.async.bulk.wait
 // those of other GPUs that a flag made visible) against accesses through the
 // asynchronous proxy (the bulk copies), in both directions.
 __device__ __forceinline__ void FenceProxyAsyncAll() { asm volatile("fence.proxy.async;" ::: "memory"); }
-__device__ __forceinline__ void FenceProxyAsyncShared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 }  // namespace dev
 }  // namespace ibcomm

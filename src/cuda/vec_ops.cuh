@@ -69,11 +69,6 @@ __device__ __forceinline__ void DiscardLine(const unsigned char* p) {
 __device__ __forceinline__ void St16Hint(void* p, uint4 v, uint64_t policy) {
   asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1,%2,%3,%4}, %5;" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(policy) : "memory");
 }
-__device__ __forceinline__ uint4 Ld16Hint(const void* p, uint64_t policy) {
-  uint4 v;
-  asm volatile("ld.global.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy) : "memory");
-  return v;
-}
 // 32 bytes from / to a 32-byte boundary in one access (sm_100).
 __device__ __forceinline__ void Ld32(const void* p, uint4* lo, uint4* hi) {
   asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"

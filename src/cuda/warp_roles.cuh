@@ -40,9 +40,6 @@ __device__ __forceinline__ unsigned LdAcquireShared(const unsigned* p) {
 __device__ __forceinline__ void StReleaseShared(unsigned* p, unsigned v) {
   asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(SmemU32(p)), "r"(v) : "memory");
 }
-__device__ __forceinline__ void AddReleaseShared(unsigned* p, unsigned v) {
-  asm volatile("red.release.cta.shared.add.u32 [%0], %1;" ::"r"(SmemU32(p)), "r"(v) : "memory");
-}
 
 // Spins until *counter >= target.  False when the call was stopped, or after
 // twice the wait limit (a safety net: the waiter's own limit fires first).
@@ -57,13 +54,6 @@ __device__ __forceinline__ bool SpinShared(const unsigned* counter, unsigned tar
       return false;
     }
   }
-}
-
-// Spins until every one of the `warps` data warps has finished `target` steps.
-__device__ __forceinline__ bool SpinAllWarpsDone(RoleSync* sync, int warps, unsigned target, uint64_t timeout_ns) {
-  for (int w = 0; w < warps; ++w)
-    if (!SpinShared(&sync->done[w], target, sync, timeout_ns)) return false;
-  return true;
 }
 
 }  // namespace dev
