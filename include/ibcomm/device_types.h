@@ -178,8 +178,9 @@ IBCOMM_HD inline void ChannelSlice(uint64_t first, uint64_t count, uint64_t slot
 // ---- how the two-shot kernels split a staging window among ranks and CTAs ----
 // [*b, *e) = part `part` of `parts` of the range [lo, hi).  Parts of 16 or more
 // times kPartAlign start on multiples of it from `lo` (512 bytes when the unit
-// is a 16-byte vector), so that a warp's accesses cover whole cache lines; the
-// last part is up to a sixteenth shorter than the others for it.
+// is a 16-byte vector), so that a warp's accesses cover whole cache lines.  Up to a
+// sixteenth of the range shifts to the front for it: of many parts the last ones
+// may be short or empty.
 constexpr uint64_t kPartAlign = 32;
 IBCOMM_HD inline void SubRange(uint64_t lo, uint64_t hi, int part, int parts, uint64_t* b, uint64_t* e) {
   const uint64_t len = hi - lo;

@@ -93,9 +93,9 @@ std::vector<Range> SplitSegments(size_t len_elements, size_t piece_elems, size_t
 // the staging holds two: a slot is whole 128-byte lines, so a piece is too.
 size_t MaxPieceElems(uint64_t stage_bytes, int regions, size_t wire_elem_bytes);
 // Staging that the ranks on one GPU cycle through together, when several share
-// it.  Eight ranks x 256 MiB, ring, on a B200 (126 MB of L2): 40 MiB 1.39 ms
-// (many small chunks), 64 MiB 1.23 ms, 96 MiB 1.34 ms, 512 MiB 1.87 ms (every
-// transfer goes to HBM and back).
+// it.  Eight ranks x 256 MiB, ring, on a B200 (126 MB of L2), called in a loop: 40
+// MiB 1.36 ms (many small chunks), 64 MiB 1.23 ms, 96 MiB 1.33 ms, 512 MiB 1.87 ms
+// (every transfer goes to HBM and back); 8 x 32 MiB 201, 166, 172, 173 us.
 constexpr uint64_t kSharedGpuStageBytes = 64ull << 20;
 // Staging a ring program uses of a rank's pool: all of it, or its share of the above
 // where several ranks are on its GPU.

@@ -160,10 +160,15 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   // together keeps its transfers there (a byte is written to staging and read back
   // 1.75 times).  Rabenseifner has the lines of its slots dropped from L2 as they are
   // read, and may then take all the staging there is, where the transfers would not
-  // fit into L2 together and are of the user's type (64 MiB per rank: 5 ranks 283 ->
-  // 267 us, 8 ranks 435 -> 424, 2 ranks 75 -> 71; 8 x 4 MiB 57 -> 59, 8 x 64 MiB with
-  // a bf16 wire 346 -> 364).  Else, with few partners, a part of L2: four regions or
-  // more leave each two slots of it, and the owners wait for the extra ranks.
+  // fit into L2 together and are of the user's type (8 x 64 MiB with a bf16 wire 346 us
+  // without, 364 with).  How many times as fast that is, by the bytes of all ranks:
+  //   ranks      2     3     4     5     6     7     8
+  //   48 MiB   0.98  1.00  1.02  1.00  0.98  1.00  0.99
+  //   64 MiB   1.02  1.15  1.00  1.05  1.01  1.00  0.99
+  //   96 MiB   1.08  1.05  0.98  1.04  1.03  1.03  1.06
+  //   256 MiB  1.08  1.10  0.99  1.03  1.07  1.05  1.03
+  // Else, with few partners, a part of L2: four regions or more leave each two slots of
+  // it, and the others wait for the extra ranks.
   const int regions = NumRegions(algo, world_size);
   const uint64_t sharers = static_cast<uint64_t>(ranks_on_gpu > 1 ? ranks_on_gpu : 1);
   const bool drop_lines = segmented && wsize == esize && sharers * len_elements * wsize >= (48ull << 20);

@@ -17,8 +17,8 @@
 namespace ibcomm {
 
 // Staging that Rabenseifner's ranks on one GPU cycle through together where a rank
-// has few partners (see kSharedGpuStageBytes; 64 MiB per rank; in 64,
-// 96 and 128 MiB: 4 ranks 192, 181, 181 us, 8 ranks no room, 435, 437).
+// has few partners (see kSharedGpuStageBytes; 64 MiB per rank, in 64, 96 and 128
+// MiB: 4 ranks 192, 181, 181 us, 8 ranks no room, 435, 437).
 constexpr uint64_t kSharedGpuHalvingBytes = 96ull << 20;
 
 // What a launch needs to know about one rank.

@@ -2,7 +2,7 @@
 //
 // One CTA per channel.  A CTA walks the rank's program; for every op it waits
 // (bounded) for the peer's data flag and for slot credit, streams its slice of
-// the chunk through registers as 16-byte vectors
+// the chunk through shared memory and, as 16-byte vectors, registers
 //     staging slot / sendbuf / recvbuf  (+ sendbuf|recvbuf) (* scale) (cast)
 //         -> recvbuf and/or the next peer's staging slot over NVLink,
 // then publishes the data flag to the receiver and returns the credit to the
@@ -29,11 +29,12 @@
 // left in series (flags, plan, fence) takes about 1.2 us, and a hand-over
 // between two ranks on one GPU about 3 us.  User data that is touched once goes
 // through L2 as evict-first, so that the staging slots of ranks sharing a GPU
-// stay there (ring 8 x 256 MiB 1.40 -> 1.23 ms).  A slot's line has one reader;
+// stay there (ring 8 x 256 MiB 1.38 -> 1.23 ms, called in a loop; 1.30-1.38 with other
+// work between the calls).  A slot's line has one reader;
 // with `drop_lines` the data warps drop it from L2 when the stage's copy has landed,
 // and the poster's fence orders that ahead of the credit that frees the slot, so
 // that dead data is not written to HBM (not the ring's, whose slots stay in L2: 8 x
-// 256 MiB 1.23 -> 1.26 ms).  Ranks sharing a B200, before and after:
+// 256 MiB 1.23 -> 1.25 ms).  Ranks sharing a B200, before and after:
 // Rabenseifner 5 x 64 MiB 908 -> 430 us, ring 8 x 32 MiB 258 -> 192 us, ring 7 x 4
 // MB 96 -> 70 us, ring 8 x 4 KiB 52 -> 46 us.
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda

@@ -113,9 +113,9 @@ cudaError_t LaunchHybridKernel(const HybridParams& h, int blocks, cudaStream_t s
 // ---- pipelined staged two-shot (staged_kernel.cu) ----
 // For buffers the peers cannot map, and for fp32 buffers that travel as
 // bf16/fp16: the message moves through the pool in windows, and inside one
-// CTA four warp groups work on up to four windows at the same time (copy in /
-// two reducers over NVLink / copy out), three buffers of each kind.  At most
-// 128 CTAs.
+// CTA groups of warps work on several windows at the same time (copy in / two
+// reducers over NVLink / copy out), with three to six buffers of each kind; or the
+// roles are split over blocks.  At most 128 CTAs that reduce.
 constexpr int kStagedMaxBuffers = 6;
 struct StagedParams {
   int32_t rank;

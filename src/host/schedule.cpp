@@ -468,7 +468,6 @@ StageLayout PlanStage(const ProgramRequest& req) {
   StageLayout st{};
   st.offset = req.stage_offset;
   st.regions = static_cast<uint32_t>(NumRegions(req.algo, req.world_size));
-  // +16 so that a slice may start at the same 16-byte phase as the user data.
   const bool pieces = req.algo == Algo::kRabenseifner && req.piece_elems != 0;
   uint64_t bytes = (pieces ? req.piece_elems : MaxChunkElems(req.ranges)) * req.wire_elem_bytes;
   st.slot_bytes = (bytes + 127) & ~uint64_t(127);
