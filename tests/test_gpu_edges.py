@@ -175,6 +175,30 @@ def test_rabenseifner_drops_lines_of_reused_slots(ws):
     world.close()
 
 
+@pytest.mark.parametrize("ws", [3, 5, 6, 7])
+def test_rabenseifner_blocks_longer_than_the_slots(ws):
+    # The message as one, in small pieces of which the slots hold a few: what the extra ranks contribute comes before
+    # all else then.  In place as well.
+    lib = ar._native.lib()
+    lib.ibcomm_set_tunable(b"IBCOMM_RABEN_PIECES", 64)
+    try:
+        world = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+        for dtype in (torch.float32, torch.bfloat16):
+            n = 64 * 16384 + 5
+            for in_place in (False, True):
+                ins = [values(n, dtype, n + r) for r in range(ws)]
+                want = torch.stack([t.double() for t in ins]).sum(0) / ws
+                outs = ins if in_place else [torch.full_like(t, 7) for t in ins]
+                world.allreduce(ins, outs, algo="rabenseifner", scale=1.0 / ws)
+                tol = 2e-2 if dtype == torch.bfloat16 else 1e-5
+                for o in outs:
+                    torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
+                    assert torch.equal(o, outs[0])
+        world.close()
+    finally:
+        lib.ibcomm_set_tunable(b"IBCOMM_RABEN_PIECES", -1)
+
+
 def test_ranks_as_rows_of_one_tensor():
     # The rows are tensors made while the call reads them.
     world = ar.EmuWorld(4)
