@@ -57,6 +57,7 @@ CUDA_SOURCES = [
     "src/cuda/nvls_kernel.cu",
     "src/cuda/oneshot_kernel.cu",
     "src/cuda/rsag_kernel.cu",
+    "src/cuda/local_kernel.cu",
     "src/cuda/hybrid_kernel.cu",
     "src/cuda/staged_kernel.cu",
     "src/cuda/copy_kernel.cu",

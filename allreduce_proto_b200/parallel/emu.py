@@ -1,6 +1,6 @@
 """Several ranks on one GPU (``ibcomm::EmuWorld``): every collective is one
-cooperative kernel launch that covers all ranks, so the real kernels, programs
-and flag protocol can be exercised on a single-GPU machine."""
+kernel launch that covers all ranks.  The kernels, programs and flag protocol of
+ranks with a GPU each can be exercised on a single-GPU machine."""
 from __future__ import annotations
 
 import ctypes as C
@@ -64,8 +64,9 @@ class EmuWorld:
         check(_native.lib().ibcomm_emu_set_bad_program_rank(self._h, rank))
 
     def set_direct_staging(self, mode) -> None:
-        """Direct algorithm: 0/False in place, 1/True staged through the pool windows one phase after the other,
-        2 staged through the pipelined kernel (needs 16-byte aligned buffers of whole 16-byte vectors)."""
+        """Direct algorithm: 0/False in place (one kernel for all ranks), 1/True staged through the pool windows one phase
+        after the other, 2 staged through the pipelined kernel (needs 16-byte aligned buffers of whole 16-byte vectors),
+        3 in place with the kernels and barriers of ranks that have a GPU each."""
         check(_native.lib().ibcomm_emu_set_direct_staging(self._h, int(mode)))
 
     @property

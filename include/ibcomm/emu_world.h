@@ -1,10 +1,11 @@
 // Several ranks on ONE GPU, for tests and for machines with fewer GPUs than
 // ranks.  Kernels of different ranks wait on each other, and nothing
 // guarantees that separate launches on one GPU run at the same time, so here
-// every collective is a single cooperative launch whose grid covers all
-// ranks (blockIdx.y = rank).  The kernels, programs, flag protocol and
-// staging layout are exactly the ones the multi-GPU path uses; only the
-// "peer" pointers are local.
+// every collective is a single launch that covers all ranks.  Where ranks
+// exchange anything through staging it is cooperative (blockIdx.y = rank), and
+// the kernels, flag protocol and staging layout are the ones the multi-GPU path
+// uses; only the "peer" pointers are local.  The direct algorithm on buffers in
+// place has a kernel of its own, since nothing has to be exchanged.
 #pragma once
 
 #include <memory>
@@ -52,8 +53,10 @@ class EmuWorld {
   // the bounds check before any memory is touched; the rank reports "bad
   // program", the others are told to stop.  -1 restores normal operation.
   void SetBadProgramRank(int r);
-  // How the direct algorithm treats the buffers: 0 in place, 1 staged through
-  // the pool window by window (as for buffers the peers cannot map).
+  // How the direct algorithm treats the buffers: 0 in place, with one kernel for
+  // all ranks; 1 staged through the pool window by window (as for buffers the
+  // peers cannot map), 2 staged through the pipelined kernel; 3 in place, with
+  // the kernels and barriers of ranks that have a GPU each.
   void SetDirectStaging(int mode);
   int last_channels() const;
 

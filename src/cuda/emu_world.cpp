@@ -24,7 +24,9 @@ struct EmuWorld::Impl {
   int last_channels = 0;
   int silent_rank = -1;
   int bad_program_rank = -1;
-  int direct_staging = 0;  // 0 in place, 1 staged window by window, 2 staged through the pipelined kernel
+  // 0 in place, by one kernel for all ranks; 1 staged window by window, 2 staged through the pipelined kernel, 3 in
+  // place, by the kernel ranks with a GPU each run.
+  int direct_staging = 0;
   int staged_max_blocks = 0;
   uint32_t last_status = 0;
   DeviceStatus last_report{};
@@ -170,16 +172,37 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
   const uint64_t timeout_ns = static_cast<uint64_t>(m.timeout_ms) * 1000000ull;
   const int cap = std::max(1, m.max_blocks / m.ws);
 
+  LocalParams local{};
+  local.op = LocalOp::kAllreduce;
+  local.world_size = m.ws;
+  local.dtype = static_cast<int32_t>(dtype);
+  local.wire = static_cast<int32_t>(wire);
+  for (int q = 0; q < m.ws; ++q) {
+    local.in[q] = sendbufs[static_cast<size_t>(q)];
+    local.out[q] = recvbufs[static_cast<size_t>(q)];
+  }
+  local.len_elements = n;
+  local.scale = scale;
+
   bool all_aligned = true;
   for (int q = 0; q < m.ws; ++q)
     all_aligned = all_aligned && ((reinterpret_cast<uintptr_t>(sendbufs[static_cast<size_t>(q)]) | reinterpret_cast<uintptr_t>(recvbufs[static_cast<size_t>(q)])) & 15u) == 0;
   const size_t wsize = DTypeSize(wire);
-  if (algo == Algo::kDirect && (wire != dtype || m.direct_staging == 2)) {
-    // The pipelined staged kernel (what ordinary buffers and 16-bit wires get on several GPUs).
-    const StagedShape sh = StagedShapeOnOneGpu(n * wsize, m.ws, m.layout.pool_bytes + m.layout.work_bytes,
-                                               m.staged_max_blocks, channels);
+  const bool pipelined = algo == Algo::kDirect && (wire != dtype || m.direct_staging == 2);
+  StagedShape sh{};
+  if (pipelined) {
+    sh = StagedShapeOnOneGpu(n * wsize, m.ws, m.layout.pool_bytes + m.layout.work_bytes, m.staged_max_blocks, channels);
     if (!all_aligned || (n * wsize) % 16 != 0 || sh.window_bytes < 4096)
       IBCOMM_FAIL(NOT_SUPPORTED, "The pipelined staged two-shot needs 16-byte aligned buffers of whole 16-byte wire vectors.\n");
+  }
+  const uint64_t half = m.layout.pool_bytes / 2 / 4096 * 4096;
+  if (algo == Algo::kDirect && !pipelined && (!all_aligned || (m.direct_staging != 0 && m.direct_staging != 3)) && half < 8192)
+    IBCOMM_FAIL(NOT_SUPPORTED, "Two-shot allreduce through the pool needs a pool of at least 16 KiB.\n");
+  if (algo == Algo::kDirect && m.direct_staging == 0 && LocalKernelTakes(local)) {
+    CUDACHECK(LaunchLocalKernel(local, stream));
+    m.last_channels = 0;
+  } else if (pipelined) {
+    // The pipelined staged kernel (what ordinary buffers and 16-bit wires get on several GPUs).
     const int ch = sh.blocks;
     std::vector<StagedParams> ps(static_cast<size_t>(m.ws));
     for (int r = 0; r < m.ws; ++r) {
@@ -220,10 +243,8 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
     CUDACHECK(LaunchStagedKernel(ps.data(), m.ws, sh.split ? 2 * ch : ch, stream));
     m.last_channels = ch;
   } else if (algo == Algo::kDirect) {
-    // The two-shot kernel with peer loads and stores.  All ranks' buffers live
-    // on this GPU, so they can be used in place; with `direct_staging` they
-    // go through the pool windows like buffers the peers cannot map.
-    const uint64_t half = m.layout.pool_bytes / 2 / 4096 * 4096;
+    // The two-shot kernel with peer loads and stores, through the pool windows like
+    // buffers the peers cannot map, or in place.
     int ch = channels > 0 ? channels : ChannelsOnOneGpu(bytes);
     ch = std::min(ch, cap);
     std::vector<NvlsParams> ps(static_cast<size_t>(m.ws));
@@ -243,12 +264,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.timeout_ns = timeout_ns;
       p.status = rr.d_status;
       p.doorbell = rr.d_doorbell;
-      bool aligned = true;
-      for (int q = 0; q < m.ws; ++q)
-        aligned = aligned && ((reinterpret_cast<uintptr_t>(sendbufs[static_cast<size_t>(q)]) | reinterpret_cast<uintptr_t>(recvbufs[static_cast<size_t>(q)])) & 15u) == 0;
-      const bool staged = m.direct_staging != 0 || !aligned;
-      if (staged && half < 8192)
-        IBCOMM_FAIL(NOT_SUPPORTED, "Two-shot allreduce through the pool needs a pool of at least 16 KiB.\n");
+      const bool staged = m.direct_staging != 3 || !all_aligned;
       p.stage_in = staged ? 1 : 0;
       p.stage_out = staged ? 1 : 0;
       for (int q = 0; q < m.ws; ++q) {
@@ -334,48 +350,63 @@ void EmuWorld::ReduceScatterOrAllGather(bool all_gather, DType dtype, const std:
   bool same_phase = true;
   auto remote_of = [&](int q) { return reinterpret_cast<uintptr_t>(all_gather ? recvbufs[static_cast<size_t>(q)] : sendbufs[static_cast<size_t>(q)]); };
   for (int q = 1; q < m.ws; ++q) same_phase = same_phase && ((remote_of(0) ^ remote_of(q)) & 15u) == 0;
-  const bool staged = m.direct_staging != 0 || !same_phase;
-  const uint64_t sub = m.layout.pool_bytes / static_cast<uint64_t>(m.ws) / 4096 * 4096;
-  if (staged && sub < 4096) IBCOMM_FAIL(NOT_SUPPORTED, "Reduce-scatter / all-gather through the pool need a larger pool.\n");
-  const int cap = std::max(1, m.max_blocks / m.ws);
-  int ch = channels > 0 ? channels : ChannelsOnOneGpu(block_bytes * static_cast<size_t>(m.ws));
-  ch = std::min(ch, cap);
-  std::vector<RsAgParams> ps(static_cast<size_t>(m.ws));
-  for (int r = 0; r < m.ws; ++r) {
-    RsAgParams& p = ps[static_cast<size_t>(r)];
-    memset(&p, 0, sizeof(p));
-    const RankResources& rr = m.ranks[static_cast<size_t>(r)];
-    p.rank = r;
-    p.world_size = m.ws;
-    p.dtype = static_cast<int32_t>(dtype);
-    p.mode = all_gather ? kRsAgAllGather : kRsAgReduceScatter;
-    p.staged = staged ? 1 : 0;
-    p.peers = rr.peers;
-    p.sendbuf = sendbufs[static_cast<size_t>(r)];
-    p.recvbuf = recvbufs[static_cast<size_t>(r)];
-    p.block_elems = block_elems;
-    p.scale = all_gather ? 1.0 : scale;
-    p.timeout_ns = static_cast<uint64_t>(m.timeout_ms) * 1000000ull;
-    p.status = rr.d_status;
-    p.doorbell = rr.d_doorbell;
+  if (m.direct_staging == 0 && same_phase) {
+    LocalParams local{};
+    local.op = all_gather ? LocalOp::kAllGather : LocalOp::kReduceScatter;
+    local.world_size = m.ws;
+    local.dtype = local.wire = static_cast<int32_t>(dtype);
     for (int q = 0; q < m.ws; ++q) {
+      local.in[q] = sendbufs[static_cast<size_t>(q)];
+      local.out[q] = recvbufs[static_cast<size_t>(q)];
+    }
+    local.len_elements = block_elems;
+    local.scale = all_gather ? 1.0 : scale;
+    CUDACHECK(LaunchLocalKernel(local, stream));
+    m.last_channels = 0;
+  } else {
+    const bool staged = m.direct_staging != 3 || !same_phase;
+    const uint64_t sub = m.layout.pool_bytes / static_cast<uint64_t>(m.ws) / 4096 * 4096;
+    if (staged && sub < 4096) IBCOMM_FAIL(NOT_SUPPORTED, "Reduce-scatter / all-gather through the pool need a larger pool.\n");
+    const int cap = std::max(1, m.max_blocks / m.ws);
+    int ch = channels > 0 ? channels : ChannelsOnOneGpu(block_bytes * static_cast<size_t>(m.ws));
+    ch = std::min(ch, cap);
+    std::vector<RsAgParams> ps(static_cast<size_t>(m.ws));
+    for (int r = 0; r < m.ws; ++r) {
+      RsAgParams& p = ps[static_cast<size_t>(r)];
+      memset(&p, 0, sizeof(p));
+      const RankResources& rr = m.ranks[static_cast<size_t>(r)];
+      p.rank = r;
+      p.world_size = m.ws;
+      p.dtype = static_cast<int32_t>(dtype);
+      p.mode = all_gather ? kRsAgAllGather : kRsAgReduceScatter;
+      p.staged = staged ? 1 : 0;
+      p.peers = rr.peers;
+      p.sendbuf = sendbufs[static_cast<size_t>(r)];
+      p.recvbuf = recvbufs[static_cast<size_t>(r)];
+      p.block_elems = block_elems;
+      p.scale = all_gather ? 1.0 : scale;
+      p.timeout_ns = static_cast<uint64_t>(m.timeout_ms) * 1000000ull;
+      p.status = rr.d_status;
+      p.doorbell = rr.d_doorbell;
+      for (int q = 0; q < m.ws; ++q) {
+        if (staged) {
+          p.peer_buf[q] = rr.peers.arena[q] + m.layout.pool_offset;
+        } else {
+          p.peer_buf[q] = all_gather ? static_cast<unsigned char*>(recvbufs[static_cast<size_t>(q)])
+                                     : static_cast<unsigned char*>(const_cast<void*>(sendbufs[static_cast<size_t>(q)]));
+        }
+      }
       if (staged) {
-        p.peer_buf[q] = rr.peers.arena[q] + m.layout.pool_offset;
+        p.sub_stride_bytes = sub;
+        p.window_elems = TwoShotWindowElems(block_elems, sub / esize, esize, 1, ch);
       } else {
-        p.peer_buf[q] = all_gather ? static_cast<unsigned char*>(recvbufs[static_cast<size_t>(q)])
-                                   : static_cast<unsigned char*>(const_cast<void*>(sendbufs[static_cast<size_t>(q)]));
+        p.sub_stride_bytes = block_bytes;
+        p.window_elems = block_elems;
       }
     }
-    if (staged) {
-      p.sub_stride_bytes = sub;
-      p.window_elems = TwoShotWindowElems(block_elems, sub / esize, esize, 1, ch);
-    } else {
-      p.sub_stride_bytes = block_bytes;
-      p.window_elems = block_elems;
-    }
+    CUDACHECK(LaunchRsAgKernel(ps.data(), m.ws, ch, stream));
+    m.last_channels = ch;
   }
-  CUDACHECK(LaunchRsAgKernel(ps.data(), m.ws, ch, stream));
-  m.last_channels = ch;
   if (async) return;
   CUDACHECK(cudaStreamSynchronize(stream));
   for (int r = 0; r < m.ws; ++r) {

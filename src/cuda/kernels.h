@@ -187,6 +187,22 @@ struct RsAgParams {
 };
 cudaError_t LaunchRsAgKernel(const RsAgParams* ranks, int n, int blocks, cudaStream_t stream);
 
+// ---- direct collectives of ranks that share a GPU, buffers in place (local_kernel.cu) ----
+enum class LocalOp : int32_t { kAllreduce, kReduceScatter, kAllGather };
+struct LocalParams {
+  LocalOp op;
+  int32_t world_size;
+  int32_t dtype;
+  int32_t wire;           // == dtype, or (allreduce) a 16-bit type that fp32 values are rounded to as if they travelled
+  const void* in[kMaxRanks];
+  void* out[kMaxRanks];
+  uint64_t len_elements;  // of the message; the halves: of a block
+  double scale;
+};
+// Whether the buffers' 16-byte boundaries lie alike, as the kernel needs.
+bool LocalKernelTakes(const LocalParams& p);
+cudaError_t LaunchLocalKernel(const LocalParams& p, cudaStream_t stream);
+
 // ---- one-shot allreduce for small messages (push to every peer, sum locally) ----
 struct OneShotParams {
   int32_t rank;

@@ -244,3 +244,82 @@ def test_staged_in_the_smallest_staging(pages):
     for o in outs:
         torch.testing.assert_close(o.double(), want, rtol=2e-2, atol=2e-2)
     world.close()
+
+
+@pytest.mark.parametrize("wire", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("ws", [2, 3, 5, 8])
+def test_direct_wire_in_place_and_through_the_pool(ws, wire):
+    # fp32 buffers with a 16-bit wire: used in place, and through the pool with the roles in every block and in blocks
+    # of their own.  The same values are rounded at the same places: the same bits.  What the pool refuses stays refused.
+    world = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+    for n in (8, 8 * ws, 8 * 1237, 8 * 512 * ws + 8, 300000, 1 << 20):
+        ins = [values(n, torch.float32, n + r) for r in range(ws)]
+        want = torch.stack([t.double() for t in ins]).sum(0) / ws
+        results = []
+        for mode, split in ((0, 0), (2, 0), (2, 1), (1, 0)):
+            world.set_direct_staging(mode)
+            ar.utils.set_tunable("IBCOMM_STAGED_SPLIT", split)
+            try:
+                outs = [torch.full_like(t, 7) for t in ins]
+                world.allreduce(ins, outs, algo="direct", scale=1.0 / ws, wire=wire)
+                bufs = [t.clone() for t in ins]
+                world.allreduce(bufs, None, algo="direct", scale=1.0 / ws, wire=wire)
+            finally:
+                ar.utils.set_tunable("IBCOMM_STAGED_SPLIT", -1)
+            results += outs + bufs
+        for o in results:
+            assert torch.equal(o, results[0])
+        torch.testing.assert_close(results[0].double(), want, rtol=2e-2, atol=2e-2)
+    for mode in (0, 2):
+        world.set_direct_staging(mode)
+        for n, offset in ((4097, 0), (4096, 1)):
+            bufs = [values(n, torch.float32, r, offset) for r in range(ws)]
+            with pytest.raises(ar.IbcommError) as e:
+                world.allreduce(bufs, None, algo="direct", wire=wire)
+            assert e.value.code == ar.NOT_SUPPORTED
+    world.close()
+
+
+@pytest.mark.parametrize("ws", [2, 3, 4, 5, 8])
+def test_direct_in_place_kernels_agree(ws):
+    # One kernel for all ranks, and each rank's own with barriers (in place, and through the pool): the same sums in rank
+    # order, so the same bits.  Lengths around a block of threads and a vector, slices that miss the boundary alike or not.
+    world = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+    for dtype in (torch.float32, torch.float64, torch.bfloat16, torch.float16, torch.int32, torch.int64):
+        k = 16 // torch.empty(0, dtype=dtype).element_size()
+        scale = 1.0 if dtype in (torch.int32, torch.int64) else 1.0 / ws
+        for n in (ws, 1, k, 128 * k - 1, 128 * k + 1, 70001):
+            for off_in, off_out in ((0, 0), (1, 1), (1, 0), (k - 1, k - 1)):
+                ins = [values(n, dtype, n + r, off_in) for r in range(ws)]
+                results = []
+                for mode in (0, 3, 1):
+                    world.set_direct_staging(mode)
+                    guard = [torch.full((n + off_out + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+                    outs = [g[off_out:off_out + n] for g in guard]
+                    world.allreduce(ins, outs, algo="direct", scale=scale)
+                    for g in guard:
+                        assert torch.all(g[:off_out] == 7) and torch.all(g[off_out + n:] == 7)
+                    results += outs
+                for o in results:
+                    assert torch.equal(o, results[0])
+                full = [values(n * ws, dtype, n + r, off_in) for r in range(ws)]
+                halves = []
+                for mode in (0, 3, 1):
+                    world.set_direct_staging(mode)
+                    guard = [torch.full((n + off_out + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+                    shards = [g[off_out:off_out + n] for g in guard]
+                    world.reduce_scatter(full, shards, scale=scale)
+                    whole = [torch.full((n * ws + off_in + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+                    outs = [g[off_in:off_in + n * ws] for g in whole]
+                    world.all_gather(shards, outs)
+                    for g in guard:
+                        assert torch.all(g[:off_out] == 7) and torch.all(g[off_out + n:] == 7)
+                    for g in whole:
+                        assert torch.all(g[:off_in] == 7) and torch.all(g[off_in + n * ws:] == 7)
+                    halves.append(outs)
+                for outs in halves:
+                    for o in outs:
+                        assert torch.equal(o, halves[0][0])
+    want = torch.stack([t.double() for t in ins]).sum(0)
+    assert torch.equal(results[0].double(), want)  # int64: exact
+    world.close()
