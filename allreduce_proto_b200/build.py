@@ -54,6 +54,7 @@ CUDA_SOURCES = [
     "src/cuda/device_context.cpp",
     "src/cuda/emu_world.cpp",
     "src/cuda/exec_kernel.cu",
+    "src/cuda/ll_kernel.cu",
     "src/cuda/nvls_kernel.cu",
     "src/cuda/oneshot_kernel.cu",
     "src/cuda/rsag_kernel.cu",

@@ -27,6 +27,9 @@ struct ArenaLayout {
   uint64_t pool_bytes = 0;
   uint64_t work_offset = 0;      // IBCOMM_WORK_GPU_MEMORY_SIZE bytes
   uint64_t work_bytes = 0;
+  // Two halves of lines_half_bytes for transfers as lines, used for nothing else; 0: none.
+  uint64_t lines_offset = 0;
+  uint64_t lines_half_bytes = 0;
   uint64_t total_bytes = 0;
 };
 // Bytes of the one-shot area: 16 MiB slots for two ranks, 4 MiB for eight.

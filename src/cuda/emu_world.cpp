@@ -21,6 +21,7 @@ struct EmuWorld::Impl {
   int timeout_ms = env::kDefaultTimeoutMs;
   int max_blocks = 0;
   int exec_max_blocks = 0;  // executor CTAs of the smaller size (two per SM)
+  int line_max_blocks = 0;
   int last_channels = 0;
   int silent_rank = -1;
   int bad_program_rank = -1;
@@ -90,6 +91,22 @@ int OneShotChannelsOnOneGpu(size_t bytes) {
   return static_cast<int>(std::min<size_t>(128, std::max<size_t>(1, bytes / (4u << 10))));
 }
 
+// Half of a rank's lines area at most: a slot for every transfer of 2 MiB by three to eight ranks.
+constexpr uint64_t kLinesHalfBytes = 16ull << 20;
+
+// Whether an op program's transfers travel as lines: `bytes` of a rank's message in the wire type.  Slots with flags
+// against lines, us (IBCOMM_LINES_MAX_KIB overrides):
+//                   64 KiB       512 KiB      1 MiB        2 MiB        4 MB
+//   ring, 8 ranks   47.3  16.4   49.6  18.5   53.3  29.3   56.6  52.1   63.6  81
+//   ring, 5 ranks   30.6  12.3   32.2  12.9   34.8  14.4   35.3  32.1   38.9  46
+//   ring, 2 ranks   14.1   6.2   15.8   6.6   16.4   7.7   16.4   8.2   17.1  10
+//   Rabenseifner 8  36.9  20.5   38.8  20.5   40.5  25.2   43.1  40.2   55.7  (same)
+//   Rabenseifner 5  26.0  12.4   26.5  12.3   27.0  18.5   28.8  25.6   36.8  (same)
+// Up to 1.2 MB a thread has one pack of a transfer (148 SMs x 512 threads x 16 bytes), from there on several.
+bool LinesPay(uint64_t bytes) {
+  return bytes <= (static_cast<uint64_t>(std::max(0, Tunable("IBCOMM_LINES_MAX_KIB", 2048))) << 10);
+}
+
 }  // namespace
 
 EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(num_ranks), impl_(new Impl()) {
@@ -100,6 +117,9 @@ EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(nu
   CUDACHECK(cudaGetDevice(&m.device));
   m.timeout_ms = env::ReadTimeoutMs();
   m.layout = MakeArenaLayout(pool_bytes ? pool_bytes : env::ReadPreAllocSize(), work_bytes ? work_bytes : env::ReadWorkGpuMemorySize(), num_ranks);
+  // Nothing is sent to a mailbox here, so lines may have that memory.
+  m.layout.lines_offset = m.layout.mailbox_offset;
+  m.layout.lines_half_bytes = std::min<uint64_t>(kLinesHalfBytes, (m.layout.pool_offset - m.layout.mailbox_offset) / 2 / 4096 * 4096);
   const size_t total = static_cast<size_t>(m.layout.total_bytes) * static_cast<size_t>(num_ranks);
   CUDACHECK(cudaMalloc(&m.arenas, total));
   CUDACHECK(cudaMemset(m.arenas, 0, total));
@@ -120,6 +140,7 @@ EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(nu
   }
   m.max_blocks = TwoShotKernelMaxCoResidentBlocks(m.device);
   m.exec_max_blocks = ExecKernelMaxCoResidentBlocks(m.device, 256);
+  m.line_max_blocks = LineKernelMaxCoResidentBlocks(m.device);
   m.staged_max_blocks = StagedKernelMaxCoResidentBlocks(m.device);
   CUDACHECK(cudaDeviceSynchronize());
 }
@@ -298,20 +319,41 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
   } else {
     // Validation (length, chunk size) happens while the first program is cut.
     std::vector<ExecParams> ps;
-    for (int r = 0; r < m.ws; ++r) {
-      const CachedProgram& cp = m.cache.Get(algo, r, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false, m.ws);
-      ps.push_back(MakeExecParams(m.ranks[static_cast<size_t>(r)], cp, dtype, wire, sendbufs[static_cast<size_t>(r)],
-                                  recvbufs[static_cast<size_t>(r)], n, scale, timeout_ns, nullptr, 0));
-      if (r == m.silent_rank) ps.back().num_ops = 0;
-      if (r == m.bad_program_rank) ps.back().len_elements = 1;
+    bool fit = true;
+    auto programs = [&](ProgramForm form) {
+      ps.clear();
+      for (int r = 0; r < m.ws; ++r) {
+        const CachedProgram& cp = m.cache.Get(algo, r, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false, m.ws, form);
+        fit = fit && LinesFit(cp.prog);
+        ps.push_back(MakeExecParams(m.ranks[static_cast<size_t>(r)], cp, dtype, wire, sendbufs[static_cast<size_t>(r)],
+                                    recvbufs[static_cast<size_t>(r)], n, scale, timeout_ns, nullptr, 0));
+        if (r == m.silent_rank) ps.back().num_ops = 0;
+        if (r == m.bad_program_rank) ps.back().len_elements = 1;
+      }
+    };
+    // Prescribed chunks and pieces, and ranks that hand over as between GPUs, keep the slots.
+    bool lines = m.direct_staging == 0 && LinesPay(n * wsize) && env::ReadChunkSize() <= 0 && Tunable("IBCOMM_RABEN_PIECES", 0) <= 0;
+    if (lines) {
+      programs(ProgramForm::kLines);
+      lines = fit;
     }
-    // A channel for every 4 KiB of a transfer: the flags of ranks on one GPU are
-    // cheap, and more channels shorten every step of the program.  One CTA per
-    // SM at most (two smaller ones per SM are no faster).
-    const uint64_t slot = ps.back().stage.slot_bytes;
-    int ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(slot / 4096, static_cast<uint64_t>(kMaxChannels)));
-    ch = std::max(1, std::min(ch, channels > 0 ? m.exec_max_blocks / m.ws : cap));
-    CUDACHECK(LaunchExecKernel(ps.data(), m.ws, ch, stream));
+    int ch;
+    if (lines) {
+      // A thread per pack of a transfer.
+      const uint64_t packs = ps.back().stage.slot_bytes / 16;
+      ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>((packs + 511) / 512, static_cast<uint64_t>(kMaxChannels)));
+      ch = std::max(1, std::min({ch, m.line_max_blocks / m.ws, kMaxChannels}));
+      CUDACHECK(LaunchLineKernel(ps.data(), m.ws, ch, m.layout.lines_half_bytes, stream));
+    } else {
+      programs(ProgramForm::kStaged);
+      // A channel for every 4 KiB of a transfer: the flags of ranks on one GPU are
+      // cheap, and more channels shorten every step of the program.  One CTA per
+      // SM at most (two smaller ones per SM are no faster).
+      const uint64_t slot = ps.back().stage.slot_bytes;
+      ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(slot / 4096, static_cast<uint64_t>(kMaxChannels)));
+      ch = std::max(1, std::min(ch, channels > 0 ? m.exec_max_blocks / m.ws : cap));
+      CUDACHECK(LaunchExecKernel(ps.data(), m.ws, ch, stream));
+    }
     m.last_channels = ch;
   }
   if (async) return;

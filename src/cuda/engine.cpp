@@ -143,7 +143,7 @@ void ProgramCache::NoteSynchronized() {
 }
 
 const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size_t len_elements, DType dtype, DType wire,
-                                       const ArenaLayout& layout, bool apply_scale, cudaStream_t stream, bool capturing, int ranks_on_gpu) {
+                                       const ArenaLayout& layout, bool apply_scale, cudaStream_t stream, bool capturing, int ranks_on_gpu, ProgramForm form) {
   const size_t esize = DTypeSize(dtype), wsize = DTypeSize(wire);
   // Read at the point of use, like the reference: a bad value fails the call.
   const long long env_chunk = env::ReadChunkSize();
@@ -151,7 +151,8 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   // The ring stages in the pool.  Rabenseifner lands its pieces in the work
   // region and, since one collective runs at a time, in the pool in front of
   // it as well (the two are adjacent in the arena).
-  const uint64_t stage_off = layout.pool_offset;
+  const bool lines = form == ProgramForm::kLines;
+  const uint64_t stage_off = lines ? layout.lines_offset : layout.pool_offset;
   int raben_div = Tunable("IBCOMM_RABEN_PIECES", 0);
   const bool asked = raben_div >= 1 && raben_div <= 1024;
   // Ranks on one GPU run Rabenseifner in segments, unless the pieces are prescribed.
@@ -171,16 +172,17 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   // it, and the others wait for the extra ranks.
   const int regions = NumRegions(algo, world_size);
   const uint64_t sharers = static_cast<uint64_t>(ranks_on_gpu > 1 ? ranks_on_gpu : 1);
-  const bool drop_lines = segmented && wsize == esize && sharers * len_elements * wsize >= (48ull << 20);
+  const bool drop_lines = segmented && !lines && wsize == esize && sharers * len_elements * wsize >= (48ull << 20);
   uint64_t stage_bytes = ring ? RingStageBytes(layout.pool_bytes, ranks_on_gpu) : layout.pool_bytes + layout.work_bytes;
-  if (segmented && !drop_lines && regions <= 3) stage_bytes = std::min<uint64_t>(stage_bytes, kSharedGpuHalvingBytes / sharers);
+  if (lines) stage_bytes = layout.lines_half_bytes / 2;  // a line holds half its bytes
+  else if (segmented && !drop_lines && regions <= 3) stage_bytes = std::min<uint64_t>(stage_bytes, kSharedGpuHalvingBytes / sharers);
   // Knobs that shape the program are part of the key: the ring's chunks per
   // rank and the number of pieces Rabenseifner cuts the message into.
-  const size_t ring_cpr = ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size), ranks_on_gpu > 1) : 0;
+  const size_t ring_cpr = lines ? 1 : ring ? RingChunksPerRank(len_elements, esize, static_cast<size_t>(world_size), ranks_on_gpu > 1) : 0;
   if (segmented) raben_div = 0;
   else if (!asked) raben_div = 8;
   Key key{static_cast<int>(algo), rank, world_size, len_elements, static_cast<int>(dtype), static_cast<int>(wire),
-          env_chunk, apply_scale, stage_off, stage_bytes, ring ? static_cast<int>(ring_cpr) : raben_div};
+          env_chunk, apply_scale, stage_off, stage_bytes, ring ? static_cast<int>(ring_cpr) : raben_div, static_cast<int>(form)};
   auto it = cache_.find(key);
   if (it != cache_.end()) {
     CachedProgram& hit = *it->second;
@@ -263,6 +265,13 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   const CachedProgram& ref = *cp;
   cache_[key] = std::move(cp);
   return ref;
+}
+
+bool LinesFit(const Program& prog) {
+  if (prog.ops.empty() || prog.ops.size() > static_cast<size_t>(kMaxLineOps)) return false;
+  for (const uint32_t sent : prog.sent_to)
+    if (sent > prog.stage.slots) return false;
+  return true;
 }
 
 ExecParams MakeExecParams(const RankResources& rr, const CachedProgram& cp, DType dtype, DType wire, const void* sendbuf,

@@ -43,6 +43,14 @@ struct StatusBlock {
   uint32_t Consume(DeviceStatus* out, cudaStream_t stream);
 };
 
+// How the ranks of a program hand over.
+enum class ProgramForm {
+  kStaged,  // through slots of the pool and the work region, with flags and credits
+  kLines,   // through slots of the lines area, each used once (ll_kernel.cu); see LinesFit
+};
+// Whether a program runs as lines: one that does not is not to be launched that way.
+bool LinesFit(const Program& prog);
+
 struct CachedProgram {
   Program prog;
   bool drop_lines = false;  // ExecParams::drop_lines
@@ -65,7 +73,8 @@ class ProgramCache {
   // Cuts the message and compiles (or finds) the program of `rank`; a new one
   // is uploaded on `stream`.  `capturing`: the call is being recorded into a graph.
   const CachedProgram& Get(Algo algo, int rank, int world_size, size_t len_elements, DType dtype, DType wire,
-                           const ArenaLayout& layout, bool apply_scale, cudaStream_t stream, bool capturing, int ranks_on_gpu = 1);
+                           const ArenaLayout& layout, bool apply_scale, cudaStream_t stream, bool capturing, int ranks_on_gpu = 1,
+                           ProgramForm form = ProgramForm::kStaged);
   // Everything issued with programs of this cache has finished (the caller
   // synchronised): the moment at which an over-full cache lets go of the
   // programs no graph refers to.
@@ -76,7 +85,7 @@ class ProgramCache {
   void SetBound(size_t entries) { bound_ = entries; }
 
  private:
-  using Key = std::tuple<int, int, int, size_t, int, int, long long, bool, uint64_t, uint64_t, int>;
+  using Key = std::tuple<int, int, int, size_t, int, int, long long, bool, uint64_t, uint64_t, int, int>;
   struct Slab {
     Op* d = nullptr;  // device memory
     Op* h = nullptr;  // pinned host memory, the upload's source

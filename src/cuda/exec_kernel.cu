@@ -45,6 +45,7 @@
 // launch (CTAs that wait on each other are co-resident).
 #include <algorithm>
 
+#include "exec_common.cuh"
 #include "flags.cuh"
 #include "ibcomm/communicator.h"
 #include "ibcomm/tunables.h"
@@ -55,16 +56,6 @@
 
 namespace ibcomm {
 namespace dev {
-
-template <typename T, typename W>
-struct ExecTraits {
-  using A = typename Acc<T>::type;
-  static constexpr int kMinBytes = sizeof(T) < sizeof(W) ? sizeof(T) : sizeof(W);
-  static constexpr int P = 16 / kMinBytes;               // elements per pack
-  static constexpr int VT = P / VecIO<T>::kN;            // 16-byte vectors per pack in the user type
-  static constexpr int VW = P / VecIO<W>::kN;            // ... in the wire type
-  static constexpr int U = VT > 1 ? 2 : 4;               // packs per thread and stage
-};
 
 constexpr int kExecServiceWarps = 3;  // waiter, loader, poster
 constexpr int kExecMaxStages = 10;
@@ -255,25 +246,6 @@ __device__ __forceinline__ void RunTile(const ExecTile& t, const ExecTile* tile,
   }
 }
 
-// Where an op's data lies.
-template <typename T, typename W>
-struct OpBuffers {
-  const T* sendbuf;
-  T* recvbuf;
-  const W* stage_in;
-  W* stage_out;
-  __device__ OpBuffers(const Op& op, const ExecParams& p)
-      : sendbuf(static_cast<const T*>(p.sendbuf)), recvbuf(static_cast<T*>(p.recvbuf)), stage_in(nullptr), stage_out(nullptr) {
-    const StageLayout& st = p.stage;
-    if (op.src_a == kSrcStage)
-      stage_in = reinterpret_cast<const W*>(p.peers.arena[p.rank] + st.offset +
-                                            (static_cast<uint64_t>(op.region_in) * st.slots + op.slot_in) * st.slot_bytes);
-    if (op.flags & kOpStoreRemote)
-      stage_out = reinterpret_cast<W*>(p.peers.arena[op.peer_out] + st.offset +
-                                       (static_cast<uint64_t>(op.region_out) * st.slots + op.slot_out) * st.slot_bytes);
-  }
-};
-
 // Element-at-a-time path for chunks that do not start on a 16-byte boundary
 // and for the few elements after the last whole pack; kU loads of each source
 // in flight per thread.
@@ -308,28 +280,6 @@ __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint
       }
     }
   }
-}
-
-// Self-check of an op before any of its addresses is formed: the message
-// range, the place inside the staging slot and the slot, region and peer
-// indices.  A failing op is reported (status "bad program") and the call
-// stops; nothing is accessed out of range and nothing traps.
-template <typename W>
-__device__ __forceinline__ bool OpInBounds(const Op& op, const ExecParams& p) {
-  if (op.elem_begin > p.len_elements || op.elem_count > p.len_elements - op.elem_begin) return false;
-  if (op.cell_begin > op.elem_begin) return false;
-  const bool reads_stage = op.src_a == kSrcStage || op.src_b == kSrcStage;
-  const bool writes_stage = (op.flags & kOpStoreRemote) != 0;
-  if (reads_stage || writes_stage) {
-    if ((op.elem_begin - op.cell_begin + op.elem_count) * sizeof(W) > p.stage.slot_bytes) return false;
-  }
-  if (reads_stage && (op.region_in >= p.stage.regions || op.slot_in >= p.stage.slots)) return false;
-  if (writes_stage && (op.region_out >= p.stage.regions || op.slot_out >= p.stage.slots || op.peer_out < 0 ||
-                       op.peer_out >= p.world_size))
-    return false;
-  if ((op.wait_in != 0 || op.post_credit != 0) && (op.peer_in < 0 || op.peer_in >= p.world_size)) return false;
-  if ((op.wait_credit != 0 || op.post_out != 0) && (op.peer_out < 0 || op.peer_out >= p.world_size)) return false;
-  return op.wait_local < static_cast<uint32_t>(p.num_ops);
 }
 
 // Position in the ring of stages.

@@ -83,8 +83,8 @@ __device__ inline void ReportFailure(const WaitCtx& w, uint32_t code, uint32_t k
 }
 
 // Sequence number of the running collective: one more than the number this
-// rank has begun before.  Every CTA of the rank calls this exactly once, with all
-// threads; `ctas` = CTAs of this rank, `scratch` is a __shared__ word.
+// rank has begun before.  Every CTA of the rank takes it exactly once: by one
+// thread, `scratch` may be read behind the CTA's next barrier; `ctas` = CTAs of this rank, `scratch` is a __shared__ word.
 //
 // ControlPage::call_word holds (calls begun << 16) | CTAs of the running call
 // that have taken their number.  The last CTA to take it advances the count:
@@ -92,13 +92,15 @@ __device__ inline void ReportFailure(const WaitCtx& w, uint32_t code, uint32_t k
 // wait for the call's end, and one atomic does for the load at the start and
 // the counter, fence and barrier at the end that it replaced (1.5-2 us of an 8 us
 // call on one GPU).
+__device__ __forceinline__ void TakeCallNumber(const PeerTable& peers, int rank, uint64_t* scratch, unsigned ctas) {
+  unsigned long long* const word = reinterpret_cast<unsigned long long*>(&Ctl(peers, rank)->call_word);
+  const unsigned long long old = atomicAdd(word, 1ull);
+  if (static_cast<unsigned>(old & 0xffffu) + 1u == ctas) atomicAdd(word, (1ull << 16) - ctas);
+  *scratch = static_cast<uint64_t>(old >> 16) + 1;
+}
+// The same with all threads of the CTA, barrier included.
 __device__ inline uint64_t BeginCollective(const PeerTable& peers, int rank, uint64_t* scratch, unsigned ctas) {
-  if (threadIdx.x == 0) {
-    unsigned long long* const word = reinterpret_cast<unsigned long long*>(&Ctl(peers, rank)->call_word);
-    const unsigned long long old = atomicAdd(word, 1ull);
-    if (static_cast<unsigned>(old & 0xffffu) + 1u == ctas) atomicAdd(word, (1ull << 16) - ctas);
-    *scratch = static_cast<uint64_t>(old >> 16) + 1;
-  }
+  if (threadIdx.x == 0) TakeCallNumber(peers, rank, scratch, ctas);
   __syncthreads();
   return *scratch;
 }

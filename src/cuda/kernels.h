@@ -50,6 +50,13 @@ cudaError_t LaunchExecKernel(const ExecParams* ranks, int n, int channels, cudaS
 int ExecKernelThreadsFor(int ctas);
 int ExecKernelMaxCoResidentBlocks(int device, int threads = 0);
 
+// The same for short messages, with transfers as lines (ll_kernel.cu).  `stage.offset` is that of an
+// area used for lines only, two halves of `half_bytes` in which the program's slots take twice their
+// bytes; no slot is used twice, and the program has at most kMaxLineOps ops.
+constexpr int kMaxLineOps = 96;
+cudaError_t LaunchLineKernel(const ExecParams* ranks, int n, int channels, uint64_t half_bytes, cudaStream_t stream);
+int LineKernelMaxCoResidentBlocks(int device);
+
 // ---- world_size == 1: out = cast(in * scale) ----
 struct CopyParams {
   const void* in;

@@ -323,3 +323,76 @@ def test_direct_in_place_kernels_agree(ws):
     want = torch.stack([t.double() for t in ins]).sum(0)
     assert torch.equal(results[0].double(), want)  # int64: exact
     world.close()
+
+
+@pytest.mark.parametrize("slots", [0, 3])
+@pytest.mark.parametrize("algo", ["ring", "rabenseifner"])
+@pytest.mark.parametrize("ws", [2, 3, 4, 5, 6, 7, 8])
+def test_short_messages_as_lines_and_through_slots(ws, algo, slots):
+    # Transfers as lines, and through the slots with flags: fewer elements than a pack per rank, packs that two ops share,
+    # a pack per thread and several, more than one channel; slices off the boundary; 16-bit wires; in place.
+    world = ar.EmuWorld(ws)
+    world.set_direct_staging(slots)
+    for dtype in (torch.float32, torch.float64, torch.bfloat16, torch.float16, torch.int32, torch.int64):
+        whole = dtype in (torch.int32, torch.int64)
+        scale = 1.0 if whole else 1.0 / ws
+        for n in (ws, 2 * ws + 1, 129, 2521, 70001):
+            for off_in, off_out in ((0, 0), (1, 1), (1, 0)):
+                for wire in (None, torch.bfloat16, torch.float16) if dtype == torch.float32 else (None,):
+                    ins = [values(n, dtype, n + r, off_in) for r in range(ws)]
+                    want = torch.stack([t.double() for t in ins]).sum(0) * scale
+                    guard = [torch.full((n + off_out + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+                    outs = [g[off_out:off_out + n] for g in guard]
+                    world.allreduce(ins, outs, algo=algo, scale=scale, wire=wire)
+                    tol = 0.0 if whole else (2e-2 if dtype in (torch.bfloat16, torch.float16) or wire is not None else (1e-5 if dtype == torch.float32 else 1e-12))
+                    for g, o in zip(guard, outs):
+                        torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
+                        assert torch.equal(o, outs[0])
+                        assert torch.all(g[:off_out] == 7) and torch.all(g[off_out + n:] == 7)
+                    world.allreduce(ins, None, algo=algo, scale=scale, wire=wire)
+                    for i in ins:
+                        torch.testing.assert_close(i.double(), want, rtol=tol, atol=tol)
+    world.close()
+
+
+@pytest.mark.parametrize("ws", [2, 5, 8])
+def test_lines_of_many_calls(ws):
+    # Calls of different lengths and algorithms back to back, other kernels between them: what earlier calls left in the
+    # lines is not taken for a transfer.  Whole numbers, so that every call's result is exact.
+    world = ar.EmuWorld(ws)
+    sizes = [ws, 300000, 1000, 4096, 70001, 131072, 64, 262144]
+    for turn in range(6):
+        calls = []
+        for k, n in enumerate(sizes):
+            ins = [torch.full((n,), float(turn + k + r), device="cuda") + torch.arange(n, device="cuda") % 13 for r in range(ws)]
+            want = torch.stack([t.double() for t in ins]).sum(0)
+            outs = [torch.full_like(t, 7) for t in ins]
+            world.allreduce(ins, outs, algo=("ring", "rabenseifner", "oneshot")[(turn + k) % 3 if n <= 262144 else 0], sync=False)
+            calls.append((outs, want))
+        torch.cuda.synchronize()
+        for outs, want in calls:
+            for o in outs:
+                assert torch.equal(o.double(), want)
+    world.close()
+
+
+@pytest.mark.parametrize("algo", ["ring", "rabenseifner"])
+def test_lines_wait_runs_out(algo):
+    # A rank that takes no part in a short call: the others' waits for its lines end, the status says that it never came,
+    # and the world stays usable.
+    world = ar.EmuWorld(4)
+    world.set_timeout_ms(200)
+    ins = [values(4096, torch.float32, r) for r in range(4)]
+    outs = [torch.zeros_like(t) for t in ins]
+    world.set_silent_rank(1)
+    with pytest.raises(ar.IbcommError) as e:
+        world.allreduce(ins, outs, algo=algo)
+    assert e.value.code == ar.TRANSPORT_ERROR
+    assert world.last_status()["code"] in (1, 2)
+    world.set_silent_rank(-1)
+    world.set_timeout_ms(5000)
+    world.allreduce(ins, outs, algo=algo)
+    want = torch.stack([t.double() for t in ins]).sum(0)
+    for o in outs:
+        torch.testing.assert_close(o.double(), want, rtol=1e-5, atol=1e-5)
+    world.close()
