@@ -32,7 +32,8 @@ constexpr int kP2pMaxSlots = 8;    // upper bound of mailbox slots per source ra
 // All words are 64-bit, written by exactly one remote rank and polled locally.
 // Values only grow: (call sequence << 32) | count.
 struct ControlPage {
-  // bar[c][s]: rank s announces "my channel c reached barrier point v".
+  // bar[c][s]: rank s announces "my channel c reached barrier point v", or how many
+  // stores into this rank's recvbuf it has finished since (Op::wait_peer).
   uint64_t bar[kMaxChannels][kMaxRanks];
   // inflag[c][s]: number of transfers rank s has completed into my staging.
   uint64_t inflag[kMaxChannels][kMaxRanks];
@@ -95,7 +96,8 @@ struct DeviceTraceRec {
 };
 
 // ---- program ops ----
-enum OpSrc : uint8_t { kSrcNone = 0, kSrcSend = 1, kSrcRecv = 2, kSrcStage = 3 };
+// kSrcPeer: sendbuf of another rank of the same launch (Op::rank_a, Op::rank_c).
+enum OpSrc : uint8_t { kSrcNone = 0, kSrcSend = 1, kSrcRecv = 2, kSrcStage = 3, kSrcPeer = 4 };
 enum OpFlags : uint8_t {
   kOpScale = 1,        // multiply by ExecParams::scale before storing
   kOpStoreLocal = 2,   // store to recvbuf[range]
@@ -105,17 +107,25 @@ enum OpFlags : uint8_t {
   kOpRoundWire = 8,
   // A later op reads what the local store leaves in recvbuf: it should stay in L2.
   kOpReadBack = 16,
+  // Values of another rank's sendbuf are rounded through the wire type before they are added, as if they had travelled.
+  kOpRoundPeer = 32,
+  // kOpReadBack for what goes into other ranks' recvbuf.
+  kOpPeersReadBack = 64,
 };
 
+// Ranks that an op tells about what it stored into their recvbuf (the others it stores to do not wait for it).
+constexpr int kMaxPeerPosts = 2;
+
+// result = (a + c) + b (* scale)
 struct Op {
   uint8_t src_a;     // OpSrc
-  uint8_t src_b;     // OpSrc (added to src_a); kSrcNone = plain copy
+  uint8_t src_b;     // OpSrc: kSrcNone, kSrcSend or kSrcRecv
   uint8_t flags;     // OpFlags
-  int8_t peer_in;    // rank whose transfer feeds kSrcStage, -1 if none
-  int8_t peer_out;   // rank that receives the remote store, -1 if none
+  int8_t peer_in;    // rank whose transfer the op waits for (it feeds kSrcStage, or lies in recvbuf), -1 if none
+  int8_t peer_out;   // rank that receives a transfer, -1 if none
   uint8_t region_in;   // staging region index on my side (one per in-peer)
   uint8_t region_out;  // staging region index on peer_out's side
-  uint8_t pad_;
+  int8_t rank_a;       // whose sendbuf src_a is (kSrcPeer)
   uint32_t slot_in;    // staging slot index inside region_in
   uint32_t slot_out;   // staging slot index inside region_out
   uint32_t wait_in;      // wait until inflag[ch][peer_in] >= base + wait_in   (0 = no wait)
@@ -132,8 +142,19 @@ struct Op {
   // to be finished first (the last of them stored into the op's cell); 0 when
   // nothing has.  Loads may run ahead of the program otherwise.
   uint32_t wait_local;
-  uint32_t pad2_;
+  // Programs of ranks that one launch runs on one GPU only: a third source, the
+  // sendbuf of rank_c (-1: none), and ranks whose recvbuf gets the value beside this
+  // rank's (a bit each).
+  int8_t rank_c;
+  uint8_t store_peers;
+  // Stores into another rank's recvbuf are counted apart, behind the entry barrier's word: wait until
+  // bar[ch][peer_in] >= base + 1 + wait_peer, and then post_peer.bar[ch][me] = base + 1 + post (0 = neither).
+  int8_t peer_told[kMaxPeerPosts];
+  uint32_t post_told[kMaxPeerPosts];
+  uint32_t wait_peer;
+  uint32_t pad_;
 };
+static_assert(sizeof(Op) == 80, "whole 16-byte vectors");
 
 // Whether a finished op's flags need a fence between what the op wrote and the
 // flags: a transfer into the peer's slot always, and the credit for a slot whose
@@ -240,6 +261,11 @@ struct ExecParams {
   DeviceStatus* status;  // device memory, fetched by the host after a failure
   uint32_t* doorbell;    // host-mapped word a failing kernel sets non-zero
   DeviceTraceRec* trace; // [channel][trace_capacity]
+  // Programs of ranks that share a GPU: everybody's buffers (null otherwise).
+  const void* peer_send[kMaxRanks];
+  void* peer_recv[kMaxRanks];
+  uint32_t present;      // ranks that the launch has blocks for, a bit each
+  uint32_t counts_for;   // ranks without blocks that this rank counts the call for (they have nothing to do in it)
 };
 
 }  // namespace ibcomm

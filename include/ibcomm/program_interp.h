@@ -31,8 +31,8 @@ template <typename T>
 class ProgramSimulator {
  public:
   ProgramSimulator(Algo algo, int world_size, size_t stage_bytes, int channels, size_t piece_elems = 0,
-                   std::vector<size_t> segments = {})
-      : algo_(algo), ws_(world_size), stage_bytes_(stage_bytes), nch_(channels), piece_elems_(piece_elems), segments_(std::move(segments)) {}
+                   std::vector<size_t> segments = {}, bool shared_gpu = false)
+      : shared_gpu_(shared_gpu), algo_(algo), ws_(world_size), stage_bytes_(stage_bytes), nch_(channels), piece_elems_(piece_elems), segments_(std::move(segments)) {}
 
   // inputs[r] is rank r's send buffer; outputs[r] receives its result.
   // `in_place` makes every rank use one buffer for both.
@@ -51,22 +51,25 @@ class ProgramSimulator {
       q.wire_elem_bytes = sizeof(T);
       q.stage_bytes = stage_bytes_;
       q.apply_scale = (scale != 1.0);
+      q.shared_gpu = shared_gpu_;
       progs.push_back(BuildProgram(q));
     }
     programs_ = progs;
     const StageLayout st = progs[0].stage;
     struct RankMem {
       std::vector<unsigned char> stage;
-      std::unique_ptr<std::atomic<uint64_t>[]> inflag, credit;
+      std::unique_ptr<std::atomic<uint64_t>[]> inflag, credit, told;
     };
     std::vector<RankMem> mem(static_cast<size_t>(ws_));
     for (auto& m : mem) {
       m.stage.assign(static_cast<size_t>(st.regions) * st.slots * st.slot_bytes, 0xAB);
       m.inflag.reset(new std::atomic<uint64_t>[static_cast<size_t>(nch_) * kMaxRanks]);
       m.credit.reset(new std::atomic<uint64_t>[static_cast<size_t>(nch_) * kMaxRanks]);
+      m.told.reset(new std::atomic<uint64_t>[static_cast<size_t>(nch_) * kMaxRanks]);
       for (int i = 0; i < nch_ * kMaxRanks; ++i) {
         m.inflag[static_cast<size_t>(i)].store(0);
         m.credit[static_cast<size_t>(i)].store(0);
+        m.told[static_cast<size_t>(i)].store(0);
       }
     }
     outputs->assign(static_cast<size_t>(ws_), std::vector<T>());
@@ -76,7 +79,8 @@ class ProgramSimulator {
     std::vector<std::string> errors(static_cast<size_t>(ws_) * static_cast<size_t>(nch_));
     auto worker = [&](int r, int ch) {
       const Program& pg = progs[static_cast<size_t>(r)];
-      const T* sendbuf = in_place ? (*outputs)[static_cast<size_t>(r)].data() : inputs[static_cast<size_t>(r)].data();
+      auto send_of = [&](int q) { return in_place ? (*outputs)[static_cast<size_t>(q)].data() : inputs[static_cast<size_t>(q)].data(); };
+      const T* sendbuf = send_of(r);
       T* recvbuf = (*outputs)[static_cast<size_t>(r)].data();
       auto wait_for = [&](std::atomic<uint64_t>& f, uint64_t target, const char* what, size_t op_index) {
         auto t0 = std::chrono::steady_clock::now();
@@ -99,7 +103,7 @@ class ProgramSimulator {
       std::vector<std::vector<T>> early(pg.ops.size());        // per op: its slice of recvbuf
       std::vector<std::vector<size_t>> due(pg.ops.size() + 1);  // by the ops that have to be finished: the ops that may load
       for (size_t i = 0; i < pg.ops.size(); ++i)
-        if (pg.ops[i].src_a == kSrcRecv || pg.ops[i].src_b == kSrcRecv) due[pg.ops[i].wait_local].push_back(i);
+        if ((pg.ops[i].src_a == kSrcRecv && pg.ops[i].wait_peer == 0) || pg.ops[i].src_b == kSrcRecv) due[pg.ops[i].wait_local].push_back(i);
       for (size_t oi = 0; oi < pg.ops.size(); ++oi) {
         for (size_t i : due[oi]) {
           const Op& ahead = pg.ops[i];
@@ -117,6 +121,9 @@ class ProgramSimulator {
         if (op.wait_credit != 0 &&
             !wait_for(me.credit[static_cast<size_t>(ch * kMaxRanks + op.peer_out)], op.wait_credit, "credit", oi))
           return;
+        if (op.wait_peer != 0 &&
+            !wait_for(me.told[static_cast<size_t>(ch * kMaxRanks + op.peer_in)], op.wait_peer, "arrival", oi))
+          return;
         T* stage_in = nullptr;
         if (op.src_a == kSrcStage)
           stage_in = reinterpret_cast<T*>(me.stage.data() + (static_cast<size_t>(op.region_in) * st.slots + op.slot_in) * st.slot_bytes);
@@ -126,17 +133,29 @@ class ProgramSimulator {
                                            (static_cast<size_t>(op.region_out) * st.slots + op.slot_out) * st.slot_bytes);
         for (uint64_t k = lo; k < hi; ++k) {
           const uint64_t g = op.cell_begin + k;
-          T v = op.src_a == kSrcStage ? stage_in[k] : (op.src_a == kSrcSend ? sendbuf[g] : early[oi][k - lo]);
+          T v;
+          switch (op.src_a) {
+            case kSrcStage: v = stage_in[k]; break;
+            case kSrcSend: v = sendbuf[g]; break;
+            case kSrcPeer: v = send_of(op.rank_a)[g]; break;
+            default: v = op.wait_peer != 0 ? recvbuf[g] : early[oi][k - lo];  // what a peer stored there, or this rank
+          }
+          if (op.rank_c >= 0) v = static_cast<T>(v + send_of(op.rank_c)[g]);
           if (op.src_b == kSrcSend) v = static_cast<T>(v + sendbuf[g]);
           else if (op.src_b == kSrcRecv) v = static_cast<T>(v + early[oi][k - lo]);
           if (op.flags & kOpScale) v = static_cast<T>(v * scale);
           if (op.flags & kOpStoreLocal) recvbuf[g] = v;
+          for (int q = 0; q < ws_; ++q)
+            if (op.store_peers >> q & 1) (*outputs)[static_cast<size_t>(q)][g] = v;
           if (stage_out != nullptr) stage_out[k] = v;
         }
         if (stage_in != nullptr) std::fill(stage_in + lo, stage_in + hi, T(-99));
         early[oi] = std::vector<T>();
         if (op.post_out != 0)
           mem[static_cast<size_t>(op.peer_out)].inflag[static_cast<size_t>(ch * kMaxRanks + r)].store(op.post_out, std::memory_order_release);
+        for (int m = 0; m < kMaxPeerPosts; ++m)
+          if (op.post_told[m] != 0)
+            mem[static_cast<size_t>(op.peer_told[m])].told[static_cast<size_t>(ch * kMaxRanks + r)].store(op.post_told[m], std::memory_order_release);
         if (op.post_credit != 0)
           mem[static_cast<size_t>(op.peer_in)].credit[static_cast<size_t>(ch * kMaxRanks + r)].store(op.post_credit, std::memory_order_release);
       }
@@ -157,6 +176,7 @@ class ProgramSimulator {
   const std::vector<Program>& programs() const { return programs_; }
 
  private:
+  bool shared_gpu_;
   Algo algo_;
   int ws_;
   size_t stage_bytes_;

@@ -51,6 +51,10 @@ struct ProgramRequest {
   uint64_t stage_offset = 0;      // where the staging area starts in the arena
   uint64_t stage_bytes = 0;       // how large it is
   bool apply_scale = false;
+  // One launch runs all ranks on one GPU and knows their buffers: a rank reads what it would be sent of another
+  // one's sendbuf there, and results go straight into the others' recvbuf.  Only partial sums pass through staging.
+  // What arrives last is not waited for, the launch's end is everybody's.
+  bool shared_gpu = false;
 };
 
 struct Program {

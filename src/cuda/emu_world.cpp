@@ -107,6 +107,18 @@ bool LinesPay(uint64_t bytes) {
   return bytes <= (static_cast<uint64_t>(std::max(0, Tunable("IBCOMM_LINES_MAX_KIB", 2048))) << 10);
 }
 
+// Whether an op program's ranks read each other's sendbuf and store into each other's recvbuf, or send as between
+// GPUs.  us, sending and sharing:
+//   Rabenseifner  2 x 64 MiB 70 56, 5 x 64 MiB 265 157, 7 x 64 MiB 458 227, 8 x 64 MiB 428 323, 8 x 8 MiB 74 59; bf16 wire
+//                 4 x 64 MiB 155 139; slices off the boundary 4 x 4 MiB 88 77
+//   ring          2 x 64 MiB 71 57, 3 x 64 MiB 117 99, 4 x 4 MiB 32 29, 5 x 4 MiB 40 37, 5 x 64 MiB 202 201, 6 x 8 MiB 61 56;
+//                 but 7 x 64 MiB 286 302, 8 x 256 MiB 1234 1331, with a ragged end 7 x 4 MB 56 66, off the boundary 80 93
+// The ring's transfers wait for each other, and a result that lies in recvbuf is there later than one in a slot.
+bool SharingPays(Algo algo, int ws, size_t bytes, bool whole_vectors) {
+  if (algo == Algo::kRabenseifner) return true;
+  return whole_vectors && (ws <= 4 || (ws <= 6 && bytes <= (size_t(16) << 20)));
+}
+
 }  // namespace
 
 EmuWorld::EmuWorld(int num_ranks, size_t pool_bytes, size_t work_bytes) : ws_(num_ranks), impl_(new Impl()) {
@@ -325,6 +337,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       for (int r = 0; r < m.ws; ++r) {
         const CachedProgram& cp = m.cache.Get(algo, r, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false, m.ws, form);
         fit = fit && LinesFit(cp.prog);
+        if (form == ProgramForm::kShared && cp.prog.ops.empty()) continue;  // an extra rank: the others read its sendbuf and store into its recvbuf
         ps.push_back(MakeExecParams(m.ranks[static_cast<size_t>(r)], cp, dtype, wire, sendbufs[static_cast<size_t>(r)],
                                     recvbufs[static_cast<size_t>(r)], n, scale, timeout_ns, nullptr, 0));
         if (r == m.silent_rank) ps.back().num_ops = 0;
@@ -345,14 +358,28 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       ch = std::max(1, std::min({ch, m.line_max_blocks / m.ws, kMaxChannels}));
       CUDACHECK(LaunchLineKernel(ps.data(), m.ws, ch, m.layout.lines_half_bytes, stream));
     } else {
-      programs(ProgramForm::kStaged);
+      const bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, all_aligned && bytes % 16 == 0);
+      programs(shared ? ProgramForm::kShared : ProgramForm::kStaged);
+      if (shared) {
+        uint32_t present = 0;
+        for (const ExecParams& p : ps) present |= 1u << p.rank;
+        for (ExecParams& p : ps) {
+          for (int q = 0; q < m.ws; ++q) {
+            p.peer_send[q] = sendbufs[static_cast<size_t>(q)];
+            p.peer_recv[q] = recvbufs[static_cast<size_t>(q)];
+          }
+          p.present = present;
+        }
+        ps.front().counts_for = ((1u << m.ws) - 1) & ~present;
+      }
+      const int rows = static_cast<int>(ps.size());
       // A channel for every 4 KiB of a transfer: the flags of ranks on one GPU are
       // cheap, and more channels shorten every step of the program.  One CTA per
       // SM at most (two smaller ones per SM are no faster).
       const uint64_t slot = ps.back().stage.slot_bytes;
       ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(slot / 4096, static_cast<uint64_t>(kMaxChannels)));
-      ch = std::max(1, std::min(ch, channels > 0 ? m.exec_max_blocks / m.ws : cap));
-      CUDACHECK(LaunchExecKernel(ps.data(), m.ws, ch, stream));
+      ch = std::max(1, std::min(ch, (channels > 0 ? m.exec_max_blocks : m.max_blocks) / rows));
+      CUDACHECK(LaunchExecKernel(ps.data(), rows, ch, stream));
     }
     m.last_channels = ch;
   }

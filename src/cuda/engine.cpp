@@ -247,6 +247,7 @@ const CachedProgram& ProgramCache::Get(Algo algo, int rank, int world_size, size
   req.stage_offset = stage_off;
   req.stage_bytes = stage_bytes;
   req.apply_scale = apply_scale;
+  req.shared_gpu = form == ProgramForm::kShared;
   std::unique_ptr<CachedProgram> cp(new CachedProgram());
   cp->prog = BuildProgram(req);
   cp->drop_lines = drop_lines;
@@ -297,6 +298,7 @@ ExecParams MakeExecParams(const RankResources& rr, const CachedProgram& cp, DTyp
   p.status = rr.d_status;
   p.doorbell = rr.d_doorbell;
   p.trace = trace;
+  p.present = (1u << rr.world_size) - 1;
   return p;
 }
 

@@ -46,6 +46,7 @@ struct StatusBlock {
 // How the ranks of a program hand over.
 enum class ProgramForm {
   kStaged,  // through slots of the pool and the work region, with flags and credits
+  kShared,  // the same for partial sums; else in the buffers of ranks that share a GPU (ProgramRequest::shared_gpu)
   kLines,   // through slots of the lines area, each used once (ll_kernel.cu); see LinesFit
 };
 // Whether a program runs as lines: one that does not is not to be launched that way.

@@ -37,6 +37,11 @@
 // 256 MiB 1.23 -> 1.25 ms).  Ranks sharing a B200, before and after:
 // Rabenseifner 5 x 64 MiB 908 -> 430 us, ring 8 x 32 MiB 258 -> 192 us, ring 7 x 4
 // MB 96 -> 70 us, ring 8 x 4 KiB 52 -> 46 us.
+// Programs of ranks that share a GPU (kShared) have ops with one to three sources, some
+// of them other ranks' buffers, and store into other ranks' recvbuf; a stage takes as many
+// packs as fit with that many sources.  5 ranks x 64 MiB Rabenseifner 271 -> 158 us, 7 x 64
+// MiB 458 -> 227, ring 2 x 64 MiB 71 -> 56.  The extra rank's work, the first step's sends
+// and the results' slots are gone: 64 block reads and writes a segment instead of 120.
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda
 // (ibcomm/allreduce_cuda_impl.h:24-33, 103-299, 470-707).
 //
@@ -59,9 +64,10 @@ namespace dev {
 
 constexpr int kExecServiceWarps = 3;  // waiter, loader, poster
 constexpr int kExecMaxStages = 10;
-// A stage holds U packs per data thread from each of two sources: 128 bytes per
-// data thread for every pair of types.  Half of that leaves a warp waiting for
-// its own shared-memory reads (5 ranks x 64 MiB Rabenseifner 496 us against 430).
+// A stage holds U packs per data thread from each of two sources, 2 U from one or
+// U / 2 from three: 128 bytes per data thread for every pair of types (96 with three).
+// Half of that leaves a warp waiting for its own shared-memory reads (5 ranks x 64 MiB
+// Rabenseifner 496 us against 430).
 constexpr int kExecStageBytesPerThread = 128;
 
 enum ExecTileFlags : uint32_t {
@@ -73,9 +79,32 @@ enum ExecTileFlags : uint32_t {
   kTileElements = 32,  // nothing in the stage: elements [lo, hi) of the op's cell, one by one
   kTileExit = 64,      // the program is over
   kTileReadBack = 128,  // the local store is read back by a later op
+  kTileThird = 256,     // source c is present
+  kTileRoundPeer = 512,  // source c, and a unless it is from staging, are rounded through the wire type
+  kTilePeersReadBack = 1024,  // what goes into other ranks' recvbuf is read there by a later op
+  kTilePeersShift = 16,  // from here up: the ranks whose recvbuf the value goes into, a bit each
 };
+// What there is of a stage and of an op only where ranks share a GPU.
+template <bool kShared>
+struct ExecTileMore {};
+template <>
+struct ExecTileMore<true> {
+  const unsigned char* tail_c;
+  uint64_t recv_off;  // where the first pack lies in every recvbuf, in bytes
+  uint32_t stride;    // 16-byte vectors of the stage from one source to the next
+};
+template <bool kShared>
+struct ExecPlanMore {};
+template <>
+struct ExecPlanMore<true> {
+  const unsigned char* src_c;
+  uint64_t recv_off;
+  uint32_t late;  // source a is another rank's work: it is there when the op's flags are
+};
+
 // What the data warps do with one stage.
-struct ExecTile {
+template <bool kShared>
+struct ExecTile : ExecTileMore<kShared> {
   uint4* local;   // recvbuf, or null
   uint4* remote;  // the next rank's staging slot, or null
   uint32_t packs;  // the one with only `tail` elements included
@@ -88,11 +117,11 @@ struct ExecTile {
   // Whole lines of the staging slot that the stage came from, to be dropped from L2.
   unsigned char* drop;
   uint32_t drop_lines;
-  uint32_t pad_;
 };
 
 // One op of this channel, worked out by a lane of the loader's warp.
-struct ExecPlan {
+template <bool kShared>
+struct ExecPlan : ExecPlanMore<kShared> {
   const unsigned char* src_a;  // address of the first pack (for staging: in the wire type)
   const unsigned char* src_b;
   unsigned char* local;
@@ -105,10 +134,11 @@ struct ExecPlan {
   uint32_t pad_;
 };
 
+template <bool kShared>
 struct ExecShared {
   RoleSync role;  // ready: ops whose flags have arrived; done[w]: ops whose stores data warp w has issued
-  ExecTile tile[kExecMaxStages];
-  ExecPlan plan[32];
+  ExecTile<kShared> tile[kExecMaxStages];
+  ExecPlan<kShared> plan[32];
   uint64_t full[kExecMaxStages];   // the stage's copies have landed and its op may store
   uint64_t empty[kExecMaxStages];  // every data warp has read the stage
 };
@@ -131,8 +161,8 @@ __device__ __forceinline__ bool RingWait(uint64_t* bar, uint32_t parity, RoleSyn
 // stage when source a comes from staging; the user's buffers are accessed up to
 // the message's end.  A slot's pack is written whole: it lies in this channel's
 // part of the slot, and nobody reads past the message's end either.
-template <typename T, typename W>
-__device__ __noinline__ void RunTailPack(const ExecTile* t, const uint4* staged, double scale) {
+template <typename T, typename W, bool kShared>
+__device__ __noinline__ void RunTailPack(const ExecTile<kShared>* t, const uint4* staged, const ExecParams& p) {
   using Tr = ExecTraits<T, W>;
   using A = typename Tr::A;
   constexpr int P = Tr::P;
@@ -141,11 +171,21 @@ __device__ __noinline__ void RunTailPack(const ExecTile* t, const uint4* staged,
 #pragma unroll
   for (int v = 0; v < Tr::VW; ++v)
     if (t->flags & kTileFromStaging) VecIO<W>::Load(staged[v], acc + v * VecIO<W>::kN);
+  const bool round_peer = kShared && (t->flags & kTileRoundPeer) && sizeof(W) != sizeof(T);
 #pragma unroll
   for (int e = 0; e < P; ++e) {
-    if (!(t->flags & kTileFromStaging)) acc[e] = e < n ? ToAcc<A, T>(reinterpret_cast<const T*>(t->tail_a)[e]) : A(0);
+    if (!(t->flags & kTileFromStaging)) {
+      acc[e] = e < n ? ToAcc<A, T>(reinterpret_cast<const T*>(t->tail_a)[e]) : A(0);
+      if (round_peer) acc[e] = ThroughWire<W, A>(acc[e]);
+    }
+    if constexpr (kShared) {
+      if ((t->flags & kTileThird) && e < n) {
+        const A c = ToAcc<A, T>(reinterpret_cast<const T*>(t->tail_c)[e]);
+        acc[e] += round_peer ? ThroughWire<W, A>(c) : c;
+      }
+    }
     if ((t->flags & kTileAdd) && e < n) acc[e] += ToAcc<A, T>(reinterpret_cast<const T*>(t->tail_b)[e]);
-    if (t->flags & kTileScale) acc[e] = ScaleAcc<A>(acc[e], scale);
+    if (t->flags & kTileScale) acc[e] = ScaleAcc<A>(acc[e], p.scale);
   }
   uint4 wq[Tr::VW];
 #pragma unroll
@@ -155,116 +195,166 @@ __device__ __noinline__ void RunTailPack(const ExecTile* t, const uint4* staged,
 #pragma unroll
     for (int v = 0; v < Tr::VW; ++v) St16(t->remote + at * Tr::VW + v, wq[v]);
   }
-  if (t->local != nullptr) {
-    if ((t->flags & kTileRoundWire) && sizeof(W) != sizeof(T)) {
+  if ((t->flags & kTileRoundWire) && sizeof(W) != sizeof(T)) {
 #pragma unroll
-      for (int v = 0; v < Tr::VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
-    }
-    T* const out = reinterpret_cast<T*>(t->local + at * Tr::VT);
+    for (int v = 0; v < Tr::VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
+  }
+  auto store = [&](T* out) {
 #pragma unroll
     for (int e = 0; e < P; ++e)
       if (e < n) out[e] = FromAcc<T, A>(acc[e]);
+  };
+  if (t->local != nullptr) store(reinterpret_cast<T*>(t->local + at * Tr::VT));
+  if constexpr (kShared) {
+    for (int q = 0; q < p.world_size; ++q)
+      if (t->flags >> (kTilePeersShift + q) & 1u) store(reinterpret_cast<T*>(static_cast<unsigned char*>(p.peer_recv[q]) + t->recv_off + static_cast<uint64_t>(at) * Tr::VT * 16u));
   }
 }
 
-// One stage: packs of P elements, U of them per thread.  `tile` is `t` in shared memory.
-template <typename T, typename W>
-__device__ __forceinline__ void RunTile(const ExecTile& t, const ExecTile* tile, const uint4* stage, uint32_t b_off, double scale, uint64_t* empty, uint64_t local_policy, unsigned tid,
-                                        unsigned nthr, int lane) {
+// One stage: packs of P elements, U of them per thread and turn.  `tile` is `t` in shared memory.
+template <typename T, typename W, bool kShared>
+__device__ __forceinline__ void RunTile(const ExecTile<kShared>& t, const ExecTile<kShared>* tile, const uint4* stage, const ExecParams& p, uint64_t* empty,
+                                        uint64_t read_back_policy, uint64_t final_policy, unsigned tid, unsigned nthr, int lane) {
   using Tr = ExecTraits<T, W>;
   using A = typename Tr::A;
   constexpr int P = Tr::P, U = Tr::U, VT = Tr::VT, VW = Tr::VW;
-  const bool from_staging = (t.flags & kTileFromStaging) != 0, add = (t.flags & kTileAdd) != 0;
+  constexpr bool kCasts = sizeof(W) != sizeof(T);
+  const bool from_staging = (t.flags & kTileFromStaging) != 0, add = (t.flags & kTileAdd) != 0, third = kShared && (t.flags & kTileThird) != 0;
+  const bool round_peer = kShared && kCasts && (t.flags & kTileRoundPeer) != 0, round_wire = kCasts && (t.flags & kTileRoundWire) != 0;
   const uint32_t whole = t.packs - (t.tail != 0 ? 1u : 0u);
-  uint4 qa[U][VT], qb[U][VT];
+  uint32_t peers = 0, stride = nthr * U * VT;
+  uint64_t recv_off = 0;
+  if constexpr (kShared) peers = t.flags >> kTilePeersShift, stride = t.stride, recv_off = t.recv_off;
+  const uint64_t local_policy = (t.flags & kTileReadBack) ? read_back_policy : final_policy;
+  const uint64_t peers_policy = (t.flags & kTilePeersReadBack) ? read_back_policy : final_policy;
+  for (unsigned l = tid; l < t.drop_lines; l += nthr) DiscardLine(t.drop + static_cast<size_t>(l) * 128u);
+  // One turn, or two where there is one source.
+  unsigned at = tid;
+  for (bool more = true; more; at += U * nthr) {
+    more = kShared && at - tid + U * nthr < whole;  // else a stage holds one turn
+    uint4 qa[U][VT], qb[U][VT], qc[U / 2][VT];
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const unsigned i = tid + static_cast<unsigned>(u) * nthr;
-    if (i < whole) {
-      if (from_staging) {
+    for (int u = 0; u < U; ++u) {
+      const unsigned i = at + static_cast<unsigned>(u) * nthr;
+      if (i < whole) {
+        if (from_staging) {
 #pragma unroll
-        for (int v = 0; v < VW; ++v) qa[u][v] = stage[i * VW + v];
-      } else {
+          for (int v = 0; v < VW; ++v) qa[u][v] = stage[i * VW + v];
+        } else {
 #pragma unroll
-        for (int v = 0; v < VT; ++v) qa[u][v] = stage[i * VT + v];
-      }
-      if (add) {
+          for (int v = 0; v < VT; ++v) qa[u][v] = stage[i * VT + v];
+        }
+        if (add) {
 #pragma unroll
-        for (int v = 0; v < VT; ++v) qb[u][v] = stage[b_off + i * VT + v];
+          for (int v = 0; v < VT; ++v) qb[u][v] = stage[stride + i * VT + v];
+        }
+        if (u < U / 2 && third) {
+#pragma unroll
+          for (int v = 0; v < VT; ++v) qc[u % (U / 2)][v] = stage[2 * stride + i * VT + v];
+        }
       }
     }
-  }
-  for (unsigned l = tid; l < t.drop_lines; l += nthr) DiscardLine(t.drop + static_cast<size_t>(l) * 128u);
-  // The stage is free for the loader once every warp has read it.
-  if (t.tail == 0) {
-    __syncwarp();
-    if (lane == 0) MbarArrive(empty);
-  }
+    // The stage is free for the loader once every warp has read it.
+    if (!more && t.tail == 0) {
+      __syncwarp();
+      if (lane == 0) MbarArrive(empty);
+    }
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const unsigned i = tid + static_cast<unsigned>(u) * nthr;
-    if (i < whole) {
-      A acc[P];
-      if (from_staging) {
+    for (int u = 0; u < U; ++u) {
+      const unsigned i = at + static_cast<unsigned>(u) * nthr;
+      if (i < whole) {
+        A acc[P];
+        if (from_staging) {
 #pragma unroll
-        for (int v = 0; v < VW; ++v) VecIO<W>::Load(qa[u][v], acc + v * VecIO<W>::kN);
-      } else {
+          for (int v = 0; v < VW; ++v) VecIO<W>::Load(qa[u][v], acc + v * VecIO<W>::kN);
+        } else {
 #pragma unroll
-        for (int v = 0; v < VT; ++v) VecIO<T>::Load(qa[u][v], acc + v * VecIO<T>::kN);
-      }
-      if (add) {
+          for (int v = 0; v < VT; ++v) VecIO<T>::Load(qa[u][v], acc + v * VecIO<T>::kN);
+          if (round_peer) {
 #pragma unroll
-        for (int v = 0; v < VT; ++v) VecIO<T>::Add(qb[u][v], acc + v * VecIO<T>::kN);
-      }
-      if (t.flags & kTileScale) {
-#pragma unroll
-        for (int e = 0; e < P; ++e) acc[e] = ScaleAcc<A>(acc[e], scale);
-      }
-      uint4 wq[VW];
-      if (t.remote != nullptr || (t.flags & kTileRoundWire)) {
-#pragma unroll
-        for (int v = 0; v < VW; ++v) wq[v] = VecIO<W>::Store(acc + v * VecIO<W>::kN);
-      }
-      if (t.remote != nullptr) {
-#pragma unroll
-        for (int v = 0; v < VW; ++v) St16(t.remote + i * VW + v, wq[v]);
-      }
-      if (t.local != nullptr) {
-        if ((t.flags & kTileRoundWire) && sizeof(W) != sizeof(T)) {
-#pragma unroll
-          for (int v = 0; v < VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
+            for (int e = 0; e < P; ++e) acc[e] = ThroughWire<W, A>(acc[e]);
+          }
         }
+        if (u < U / 2 && third) {
+          A c[P];
 #pragma unroll
-        for (int v = 0; v < VT; ++v) St16Hint(t.local + i * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), local_policy);
+          for (int v = 0; v < VT; ++v) VecIO<T>::Load(qc[u % (U / 2)][v], c + v * VecIO<T>::kN);
+#pragma unroll
+          for (int e = 0; e < P; ++e) acc[e] += round_peer ? ThroughWire<W, A>(c[e]) : c[e];
+        }
+        if (add) {
+#pragma unroll
+          for (int v = 0; v < VT; ++v) VecIO<T>::Add(qb[u][v], acc + v * VecIO<T>::kN);
+        }
+        if (t.flags & kTileScale) {
+#pragma unroll
+          for (int e = 0; e < P; ++e) acc[e] = ScaleAcc<A>(acc[e], p.scale);
+        }
+        uint4 wq[VW];
+        if (t.remote != nullptr || round_wire) {
+#pragma unroll
+          for (int v = 0; v < VW; ++v) wq[v] = VecIO<W>::Store(acc + v * VecIO<W>::kN);
+        }
+        if (t.remote != nullptr) {
+#pragma unroll
+          for (int v = 0; v < VW; ++v) St16(t.remote + i * VW + v, wq[v]);
+        }
+        if (t.local != nullptr || peers != 0) {
+          if (round_wire) {
+#pragma unroll
+            for (int v = 0; v < VW; ++v) VecIO<W>::Load(wq[v], acc + v * VecIO<W>::kN);
+          }
+          uint4 out[VT];
+#pragma unroll
+          for (int v = 0; v < VT; ++v) out[v] = VecIO<T>::Store(acc + v * VecIO<T>::kN);
+          if (t.local != nullptr) {
+#pragma unroll
+            for (int v = 0; v < VT; ++v) St16Hint(t.local + i * VT + v, out[v], local_policy);
+          }
+          if (kShared && peers != 0) {
+#pragma unroll
+            for (int q = 0; q < kMaxRanks; ++q) {
+              if (peers >> q & 1u) {
+                uint4* const dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(p.peer_recv[q]) + recv_off);
+#pragma unroll
+                for (int v = 0; v < VT; ++v) St16Hint(dst + i * VT + v, out[v], peers_policy);
+              }
+            }
+          }
+        }
       }
     }
   }
   if (t.tail != 0) {
-    if (whole % nthr == tid) RunTailPack<T, W>(tile, stage + whole * VW, scale);
+    if (whole % nthr == tid) RunTailPack<T, W, kShared>(tile, stage + whole * VW, p);
     __syncwarp();
     if (lane == 0) MbarArrive(empty);
   }
 }
 
-// Element-at-a-time path for chunks that do not start on a 16-byte boundary
-// and for the few elements after the last whole pack; kU loads of each source
-// in flight per thread.
-template <typename T, typename W>
+// Element-at-a-time path for chunks that do not start on a 16-byte boundary;
+// kU loads of each source in flight per thread.
+template <typename T, typename W, bool kShared>
 __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint64_t hi, unsigned tid, unsigned nthr) {
   using A = typename Acc<T>::type;
   constexpr int kU = 8;
   const OpBuffers<T, W> buf(op, p);
+  const T* a_src = op.src_a == kSrcSend ? buf.sendbuf : (kShared && op.src_a == kSrcPeer ? static_cast<const T*>(p.peer_send[op.rank_a]) : buf.recvbuf);
   const T* b_src = op.src_b == kSrcSend ? buf.sendbuf : (op.src_b == kSrcRecv ? buf.recvbuf : nullptr);
+  const T* c_src = kShared && op.rank_c >= 0 ? static_cast<const T*>(p.peer_send[op.rank_c]) : nullptr;
+  const bool round_peer = kShared && (op.flags & kOpRoundPeer) && sizeof(W) != sizeof(T);
+  auto of_peer = [&](T v) -> A { return round_peer ? ThroughWire<W, A>(ToAcc<A, T>(v)) : ToAcc<A, T>(v); };
   for (uint64_t k0 = lo + tid; k0 < hi; k0 += static_cast<uint64_t>(nthr) * kU) {
     A a[kU];
-    T b[kU];
+    T b[kU], c[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const uint64_t k = k0 + static_cast<uint64_t>(u) * nthr;
       if (k < hi) {
         if (op.src_a == kSrcStage) a[u] = ToAcc<A, W>(LdScalarStrong<W>(buf.stage_in + k));
-        else a[u] = ToAcc<A, T>((op.src_a == kSrcSend ? buf.sendbuf : buf.recvbuf)[op.cell_begin + k]);
+        else a[u] = kShared && op.src_a == kSrcPeer ? of_peer(a_src[op.cell_begin + k]) : (kShared && op.src_a == kSrcRecv ? ToAcc<A, T>(LdScalarStrong<T>(a_src + op.cell_begin + k)) : ToAcc<A, T>(a_src[op.cell_begin + k]));
         if (b_src != nullptr) b[u] = b_src[op.cell_begin + k];
+        if (c_src != nullptr) c[u] = c_src[op.cell_begin + k];
       }
     }
 #pragma unroll
@@ -272,11 +362,14 @@ __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint
       const uint64_t k = k0 + static_cast<uint64_t>(u) * nthr;
       if (k < hi) {
         A v = a[u];
+        if (c_src != nullptr) v += of_peer(c[u]);
         if (b_src != nullptr) v += ToAcc<A, T>(b[u]);
         if (op.flags & kOpScale) v = ScaleAcc<A>(v, p.scale);
-        if ((op.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) v = ToAcc<A, W>(FromAcc<W, A>(v));
+        if ((op.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) v = ThroughWire<W, A>(v);
         if (op.flags & kOpStoreLocal) buf.recvbuf[op.cell_begin + k] = FromAcc<T, A>(v);
         if (op.flags & kOpStoreRemote) buf.stage_out[k] = FromAcc<W, A>(v);
+        for (int q = 0; kShared && q < p.world_size; ++q)
+          if (op.store_peers >> q & 1) static_cast<T*>(p.peer_recv[q])[op.cell_begin + k] = FromAcc<T, A>(v);
       }
     }
   }
@@ -295,12 +388,11 @@ struct RingPos {
 // The lanes work out 32 ops at a time (an op is a 64-byte load and a division,
 // 1.5 us one after the other); lane 0 then only issues copies.  Returns after it
 // has handed out the exit stage (or could not, because the data warps gave up).
-template <typename T, typename W>
-__device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* smem, int stages, int ch, int nch, int data_warps, int lane) {
+template <typename T, typename W, bool kShared>
+__device__ void LoaderBody(const ExecParams& p, ExecShared<kShared>* sh, unsigned char* smem, int stages, int ch, int nch, int data_warps, int lane) {
   using Tr = ExecTraits<T, W>;
   const unsigned nthr = static_cast<unsigned>(data_warps) * 32u;
-  const uint32_t tile_packs = nthr * Tr::U;
-  const uint32_t half_bytes = tile_packs * Tr::VT * 16u;  // source a, then source b
+  const uint32_t stage_bytes = nthr * static_cast<uint32_t>(kExecStageBytesPerThread);
   // The user's data is read once, sendbuf and what is read back from recvbuf.
   const uint64_t user_policy = PolicyEvictFirst();
   RingPos pos(stages);
@@ -328,7 +420,7 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
     bool in_bounds = true;
     if (lane < in_batch) {
       const Op op = p.ops[first + lane];
-      in_bounds = OpInBounds<W>(op, p);
+      in_bounds = OpInBounds<W, kShared>(op, p);
       if (in_bounds) {
         uint64_t lo, hi;
         ChannelSlice(op.elem_begin - op.cell_begin, op.elem_count, p.stage.slot_bytes / sizeof(W), nch, ch, &lo, &hi);
@@ -336,7 +428,11 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
         const uint64_t g0 = op.cell_begin + lo;
         const bool uses_send = op.src_a == kSrcSend || op.src_b == kSrcSend;
         const bool uses_recv = op.src_a == kSrcRecv || op.src_b == kSrcRecv || (op.flags & kOpStoreLocal);
-        uintptr_t bits = 0;
+        const T* const peer_a = kShared && op.src_a == kSrcPeer ? static_cast<const T*>(p.peer_send[op.rank_a]) + g0 : nullptr;
+        const T* const peer_c = kShared && op.rank_c >= 0 ? static_cast<const T*>(p.peer_send[op.rank_c]) + g0 : nullptr;
+        uintptr_t bits = reinterpret_cast<uintptr_t>(peer_a) | reinterpret_cast<uintptr_t>(peer_c);
+        for (int q = 0; kShared && q < p.world_size; ++q)
+          if (op.store_peers >> q & 1) bits |= reinterpret_cast<uintptr_t>(static_cast<T*>(p.peer_recv[q]) + g0);
         if (uses_send) bits |= reinterpret_cast<uintptr_t>(buf.sendbuf + g0);
         if (uses_recv) bits |= reinterpret_cast<uintptr_t>(buf.recvbuf + g0);
         // The place inside a staging slot follows the cell, not the user buffer: a
@@ -347,11 +443,17 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
         auto source = [&](uint8_t src) -> const unsigned char* {
           if (src == kSrcStage) return reinterpret_cast<const unsigned char*>(buf.stage_in + lo);
           if (src == kSrcNone) return nullptr;
+          if (src == kSrcPeer) return reinterpret_cast<const unsigned char*>(peer_a);
           return reinterpret_cast<const unsigned char*>((src == kSrcSend ? buf.sendbuf : buf.recvbuf) + g0);
         };
-        ExecPlan& pl = sh->plan[lane];
+        ExecPlan<kShared>& pl = sh->plan[lane];
         pl.src_a = source(op.src_a);
         pl.src_b = source(op.src_b);
+        if constexpr (kShared) {
+          pl.src_c = reinterpret_cast<const unsigned char*>(peer_c);
+          pl.recv_off = g0 * sizeof(T);
+          pl.late = op.src_a == kSrcStage || op.wait_peer != 0 ? 1 : 0;
+        }
         pl.local = (op.flags & kOpStoreLocal) ? reinterpret_cast<unsigned char*>(buf.recvbuf + g0) : nullptr;
         pl.remote = buf.stage_out != nullptr ? reinterpret_cast<unsigned char*>(buf.stage_out + lo) : nullptr;
         const bool in_packs = lo < hi && (bits & 15u) == 0;
@@ -361,7 +463,9 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
         pl.hi = hi;
         pl.flags = (op.src_a == kSrcStage ? kTileFromStaging : 0u) | (op.src_b != kSrcNone ? kTileAdd : 0u) |
                    ((op.flags & kOpScale) ? kTileScale : 0u) | ((op.flags & kOpRoundWire) ? kTileRoundWire : 0u) |
-                   ((op.flags & kOpReadBack) ? kTileReadBack : 0u);
+                   ((op.flags & kOpReadBack) ? kTileReadBack : 0u) | (peer_c != nullptr ? kTileThird : 0u) |
+                   ((op.flags & kOpRoundPeer) ? kTileRoundPeer : 0u) | ((op.flags & kOpPeersReadBack) ? kTilePeersReadBack : 0u) |
+                   (static_cast<uint32_t>(op.store_peers) << kTilePeersShift);
         pl.wait_local = op.wait_local;
       }
     }
@@ -387,7 +491,7 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
       }
       int alive = 1;
       if (lane == 0) {
-        const ExecPlan pl = sh->plan[k];
+        const ExecPlan<kShared> pl = sh->plan[k];
         // The flags of op `oi` have arrived: one look may cover several ops, and
         // one proxy fence what all of them read from staging (written by
         // ordinary stores of the peers that the waiter's acquire made visible).
@@ -401,16 +505,29 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
         const bool a_staged = (pl.flags & kTileFromStaging) != 0;
         const bool drop = p.drop_lines != 0;
         const uint64_t a_step = static_cast<uint64_t>(a_staged ? Tr::VW : Tr::VT) * 16u;
+        const unsigned char* src_c = nullptr;
+        bool late = a_staged;
+        uint32_t tile_packs = nthr * Tr::U;
+        if constexpr (kShared) {
+          src_c = pl.src_c;
+          late = pl.late != 0;
+          tile_packs = nthr * static_cast<uint32_t>(src_c != nullptr ? Tr::U / 2 : (pl.src_b != nullptr ? Tr::U : 2 * Tr::U));
+        }
+        const uint32_t source_bytes = tile_packs * Tr::VT * 16u;
         for (uint64_t j = 0; j < pl.packs; j += tile_packs) {
           if (!next_stage()) {
             alive = -1;
             break;
           }
           const uint32_t n = pl.packs - j < tile_packs ? static_cast<uint32_t>(pl.packs - j) : tile_packs;
-          unsigned char* dst = smem + static_cast<size_t>(s) * 2 * half_bytes;
-          ExecTile& t = sh->tile[s];
+          unsigned char* dst = smem + static_cast<size_t>(s) * stage_bytes;
+          ExecTile<kShared>& t = sh->tile[s];
           t.local = pl.local != nullptr ? reinterpret_cast<uint4*>(pl.local + j * Tr::VT * 16u) : nullptr;
           t.remote = pl.remote != nullptr ? reinterpret_cast<uint4*>(pl.remote + j * Tr::VW * 16u) : nullptr;
+          if constexpr (kShared) {
+            t.recv_off = pl.recv_off + j * Tr::VT * 16u;
+            t.stride = source_bytes / 16u;
+          }
           t.packs = n;
           t.op = oi;
           const bool last = j + n >= pl.packs;
@@ -427,18 +544,18 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           if (t.tail != 0) {
             t.tail_a = pl.src_a + (j + whole) * Tr::VT * 16u;
             t.tail_b = pl.src_b + (j + whole) * Tr::VT * 16u;
+            if constexpr (kShared) t.tail_c = src_c + (j + whole) * Tr::VT * 16u;
           }
           // What does not depend on a peer first, then the op's flags, then the staging slot.
           // The user's buffers end where the message ends; a slot holds whole packs.
           const uint32_t user_bytes = whole * Tr::VT * 16u, a_bytes = n * static_cast<uint32_t>(a_step);
-          if (pl.src_b != nullptr && whole != 0) {
+          auto load_user = [&](uint32_t source, const unsigned char* from) {
             MbarExpectTxOnly(&sh->full[s], user_bytes);
-            BulkLoadHint(dst + half_bytes, pl.src_b + j * Tr::VT * 16u, user_bytes, &sh->full[s], user_policy);
-          }
-          if (!a_staged && whole != 0) {
-            MbarExpectTxOnly(&sh->full[s], user_bytes);
-            BulkLoadHint(dst, pl.src_a + j * a_step, user_bytes, &sh->full[s], user_policy);
-          }
+            BulkLoadHint(dst + source * source_bytes, from + j * Tr::VT * 16u, user_bytes, &sh->full[s], user_policy);
+          };
+          if (pl.src_b != nullptr && whole != 0) load_user(1, pl.src_b);
+          if (src_c != nullptr && whole != 0) load_user(2, src_c);
+          if (!late && whole != 0) load_user(0, pl.src_a);
           if (!get_ready()) {
             alive = 0;
             break;
@@ -446,6 +563,8 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           if (a_staged) {
             MbarExpectTxOnly(&sh->full[s], a_bytes);
             BulkLoad(dst, pl.src_a + j * a_step, a_bytes, &sh->full[s]);
+          } else if (late && whole != 0) {
+            load_user(0, pl.src_a);
           }
           MbarArrive(&sh->full[s]);
         }
@@ -456,7 +575,7 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
           } else if (!get_ready()) {
             alive = 0;
           } else {
-            ExecTile& t = sh->tile[s];
+            ExecTile<kShared>& t = sh->tile[s];
             t.flags = kTileElements | kTileLastOfOp;
             t.op = oi;
             t.lo = pl.lo;
@@ -476,37 +595,39 @@ __device__ void LoaderBody(const ExecParams& p, ExecShared* sh, unsigned char* s
 }
 
 // The waiter: a warp that looks at all of this channel's flags at once (lane q:
-// data from rank q, lane 8 + q: credit from rank q) and releases every op whose
+// data from rank q, lane 8 + q: credit from rank q, lane 16 + q: rank q's stores into
+// recvbuf) and releases every op whose
 // flags are there.  Lane k holds op first + k.
-template <typename W>
+template <typename W, bool kShared>
 __device__ void WaiterBody(const ExecParams& p, const WaitCtx& w, RoleSync* sync, uint64_t base, int ch, int lane, DeviceTraceRec* trace) {
   static_assert(kMaxRanks == 8, "one lane per flag");
   ControlPage* const me = Ctl(p.peers, p.rank);
-  const uint64_t* const my_flag = lane < 8 ? &me->inflag[ch][lane] : &me->credit[ch][lane & 7];
-  const bool watches = lane < 16 && (lane & 7) < p.world_size;
+  const uint64_t* const my_flag = lane < 8 ? &me->inflag[ch][lane] : (lane < 16 ? &me->credit[ch][lane & 7] : &me->bar[ch][lane & 7]);
+  const bool watches = lane < (kShared ? 24 : 16) && (lane & 7) < p.world_size;
   const bool one_gpu = p.peers.one_gpu != 0;
   const uint64_t* const abort_word = &me->abort_seq;
   uint64_t seen = 0;
   for (int first = 0; first < p.num_ops; first += 32) {
     const int mine = first + lane;
-    uint64_t need_data = 0, need_credit = 0;
-    int from = 0, to = 0;
+    uint64_t need_data = 0, need_credit = 0;  // of data: a transfer into staging, or a store into recvbuf
+    int from = 0, to = 0;                     // lanes that look at it
     bool bad = false;
     uint64_t elem_begin = 0, elem_count = 0;
     if (mine < p.num_ops) {
       const Op op = p.ops[mine];
-      bad = !OpInBounds<W>(op, p);
+      bad = !OpInBounds<W, kShared>(op, p);
       elem_begin = op.elem_begin;
       elem_count = op.elem_count;
       if (!bad && op.wait_in != 0) need_data = base | op.wait_in, from = op.peer_in;
-      if (!bad && op.wait_credit != 0) need_credit = base | op.wait_credit, to = op.peer_out;
+      if (!bad && op.wait_peer != 0) need_data = (base | 1u) + op.wait_peer, from = 16 + op.peer_in;
+      if (!bad && op.wait_credit != 0) need_credit = base | op.wait_credit, to = 8 + op.peer_out;
     }
     const int in_batch = p.num_ops - first < 32 ? p.num_ops - first : 32;
     int released = 0;
     uint64_t t0 = GlobalTimerNs();
     for (uint32_t spin = 0; released < in_batch; ++spin) {
       if (watches) seen = LdAcquirePeers(my_flag, one_gpu);
-      const uint64_t data = __shfl_sync(0xffffffffu, seen, from), credit = __shfl_sync(0xffffffffu, seen, 8 + to);
+      const uint64_t data = __shfl_sync(0xffffffffu, seen, from), credit = __shfl_sync(0xffffffffu, seen, to);
       const bool go = !bad && (need_data == 0 || data >= need_data) && (need_credit == 0 || credit >= need_credit);
       const unsigned blocked = ~__ballot_sync(0xffffffffu, go || lane < released);
       const int upto = blocked == 0 ? 32 : __ffs(static_cast<int>(blocked)) - 1;
@@ -530,10 +651,10 @@ __device__ void WaiterBody(const ExecParams& p, const WaitCtx& w, RoleSync* sync
           const bool on_data = need_data != 0 && data < need_data;
           const uint32_t kind = on_data ? kWaitData : kWaitCredit;
           if (LdRelaxedSys(abort_word) == w.seq) {
-            ReportFailure(w, kStatusPeerAbort, kind, on_data ? from : to, mine, on_data ? need_data : need_credit, on_data ? data : credit);
+            ReportFailure(w, kStatusPeerAbort, kind, (on_data ? from : to) & 7, mine, on_data ? need_data : need_credit, on_data ? data : credit);
             give_up = 1;
           } else if (GlobalTimerNs() - t0 > p.timeout_ns) {
-            ReportFailure(w, kStatusWaitTimeout, kind, on_data ? from : to, mine, on_data ? need_data : need_credit, on_data ? data : credit);
+            ReportFailure(w, kStatusWaitTimeout, kind, (on_data ? from : to) & 7, mine, on_data ? need_data : need_credit, on_data ? data : credit);
             BroadcastAbort(w);
             give_up = 1;
           }
@@ -550,8 +671,8 @@ __device__ void WaiterBody(const ExecParams& p, const WaitCtx& w, RoleSync* sync
 
 // Body of the executor for one CTA: warps [0, data_warps) move data, then the
 // waiter's, the loader's and the poster's warp.
-template <typename T, typename W>
-__device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsigned char* smem, int stages) {
+template <typename T, typename W, bool kShared>
+__device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared<kShared>* sh, unsigned char* smem, int stages) {
   using Tr = ExecTraits<T, W>;
   const int ch = blockIdx.x, nch = gridDim.x;
   RoleSync* const sync = &sh->role;
@@ -570,7 +691,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
 
   // Entry barrier per channel: every peer's channel `ch` has started this
   // call, hence finished the previous one, so staging slots are free.
-  if (threadIdx.x < p.world_size && threadIdx.x != p.rank) {
+  if (threadIdx.x < p.world_size && threadIdx.x != p.rank && (p.present >> threadIdx.x & 1u)) {
     StReleasePeers(&Ctl(p.peers, threadIdx.x)->bar[ch][p.rank], base | 1u, p.peers.one_gpu != 0);
     if (!WaitGE(&me->bar[ch][threadIdx.x], base | 1u, w, kWaitBarrier, threadIdx.x, -1)) *stop = 1;
   }
@@ -581,7 +702,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
   const int data_warps = static_cast<int>(blockDim.x) / 32 - kExecServiceWarps;
   const int warp = static_cast<int>(threadIdx.x) / 32, lane = static_cast<int>(threadIdx.x) % 32;
   const unsigned nthr = static_cast<unsigned>(data_warps) * 32u;
-  const uint32_t half_vecs = nthr * Tr::U * Tr::VT;
+  const uint32_t stage_vecs = nthr * kExecStageBytesPerThread / 16u;
 
   if (warp < data_warps) {
     // A result nobody reads back should leave L2 before the staging slots and the partial
@@ -590,15 +711,15 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
     for (RingPos pos(stages);; pos.Next()) {
       const uint32_t s = pos.s;
       if (!RingWait(&sh->full[s], pos.parity, sync, p.timeout_ns)) break;
-      const ExecTile t = sh->tile[s];
+      const ExecTile<kShared> t = sh->tile[s];
       if (t.flags & kTileExit) break;
       if (t.flags & kTileElements) {
         __syncwarp();
         if (lane == 0) MbarArrive(&sh->empty[s]);
-        RunElements<T, W>(p.ops[t.op], p, t.lo, t.hi, threadIdx.x, nthr);
+        RunElements<T, W, kShared>(p.ops[t.op], p, t.lo, t.hi, threadIdx.x, nthr);
       } else {
-        RunTile<T, W>(t, &sh->tile[s], reinterpret_cast<const uint4*>(smem) + static_cast<size_t>(s) * 2 * half_vecs, half_vecs, p.scale, &sh->empty[s],
-                      (t.flags & kTileReadBack) ? partial_policy : final_policy, threadIdx.x, nthr, lane);
+        RunTile<T, W, kShared>(t, &sh->tile[s], reinterpret_cast<const uint4*>(smem) + static_cast<size_t>(s) * stage_vecs, p, &sh->empty[s],
+                      partial_policy, final_policy, threadIdx.x, nthr, lane);
       }
       if (t.flags & kTileLastOfOp) {
         __syncwarp();
@@ -606,22 +727,26 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
       }
     }
   } else if (warp == data_warps) {
-    WaiterBody<W>(p, w, sync, base, ch, lane, trace);
+    WaiterBody<W, kShared>(p, w, sync, base, ch, lane, trace);
   } else if (warp == data_warps + 1) {
-    LoaderBody<T, W>(p, sh, smem, stages, ch, nch, data_warps, lane);
+    LoaderBody<T, W, kShared>(p, sh, smem, stages, ch, nch, data_warps, lane);
   } else {
     // Poster: when every data warp has issued an op's stores, make them visible
     // to the peers and publish the op's flags.  Lane k holds op first + k.
     for (int first = 0; first < p.num_ops; first += 32) {
       const int mine = first + lane;
       uint32_t post_out = 0, post_credit = 0;
-      int peers = 0;
+      uint32_t told[kMaxPeerPosts] = {};
+      int peers = 0, told_peers = 0;
       if (mine < p.num_ops) {
         const Op op = p.ops[mine];
         post_out = op.post_out;
         post_credit = op.post_credit;
         peers = (static_cast<uint8_t>(op.peer_in) << 8) | static_cast<uint8_t>(op.peer_out);
+#pragma unroll
+        for (int m = 0; m < kMaxPeerPosts; ++m) told[m] = op.post_told[m], told_peers |= static_cast<uint8_t>(op.peer_told[m]) << (8 * m);
       }
+      const bool tells = kShared && __any_sync(0xffffffffu, told[0] != 0);
       const int end = first + 32 < p.num_ops ? first + 32 : p.num_ops;
       int posted = first;
       while (posted < end) {
@@ -632,7 +757,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
         unsigned upto = lane < data_warps ? LdAcquireShared(&sync->done[lane]) : 0xffffffffu;
         upto = __reduce_min_sync(0xffffffffu, upto);
         const int until = static_cast<int>(upto) < end ? static_cast<int>(upto) : end;
-        const bool fence = __any_sync(0xffffffffu, mine >= posted && mine < until && FlagsNeedFence(post_out, post_credit, p.drop_lines != 0));
+        const bool fence = __any_sync(0xffffffffu, mine >= posted && mine < until && FlagsNeedFence(post_out | told[0], post_credit, p.drop_lines != 0));
         __syncwarp();  // what the other lanes acquired is ordered before lane 0's fence
         if (fence && lane == 0) FencePeers(p.peers.one_gpu != 0);
         for (; posted < until; ++posted) {
@@ -644,18 +769,27 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared* sh, unsi
             if (credit != 0) StRelaxedSys(&Ctl(p.peers, who >> 8)->credit[ch][p.rank], base | credit);
             if (trace != nullptr && posted < p.trace_capacity) trace[posted].t_done = GlobalTimerNs();
           }
+          if (tells) {
+            const int whom = __shfl_sync(0xffffffffu, told_peers, k);
+#pragma unroll
+            for (int m = 0; m < kMaxPeerPosts; ++m) {
+              const uint32_t n = __shfl_sync(0xffffffffu, told[m], k);
+              if (lane == 0 && n != 0) StRelaxedSys(&Ctl(p.peers, whom >> (8 * m) & 0xff)->bar[ch][p.rank], (base | 1u) + n);
+            }
+          }
         }
       }
     }
   }
 }
 
-template <typename T, typename W>
+// kShared: programs of ranks that share a GPU and its memory (ProgramRequest::shared_gpu).
+template <typename T, typename W, bool kShared>
 __global__ void __launch_bounds__(kExecThreads, 1)
 ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all, int stages) {
   const ExecParams& p = all.rank[blockIdx.y];
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ ExecShared s_exec;
+  __shared__ ExecShared<kShared> s_exec;
   __shared__ uint64_t s_seq;
   {
     if (threadIdx.x == 0) {
@@ -669,8 +803,11 @@ ExecKernel(const __grid_constant__ RankBlocks<ExecParams> all, int stages) {
   }
   if (p.world_size <= 1) return;
   const uint64_t seq = BeginCollective(p.peers, p.rank, &s_seq, gridDim.x);
+  // Ranks without blocks in this launch count the call all the same.
+  if (kShared && blockIdx.x == 0 && threadIdx.x < kMaxRanks && (p.counts_for >> threadIdx.x & 1u))
+    atomicAdd(reinterpret_cast<unsigned long long*>(&Ctl(p.peers, static_cast<int>(threadIdx.x))->call_word), 1ull << 16);
   // num_ops <= 0: this rank sits the call out (test hook), but still counts it.
-  if (p.num_ops > 0) ExecBody<T, W>(p, seq, &s_exec, smem, stages);
+  if (p.num_ops > 0) ExecBody<T, W, kShared>(p, seq, &s_exec, smem, stages);
 }
 
 }  // namespace dev
@@ -691,15 +828,21 @@ static size_t ExecSmemBytes(int threads) {
   return static_cast<size_t>(ExecStages(threads)) * static_cast<size_t>((threads - 32 * dev::kExecServiceWarps) * dev::kExecStageBytesPerThread);
 }
 
-template <typename T, typename W>
-static cudaError_t Launch(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
+template <typename T, typename W, bool kShared>
+static cudaError_t LaunchOne(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
   // Beyond one CTA per SM, two smaller CTAs share an SM: while one waits for a
   // flag, the other streams.
   const int threads = ExecKernelThreadsFor(channels * n);
   const size_t smem = ExecSmemBytes(threads);
-  const cudaError_t e = AllowSharedMemory(dev::ExecKernel<T, W>, smem);
+  const auto kernel = dev::ExecKernel<T, W, kShared>;
+  const cudaError_t e = AllowSharedMemory(kernel, smem);
   if (e != cudaSuccess) return e;
-  return LaunchRanks(dev::ExecKernel<T, W>, ranks, n, channels, threads, smem, stream, ExecStages(threads));
+  return LaunchRanks(kernel, ranks, n, channels, threads, smem, stream, ExecStages(threads));
+}
+template <typename T, typename W>
+static cudaError_t Launch(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
+  // Programs that name other ranks' buffers come with them.
+  return ranks->peer_recv[0] != nullptr ? LaunchOne<T, W, true>(ranks, n, channels, stream) : LaunchOne<T, W, false>(ranks, n, channels, stream);
 }
 
 cudaError_t LaunchExecKernel(const ExecParams* ranks, int n, int channels, cudaStream_t stream) {
@@ -721,8 +864,8 @@ int ExecKernelMaxCoResidentBlocks(int device, int threads) {
   int per_sm = 0, sms = 0;
   if (threads <= 0) threads = kExecThreads;
   const size_t smem = ExecSmemBytes(threads);
-  if (AllowSharedMemory(dev::ExecKernel<float, float>, smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::ExecKernel<float, float>, threads, smem) != cudaSuccess) return 0;
+  if (AllowSharedMemory(dev::ExecKernel<float, float, true>, smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::ExecKernel<float, float, true>, threads, smem) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
   return per_sm * sms;
 }

@@ -99,7 +99,7 @@ __device__ void LineBody(const ExecParams& p, uint64_t half_bytes, LinePlan* pla
   bool bad = false;
   if (static_cast<int>(tid) < p.num_ops) {
     const Op op = p.ops[tid];
-    bad = !OpInBounds<W>(op, p);
+    bad = !OpInBounds<W, false>(op, p);
     plan[tid].bad = bad ? 1 : 0;
     if (!bad) {
       uint64_t lo0, unused, lo, hi;

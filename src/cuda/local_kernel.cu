@@ -29,12 +29,6 @@ namespace dev {
 // A thread per vector: blocks of 64 to 256 are within 1 % of each other.
 constexpr int kLocalThreads = 128;
 
-// A value of the buffers' type as it comes out of the wire type W.
-template <typename W, typename A>
-__device__ __forceinline__ A ThroughWire(A v) {
-  return ToAcc<A, W>(FromAcc<W, A>(v));
-}
-
 // kR: ranks at most (2, 4 or 8), so that all their loads are in flight and in registers.
 template <typename T, typename W, LocalOp kOp, int kR>
 __global__ void __launch_bounds__(kLocalThreads) LocalKernel(const __grid_constant__ LocalParams p) {

@@ -32,6 +32,9 @@ template <> __device__ __forceinline__ long long ScaleAcc<long long>(long long v
   return static_cast<long long>(static_cast<double>(v) * s);
 }
 
+// A value of the buffers' type as it comes out of the wire type W.
+template <typename W, typename A> __device__ __forceinline__ A ThroughWire(A v) { return ToAcc<A, W>(FromAcc<W, A>(v)); }
+
 // Raw 16-byte accesses.  "Strong" loads bypass L1 (data written by a peer
 // over NVLink); weak loads may be cached.
 __device__ __forceinline__ uint4 Ld16Strong(const void* p) {

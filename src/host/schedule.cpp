@@ -20,6 +20,7 @@ struct Builder {
   Program prog;
   uint32_t slots;
   std::vector<int> my_in_peers;
+  uint32_t told[kMaxRanks] = {0}, heard[kMaxRanks] = {0};  // stores into another rank's recvbuf, and into this one's
 
   explicit Builder(const ProgramRequest& r) : req(r) {
     prog.stage = PlanStage(r);
@@ -39,6 +40,8 @@ struct Builder {
     Op op{};
     op.peer_in = -1;
     op.peer_out = -1;
+    op.rank_a = op.rank_c = -1;
+    for (int8_t& p : op.peer_told) p = -1;
     op.elem_begin = g.first;
     op.elem_count = g.second - g.first;
     op.cell_begin = g.first;
@@ -82,11 +85,45 @@ struct Builder {
 
   void AttachIn(Op* op, int from) {
     uint32_t k = prog.received_from[from]++;
+    op->src_a = kSrcStage;
     op->peer_in = static_cast<int8_t>(from);
     op->region_in = static_cast<uint8_t>(RegionOf(req.rank, from));
     op->slot_in = k % slots;
     op->wait_in = k + 1;
     op->post_credit = k + 1;
+  }
+
+  // ---- ranks on one GPU (ProgramRequest::shared_gpu) ----
+  // Source a (or c) is rank `who`'s sendbuf.
+  void PullA(Op* op, int who) {
+    op->src_a = kSrcPeer;
+    op->rank_a = static_cast<int8_t>(who);
+    op->flags |= kOpRoundPeer;
+  }
+  void PullC(Op* op, int who) {
+    op->rank_c = static_cast<int8_t>(who);
+    op->flags |= kOpRoundPeer;
+  }
+  // The value goes into `to`'s recvbuf; `read_on`: and is read there by an op of that rank.
+  void StoreTo(Op* op, int to, bool read_on) {
+    op->store_peers = static_cast<uint8_t>(op->store_peers | (1u << to));
+    if (!read_on) return;
+    op->flags |= kOpPeersReadBack;
+    int m = 0;
+    while (m < kMaxPeerPosts && op->post_told[m] != 0) ++m;
+    if (m == kMaxPeerPosts) IBCOMM_FAIL(INVALID_ARGUMENT, "schedule: an op tells too many ranks.\n");
+    op->peer_told[m] = static_cast<int8_t>(to);
+    op->post_told[m] = ++told[to];
+  }
+  // Source a is what `from` stored into recvbuf.
+  void TakeArrived(Op* op, int from) {
+    op->src_a = kSrcRecv;
+    op->peer_in = static_cast<int8_t>(from);
+    op->wait_peer = ++heard[from];
+  }
+  void Finish(Op* op) {
+    op->flags |= kOpStoreLocal | kOpRoundWire;
+    if (req.apply_scale) op->flags |= kOpScale;
   }
 
   // Plain send of a chunk taken from `src` (sendbuf or recvbuf).
@@ -100,7 +137,6 @@ struct Builder {
   // Receive a chunk; optionally add `add` to it, store locally and/or forward.
   void Recv(const Range& g, int from, OpSrc add, bool store_local, bool scale, int forward_to) {
     Op op = Base(g);
-    op.src_a = kSrcStage;
     op.src_b = add;
     if (store_local) op.flags |= kOpStoreLocal;
     if (scale) op.flags |= kOpRoundWire;
@@ -166,6 +202,46 @@ std::vector<int> ChunksOfBlocks(const std::vector<std::vector<int>>& blocks, int
   return out;
 }
 
+// The ring of ranks that share a GPU.  The steps, the order of the additions and the owners are those of BuildRing.
+// The first step's partner is read where it is, and a result travels from recvbuf to recvbuf: 34 reads and writes
+// per eight elements and rank instead of 44 (8 ranks).
+template <typename ChunkAt>
+void BuildRingOnOneGpu(Builder* bld, size_t positions, size_t group, ChunkAt at) {
+  const ProgramRequest& q = bld->req;
+  const int ws = q.world_size, r = q.rank;
+  const int from = Mod(r - 1, ws), to = Mod(r + 1, ws);
+  for (size_t i0 = 0; i0 < positions; i0 += group) {
+    const size_t i1 = std::min(positions, i0 + group);
+    for (int k = 0; k <= ws - 2; ++k) {  // reduce-scatter
+      for (size_t i = i0; i < i1; ++i) {
+        const int c = at(Mod(r - 1 - k, ws), i);
+        if (c < 0) continue;
+        Op op = bld->Base(bld->ChunkRange(c));
+        op.src_b = kSrcSend;
+        if (k == 0) bld->PullA(&op, from);
+        else bld->AttachIn(&op, from);
+        if (k < ws - 2) {
+          bld->AttachOut(&op, to);
+        } else {
+          bld->Finish(&op);
+          bld->StoreTo(&op, to, ws > 2);
+        }
+        bld->prog.ops.push_back(op);
+      }
+    }
+    for (int k = 0; k <= ws - 3; ++k) {  // all-gather
+      for (size_t i = i0; i < i1; ++i) {
+        const int c = at(Mod(r - k, ws), i);
+        if (c < 0) continue;
+        Op op = bld->Base(bld->ChunkRange(c));
+        bld->TakeArrived(&op, from);
+        bld->StoreTo(&op, to, k < ws - 3);
+        bld->prog.ops.push_back(op);
+      }
+    }
+  }
+}
+
 void BuildRing(Builder* bld) {
   const ProgramRequest& q = bld->req;
   const int ws = q.world_size, r = q.rank;
@@ -190,6 +266,7 @@ void BuildRing(Builder* bld) {
   // each waiting for the other's hand-over (4 us on one GPU), so half the
   // slots are left to run ahead into.
   const size_t group = std::max<size_t>(1, std::min<size_t>(positions, bld->slots / 2));
+  if (q.shared_gpu) return BuildRingOnOneGpu(bld, positions, group, at);
   for (size_t i0 = 0; i0 < positions; i0 += group) {
     const size_t i1 = std::min(positions, i0 + group);
     for (size_t i = i0; i < i1; ++i) {
@@ -252,6 +329,16 @@ struct Halving {
     std::vector<Piece> out = Kept(v ^ (1 << (s + 1)), s + 1);
     const std::vector<Piece> rest = Pieces(v, s + 2);
     out.insert(out.end(), rest.begin(), rest.end());
+    return out;
+  }
+  // What rank `v` stores into its partner's recvbuf in step `t` of the doubling, in order (ranks on one GPU): its own
+  // block, then what came in the steps before.
+  std::vector<Piece> Delivered(int v, int t) const {
+    std::vector<Piece> out = Own(v);
+    for (int u = 0; u < t; ++u) {
+      const std::vector<Piece> came = Delivered(DoublingPartner(v, u), u);
+      out.insert(out.end(), came.begin(), came.end());
+    }
     return out;
   }
   int DoublingPartner(int v, int t) const { return v ^ (1 << (exp - 1 - t)); }
@@ -378,6 +465,84 @@ void BuildHalvingDoubling(Builder* bld, const Segment& segment) {
   }
 }
 
+// Halving and doubling of one segment by ranks that share a GPU.  The first step's partner and the extra ranks'
+// contributions are read where they are, final blocks go straight to every rank that the doubling takes them to from
+// here, and extra ranks have nothing to do.  An extra rank's contribution is added to a sum of two (its partner's, in
+// the op (a + c) + b), so that every sum is as long at its last additions as where extra ranks are folded first:
+//   one: in the last step, by the owner;  two: in the first step, by the two ranks that keep the block, one each;
+//   three: in the first step, two of them by the owner (one to each term), one by the other rank.
+void BuildHalvingDoublingOnOneGpu(Builder* bld, const Segment& segment) {
+  using Piece = Builder::Piece;
+  const int ws = bld->req.world_size, r = bld->req.rank;
+  const int p = static_cast<int>(util::FloorPow2(static_cast<uint64_t>(ws)));
+  const int extra = ws - p;
+  const int exp = util::GetExpOfTwo(static_cast<uint64_t>(p));
+  auto real_rank = [extra](int v) { return v < extra ? 2 * v + 1 : v + extra; };
+  const std::vector<std::vector<int>> blocks = SegmentBlocks(segment, p);
+  const Halving half{*bld, blocks, p, exp};
+  const int vrank = r < 2 * extra ? r / 2 : r - extra;
+  const size_t slots = bld->slots;
+
+  // The extra rank whose contribution this rank adds to a piece in step `s`, or -1.
+  auto joins = [&](const Piece& g, int s) -> int {
+    if (extra == 0 || g.owner < 0) return -1;
+    if (extra == 1) return s == exp - 1 ? 0 : -1;
+    if (s != 0) return -1;
+    return g.owner == vrank ? 2 * (extra - 2) : 2 * (extra == 2 ? 1 : 2);
+  };
+  size_t sent = 0;  // of what this step sends, forwarded during the one before
+  for (int s = 0; s < exp; ++s) {
+    const int peer = real_rank(vrank ^ (1 << s));
+    const std::vector<Piece> sends = s == 0 ? std::vector<Piece>() : half.Kept(vrank ^ (1 << s), s);
+    const std::vector<Piece> arrivals = half.Kept(vrank, s);
+    const bool last = s + 1 == exp;
+    const int next = last ? -1 : real_rank(vrank ^ (1 << (s + 1)));
+    const size_t forward = last ? 0 : std::min(half.Kept(vrank ^ (1 << (s + 1)), s + 1).size(), slots);
+    size_t si = sent;
+    while (si < sends.size() && si < slots) bld->Send(sends[si++].range, kSrcRecv, peer);
+    for (size_t ri = 0; ri < arrivals.size(); ++ri) {
+      const Piece& g = arrivals[ri];
+      OpSrc mine = s == 0 ? kSrcSend : kSrcRecv;
+      if (extra == 3 && s == 0 && g.owner == vrank) {
+        Op first = bld->Base(g.range);
+        bld->PullA(&first, 0);
+        first.src_b = kSrcSend;
+        first.flags |= kOpStoreLocal;
+        bld->prog.ops.push_back(first);
+        mine = kSrcRecv;
+      }
+      Op op = bld->Base(g.range);
+      op.src_b = mine;
+      if (s == 0) bld->PullA(&op, peer);
+      else bld->AttachIn(&op, peer);
+      if (const int x = joins(g, s); x >= 0) bld->PullC(&op, x);
+      if (last) {
+        bld->Finish(&op);
+        for (int t = 0; t < exp; ++t) bld->StoreTo(&op, real_rank(half.DoublingPartner(vrank, t)), t + 1 < exp);
+        for (int x = 0; x < extra; ++x) bld->StoreTo(&op, 2 * x, false);
+      } else if (ri < forward) {
+        bld->AttachOut(&op, next);
+      } else {
+        op.flags |= kOpStoreLocal;
+      }
+      bld->prog.ops.push_back(op);
+      if (si < sends.size()) bld->Send(sends[si++].range, kSrcRecv, peer);
+    }
+    while (si < sends.size()) bld->Send(sends[si++].range, kSrcRecv, peer);
+    sent = forward;
+  }
+  // What comes in one step of the doubling goes to the partners of all later ones at once.
+  for (int t = 0; t + 1 < exp; ++t) {
+    const int vpeer = half.DoublingPartner(vrank, t);
+    for (const Piece& g : half.Delivered(vpeer, t)) {
+      Op op = bld->Base(g.range);
+      bld->TakeArrived(&op, real_rank(vpeer));
+      for (int u = t + 1; u < exp; ++u) bld->StoreTo(&op, real_rank(half.DoublingPartner(vrank, u)), u + 1 < exp);
+      bld->prog.ops.push_back(op);
+    }
+  }
+}
+
 // An extra rank hands every block of its message to the rank that adds it (Joiner) and
 // gets the results back from the owners.  Piece by piece over the blocks, so that all of
 // them have something to work on.  It sends a segment ahead of the one it receives if the
@@ -423,7 +588,12 @@ void BuildRabenseifner(Builder* bld) {
     segments.emplace_back(q.segments[k], k + 1 < q.segments.size() ? q.segments[k + 1] : q.ranges.size());
   if (segments.empty()) segments.emplace_back(0, q.ranges.size());
   const int extra = q.world_size - static_cast<int>(util::FloorPow2(static_cast<uint64_t>(q.world_size)));
-  if (q.rank < 2 * extra && (q.rank & 1) == 0) return BuildExtraRank(bld, segments);
+  const bool is_extra = q.rank < 2 * extra && (q.rank & 1) == 0;
+  if (q.shared_gpu) {
+    for (size_t k = 0; k < segments.size() && !is_extra; ++k) BuildHalvingDoublingOnOneGpu(bld, segments[k]);
+    return;
+  }
+  if (is_extra) return BuildExtraRank(bld, segments);
   for (const Segment& g : segments) BuildHalvingDoubling(bld, g);
 }
 
@@ -587,8 +757,12 @@ std::string ValidateProgram(const Program& prog, uint64_t len_elements, size_t w
   for (size_t i = 0; i < prog.ops.size(); ++i) {
     const Op& op = prog.ops[i];
     const char* why = nullptr;
-    const bool reads_stage = op.src_a == kSrcStage || op.src_b == kSrcStage;
+    const bool reads_stage = op.src_a == kSrcStage;
     const bool writes_stage = (op.flags & kOpStoreRemote) != 0;
+    auto is_rank = [world_size](int r) { return r >= 0 && r < world_size; };
+    bool told_ok = true;
+    for (int m = 0; m < kMaxPeerPosts; ++m) told_ok = told_ok && (op.post_told[m] == 0 || is_rank(op.peer_told[m]));
+    told_ok = told_ok && (op.wait_peer == 0 || is_rank(op.peer_in));
     if (op.elem_begin > len_elements || op.elem_count > len_elements - op.elem_begin) {
       why = "range outside the message";
     } else if (op.cell_begin > op.elem_begin) {
@@ -604,6 +778,10 @@ std::string ValidateProgram(const Program& prog, uint64_t len_elements, size_t w
       why = "peer_out is not a rank";
     } else if ((op.wait_in != 0 || op.post_credit != 0) && (op.peer_in < 0 || op.peer_in >= world_size)) {
       why = "peer_in is not a rank";
+    } else if ((op.src_a == kSrcPeer && !is_rank(op.rank_a)) || (op.rank_c != -1 && !is_rank(op.rank_c)) || (op.store_peers >> world_size) != 0 || !told_ok) {
+      why = "names a rank that is none";
+    } else if (op.src_b == kSrcStage || op.src_b == kSrcPeer) {
+      why = "second source is not this rank's";
     } else if (op.wait_local > i) {
       why = "waits for an op that comes later";
     }
@@ -613,12 +791,12 @@ std::string ValidateProgram(const Program& prog, uint64_t len_elements, size_t w
 }
 
 std::string DescribeOp(const Op& op) {
-  static const char* const src[] = {"-", "send", "recv", "stage"};
+  static const char* const src[] = {"-", "send", "recv", "stage", "peer", "?", "?", "?"};
   char buf[256];
   snprintf(buf, sizeof(buf),
            "[%llu+%llu] a=%s b=%s%s%s%s in=%d(r%u s%u w%u c%u) out=%d(r%u s%u w%u p%u)",
            static_cast<unsigned long long>(op.elem_begin), static_cast<unsigned long long>(op.elem_count),
-           src[op.src_a & 3], src[op.src_b & 3], (op.flags & kOpScale) ? " scale" : "",
+           src[op.src_a & 7], src[op.src_b & 7], (op.flags & kOpScale) ? " scale" : "",
            (op.flags & kOpStoreLocal) ? " local" : "", (op.flags & kOpStoreRemote) ? " remote" : "", op.peer_in,
            op.region_in, op.slot_in, op.wait_in, op.post_credit, op.peer_out, op.region_out, op.slot_out,
            op.wait_credit, op.post_out);

@@ -13,7 +13,7 @@ using namespace ibcomm;
 
 template <typename T>
 static bool RunCase(Algo algo, int ws, size_t n, int64_t env_chunk, size_t stage_bytes, int nch, bool in_place,
-                    double scale, size_t max_chunk_bytes = 0, size_t piece_elems = 0, size_t segment_pieces = 0) {
+                    double scale, size_t max_chunk_bytes = 0, size_t piece_elems = 0, size_t segment_pieces = 0, bool shared_gpu = false) {
   std::vector<size_t> segments;
   std::vector<Range> ranges = segment_pieces == 0 ? SplitForDevice(n, sizeof(T), static_cast<size_t>(ws), env_chunk, max_chunk_bytes)
                                                   : SplitSegments(n, piece_elems, segment_pieces, &segments);
@@ -21,7 +21,7 @@ static bool RunCase(Algo algo, int ws, size_t n, int64_t env_chunk, size_t stage
   std::mt19937 gen(static_cast<unsigned>(n * 31 + static_cast<size_t>(ws)));
   for (int r = 0; r < ws; ++r)
     for (size_t i = 0; i < n; ++i) in[static_cast<size_t>(r)][i] = static_cast<T>(static_cast<int>(gen() % 2001) - 1000);
-  ProgramSimulator<T> sim(algo, ws, stage_bytes, nch, piece_elems, segments);
+  ProgramSimulator<T> sim(algo, ws, stage_bytes, nch, piece_elems, segments, shared_gpu);
   SimResult res = sim.Run(ranges, in, &out, scale, in_place);
   if (!res.ok) {
     fprintf(stderr, "%s ws=%d n=%zu: %s", AlgoName(algo), ws, n, res.error.c_str());
@@ -126,6 +126,25 @@ MINI_TEST(RabenseifnerSegments) {
   }
 }
 
+MINI_TEST(RanksOnOneGpu) {
+  // Programs that read the other ranks' sendbuf and store into their recvbuf: all world sizes, in place (a buffer is
+  // overwritten with results while others still have to have read it), few and many slots, short and ragged lengths.
+  for (int ws = 2; ws <= 8; ++ws)
+    for (bool in_place : {false, true}) {
+      for (size_t n : {size_t(ws), size_t(2 * ws + 1), size_t(2521), size_t(40007)})
+        for (int nch : {1, 3}) {
+          CHECK_TRUE(RunCase<int>(Algo::kRing, ws, n, 0, size_t(1) << 22, nch, in_place, 1.0, 0, 0, 0, true));
+          CHECK_TRUE(RunCase<double>(Algo::kRing, ws, n, 0, 65536, nch, in_place, 0.5, 16384, 0, 0, true));
+          CHECK_TRUE(RunCase<int>(Algo::kRabenseifner, ws, n, 0, size_t(1) << 22, nch, in_place, 1.0, 0, 1000, 0, true));
+        }
+      const size_t p = ws < 4 ? 2 : ws < 8 ? 4 : 8, regions = static_cast<size_t>(NumRegions(Algo::kRabenseifner, ws));
+      for (size_t own : {size_t(1), size_t(3)})
+        for (size_t n : {own * p * 256, 2 * own * p * 256 - 5, 20003 + 4 * own * p * 256})
+          for (size_t slots : {size_t(2), 4 * own + 1})
+            CHECK_TRUE(RunCase<double>(Algo::kRabenseifner, ws, n, 0, slots * regions * 256 * 8, 2, in_place, 0.25, 0, 256, own * p, true));
+    }
+}
+
 // A partial sum as what it costs in precision: every addition rounds a sum of so many
 // terms, and the error of a rounding grows with the sum.
 struct Rounded {
@@ -148,12 +167,13 @@ MINI_TEST(RabenseifnerRoundsLikeAFold) {
     const int p = ws < 4 ? 2 : ws < 8 ? 4 : 8, exp = util::GetExpOfTwo(static_cast<uint64_t>(p));
     const size_t n = 3001, piece = 128;
     for (size_t slots : {size_t(2), size_t(64)})  // contributions of extra ranks before all else, and where they are needed
-      for (bool in_segments : {false, true}) {
+      for (int form = 0; form < 3; ++form) {
+        const bool in_segments = form != 0, shared_gpu = form == 2;
         std::vector<size_t> segments;
         const std::vector<Range> ranges = in_segments ? SplitSegments(n, piece, 4 * static_cast<size_t>(p), &segments)
                                                       : SplitForDevice(n, sizeof(Rounded), static_cast<size_t>(ws), 0, 0);
         const size_t stage = slots * static_cast<size_t>(NumRegions(Algo::kRabenseifner, ws)) * piece * sizeof(Rounded);
-        ProgramSimulator<Rounded> sim(Algo::kRabenseifner, ws, stage, 1, piece, segments);
+        ProgramSimulator<Rounded> sim(Algo::kRabenseifner, ws, stage, 1, piece, segments, shared_gpu);
         std::vector<std::vector<Rounded>> out;
         CHECK_TRUE(sim.Run(ranges, std::vector<std::vector<Rounded>>(static_cast<size_t>(ws), std::vector<Rounded>(n)), &out, 1.0, false).ok);
         int worst = 0, terms = 0;
@@ -287,6 +307,12 @@ MINI_TEST(ValidateProgramFindsOutOfBoundsOps) {
         for (Op& op : bad.ops)
           if (op.flags & kOpStoreRemote) { op.slot_out = bad.stage.slots; break; }
         CHECK_TRUE(ValidateProgram(bad, n, 4, ws).find("output slot") != std::string::npos);
+        q.shared_gpu = true;
+        Program shared = BuildProgram(q);
+        CHECK_TRUE(ValidateProgram(shared, n, 4, ws).empty());
+        for (Op& op : shared.ops)
+          if (op.store_peers != 0) { op.store_peers = static_cast<uint8_t>(1u << ws); break; }
+        CHECK_TRUE(shared.ops.empty() || ws == 8 || ValidateProgram(shared, n, 4, ws).find("a rank that is none") != std::string::npos);
         bad = p;
         bad.stage.slot_bytes = 64;
         CHECK_TRUE(ValidateProgram(bad, n, 4, ws).find("does not fit") != std::string::npos);

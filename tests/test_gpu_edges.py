@@ -396,3 +396,67 @@ def test_lines_wait_runs_out(algo):
     for o in outs:
         torch.testing.assert_close(o.double(), want, rtol=1e-5, atol=1e-5)
     world.close()
+
+
+@pytest.fixture
+def slots_only():
+    # Messages of every length through the executor with slots and flags.
+    ar.utils.set_tunable("IBCOMM_LINES_MAX_KIB", 0)
+    yield
+    ar.utils.set_tunable("IBCOMM_LINES_MAX_KIB", -1)
+
+
+@pytest.mark.parametrize("mode", [0, 3])
+@pytest.mark.parametrize("algo", ["ring", "rabenseifner"])
+@pytest.mark.parametrize("ws", [2, 3, 4, 5, 6, 7, 8])
+def test_op_programs_of_ranks_that_share_memory(slots_only, ws, algo, mode):
+    # Programs that read the other ranks' sendbuf and store into their recvbuf, and those that send as between GPUs:
+    # ragged ends, slices off the boundary, stages of one, two and three sources, few slots that are used many times, in
+    # place (a buffer is overwritten while others still have to have read it), 16-bit wires.
+    for pool in (0, 1 << 20):
+        world = ar.EmuWorld(ws, pool, pool)
+        world.set_direct_staging(mode)
+        for dtype in (torch.float32, torch.float64, torch.bfloat16, torch.int64) if pool == 0 else (torch.float32, torch.bfloat16):
+            whole = dtype == torch.int64
+            scale = 1.0 if whole else 1.0 / ws
+            for n, offset in ((4 * ws, 0), (2521, 0), (2521, 1), (8 * 512 * ws + 5, 0), (8 * 512 * ws, 0), (1 << 20, 0), (1000003, 0)):
+                for wire in (None, torch.bfloat16) if dtype == torch.float32 else (None,):
+                    ins = [values(n, dtype, n + r, offset) for r in range(ws)]
+                    want = torch.stack([t.double() for t in ins]).sum(0) * scale
+                    guard = [torch.full((n + offset + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+                    outs = [g[offset:offset + n] for g in guard]
+                    tol = 0.0 if whole else (2e-2 if dtype == torch.bfloat16 or wire is not None else (1e-5 if dtype == torch.float32 else 1e-12))
+                    for call in range(2):
+                        world.allreduce(ins, outs, algo=algo, scale=scale, wire=wire)
+                    world.allreduce(ins, None, algo=algo, scale=scale, wire=wire)
+                    for g, o, i in zip(guard, outs, ins):
+                        torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
+                        assert torch.equal(o, outs[0]) and torch.equal(i, o)
+                        assert torch.all(g[:offset] == 7) and torch.all(g[offset + n:] == 7)
+        world.close()
+
+
+@pytest.mark.parametrize("mode", [0, 3])
+@pytest.mark.parametrize("algo,ws", [("ring", 4), ("rabenseifner", 4), ("rabenseifner", 5)])
+def test_executor_gives_up_cleanly(slots_only, algo, ws, mode):
+    # A rank that takes no part, and one whose ops fail their self-check, with and without ranks that have no blocks in the
+    # launch; the calls are counted for those too, so the world stays usable by every kernel.
+    world = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+    world.set_direct_staging(mode)
+    ins = [values(8192, torch.float32, r) for r in range(ws)]
+    outs = [torch.zeros_like(t) for t in ins]
+    want = torch.stack([t.double() for t in ins]).sum(0)
+    for hook, codes in ((world.set_silent_rank, (1, 2)), (world.set_bad_program_rank, (3,))):
+        world.set_timeout_ms(200)
+        hook(1)
+        with pytest.raises(ar.IbcommError) as e:
+            world.allreduce(ins, outs, algo=algo)
+        assert e.value.code == ar.TRANSPORT_ERROR
+        assert world.last_status()["code"] in codes
+        hook(-1)
+        world.set_timeout_ms(5000)
+        for other in (algo, "oneshot", "ring", algo):
+            world.allreduce(ins, outs, algo=other)
+            for o in outs:
+                torch.testing.assert_close(o.double(), want, rtol=1e-5, atol=1e-5)
+    world.close()
