@@ -159,6 +159,9 @@ struct StagedParams {
   int32_t load_groups, reduce_groups, store_groups;
   int32_t copy_warps;  // unsplit, copies by the threads: warps of the loader and of the storer (0: three each)
   int32_t drop_lines;  // 1: lines of the windows leave L2 unwritten once their reader has them
+  // 1: a result is stored once, in its reducer's pool, and the ranks' storers load it there (ranks on one GPU, copies by the
+  // threads); 0: the reducer stores it into every rank's pool.
+  int32_t pull_results;
   int32_t posters;  // split mode: a poster warp per reducer group fences and publishes behind the data warps
 };
 cudaError_t LaunchStagedKernel(const StagedParams* ranks, int n, int blocks, cudaStream_t stream);

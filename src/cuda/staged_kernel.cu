@@ -50,7 +50,11 @@
 // rounds in flight (AsyncRounds, twoshot_common.cuh): B200, 4 ranks x 64 MiB 203
 // -> 170 us, 8 x 25 MiB bucket with a bf16 wire 183 -> 156 us.
 //
-// A line of a window has one reader (a shard's reducer, or the storer).  Ranks on one
+// Ranks on one GPU, more than two of them, write a result once, into the reducer's own output window, and the storers of
+// the other ranks load it from there (`pull_results`); the flags are the same, since a window is emptied when every
+// rank's storer says so.
+//
+// A line of an input window, and without that of an output window, has one reader (a shard's reducer, or the storer).  Ranks on one
 // GPU have it drop the line from L2 (`drop_lines`) once its warp holds the data and
 // before the flag that frees the window, which orders the two: less of what is dead
 // is written to HBM (half of the staging stores before).  One discard per lane and round;
@@ -174,10 +178,12 @@ __device__ __forceinline__ void RolePost(RoleCtx& c, int row, uint64_t flag_wind
 // first element.  A range is a round or two, so the loads have to run over its end.
 struct CopyParts {
   uint64_t from[kMaxRanks], to[kMaxRanks];
+  const unsigned char* results[kMaxRanks];  // staging memory the storer takes a part's results from
   int parts;
   __device__ __forceinline__ int count() const { return parts; }
   __device__ __forceinline__ uint64_t begin(int q) const { return from[q]; }
   __device__ __forceinline__ uint64_t end(int q) const { return to[q]; }
+  __device__ __forceinline__ const unsigned char* data(int q) const { return results[q]; }
 };
 
 template <typename T, typename W>
@@ -187,7 +193,7 @@ __device__ __forceinline__ void CastIn(unsigned char* smem, uint4* wire, const u
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
   AsyncRounds<kRoundVecs / VT>(
       smem, parts, static_cast<unsigned>(tid), static_cast<unsigned>(nthr),
-      [&](uint64_t vec, uint32_t slot, uint32_t stride) {
+      [&](const unsigned char*, uint64_t vec, uint32_t slot, uint32_t stride) {
 #pragma unroll
         for (int v = 0; v < VT; ++v) CpAsync16Hint(slot + static_cast<uint32_t>(v) * stride, user + vec * VT + v, policy);
       },
@@ -200,14 +206,15 @@ __device__ __forceinline__ void CastIn(unsigned char* smem, uint4* wire, const u
       });
 }
 
+// `off`: of the window in a staging memory.
 template <typename T, typename W>
-__device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const uint4* wire, const CopyParts& parts, uint64_t policy, bool drop, int tid, int nthr) {
+__device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, uint64_t off, const CopyParts& parts, uint64_t policy, const unsigned char* drop, int tid, int nthr) {
   using A = typename Acc<T>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
   AsyncRounds<kRoundVecs>(
       smem, parts, static_cast<unsigned>(tid), static_cast<unsigned>(nthr),
-      [&](uint64_t vec, uint32_t slot, uint32_t) { CpAsync16(slot, wire + vec); },
+      [&](const unsigned char* at, uint64_t vec, uint32_t slot, uint32_t) { CpAsync16(slot, at + off + vec * 16); },
       [&](uint64_t vec, const unsigned char* slot, uint32_t) {
         A acc[P];
         VecIO<W>::Load(*reinterpret_cast<const uint4*>(slot), acc);
@@ -215,7 +222,7 @@ __device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const 
         for (int v = 0; v < VT; ++v) St16Hint(user + vec * VT + v, VecIO<T>::Store(acc + v * VecIO<T>::kN), policy);
       },
       Dropping([&](int, uint64_t vec) {
-        if (drop) DropLine(reinterpret_cast<const unsigned char*>(wire + vec));
+        if (drop != nullptr) DropLine(drop + vec * 16);
       }));
 }
 
@@ -357,12 +364,14 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   auto fill_parts = [&](CopyParts* cp, uint64_t nv) {
     cp->parts = 0;
     cp->from[0] = cp->to[0] = 0;
+    cp->results[0] = nullptr;
     for (int s = 0; s < ws; ++s) {
       uint64_t b, e;
       part(s, nv, &b, &e);
       if ((kOwnInPlace && s == me) || b >= e) continue;
       cp->from[cp->parts] = b;
       cp->to[cp->parts] = e;
+      cp->results[cp->parts] = p.stage[p.pull_results != 0 ? s : me];
       ++cp->parts;
     }
   };
@@ -506,7 +515,8 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         }
         FenceProxyAsyncAll();
       } else if (!tma) {
-        CastOut<T, W>(smem, reinterpret_cast<uint4*>(user), reinterpret_cast<const uint4*>(win), parts_of(nv), once, p.drop_lines != 0, c.tid, c.nthr);
+        const unsigned char* const drop = p.drop_lines != 0 && p.pull_results == 0 ? win : nullptr;
+        CastOut<T, W>(smem, reinterpret_cast<uint4*>(user), p.out_off[j], parts_of(nv), once, drop, c.tid, c.nthr);
       }
       RolePost(c, kRowOutFree, k, SG, base | (k + 1));
       if (role_w != 0 && gtid == 0) trace[2 * role_w + k].t_done = GlobalTimerNs();
@@ -571,7 +581,14 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
             }
           }
         }
+        // Results: to every rank's pool, or once to this rank's, where the others' storers fetch them.
+        unsigned char* const own_out = p.stage[me] + p.out_off[j];
         auto store = [&](uint64_t idx, uint4 r) {
+          if (p.pull_results != 0) {
+            St16(own_out + idx * 16, r);
+            if (kOwnInPlace) St16(static_cast<unsigned char*>(p.recvbuf) + v0 * 16 + idx * 16, r);
+            return;
+          }
 #pragma unroll
           for (int q = 0; q < kR; ++q)
             if (q < ws) St16(to[q] + idx * 16, r);

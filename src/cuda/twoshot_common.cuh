@@ -142,14 +142,16 @@ struct OneRange {
   __device__ __forceinline__ int count() const { return 1; }
   __device__ __forceinline__ uint64_t begin(int) const { return b; }
   __device__ __forceinline__ uint64_t end(int) const { return e; }
+  __device__ __forceinline__ const unsigned char* data(int) const { return nullptr; }
 };
 template <typename Ranges>
 struct RoundCursor {
   int q;
   uint64_t base, end;
-  __device__ __forceinline__ explicit RoundCursor(const Ranges& r) : q(0), base(r.begin(0)), end(r.end(0)) { Settle(r); }
+  const unsigned char* at;
+  __device__ __forceinline__ explicit RoundCursor(const Ranges& r) : q(0), base(r.begin(0)), end(r.end(0)), at(r.data(0)) { Settle(r); }
   __device__ __forceinline__ void Settle(const Ranges& r) {
-    while (base >= end && ++q < r.count()) base = r.begin(q), end = r.end(q);
+    while (base >= end && ++q < r.count()) base = r.begin(q), end = r.end(q), at = r.data(q);
   }
   __device__ __forceinline__ void Next(const Ranges& r, uint64_t step) {
     base += step;
@@ -178,8 +180,8 @@ __device__ __forceinline__ DropLines<Fn> Dropping(Fn fn) {
 }
 
 // Every item of `ranges` over `nthr` threads numbered `tid`, kU items per thread
-// and round, each of kRoundVecs / kU vectors: `issue(item, smem, stride)` starts
-// the loads of one item into slots `smem`, `smem + stride`, ..., `use(item, slots,
+// and round, each of kRoundVecs / kU vectors: `issue(at, item, smem, stride)` starts
+// the loads of one item of a range whose data lies at `at` into slots `smem`, `smem + stride`, ..., `use(item, slots,
 // stride)` consumes it.  `smem`: kRoundSmemPerThread bytes for every thread of the
 // block.  The loads run over the ends of ranges.  `drop(v, item)` is called for the
 // vectors v of items item .. item + 7 when the warp has them: a round is 32 lines of 8
@@ -199,7 +201,7 @@ __device__ __forceinline__ void AsyncRounds(unsigned char* smem, const Ranges& r
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
         const uint64_t idx = in.base + tid + static_cast<uint64_t>(u) * nthr;
-        if (idx < in.end) issue(idx, mine_u32 + ahead + static_cast<uint32_t>(u * kV) * stride, stride);
+        if (idx < in.end) issue(in.at, idx, mine_u32 + ahead + static_cast<uint32_t>(u * kV) * stride, stride);
       }
       in.Next(ranges, step);
     }
@@ -237,7 +239,7 @@ __device__ __forceinline__ void PeerReduce(unsigned char* smem, unsigned char* c
   static_assert(kRoundVecs % kR == 0, "a round holds whole items");
   AsyncRounds<kRoundVecs / kR>(
       smem, OneRange{b, e}, tid, nthr,
-      [&](uint64_t idx, uint32_t slot, uint32_t stride) {
+      [&](const unsigned char*, uint64_t idx, uint32_t slot, uint32_t stride) {
 #pragma unroll
         for (int q = 0; q < kR; ++q)
           if (q < ws) CpAsync16(slot + static_cast<uint32_t>(q) * stride, peer[q] + off + idx * 16);
