@@ -64,9 +64,10 @@ class EmuWorld:
         check(_native.lib().ibcomm_emu_set_bad_program_rank(self._h, rank))
 
     def set_direct_staging(self, mode) -> None:
-        """Direct algorithm: 0/False in place (one kernel for all ranks), 1/True staged through the pool windows one phase
-        after the other, 2 staged through the pipelined kernel (needs 16-byte aligned buffers of whole 16-byte vectors),
-        3 in place with the kernels and barriers of ranks that have a GPU each."""
+        """0/False: the ranks share a GPU and its memory (direct and one-shot: one kernel for all ranks; op programs:
+        lines, or each other's buffers).  Else the kernels and programs of ranks that have a GPU each, and the direct
+        algorithm: 1/True staged through the pool windows one phase after the other, 2 staged through the pipelined
+        kernel (needs 16-byte aligned buffers of whole 16-byte vectors), 3 in place with barriers."""
         check(_native.lib().ibcomm_emu_set_direct_staging(self._h, int(mode)))
 
     @property

@@ -4,8 +4,8 @@
 // every collective is a single launch that covers all ranks.  Where ranks
 // exchange anything through staging it is cooperative (blockIdx.y = rank), and
 // the kernels, flag protocol and staging layout are the ones the multi-GPU path
-// uses; only the "peer" pointers are local.  The direct algorithm on buffers in
-// place has a kernel of its own, since nothing has to be exchanged.
+// uses; only the "peer" pointers are local.  The direct and the one-shot algorithm
+// on buffers in place have a kernel of their own, since nothing has to be exchanged.
 #pragma once
 
 #include <memory>
@@ -53,10 +53,12 @@ class EmuWorld {
   // the bounds check before any memory is touched; the rank reports "bad
   // program", the others are told to stop.  -1 restores normal operation.
   void SetBadProgramRank(int r);
-  // How the direct algorithm treats the buffers: 0 in place, with one kernel for
-  // all ranks; 1 staged through the pool window by window (as for buffers the
-  // peers cannot map), 2 staged through the pipelined kernel; 3 in place, with
-  // the kernels and barriers of ranks that have a GPU each.
+  // How the ranks treat the buffers.  0: they share a GPU.  The direct and the
+  // one-shot algorithm run one kernel for all ranks, short op programs hand over in
+  // lines, long ones use each other's buffers.  Else as ranks that have a GPU each,
+  // and the direct algorithm: 1 staged through the pool window by window (as for buffers the
+  // peers cannot map), 2 staged through the pipelined kernel, 3 in place with
+  // barriers.
   void SetDirectStaging(int mode);
   int last_channels() const;
 

@@ -234,7 +234,13 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
   const uint64_t half = m.layout.pool_bytes / 2 / 4096 * 4096;
   if (algo == Algo::kDirect && !pipelined && (!all_aligned || (m.direct_staging != 0 && m.direct_staging != 3)) && half < 8192)
     IBCOMM_FAIL(NOT_SUPPORTED, "Two-shot allreduce through the pool needs a pool of at least 16 KiB.\n");
-  if (algo == Algo::kDirect && m.direct_staging == 0 && LocalKernelTakes(local)) {
+  if (algo == Algo::kOneShot) {
+    if (bytes > m.layout.oneshot_slot_bytes)
+      IBCOMM_FAIL(INVALID_ARGUMENT, "One-shot allreduce handles at most %llu bytes (got %zu).\n",
+                  static_cast<unsigned long long>(m.layout.oneshot_slot_bytes), bytes);
+    local.wire = local.dtype;  // it has no other
+  }
+  if ((algo == Algo::kDirect || algo == Algo::kOneShot) && m.direct_staging == 0 && LocalKernelTakes(local)) {
     CUDACHECK(LaunchLocalKernel(local, stream));
     m.last_channels = 0;
   } else if (pipelined) {
@@ -322,9 +328,6 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
     CUDACHECK(LaunchNvlsKernel(ps.data(), m.ws, ch, stream));
     m.last_channels = ch;
   } else if (algo == Algo::kOneShot) {
-    if (bytes > m.layout.oneshot_slot_bytes)
-      IBCOMM_FAIL(INVALID_ARGUMENT, "One-shot allreduce handles at most %llu bytes (got %zu).\n",
-                  static_cast<unsigned long long>(m.layout.oneshot_slot_bytes), bytes);
     std::vector<OneShotParams> ps;
     for (int r = 0; r < m.ws; ++r)
       ps.push_back(MakeOneShotParams(m.ranks[static_cast<size_t>(r)], dtype, sendbufs[static_cast<size_t>(r)],

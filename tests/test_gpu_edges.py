@@ -491,3 +491,31 @@ def test_staged_results_fetched_from_their_reducer(ws, dtype, wire):
         for o in results:
             assert torch.equal(o, results[0])
     world.close()
+
+
+@pytest.mark.parametrize("mode", [0, 3])
+@pytest.mark.parametrize("ws", [2, 3, 5, 8])
+def test_one_shot_pushed_and_in_place(ws, mode):
+    # The push into every rank's slot, several calls in a row on slots that alternate, and one kernel for all ranks: every
+    # element type, a wire type that one-shot does not have, ragged ends, slices that miss the boundary alike or not.
+    world = ar.EmuWorld(ws)
+    world.set_direct_staging(mode)
+    for dtype in (torch.float32, torch.float64, torch.bfloat16, torch.float16, torch.int32, torch.int64):
+        whole = dtype in (torch.int32, torch.int64)
+        scale = 1.0 if whole else 0.5
+        for n in (1, 7, 2048, 2049, 70001):
+            for off_in, off_out in ((0, 0), (1, 1), (1, 0)):
+                ins = [values(n, dtype, n + r, off_in) for r in range(ws)]
+                acc = ins[0].float() if dtype in (torch.bfloat16, torch.float16) else ins[0].clone()
+                for t in ins[1:]:
+                    acc += t
+                want = acc.to(dtype) if whole else (acc * scale).to(dtype)
+                guard = [torch.full((n + off_out + 8,), 7, device="cuda", dtype=dtype) for _ in range(ws)]
+                outs = [g[off_out:off_out + n] for g in guard]
+                for call in range(3):
+                    world.allreduce(ins, outs, algo="oneshot", scale=scale, wire=torch.bfloat16 if dtype == torch.float32 else None, sync=False)
+                world.allreduce(ins, None, algo="oneshot", scale=scale)
+                for g, o, i in zip(guard, outs, ins):
+                    assert torch.equal(o, want) and torch.equal(i, want)
+                    assert torch.all(g[:off_out] == 7) and torch.all(g[off_out + n:] == 7)
+    world.close()
