@@ -44,6 +44,9 @@ struct StagedShape {
   int load_groups, reduce_groups, store_groups;
 };
 
+// From which message on results are fetched from their reducers.
+constexpr size_t kPullBytes = 8u << 20;
+
 // `bytes`: of a rank's message in the wire type; `resident`: blocks of the kernel
 // the GPU holds at once.  Measured on a B200 (the knobs override each choice):
 //  * The windows of all ranks share one L2.  A line leaves it unwritten as soon as its
@@ -58,7 +61,8 @@ struct StagedShape {
 //    MiB: 170 against 200 with bulk copies).
 //  * A result is stored once, in its reducer's pool, and loaded there by the other ranks' storers: of 8 ranks, 2.0 times
 //    the results' bytes are written instead of 2.75, and the output windows fill an eighth of their lines.  Their lines
-//    have several readers and stay.  4 ranks x 64 MiB 163 -> 146 us, 8 x 32 MiB 189 -> 159, 5 x 64 MiB 225 -> 202.
+//    have several readers and stay.  4 ranks x 64 MiB 168 -> 145 us, 8 x 32 MiB 189 -> 157, 5 x 64 MiB 225 -> 199, 8 x 12 MiB
+//    79 -> 67; at 4 MiB and less within 2 %.
 //  * Four warps load, four store, eight reduce: 5 ranks x 64 MiB 229 us against 239
 //    with five, 2 x 12 MiB 21 against 23 (but 8 x 64 MiB 368 against 360).
 //  * A block per 16 KiB: with one per 128 KiB a 0.5 MiB message on 5 ranks takes
@@ -113,13 +117,13 @@ bool LinesPay(uint64_t bytes) {
 // Whether an op program's ranks read each other's sendbuf and store into each other's recvbuf, or send as between
 // GPUs.  us, sending and sharing:
 //   Rabenseifner  2 x 64 MiB 70 56, 5 x 64 MiB 265 157, 7 x 64 MiB 458 227, 8 x 64 MiB 428 323, 8 x 8 MiB 74 59; bf16 wire
-//                 4 x 64 MiB 155 139; slices off the boundary 4 x 4 MiB 88 77
+//                 4 x 64 MiB 155 139; slices off the boundary 4 x 4 MiB 88 77, 6 x 4 MB 185 84, 8 x 4 MB 197 206
 //   ring          2 x 64 MiB 71 57, 3 x 64 MiB 117 99, 4 x 4 MiB 32 29, 5 x 4 MiB 40 37, 5 x 64 MiB 202 201, 6 x 8 MiB 61 56;
 //                 but 7 x 64 MiB 286 302, 8 x 256 MiB 1234 1331, with a ragged end 7 x 4 MB 56 66, off the boundary 80 93
 // The ring's transfers wait for each other, and a result that lies in recvbuf is there later than one in a slot.
-bool SharingPays(Algo algo, int ws, size_t bytes, bool whole_vectors) {
-  if (algo == Algo::kRabenseifner) return true;
-  return whole_vectors && (ws <= 4 || (ws <= 6 && bytes <= (size_t(16) << 20)));
+bool SharingPays(Algo algo, int ws, size_t bytes, bool aligned) {
+  if (algo == Algo::kRabenseifner) return aligned || ws < 8;
+  return aligned && bytes % 16 == 0 && (ws <= 4 || (ws <= 6 && bytes <= (size_t(16) << 20)));
 }
 
 }  // namespace
@@ -259,8 +263,8 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.use_tma = (wire == dtype && Tunable("IBCOMM_STAGED_TMA", 0) != 0) ? 1 : 0;
       p.copy_warps = 4;
       p.drop_lines = p.use_tma == 0 ? 1 : 0;
-      // Between two ranks a result is stored once either way (2 x 12 MiB 22.8 us so, 24.1 with loads).
-      p.pull_results = p.use_tma == 0 && m.ws > 2 ? 1 : 0;
+      // Between two ranks a result is stored once either way, and what is short waits rather than streams.
+      p.pull_results = p.use_tma == 0 && m.ws > 2 && n * wsize >= kPullBytes ? 1 : 0;
       p.peers = rr.peers;
       p.sendbuf = sendbufs[static_cast<size_t>(r)];
       p.recvbuf = recvbufs[static_cast<size_t>(r)];
@@ -366,7 +370,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       ch = std::max(1, std::min({ch, m.line_max_blocks / m.ws, kMaxChannels}));
       CUDACHECK(LaunchLineKernel(ps.data(), m.ws, ch, m.layout.lines_half_bytes, stream));
     } else {
-      const bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, all_aligned && bytes % 16 == 0);
+      const bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, all_aligned);
       programs(shared ? ProgramForm::kShared : ProgramForm::kStaged);
       if (shared) {
         uint32_t present = 0;

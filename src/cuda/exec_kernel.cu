@@ -339,10 +339,15 @@ __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint
   using A = typename Acc<T>::type;
   constexpr int kU = 8;
   const OpBuffers<T, W> buf(op, p);
-  const T* a_src = op.src_a == kSrcSend ? buf.sendbuf : (kShared && op.src_a == kSrcPeer ? static_cast<const T*>(p.peer_send[op.rank_a]) : buf.recvbuf);
   const T* b_src = op.src_b == kSrcSend ? buf.sendbuf : (op.src_b == kSrcRecv ? buf.recvbuf : nullptr);
-  const T* c_src = kShared && op.rank_c >= 0 ? static_cast<const T*>(p.peer_send[op.rank_c]) : nullptr;
-  const bool round_peer = kShared && (op.flags & kOpRoundPeer) && sizeof(W) != sizeof(T);
+  // What is another rank's: sources, and (rounded through the wire type) their values.
+  const T *peer_a = nullptr, *peer_c = nullptr;
+  bool round_peer = false;
+  if constexpr (kShared) {
+    if (op.src_a == kSrcPeer) peer_a = static_cast<const T*>(p.peer_send[op.rank_a]);
+    if (op.rank_c >= 0) peer_c = static_cast<const T*>(p.peer_send[op.rank_c]);
+    round_peer = (op.flags & kOpRoundPeer) && sizeof(W) != sizeof(T);
+  }
   auto of_peer = [&](T v) -> A { return round_peer ? ThroughWire<W, A>(ToAcc<A, T>(v)) : ToAcc<A, T>(v); };
   for (uint64_t k0 = lo + tid; k0 < hi; k0 += static_cast<uint64_t>(nthr) * kU) {
     A a[kU];
@@ -351,10 +356,17 @@ __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint
     for (int u = 0; u < kU; ++u) {
       const uint64_t k = k0 + static_cast<uint64_t>(u) * nthr;
       if (k < hi) {
-        if (op.src_a == kSrcStage) a[u] = ToAcc<A, W>(LdScalarStrong<W>(buf.stage_in + k));
-        else a[u] = kShared && op.src_a == kSrcPeer ? of_peer(a_src[op.cell_begin + k]) : (kShared && op.src_a == kSrcRecv ? ToAcc<A, T>(LdScalarStrong<T>(a_src + op.cell_begin + k)) : ToAcc<A, T>(a_src[op.cell_begin + k]));
+        if (op.src_a == kSrcStage) {
+          a[u] = ToAcc<A, W>(LdScalarStrong<W>(buf.stage_in + k));
+        } else if (kShared && peer_a != nullptr) {
+          a[u] = of_peer(peer_a[op.cell_begin + k]);
+        } else if (kShared && op.src_a == kSrcRecv) {
+          a[u] = ToAcc<A, T>(LdScalarStrong<T>(buf.recvbuf + op.cell_begin + k));  // another rank may have stored it
+        } else {
+          a[u] = ToAcc<A, T>((op.src_a == kSrcSend ? buf.sendbuf : buf.recvbuf)[op.cell_begin + k]);
+        }
         if (b_src != nullptr) b[u] = b_src[op.cell_begin + k];
-        if (c_src != nullptr) c[u] = c_src[op.cell_begin + k];
+        if (kShared && peer_c != nullptr) c[u] = peer_c[op.cell_begin + k];
       }
     }
 #pragma unroll
@@ -362,14 +374,16 @@ __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint
       const uint64_t k = k0 + static_cast<uint64_t>(u) * nthr;
       if (k < hi) {
         A v = a[u];
-        if (c_src != nullptr) v += of_peer(c[u]);
+        if (kShared && peer_c != nullptr) v += of_peer(c[u]);
         if (b_src != nullptr) v += ToAcc<A, T>(b[u]);
         if (op.flags & kOpScale) v = ScaleAcc<A>(v, p.scale);
         if ((op.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) v = ThroughWire<W, A>(v);
         if (op.flags & kOpStoreLocal) buf.recvbuf[op.cell_begin + k] = FromAcc<T, A>(v);
         if (op.flags & kOpStoreRemote) buf.stage_out[k] = FromAcc<W, A>(v);
-        for (int q = 0; kShared && q < p.world_size; ++q)
-          if (op.store_peers >> q & 1) static_cast<T*>(p.peer_recv[q])[op.cell_begin + k] = FromAcc<T, A>(v);
+        if constexpr (kShared) {
+          for (int q = 0; q < p.world_size; ++q)
+            if (op.store_peers >> q & 1) static_cast<T*>(p.peer_recv[q])[op.cell_begin + k] = FromAcc<T, A>(v);
+        }
       }
     }
   }
@@ -619,7 +633,7 @@ __device__ void WaiterBody(const ExecParams& p, const WaitCtx& w, RoleSync* sync
       elem_begin = op.elem_begin;
       elem_count = op.elem_count;
       if (!bad && op.wait_in != 0) need_data = base | op.wait_in, from = op.peer_in;
-      if (!bad && op.wait_peer != 0) need_data = (base | 1u) + op.wait_peer, from = 16 + op.peer_in;
+      if (kShared && !bad && op.wait_peer != 0) need_data = (base | 1u) + op.wait_peer, from = 16 + op.peer_in;
       if (!bad && op.wait_credit != 0) need_credit = base | op.wait_credit, to = 8 + op.peer_out;
     }
     const int in_batch = p.num_ops - first < 32 ? p.num_ops - first : 32;
@@ -743,8 +757,10 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared<kShared>*
         post_out = op.post_out;
         post_credit = op.post_credit;
         peers = (static_cast<uint8_t>(op.peer_in) << 8) | static_cast<uint8_t>(op.peer_out);
+        if constexpr (kShared) {
 #pragma unroll
-        for (int m = 0; m < kMaxPeerPosts; ++m) told[m] = op.post_told[m], told_peers |= static_cast<uint8_t>(op.peer_told[m]) << (8 * m);
+          for (int m = 0; m < kMaxPeerPosts; ++m) told[m] = op.post_told[m], told_peers |= static_cast<uint8_t>(op.peer_told[m]) << (8 * m);
+        }
       }
       const bool tells = kShared && __any_sync(0xffffffffu, told[0] != 0);
       const int end = first + 32 < p.num_ops ? first + 32 : p.num_ops;
@@ -757,7 +773,7 @@ __device__ void ExecBody(const ExecParams& p, uint64_t seq, ExecShared<kShared>*
         unsigned upto = lane < data_warps ? LdAcquireShared(&sync->done[lane]) : 0xffffffffu;
         upto = __reduce_min_sync(0xffffffffu, upto);
         const int until = static_cast<int>(upto) < end ? static_cast<int>(upto) : end;
-        const bool fence = __any_sync(0xffffffffu, mine >= posted && mine < until && FlagsNeedFence(post_out | told[0], post_credit, p.drop_lines != 0));
+        const bool fence = __any_sync(0xffffffffu, mine >= posted && mine < until && FlagsNeedFence(kShared ? post_out | told[0] : post_out, post_credit, p.drop_lines != 0));
         __syncwarp();  // what the other lanes acquired is ordered before lane 0's fence
         if (fence && lane == 0) FencePeers(p.peers.one_gpu != 0);
         for (; posted < until; ++posted) {

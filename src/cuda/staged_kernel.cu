@@ -206,15 +206,15 @@ __device__ __forceinline__ void CastIn(unsigned char* smem, uint4* wire, const u
       });
 }
 
-// `off`: of the window in a staging memory.
-template <typename T, typename W>
-__device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, uint64_t off, const CopyParts& parts, uint64_t policy, const unsigned char* drop, int tid, int nthr) {
+// `off`: of the window in this rank's staging memory, at `own`, or (kPull) in that of the parts' reducers.
+template <typename T, typename W, bool kPull>
+__device__ __forceinline__ void CastOut(unsigned char* smem, uint4* user, const unsigned char* own, uint64_t off, const CopyParts& parts, uint64_t policy, const unsigned char* drop, int tid, int nthr) {
   using A = typename Acc<T>::type;
   constexpr int P = 16 / static_cast<int>(sizeof(W));
   constexpr int VT = P * static_cast<int>(sizeof(T)) / 16;
   AsyncRounds<kRoundVecs>(
       smem, parts, static_cast<unsigned>(tid), static_cast<unsigned>(nthr),
-      [&](const unsigned char* at, uint64_t vec, uint32_t slot, uint32_t) { CpAsync16(slot, at + off + vec * 16); },
+      [&](const unsigned char* at, uint64_t vec, uint32_t slot, uint32_t) { CpAsync16(slot, (kPull ? at : own) + off + vec * 16); },
       [&](uint64_t vec, const unsigned char* slot, uint32_t) {
         A acc[P];
         VecIO<W>::Load(*reinterpret_cast<const uint4*>(slot), acc);
@@ -290,7 +290,9 @@ __device__ inline bool BulkCopyPieces(BulkRing& ring, unsigned char* const* dst,
   return ok;
 }
 
-template <typename T, typename W, bool kMultimem, int kR>
+// kPull: results are fetched from their reducers (StagedParams::pull_results); a kernel of its own, since the other one's
+// storers then wait 10 % longer (2 x 4 MiB 14.5 -> 16.1 us).
+template <typename T, typename W, bool kMultimem, int kR, bool kPull>
 __global__ void __launch_bounds__(kStagedThreads, 1)
 StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
   static_assert(sizeof(W) <= sizeof(T), "the wire type is never wider than the buffer type");
@@ -371,7 +373,7 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
       if ((kOwnInPlace && s == me) || b >= e) continue;
       cp->from[cp->parts] = b;
       cp->to[cp->parts] = e;
-      cp->results[cp->parts] = p.stage[p.pull_results != 0 ? s : me];
+      cp->results[cp->parts] = p.stage[s];
       ++cp->parts;
     }
   };
@@ -515,8 +517,8 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         }
         FenceProxyAsyncAll();
       } else if (!tma) {
-        const unsigned char* const drop = p.drop_lines != 0 && p.pull_results == 0 ? win : nullptr;
-        CastOut<T, W>(smem, reinterpret_cast<uint4*>(user), p.out_off[j], parts_of(nv), once, drop, c.tid, c.nthr);
+        const unsigned char* const drop = p.drop_lines != 0 && !kPull ? win : nullptr;
+        CastOut<T, W, kPull>(smem, reinterpret_cast<uint4*>(user), p.stage[me], p.out_off[j], parts_of(nv), once, drop, c.tid, c.nthr);
       }
       RolePost(c, kRowOutFree, k, SG, base | (k + 1));
       if (role_w != 0 && gtid == 0) trace[2 * role_w + k].t_done = GlobalTimerNs();
@@ -584,14 +586,14 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
         // Results: to every rank's pool, or once to this rank's, where the others' storers fetch them.
         unsigned char* const own_out = p.stage[me] + p.out_off[j];
         auto store = [&](uint64_t idx, uint4 r) {
-          if (p.pull_results != 0) {
+          if constexpr (kPull) {
             St16(own_out + idx * 16, r);
             if (kOwnInPlace) St16(static_cast<unsigned char*>(p.recvbuf) + v0 * 16 + idx * 16, r);
-            return;
-          }
+          } else {
 #pragma unroll
-          for (int q = 0; q < kR; ++q)
-            if (q < ws) St16(to[q] + idx * 16, r);
+            for (int q = 0; q < kR; ++q)
+              if (q < ws) St16(to[q] + idx * 16, r);
+          }
         };
         // Vector v of an item is rank v's; this rank's own is the user's.
         auto drop = [&](int v, uint64_t idx) {
@@ -633,9 +635,9 @@ StagedKernel(const __grid_constant__ RankBlocks<StagedParams> all) {
 
 }  // namespace dev
 
-template <typename T, typename W, bool kMultimem, int kR>
+template <typename T, typename W, bool kMultimem, int kR, bool kPull = false>
 static cudaError_t LaunchStagedOne(const StagedParams* ranks, int n, int blocks, cudaStream_t stream) {
-  auto kernel = dev::StagedKernel<T, W, kMultimem, kR>;
+  auto kernel = dev::StagedKernel<T, W, kMultimem, kR, kPull>;
   const cudaError_t e = AllowSharedMemory(kernel, dev::kStagedSmemBytes);
   if (e != cudaSuccess) return e;
   return LaunchRanks(kernel, ranks, n, blocks, dev::kStagedThreads, dev::kStagedSmemBytes, stream);
@@ -650,6 +652,9 @@ static cudaError_t LaunchStagedTyped(const StagedParams* ranks, int n, int block
       return cudaErrorInvalidValue;
     }
   }
+  if (ranks->pull_results != 0)
+    return ranks->world_size <= 4 ? LaunchStagedOne<T, W, false, 4, true>(ranks, n, blocks, stream)
+                                  : LaunchStagedOne<T, W, false, kMaxRanks, true>(ranks, n, blocks, stream);
   switch (dev::RankClass(ranks->world_size)) {
     case 2: return LaunchStagedOne<T, W, false, 2>(ranks, n, blocks, stream);
     case 4: return LaunchStagedOne<T, W, false, 4>(ranks, n, blocks, stream);
@@ -675,7 +680,7 @@ cudaError_t LaunchStagedKernel(const StagedParams* ranks, int n, int blocks, cud
 
 int StagedKernelMaxCoResidentBlocks(int device) {
   int per_sm = 0, sms = 0;
-  auto kernel = dev::StagedKernel<float, float, false, kMaxRanks>;
+  auto kernel = dev::StagedKernel<float, float, false, kMaxRanks, true>;
   if (AllowSharedMemory(kernel, dev::kStagedSmemBytes) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, dev::kStagedThreads, dev::kStagedSmemBytes) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
