@@ -465,26 +465,28 @@ def test_executor_gives_up_cleanly(slots_only, algo, ws, mode):
 @pytest.mark.parametrize("dtype,wire", [(torch.float32, None), (torch.bfloat16, None), (torch.float32, torch.bfloat16)])
 @pytest.mark.parametrize("ws", [2, 3, 4, 7, 8])
 def test_staged_results_fetched_from_their_reducer(ws, dtype, wire):
-    # Results that the storers fetch from their reducers' windows (more than two ranks, copies by the threads) and that are
-    # stored into every rank's window (bulk copies): windows that are reused many times, a short last one, parts that end
-    # inside a line, one channel and several, calls back to back.
+    # Results that the storers fetch from their reducers' windows (more than two ranks, 8 MiB or more, copies by the threads)
+    # and that are stored into every rank's window: windows that are reused many times, a short last one, parts that end
+    # inside a line, several channels, copy roles in blocks of their own, calls back to back.
     world = ar.EmuWorld(ws, 128 << 10, 128 << 10)
     world.set_direct_staging(2)
     k = 8 if wire is not None or dtype == torch.bfloat16 else 4
-    for n in (k, k * ws, k * 1237, k * 16384 + k, 600000):
+    from_8_mib = (8 << 20) * k // 16
+    for n in (k * ws, k * 1237, from_8_mib - k, from_8_mib, from_8_mib + k * 5003):
         ins = [values(n, dtype, n + r) for r in range(ws)]
         results = []
-        for tma in (0, 1):
+        for tma, split, channels in ((0, 0, 0), (0, 0, 3), (0, 1, 0), (1, 0, 0)):
             ar.utils.set_tunable("IBCOMM_STAGED_TMA", tma)
+            ar.utils.set_tunable("IBCOMM_STAGED_SPLIT", split)
             try:
-                for channels in (0, 1, 3):
-                    outs = [torch.full_like(t, 7) for t in ins]
-                    for call in range(2):
-                        world.allreduce(ins, outs, algo="direct", scale=1.0 / ws, wire=wire, channels=channels, sync=False)
-                    torch.cuda.synchronize()
-                    results += outs
+                outs = [torch.full_like(t, 7) for t in ins]
+                for call in range(2):
+                    world.allreduce(ins, outs, algo="direct", scale=1.0 / ws, wire=wire, channels=channels, sync=False)
+                torch.cuda.synchronize()
+                results += outs
             finally:
                 ar.utils.set_tunable("IBCOMM_STAGED_TMA", -1)
+                ar.utils.set_tunable("IBCOMM_STAGED_SPLIT", -1)
         want = torch.stack([t.double() for t in ins]).sum(0) / ws
         tol = 1e-5 if dtype == torch.float32 and wire is None else 2e-2
         torch.testing.assert_close(results[0].double(), want, rtol=tol, atol=tol)
