@@ -101,17 +101,18 @@ int OneShotChannelsOnOneGpu(size_t bytes) {
 // Half of a rank's lines area at most: a slot for every transfer of 2 MiB by three to eight ranks.
 constexpr uint64_t kLinesHalfBytes = 16ull << 20;
 
-// Whether an op program's transfers travel as lines: `bytes` of a rank's message in the wire type.  Slots with flags
-// against lines, us (IBCOMM_LINES_MAX_KIB overrides):
+// Whether an op program's transfers travel as lines: `bytes` of a rank's message in the wire type.  Slots with flags (as
+// SharingPays says) against lines, us (IBCOMM_LINES_MAX_KIB overrides):
 //                   64 KiB       512 KiB      1 MiB        2 MiB        4 MB
-//   ring, 8 ranks   47.3  16.4   49.6  18.5   53.3  29.3   56.6  52.1   63.6  81
-//   ring, 5 ranks   30.6  12.3   32.2  12.9   34.8  14.4   35.3  32.1   38.9  46
-//   ring, 2 ranks   14.1   6.2   15.8   6.6   16.4   7.7   16.4   8.2   17.1  10
-//   Rabenseifner 8  36.9  20.5   38.8  20.5   40.5  25.2   43.1  40.2   55.7  (same)
-//   Rabenseifner 5  26.0  12.4   26.5  12.3   27.0  18.5   28.8  25.6   36.8  (same)
-// Up to 1.2 MB a thread has one pack of a transfer (148 SMs x 512 threads x 16 bytes), from there on several.
-bool LinesPay(uint64_t bytes) {
-  return bytes <= (static_cast<uint64_t>(std::max(0, Tunable("IBCOMM_LINES_MAX_KIB", 2048))) << 10);
+//   ring, 8 ranks   47.5  15.0   49.9  16.4   53.4  30.7   57.2  48.4   63.5  81
+//   ring, 5 ranks   28.7  11.6   29.0  12.3   31.8  13.2   33.4  29.9   40.4  47
+//   ring, 2 ranks    8.2   6.2    9.0   6.3    9.8   7.2   10.3   8.2   17.8  10
+//   Rabenseifner 8  25.1  16.4   26.7  18.5   28.7  23.3   30.8  38.5
+//   Rabenseifner 5  16.4  12.3   16.4  12.2   18.5  13.2   20.5  28.4
+//   Rabenseifner 3   8.2   8.2    8.2   8.2    8.9  10.0   10.3  12.4
+bool LinesPay(Algo algo, uint64_t bytes) {
+  const int most = Tunable("IBCOMM_LINES_MAX_KIB", algo == Algo::kRing ? 2048 : 1024);
+  return bytes <= (static_cast<uint64_t>(std::max(0, most)) << 10);
 }
 
 // Whether an op program's ranks read each other's sendbuf and store into each other's recvbuf, or send as between
@@ -357,7 +358,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       }
     };
     // Prescribed chunks and pieces, and ranks that hand over as between GPUs, keep the slots.
-    bool lines = m.direct_staging == 0 && LinesPay(n * wsize) && env::ReadChunkSize() <= 0 && Tunable("IBCOMM_RABEN_PIECES", 0) <= 0;
+    bool lines = m.direct_staging == 0 && LinesPay(algo, n * wsize) && env::ReadChunkSize() <= 0 && Tunable("IBCOMM_RABEN_PIECES", 0) <= 0;
     if (lines) {
       programs(ProgramForm::kLines);
       lines = fit;

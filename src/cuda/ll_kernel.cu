@@ -6,9 +6,9 @@
 // exec_kernel.cu one passes through six parties (data warps, poster with its fence,
 // flag, waiter, loader, bulk copy): 3-4 us on one GPU.  Here a thread reads the lines of
 // its packs until they are there, adds, and stores the next rank's lines: B200, us,
-// ring of 8 x 64 KiB 47.3 -> 16.4, 8 x 512 KiB 49.6 -> 18.5, 5 x 1 MiB 34.8 -> 14.4;
-// Rabenseifner 8 x 64 KiB 36.9 -> 20.5.  Beyond a pack per thread (1.2 MB) a step takes
-// as many trips to L2 as a thread has rounds of packs, and the bytes count twice.
+// ring of 8 x 64 KiB 47.3 -> 15.0, 8 x 512 KiB 49.6 -> 16.4, 5 x 1 MiB 34.8 -> 13.2;
+// Rabenseifner 8 x 64 KiB 36.9 -> 16.4.  Where a transfer fills the threads (1 MiB and
+// more) the looks and the doubled bytes are what L2 carries.
 //
 // A pack's place in its cell decides which channel and thread handle it, in every op
 // and on every rank.  So what an op reads from recvbuf was stored by the thread that
@@ -89,7 +89,7 @@ template <typename T, typename W>
 __device__ void LineBody(const ExecParams& p, uint64_t half_bytes, LinePlan* plan, const uint64_t* s_seq) {
   using Tr = ExecTraits<T, W>;
   using A = typename Tr::A;
-  constexpr int P = Tr::P, VT = Tr::VT, U = Tr::U;
+  constexpr int P = Tr::P, VT = Tr::VT;
   static_assert(Tr::VW == 1, "the wire type is never wider than the buffer type: a pack travels as one vector");
   const int ch = blockIdx.x, nch = gridDim.x;
   const unsigned tid = threadIdx.x;
@@ -161,87 +161,65 @@ __device__ void LineBody(const ExecParams& p, uint64_t half_bytes, LinePlan* pla
     const LinePlan pl = plan[oi];
     const uint32_t j0 = pl.lo / P, j1 = (pl.hi + P - 1) / P;
     const bool aligned = pl.aligned != 0;
-    for (uint32_t j = j0 + ((tid - j0) & (kLineThreads - 1)); j < j1; j += U * kLineThreads) {
-      uint4 a[U][VT], b[U][VT];
-      uint32_t e0[U], e1[U];
-      // The first pack's lines are looked for first; by the time they are there, so are the others' as a rule.  Looking
-      // for all of them keeps L2 busy.
-      unsigned missing = pl.lines_in != nullptr ? 1u : 0u, rest = 0;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint32_t ju = j + static_cast<uint32_t>(u) * kLineThreads;
-        e0[u] = e1[u] = 0;
-        if (ju < j1) {
-          e0[u] = pl.lo > ju * P ? pl.lo - ju * P : 0;
-          e1[u] = pl.hi < ju * P + P ? pl.hi - ju * P : P;
-          if (pl.user_b != nullptr) LdPack<T, VT, P>(pl.user_b + static_cast<size_t>(ju) * VT * 16, e0[u], e1[u], aligned, b[u]);
-          if (pl.user_a != nullptr) LdPack<T, VT, P>(pl.user_a + static_cast<size_t>(ju) * VT * 16, e0[u], e1[u], aligned, a[u]);
-          if (pl.lines_in != nullptr && u != 0) rest |= 1u << u;
-        }
-      }
-      LineWait wait;
-      while (missing != 0) {
-        Lines l[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (missing & (1u << u)) l[u] = LdLines(pl.lines_in + parity_off + static_cast<size_t>(j + static_cast<uint32_t>(u) * kLineThreads) * 16, apart);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if ((missing & (1u << u)) && HaveArrived(l[u], number)) {
-            a[u][0] = DataOf(l[u]);
-            missing &= ~(1u << u);
+    for (uint32_t j = j0 + ((tid - j0) & (kLineThreads - 1)); j < j1; j += kLineThreads) {
+      uint4 a[VT], b[VT];
+      const uint32_t e0 = pl.lo > j * P ? pl.lo - j * P : 0, e1 = pl.hi < j * P + P ? pl.hi - j * P : P;
+      const size_t at = static_cast<size_t>(j) * VT * 16, line = static_cast<size_t>(j) * 16 + parity_off;
+      // What does not depend on a peer is on its way while the lines are looked for.
+      if (pl.user_b != nullptr) LdPack<T, VT, P>(pl.user_b + at, e0, e1, aligned, b);
+      if (pl.user_a != nullptr) LdPack<T, VT, P>(pl.user_a + at, e0, e1, aligned, a);
+      if (pl.lines_in != nullptr) {
+        LineWait wait;
+        for (;;) {
+          const Lines l = LdLines(pl.lines_in + line, apart);
+          if (HaveArrived(l, number)) {
+            a[0] = DataOf(l);
+            break;
           }
-        if (missing == 0) {
-          missing = rest;
-          rest = 0;
-          continue;
-        }
-        const uint32_t over = wait.Again(w);
-        if (over != kStatusOk) {
-          // A rank that never came says more than the one before this, which waits for it too.
-          int peer = pl.peer_in;
-          uint32_t kind = kWaitData;
-          for (int q = p.world_size - 1; q >= 0; --q)
-            if (q != p.rank && LdRelaxedSys(&Ctl(p.peers, p.rank)->bar[ch][q]) < (base | 1u)) peer = q, kind = kWaitBarrier;
-          LineWaitOver(w, over, kind, peer, oi, base | 1u);
-          return;
+          const uint32_t over = wait.Again(w);
+          if (over != kStatusOk) {
+            // A rank that never came says more than the one before this, which waits for it too.
+            int peer = pl.peer_in;
+            uint32_t kind = kWaitData;
+            for (int q = p.world_size - 1; q >= 0; --q)
+              if (q != p.rank && LdRelaxedSys(&Ctl(p.peers, p.rank)->bar[ch][q]) < (base | 1u)) peer = q, kind = kWaitBarrier;
+            LineWaitOver(w, over, kind, peer, oi, base | 1u);
+            return;
+          }
         }
       }
+      A acc[P];
+      if (pl.lines_in != nullptr) {
+        VecIO<W>::Load(a[0], acc);
+      } else {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint32_t ju = j + static_cast<uint32_t>(u) * kLineThreads;
-        if (ju >= j1) continue;
-        A acc[P];
-        if (pl.lines_in != nullptr) {
-          VecIO<W>::Load(a[u][0], acc);
-        } else {
+        for (int v = 0; v < VT; ++v) VecIO<T>::Load(a[v], acc + v * VecIO<T>::kN);
+      }
+      if (pl.user_b != nullptr) {
 #pragma unroll
-          for (int v = 0; v < VT; ++v) VecIO<T>::Load(a[u][v], acc + v * VecIO<T>::kN);
-        }
-        if (pl.user_b != nullptr) {
+        for (int v = 0; v < VT; ++v) VecIO<T>::Add(b[v], acc + v * VecIO<T>::kN);
+      }
+      if (pl.flags & kOpScale) {
 #pragma unroll
-          for (int v = 0; v < VT; ++v) VecIO<T>::Add(b[u][v], acc + v * VecIO<T>::kN);
-        }
-        if (pl.flags & kOpScale) {
+        for (int e = 0; e < P; ++e) acc[e] = ScaleAcc<A>(acc[e], p.scale);
+      }
+      const uint4 wire = VecIO<W>::Store(acc);
+      if (pl.lines_out != nullptr) StLines(pl.lines_out + line, apart, wire, number);
+      if (pl.local != nullptr) {
+        if ((pl.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) VecIO<W>::Load(wire, acc);
+        uint4 out[VT];
 #pragma unroll
-          for (int e = 0; e < P; ++e) acc[e] = ScaleAcc<A>(acc[e], p.scale);
-        }
-        const uint4 wire = VecIO<W>::Store(acc);
-        if (pl.lines_out != nullptr) StLines(pl.lines_out + parity_off + static_cast<size_t>(ju) * 16, apart, wire, number);
-        if (pl.local != nullptr) {
-          if ((pl.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) VecIO<W>::Load(wire, acc);
-          uint4 out[VT];
-#pragma unroll
-          for (int v = 0; v < VT; ++v) out[v] = VecIO<T>::Store(acc + v * VecIO<T>::kN);
-          StPack<T, VT, P>(pl.local + static_cast<size_t>(ju) * VT * 16, e0[u], e1[u], aligned, out);
-        }
+        for (int v = 0; v < VT; ++v) out[v] = VecIO<T>::Store(acc + v * VecIO<T>::kN);
+        StPack<T, VT, P>(pl.local + at, e0, e1, aligned, out);
       }
     }
   }
 }
 
+// Two blocks per SM: a pack at a time in 64 registers.  With four in 120, one block per SM, 8 ranks x 512 KiB take 18.5 us
+// instead of 16.4 (ring) and 20.5 instead of 18.5 (Rabenseifner).
 template <typename T, typename W>
-__global__ void __launch_bounds__(kLineThreads, 1)
+__global__ void __launch_bounds__(kLineThreads, 2)
 LineKernel(const __grid_constant__ RankBlocks<ExecParams> all, uint64_t half_bytes) {
   const ExecParams& p = all.rank[blockIdx.y];
   __shared__ LinePlan s_plan[kMaxLineOps];
