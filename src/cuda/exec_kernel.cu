@@ -64,8 +64,9 @@ namespace dev {
 
 constexpr int kExecServiceWarps = 3;  // waiter, loader, poster
 constexpr int kExecMaxStages = 10;
-// A stage holds U packs per data thread from each of two sources, 2 U from one or
-// U / 2 from three: 128 bytes per data thread for every pair of types (96 with three).
+// A stage holds U packs per data thread from each of two sources: 128 bytes per data thread
+// for every pair of types.  Where ranks share a GPU it takes 2 U from one source (5 ranks x
+// 64 MiB Rabenseifner 160 -> 157 us; the ring of ranks that send 3 % slower) and U / 2 from three.
 // Half of that leaves a warp waiting for its own shared-memory reads (5 ranks x 64 MiB
 // Rabenseifner 496 us against 430).
 constexpr int kExecStageBytesPerThread = 128;
