@@ -56,7 +56,8 @@ class EmuWorld:
         check(_native.lib().ibcomm_emu_set_timeout_ms(self._h, ms))
 
     def set_silent_rank(self, rank: int) -> None:
-        """Test hook: ``rank`` skips the following collectives (-1: nobody does)."""
+        """Test hook: ``rank`` skips the following ring and Rabenseifner calls, and those of the pipelined staged kernel
+        (-1: nobody does)."""
         check(_native.lib().ibcomm_emu_set_silent_rank(self._h, rank))
 
     def set_bad_program_rank(self, rank: int) -> None:

@@ -113,8 +113,8 @@ int ibcomm_emu_set_timeout_ms(ibcomm_emu* w, int ms);
 int ibcomm_emu_rsag(ibcomm_emu* w, int all_gather, int dtype, const void* const* sendbufs, void* const* recvbufs,
                     size_t block_elements, double scale, int channels, void* stream, int async);
 int ibcomm_emu_last_channels(ibcomm_emu* w);
-/* Test hook: rank `rank` does not take part in the following collectives
- * (-1 = everybody takes part), so its peers' bounded waits run out. */
+/* Test hook: rank `rank` does not take part in the following ring and Rabenseifner calls and in those of the pipelined
+ * staged kernel (-1 = everybody takes part), so its peers' bounded waits run out. */
 int ibcomm_emu_set_silent_rank(ibcomm_emu* w, int rank);
 /* Test hook: rank `rank` fails the executor's per-op bounds check (-1 = nobody);
  * no memory is touched out of range, the call reports "bad program". */

@@ -44,9 +44,11 @@ class EmuWorld {
   // first failure report among the ranks.
   uint32_t LastStatus(DeviceStatus* report) const;
   void SetTimeoutMs(int ms);
-  // Test hook: rank `r` takes no part in the following collectives (its CTAs
-  // return at once), so its peers' bounded waits run out and they report a
-  // timeout; nothing faults or hangs.  -1 restores normal operation.
+  // Test hook: rank `r` takes no part in the following ring and Rabenseifner calls
+  // and in those of the pipelined staged kernel (SetDirectStaging(2), or a 16-bit
+  // wire; its CTAs return at once), so its peers' bounded waits run out and they
+  // report a timeout; nothing faults or hangs.  The other collectives take no notice.
+  // -1 restores normal operation.
   void SetSilentRank(int r);
   // Test hook for the executor's self-check: rank `r` is told a message length
   // of one element for programs cut for the real length, so its first op fails

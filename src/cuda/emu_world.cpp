@@ -245,7 +245,9 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
                   static_cast<unsigned long long>(m.layout.oneshot_slot_bytes), bytes);
     local.wire = local.dtype;  // it has no other
   }
-  if ((algo == Algo::kDirect || algo == Algo::kOneShot) && m.direct_staging == 0 && LocalKernelTakes(local)) {
+  // Ranks wait for each other in the staged kernel only, so that is where one that stays away is noticed.
+  const bool silent = pipelined && m.silent_rank >= 0;
+  if ((algo == Algo::kDirect || algo == Algo::kOneShot) && m.direct_staging == 0 && !silent && LocalKernelTakes(local)) {
     CUDACHECK(LaunchLocalKernel(local, stream));
     m.last_channels = 0;
   } else if (pipelined) {
@@ -344,13 +346,16 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
   } else {
     // Validation (length, chunk size) happens while the first program is cut.
     std::vector<ExecParams> ps;
-    bool fit = true;
+    bool fit = true, hooked_has_ops = true;
     auto programs = [&](ProgramForm form) {
       ps.clear();
       for (int r = 0; r < m.ws; ++r) {
         const CachedProgram& cp = m.cache.Get(algo, r, m.ws, n, dtype, wire, m.layout, scale != 1.0, stream, false, m.ws, form);
         fit = fit && LinesFit(cp.prog);
-        if (form == ProgramForm::kShared && cp.prog.ops.empty()) continue;  // an extra rank: the others read its sendbuf and store into its recvbuf
+        if (form == ProgramForm::kShared && cp.prog.ops.empty()) {  // an extra rank: the others read its sendbuf and store into its recvbuf
+          if (r == m.silent_rank || r == m.bad_program_rank) hooked_has_ops = false;
+          continue;
+        }
         ps.push_back(MakeExecParams(m.ranks[static_cast<size_t>(r)], cp, dtype, wire, sendbufs[static_cast<size_t>(r)],
                                     recvbufs[static_cast<size_t>(r)], n, scale, timeout_ns, nullptr, 0));
         if (r == m.silent_rank) ps.back().num_ops = 0;
@@ -371,8 +376,13 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       ch = std::max(1, std::min({ch, m.line_max_blocks / m.ws, kMaxChannels}));
       CUDACHECK(LaunchLineKernel(ps.data(), m.ws, ch, m.layout.lines_half_bytes, stream));
     } else {
-      const bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, all_aligned);
+      bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, all_aligned);
       programs(shared ? ProgramForm::kShared : ProgramForm::kStaged);
+      if (!hooked_has_ops) {
+        // A rank that is to stay away, or to fail its self-check, needs ops of its own for that.
+        shared = false;
+        programs(ProgramForm::kStaged);
+      }
       if (shared) {
         uint32_t present = 0;
         for (const ExecParams& p : ps) present |= 1u << p.rank;

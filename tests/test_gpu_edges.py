@@ -521,3 +521,48 @@ def test_one_shot_pushed_and_in_place(ws, mode):
                     assert torch.equal(o, want) and torch.equal(i, want)
                     assert torch.all(g[:off_out] == 7) and torch.all(g[off_out + n:] == 7)
     world.close()
+
+
+@pytest.mark.parametrize("hook,codes", [("silent", (1, 2)), ("bad_program", (3,))])
+@pytest.mark.parametrize("ws,rank", [(3, 0), (5, 0), (6, 2), (7, 4)])
+def test_hooks_reach_extra_ranks(ws, rank, hook, codes):
+    # Ranks that have no blocks where ranks share buffers: one that is to stay away, or to fail its self-check, still does.
+    # Longer than what goes as lines.
+    world = ar.EmuWorld(ws)
+    world.set_timeout_ms(200)
+    ins = [values(2000000, torch.float32, r) for r in range(ws)]
+    outs = [torch.zeros_like(t) for t in ins]
+    set_hook = world.set_silent_rank if hook == "silent" else world.set_bad_program_rank
+    set_hook(rank)
+    with pytest.raises(ar.IbcommError) as e:
+        world.allreduce(ins, outs, algo="rabenseifner")
+    assert e.value.code == ar.TRANSPORT_ERROR
+    assert world.last_status()["code"] in codes
+    set_hook(-1)
+    world.set_timeout_ms(5000)
+    for algo in ("rabenseifner", "ring"):
+        world.allreduce(ins, outs, algo=algo)
+        want = torch.stack([t.double() for t in ins]).sum(0)
+        for o in outs:
+            torch.testing.assert_close(o.double(), want, rtol=1e-5, atol=1e-5)
+    world.close()
+
+
+def test_silent_rank_of_direct_with_16_bit_wire():
+    # The others wait for it in the staged kernel, although the buffers could be used in place.
+    world = ar.EmuWorld(4)
+    world.set_timeout_ms(200)
+    ins = [values(1 << 16, torch.float32, r) for r in range(4)]
+    outs = [torch.zeros_like(t) for t in ins]
+    world.set_silent_rank(1)
+    with pytest.raises(ar.IbcommError) as e:
+        world.allreduce(ins, outs, algo="direct", wire=torch.bfloat16)
+    assert e.value.code == ar.TRANSPORT_ERROR
+    assert world.last_status()["code"] in (1, 2)
+    world.set_silent_rank(-1)
+    world.set_timeout_ms(5000)
+    world.allreduce(ins, outs, algo="direct", wire=torch.bfloat16)
+    want = torch.stack([t.double() for t in ins]).sum(0)
+    for o in outs:
+        torch.testing.assert_close(o.double(), want, rtol=2e-2, atol=2e-2)
+    world.close()
