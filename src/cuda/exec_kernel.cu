@@ -333,23 +333,35 @@ __device__ __forceinline__ void RunTile(const ExecTile<kShared>& t, const ExecTi
   }
 }
 
-// Element-at-a-time path for chunks that do not start on a 16-byte boundary;
-// kU loads of each source in flight per thread.
+// Element-at-a-time path for chunks that do not start on a 16-byte boundary; kU
+// loads of each source in flight per thread.  Bound by instructions: what the op says
+// is read once, not for every element (it lies in global memory, which the stores
+// below may change for all the compiler knows), and four loads keep this path and the
+// tiles, which share its registers, from spilling.  With eight and the op's fields read
+// anew, us: ring 8 x 4 MiB 199 -> 99, Rabenseifner 8 x 4 MiB 214 -> 113, 4 x 4 MiB of
+// fp64 75 -> 33; aligned, ring 4 x 64 MiB of fp64 180 -> 157.  With eight and the fields
+// read once the same here, but the aligned ring of 4 to 6 ranks that share buffers 7 % slower.
 template <typename T, typename W, bool kShared>
 __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint64_t hi, unsigned tid, unsigned nthr) {
   using A = typename Acc<T>::type;
-  constexpr int kU = 8;
+  constexpr int kU = 4;
   const OpBuffers<T, W> buf(op, p);
   const T* b_src = op.src_b == kSrcSend ? buf.sendbuf : (op.src_b == kSrcRecv ? buf.recvbuf : nullptr);
   // What is another rank's: sources, and (rounded through the wire type) their values.
   const T *peer_a = nullptr, *peer_c = nullptr;
   bool round_peer = false;
   if constexpr (kShared) {
-    if (op.src_a == kSrcPeer) peer_a = static_cast<const T*>(p.peer_send[op.rank_a]);
-    if (op.rank_c >= 0) peer_c = static_cast<const T*>(p.peer_send[op.rank_c]);
+    if (op.src_a == kSrcPeer) peer_a = static_cast<const T*>(p.peer_send[op.rank_a]) + op.cell_begin;
+    if (op.rank_c >= 0) peer_c = static_cast<const T*>(p.peer_send[op.rank_c]) + op.cell_begin;
     round_peer = (op.flags & kOpRoundPeer) && sizeof(W) != sizeof(T);
   }
+  const uint64_t cell_begin = op.cell_begin;
+  const uint8_t src_a = op.src_a, flags = op.flags, store_peers = op.store_peers;
+  const T* const a_src = (src_a == kSrcSend ? buf.sendbuf : buf.recvbuf) + op.cell_begin;
+  if (b_src != nullptr) b_src += op.cell_begin;
+  T* const out = buf.recvbuf + op.cell_begin;
   auto of_peer = [&](T v) -> A { return round_peer ? ThroughWire<W, A>(ToAcc<A, T>(v)) : ToAcc<A, T>(v); };
+#pragma unroll 1
   for (uint64_t k0 = lo + tid; k0 < hi; k0 += static_cast<uint64_t>(nthr) * kU) {
     A a[kU];
     T b[kU], c[kU];
@@ -357,17 +369,17 @@ __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint
     for (int u = 0; u < kU; ++u) {
       const uint64_t k = k0 + static_cast<uint64_t>(u) * nthr;
       if (k < hi) {
-        if (op.src_a == kSrcStage) {
+        if (src_a == kSrcStage) {
           a[u] = ToAcc<A, W>(LdScalarStrong<W>(buf.stage_in + k));
         } else if (kShared && peer_a != nullptr) {
-          a[u] = of_peer(peer_a[op.cell_begin + k]);
-        } else if (kShared && op.src_a == kSrcRecv) {
-          a[u] = ToAcc<A, T>(LdScalarStrong<T>(buf.recvbuf + op.cell_begin + k));  // another rank may have stored it
+          a[u] = of_peer(peer_a[k]);
+        } else if (kShared && src_a == kSrcRecv) {
+          a[u] = ToAcc<A, T>(LdScalarStrong<T>(out + k));  // another rank may have stored it
         } else {
-          a[u] = ToAcc<A, T>((op.src_a == kSrcSend ? buf.sendbuf : buf.recvbuf)[op.cell_begin + k]);
+          a[u] = ToAcc<A, T>(a_src[k]);
         }
-        if (b_src != nullptr) b[u] = b_src[op.cell_begin + k];
-        if (kShared && peer_c != nullptr) c[u] = peer_c[op.cell_begin + k];
+        if (b_src != nullptr) b[u] = b_src[k];
+        if (kShared && peer_c != nullptr) c[u] = peer_c[k];
       }
     }
 #pragma unroll
@@ -377,13 +389,13 @@ __device__ void RunElements(const Op& op, const ExecParams& p, uint64_t lo, uint
         A v = a[u];
         if (kShared && peer_c != nullptr) v += of_peer(c[u]);
         if (b_src != nullptr) v += ToAcc<A, T>(b[u]);
-        if (op.flags & kOpScale) v = ScaleAcc<A>(v, p.scale);
-        if ((op.flags & kOpRoundWire) && sizeof(W) != sizeof(T)) v = ThroughWire<W, A>(v);
-        if (op.flags & kOpStoreLocal) buf.recvbuf[op.cell_begin + k] = FromAcc<T, A>(v);
-        if (op.flags & kOpStoreRemote) buf.stage_out[k] = FromAcc<W, A>(v);
+        if (flags & kOpScale) v = ScaleAcc<A>(v, p.scale);
+        if ((flags & kOpRoundWire) && sizeof(W) != sizeof(T)) v = ThroughWire<W, A>(v);
+        if (flags & kOpStoreLocal) out[k] = FromAcc<T, A>(v);
+        if (flags & kOpStoreRemote) buf.stage_out[k] = FromAcc<W, A>(v);
         if constexpr (kShared) {
           for (int q = 0; q < p.world_size; ++q)
-            if (op.store_peers >> q & 1) static_cast<T*>(p.peer_recv[q])[op.cell_begin + k] = FromAcc<T, A>(v);
+            if (store_peers >> q & 1) static_cast<T*>(p.peer_recv[q])[cell_begin + k] = FromAcc<T, A>(v);
         }
       }
     }
