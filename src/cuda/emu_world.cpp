@@ -401,7 +401,8 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       // SM at most (two smaller ones per SM are no faster).
       const uint64_t slot = ps.back().stage.slot_bytes;
       ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(slot / 4096, static_cast<uint64_t>(kMaxChannels)));
-      ch = std::max(1, std::min(ch, (channels > 0 ? m.exec_max_blocks : m.max_blocks) / rows));
+      // A short program may leave one rank with blocks, which the GPU holds more of than there are flags.
+      ch = std::max(1, std::min({ch, (channels > 0 ? m.exec_max_blocks : m.max_blocks) / rows, kMaxChannels}));
       CUDACHECK(LaunchExecKernel(ps.data(), rows, ch, stream));
     }
     m.last_channels = ch;

@@ -566,3 +566,16 @@ def test_silent_rank_of_direct_with_16_bit_wire():
     for o in outs:
         torch.testing.assert_close(o.double(), want, rtol=2e-2, atol=2e-2)
     world.close()
+
+
+def test_one_rank_with_blocks_in_prescribed_channels(slots_only):
+    # One piece, one rank that sums it: as many blocks as there are flags of a rank (256) at most.
+    world = ar.EmuWorld(2)
+    for n in (2, 31):
+        ins = [values(n, torch.float32, n + r) for r in range(2)]
+        outs = [torch.full_like(t, 7) for t in ins]
+        world.allreduce(ins, outs, algo="rabenseifner", channels=1000)
+        assert 1 <= world.last_channels <= 256
+        for o in outs:
+            torch.testing.assert_close(o, ins[0] + ins[1], rtol=1e-6, atol=1e-6)
+    world.close()
