@@ -110,9 +110,15 @@ constexpr uint64_t kLinesHalfBytes = 16ull << 20;
 //   Rabenseifner 8  25.1  16.4   26.7  18.5   28.7  23.3   30.8  38.5
 //   Rabenseifner 5  16.4  12.3   16.4  12.2   18.5  13.2   20.5  28.4
 //   Rabenseifner 3   8.2   8.2    8.2   8.2    8.9  10.0   10.3  12.4
-bool LinesPay(Algo algo, uint64_t bytes) {
+// One bound for all world sizes, although two ranks' rings are better off as lines up to 4 MB and three ranks'
+// Rabenseifner is not at 1 MiB.
+// `turns`: packs of a transfer that a thread handles one after the other, more than one where the caller prescribes fewer
+// channels than a pack per thread takes.  Each turn waits for lines anew (ring, 8 ranks x 2 MiB in 32, 16, 8 and 4 channels
+// 46, 50, 67 and 113 us as lines, 58, 56, 60 and 76 through slots), so the bound is that of the turns together; from five on
+// lines gain little or nothing (5 ranks x 256 KiB in one channel, seven turns, 44 us against 43).
+bool LinesPay(Algo algo, uint64_t bytes, uint64_t turns) {
   const int most = Tunable("IBCOMM_LINES_MAX_KIB", algo == Algo::kRing ? 2048 : 1024);
-  return bytes <= (static_cast<uint64_t>(std::max(0, most)) << 10);
+  return turns <= 4 && bytes * turns <= (static_cast<uint64_t>(std::max(0, most)) << 10);
 }
 
 // Whether an op program's ranks read each other's sendbuf and store into each other's recvbuf, or send as between
@@ -363,17 +369,17 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       }
     };
     // Prescribed chunks and pieces, and ranks that hand over as between GPUs, keep the slots.
-    bool lines = m.direct_staging == 0 && LinesPay(algo, n * wsize) && env::ReadChunkSize() <= 0 && Tunable("IBCOMM_RABEN_PIECES", 0) <= 0;
+    bool lines = m.direct_staging == 0 && LinesPay(algo, n * wsize, 1) && env::ReadChunkSize() <= 0 && Tunable("IBCOMM_RABEN_PIECES", 0) <= 0;
+    int ch = 0;
     if (lines) {
       programs(ProgramForm::kLines);
-      lines = fit;
-    }
-    int ch;
-    if (lines) {
       // A thread per pack of a transfer.
-      const uint64_t packs = ps.back().stage.slot_bytes / 16;
-      ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>((packs + 511) / 512, static_cast<uint64_t>(kMaxChannels)));
+      const uint64_t blocks = (ps.back().stage.slot_bytes / 16 + 511) / 512;
+      ch = channels > 0 ? channels : static_cast<int>(std::min<uint64_t>(blocks, static_cast<uint64_t>(kMaxChannels)));
       ch = std::max(1, std::min({ch, m.line_max_blocks / m.ws, kMaxChannels}));
+      lines = fit && LinesPay(algo, n * wsize, (blocks + static_cast<uint64_t>(ch) - 1) / static_cast<uint64_t>(ch));
+    }
+    if (lines) {
       CUDACHECK(LaunchLineKernel(ps.data(), m.ws, ch, m.layout.lines_half_bytes, stream));
     } else {
       bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, all_aligned);

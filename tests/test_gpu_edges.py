@@ -579,3 +579,27 @@ def test_one_rank_with_blocks_in_prescribed_channels(slots_only):
         for o in outs:
             torch.testing.assert_close(o, ins[0] + ins[1], rtol=1e-6, atol=1e-6)
     world.close()
+
+
+@pytest.mark.parametrize("mode", [0, 3])
+@pytest.mark.parametrize("algo", ["ring", "rabenseifner"])
+@pytest.mark.parametrize("ws", [2, 3, 5, 8])
+def test_op_programs_in_prescribed_channels(ws, algo, mode):
+    # Few channels for what goes as lines otherwise (packs that a thread handles one after the other, up to four and more),
+    # for programs that share buffers and for those that send; more channels than there are packs, or than the GPU holds.
+    world = ar.EmuWorld(ws)
+    world.set_direct_staging(mode)
+    for n in (ws, 2521, 16384, 65536 + 5, 262144, 600001):
+        for dtype in (torch.float32, torch.bfloat16):
+            ins = [values(n, dtype, n + r) for r in range(ws)]
+            want = torch.stack([t.double() for t in ins]).sum(0) / ws
+            tol = 1e-5 if dtype == torch.float32 else 2e-2
+            for channels in (1, 2, 3, 8, 31, 1000):
+                outs = [torch.full_like(t, 7) for t in ins]
+                for call in range(2):
+                    world.allreduce(ins, outs, algo=algo, scale=1.0 / ws, channels=channels)
+                assert 1 <= world.last_channels <= channels
+                for o in outs:
+                    torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
+                    assert torch.equal(o, outs[0])
+    world.close()
