@@ -122,15 +122,39 @@ bool LinesPay(Algo algo, uint64_t bytes, uint64_t turns) {
 }
 
 // Whether an op program's ranks read each other's sendbuf and store into each other's recvbuf, or send as between
-// GPUs.  us, sending and sharing:
-//   Rabenseifner  2 x 64 MiB 70 56, 5 x 64 MiB 265 157, 7 x 64 MiB 458 227, 8 x 64 MiB 428 323, 8 x 8 MiB 74 59; bf16 wire
-//                 4 x 64 MiB 155 139; slices off the boundary 4 x 4 MiB 88 77, 6 x 4 MB 185 84, 8 x 4 MB 197 206
-//   ring          2 x 64 MiB 71 57, 3 x 64 MiB 117 99, 4 x 4 MiB 32 29, 5 x 4 MiB 40 37, 5 x 64 MiB 202 201, 6 x 8 MiB 61 56;
-//                 but 7 x 64 MiB 286 302, 8 x 256 MiB 1234 1331, with a ragged end 7 x 4 MB 56 66, off the boundary 80 93
-// The ring's transfers wait for each other, and a result that lies in recvbuf is there later than one in a slot.
-bool SharingPays(Algo algo, int ws, size_t bytes, bool aligned) {
-  if (algo == Algo::kRabenseifner) return aligned || ws < 8;
-  return aligned && bytes % 16 == 0 && (ws <= 4 || (ws <= 6 && bytes <= (size_t(16) << 20)));
+// GPUs.  `bytes` of a rank's message, `wire_bytes` of it in the wire type, `words`: of 4-byte elements that travel as they
+// are; `channels` prescribed or 0.  Rabenseifner always (.28 to .97 in 2600 calls of 2 to 8 ranks).  The ring's
+// transfers wait for each other, and a result that lies in recvbuf is there later than one in a slot, which does not show as
+// long as the ranks are few and the parts short.  Sharing as a multiple of the time of sending, ring:
+//                        4 MiB  8    12    16    24    32    64   128
+//   2 ranks fp32          .67  .70   .73   .76   .79   .76   .76   .75
+//   3 ranks fp32 / bf16   .83  .81   .86   .85   .88   .81   .85   .84    /  .81  .86  .86  .88  .94  .88  .88  .92
+//   4 ranks fp32          .87  .87   .88   .92   .98   .99   .97   .96
+//           bf16          .89  .90   .92   .96  1.05  1.04  1.04  1.03
+//           fp64          .90  .88   .92   .94  1.01  1.03  1.00   .99
+//           bf16 wire     .91  .89   .91   .92   .93   .99  1.03  1.01
+//   6 ranks fp32          .93  .93   .95  1.00  1.05  1.00  1.01  1.03
+//           bf16 / fp64   .96  .96  1.00  1.06  1.12  1.08  1.08  1.11    /  .96  .94  .98  1.03
+//           bf16 wire     .96  .93   .95   .96  1.00  1.04  1.03  1.02
+//   8 ranks fp32          .98  .97  1.00  1.03  1.08  1.10  1.09  1.08
+//   ragged ends 4 ranks 1.00 to 1.05, 5 ranks 1.10 to 1.15; slices off the boundary 3 ranks .86 to .97, 4 ranks 1.06 to 1.14
+//   in prescribed channels, bytes a channel:  256 KiB   512 KiB    1 MiB    2 MiB
+//   3 ranks fp32, 2 to 16 channels              .80       .90      1.01     1.00
+//   5 ranks fp32, 2 to 16 channels              .91       .92      1.05     1.16
+//   6 ranks fp32, one / two channels         1.01 .96  1.05 .96  1.07 1.07  1.21
+//   and beyond a block per SM, 4 ranks in 48 channels 8 MiB .93, 16 MiB 1.10; 5 ranks in 32 channels 4 MiB .95, 8 MiB 1.05
+bool SharingPays(Algo algo, int ws, size_t bytes, size_t wire_bytes, bool words, bool aligned, int channels) {
+  if (algo == Algo::kRabenseifner) return true;
+  if (!aligned || bytes % 16 != 0 || ws > 6) return false;
+  if (ws == 2) return true;
+  if (channels > 0) {
+    size_t most = channels == 1 ? size_t(256) << 10 : static_cast<size_t>(channels) << 19;
+    if (ws > 3 && channels * ws > 148) most = std::min(most, size_t(4) << 20);
+    if (bytes > most) return false;
+  }
+  if (ws == 3) return true;
+  if (ws == 4) return words || wire_bytes <= (size_t(16) << 20);
+  return wire_bytes <= (size_t(words ? 16 : 12) << 20);
 }
 
 }  // namespace
@@ -382,7 +406,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
     if (lines) {
       CUDACHECK(LaunchLineKernel(ps.data(), m.ws, ch, m.layout.lines_half_bytes, stream));
     } else {
-      bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, all_aligned);
+      bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, n * wsize, esize == 4 && wsize == 4, all_aligned, std::min(channels, m.exec_max_blocks / m.ws));
       programs(shared ? ProgramForm::kShared : ProgramForm::kStaged);
       if (!hooked_has_ops) {
         // A rank that is to stay away, or to fail its self-check, needs ops of its own for that.
