@@ -114,11 +114,13 @@ constexpr uint64_t kLinesHalfBytes = 16ull << 20;
 // Rabenseifner is not at 1 MiB.
 // `turns`: packs of a transfer that a thread handles one after the other, more than one where the caller prescribes fewer
 // channels than a pack per thread takes.  Each turn waits for lines anew (ring, 8 ranks x 2 MiB in 32, 16, 8 and 4 channels
-// 46, 50, 67 and 113 us as lines, 58, 56, 60 and 76 through slots), so the bound is that of the turns together; from five on
-// lines gain little or nothing (5 ranks x 256 KiB in one channel, seven turns, 44 us against 43).
+// 46, 50, 67 and 113 us as lines, 58, 56, 60 and 76 through slots), so there is a bound of all turns together, half as much
+// again as that of one; from five on lines gain little or nothing (5 ranks x 256 KiB in one channel, seven turns, 44 us
+// against 43).
 bool LinesPay(Algo algo, uint64_t bytes, uint64_t turns) {
   const int most = Tunable("IBCOMM_LINES_MAX_KIB", algo == Algo::kRing ? 2048 : 1024);
-  return turns <= 4 && bytes * turns <= (static_cast<uint64_t>(std::max(0, most)) << 10);
+  const uint64_t bound = static_cast<uint64_t>(std::max(0, most)) << 10;
+  return turns <= 4 && bytes <= bound && bytes * turns <= bound + bound / 2;
 }
 
 // Whether an op program's ranks read each other's sendbuf and store into each other's recvbuf, or send as between
