@@ -33,7 +33,8 @@ class EmuWorld:
     def allreduce(self, sendbufs: Sequence[torch.Tensor], recvbufs: Optional[Sequence[torch.Tensor]] = None, *,
                   algo: str = "ring", scale: float = 1.0, wire=None, channels: int = 0,
                   stream: Optional[torch.cuda.Stream] = None, sync: bool = True):
-        """``recvbufs[r]`` = scale * sum over r of ``sendbufs[r]`` for every emulated rank."""
+        """``recvbufs[r]`` = scale * sum over r of ``sendbufs[r]`` for every emulated rank.  ``channels``: blocks that a
+        rank may have at most, 0 leaves them to the library."""
         if recvbufs is None:
             recvbufs = sendbufs
         _native.fast().emu_allreduce(self._h.value, self.num_ranks, sendbufs, recvbufs, ALGO_CODES[algo], scale,
@@ -73,6 +74,7 @@ class EmuWorld:
 
     @property
     def last_channels(self) -> int:
+        """Blocks per rank of the last collective, 0 where one kernel ran for all ranks."""
         return _native.lib().ibcomm_emu_last_channels(self._h)
 
     def last_status(self) -> dict:

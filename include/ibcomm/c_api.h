@@ -112,6 +112,7 @@ int ibcomm_emu_allreduce(ibcomm_emu* w, int algo, int dtype, const void* const* 
 int ibcomm_emu_set_timeout_ms(ibcomm_emu* w, int ms);
 int ibcomm_emu_rsag(ibcomm_emu* w, int all_gather, int dtype, const void* const* sendbufs, void* const* recvbufs,
                     size_t block_elements, double scale, int channels, void* stream, int async);
+/* Blocks per rank of the last collective, 0 where one kernel ran for all ranks (which takes no prescribed `channels`). */
 int ibcomm_emu_last_channels(ibcomm_emu* w);
 /* Test hook: rank `rank` does not take part in the following ring and Rabenseifner calls and in those of the pipelined
  * staged kernel (-1 = everybody takes part), so its peers' bounded waits run out. */
@@ -119,7 +120,10 @@ int ibcomm_emu_set_silent_rank(ibcomm_emu* w, int rank);
 /* Test hook: rank `rank` fails the executor's per-op bounds check (-1 = nobody);
  * no memory is touched out of range, the call reports "bad program". */
 int ibcomm_emu_set_bad_program_rank(ibcomm_emu* w, int rank);
-/* Direct algorithm: in place (0, default) or staged through the pool windows (1). */
+/* How the ranks treat the buffers.  0 (default): they share a GPU and its memory; direct, one-shot, reduce-scatter and
+ * all-gather run one kernel for all ranks, short ring and Rabenseifner calls hand over in lines, long ones use each other's
+ * buffers.  Else as ranks with a GPU each, and the direct algorithm: 1 staged through the pool windows, 2 staged through
+ * the pipelined kernel, 3 in place with barriers. */
 int ibcomm_emu_set_direct_staging(ibcomm_emu* w, int on);
 typedef struct {
   uint32_t code;

@@ -26,7 +26,8 @@ class EmuWorld {
   int num_ranks() const { return ws_; }
 
   // Device pointers, one per rank.  Runs on `stream` (0 = default stream) and
-  // returns after synchronising unless `async`.
+  // returns after synchronising unless `async`.  `channels`: blocks that a rank may
+  // have at most, 0 leaves them to the library.
   void Allreduce(Algo algo, DType dtype, const std::vector<const void*>& sendbufs,
                  const std::vector<void*>& recvbufs, size_t len_elements, double scale = 1.0,
                  DType wire = DType::kFloat32, int channels = 0, void* stream = nullptr, bool async = false);
@@ -56,12 +57,13 @@ class EmuWorld {
   // program", the others are told to stop.  -1 restores normal operation.
   void SetBadProgramRank(int r);
   // How the ranks treat the buffers.  0: they share a GPU.  The direct and the
-  // one-shot algorithm run one kernel for all ranks, short op programs hand over in
-  // lines, long ones use each other's buffers.  Else as ranks that have a GPU each,
+  // one-shot algorithm run one kernel for all ranks (unless `channels` are prescribed),
+  // short op programs hand over in lines, long ones use each other's buffers.  Else as ranks that have a GPU each,
   // and the direct algorithm: 1 staged through the pool window by window (as for buffers the
   // peers cannot map), 2 staged through the pipelined kernel, 3 in place with
   // barriers.
   void SetDirectStaging(int mode);
+  // Blocks per rank of the last collective, 0 where one kernel ran for all ranks.
   int last_channels() const;
 
   struct Impl;

@@ -277,9 +277,11 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
                   static_cast<unsigned long long>(m.layout.oneshot_slot_bytes), bytes);
     local.wire = local.dtype;  // it has no other
   }
-  // Ranks wait for each other in the staged kernel only, so that is where one that stays away is noticed.
+  // Ranks wait for each other in the staged kernel only, so that is where one that stays away is noticed.  The kernel for all
+  // ranks has as many blocks as there are vectors; where the caller says how many a rank may have, those with channels run.
   const bool silent = pipelined && m.silent_rank >= 0;
-  if ((algo == Algo::kDirect || algo == Algo::kOneShot) && m.direct_staging == 0 && !silent && LocalKernelTakes(local)) {
+  const bool one_kernel = m.direct_staging == 0 && channels <= 0 && !silent;
+  if ((algo == Algo::kDirect || algo == Algo::kOneShot) && one_kernel && LocalKernelTakes(local)) {
     CUDACHECK(LaunchLocalKernel(local, stream));
     m.last_channels = 0;
   } else if (pipelined) {
@@ -347,7 +349,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
       p.timeout_ns = timeout_ns;
       p.status = rr.d_status;
       p.doorbell = rr.d_doorbell;
-      const bool staged = m.direct_staging != 3 || !all_aligned;
+      const bool staged = (m.direct_staging != 0 && m.direct_staging != 3) || !all_aligned;
       p.stage_in = staged ? 1 : 0;
       p.stage_out = staged ? 1 : 0;
       for (int q = 0; q < m.ws; ++q) {
@@ -475,7 +477,7 @@ void EmuWorld::ReduceScatterOrAllGather(bool all_gather, DType dtype, const std:
   bool same_phase = true;
   auto remote_of = [&](int q) { return reinterpret_cast<uintptr_t>(all_gather ? recvbufs[static_cast<size_t>(q)] : sendbufs[static_cast<size_t>(q)]); };
   for (int q = 1; q < m.ws; ++q) same_phase = same_phase && ((remote_of(0) ^ remote_of(q)) & 15u) == 0;
-  if (m.direct_staging == 0 && same_phase) {
+  if (m.direct_staging == 0 && same_phase && channels <= 0) {
     LocalParams local{};
     local.op = all_gather ? LocalOp::kAllGather : LocalOp::kReduceScatter;
     local.world_size = m.ws;
@@ -489,7 +491,7 @@ void EmuWorld::ReduceScatterOrAllGather(bool all_gather, DType dtype, const std:
     CUDACHECK(LaunchLocalKernel(local, stream));
     m.last_channels = 0;
   } else {
-    const bool staged = m.direct_staging != 3 || !same_phase;
+    const bool staged = (m.direct_staging != 0 && m.direct_staging != 3) || !same_phase;
     const uint64_t sub = m.layout.pool_bytes / static_cast<uint64_t>(m.ws) / 4096 * 4096;
     if (staged && sub < 4096) IBCOMM_FAIL(NOT_SUPPORTED, "Reduce-scatter / all-gather through the pool need a larger pool.\n");
     const int cap = std::max(1, m.max_blocks / m.ws);

@@ -603,3 +603,35 @@ def test_op_programs_in_prescribed_channels(ws, algo, mode):
                     torch.testing.assert_close(o.double(), want, rtol=tol, atol=tol)
                     assert torch.equal(o, outs[0])
     world.close()
+
+
+@pytest.mark.parametrize("ws", [2, 3, 8])
+def test_prescribed_channels_of_buffers_in_place(ws):
+    # Direct (with and without a 16-bit wire), one-shot and the halves keep to the blocks that the caller allows; the bits are
+    # those of the kernel that runs for all ranks otherwise.
+    world = ar.EmuWorld(ws)
+    for n in (8 * ws, 8 * 1237, 65536):
+        ins = [values(n, torch.float32, n + r) for r in range(ws)]
+        for algo, wire in (("direct", None), ("direct", torch.bfloat16), ("oneshot", None)):
+            want = [torch.full_like(t, 7) for t in ins]
+            world.allreduce(ins, want, algo=algo, scale=1.0 / ws, wire=wire)
+            for channels in (1, 3, 8):
+                outs = [torch.full_like(t, 7) for t in ins]
+                world.allreduce(ins, outs, algo=algo, scale=1.0 / ws, wire=wire, channels=channels)
+                assert world.last_channels == channels
+                for o, t in zip(outs, want):
+                    assert torch.equal(o, t)
+        block = n // ws
+        full = [t[:block * ws] for t in ins]
+        shards = [torch.full((block,), 7.0, device="cuda") for _ in range(ws)]
+        world.reduce_scatter(full, shards, scale=0.5)
+        for channels in (1, 3, 8):
+            again = [torch.full_like(t, 7) for t in shards]
+            world.reduce_scatter(full, again, scale=0.5, channels=channels)
+            assert world.last_channels == channels
+            whole = [torch.full_like(t, 7) for t in full]
+            world.all_gather(shards, whole, channels=channels)
+            assert world.last_channels == channels
+            for r in range(ws):
+                assert torch.equal(again[r], shards[r]) and torch.equal(whole[r], torch.cat(shards))
+    world.close()
