@@ -35,7 +35,7 @@ def test_copy_scale_quanta_heads_and_tails(types, offsets):
         assert torch.all(guard[:offsets[1]] == 7) and torch.all(guard[offsets[1] + n:] == 7), n
 
 
-@pytest.mark.parametrize("staged", [0, 1])
+@pytest.mark.parametrize("staged", [0, 1, 3])
 @pytest.mark.parametrize("offset", [0, 1, 3])
 @pytest.mark.parametrize("ws", [2, 3, 8])
 def test_reduce_scatter_and_all_gather_ragged_blocks(ws, offset, staged):
@@ -64,12 +64,14 @@ def test_reduce_scatter_and_all_gather_ragged_blocks(ws, offset, staged):
     world.close()
 
 
+@pytest.mark.parametrize("mode", [0, 3])
 @pytest.mark.parametrize("algo", ["oneshot", "direct", "ring", "rabenseifner"])
 @pytest.mark.parametrize("ws", [2, 3, 5, 8])
-def test_allreduce_ragged_ends(ws, algo):
+def test_allreduce_ragged_ends(ws, algo, mode):
     # Lengths around a vector, a round of loads per thread, a stage of the executor and a part on cache lines, all with
     # a ragged end; slices off the boundary; 16-bit wires where there are op programs.
     world = ar.EmuWorld(ws)
+    world.set_direct_staging(mode)
     wires = [None, torch.bfloat16] if algo in ("ring", "rabenseifner") else [None]
     for dtype in (torch.float32, torch.bfloat16, torch.float64):
         for offset in (0, 1):
@@ -88,15 +90,17 @@ def test_allreduce_ragged_ends(ws, algo):
     world.close()
 
 
+@pytest.mark.parametrize("mode", [0, 3])
 @pytest.mark.parametrize("in_place", [False, True])
 @pytest.mark.parametrize("ws", [2, 3, 4, 5, 6, 7, 8])
-def test_rabenseifner_segments(ws, in_place):
+def test_rabenseifner_segments(ws, in_place, mode):
     # A small staging area makes segments of a few pieces: one, an exact number of them, a last one that is shorter
     # or lacks blocks, and many; partial sums read back from recvbuf.
     p = 1 << (ws.bit_length() - 1)
     regions = max(p.bit_length() - 1 + ws - p, p if ws != p else 0)
     area = 2 * regions * 65536
     world = ar.EmuWorld(ws, area // 2, area // 2)
+    world.set_direct_staging(mode)
     for wire, size in ((None, 4), (torch.bfloat16, 2)):
         piece = 65536 // size
         for n in (p, piece * p, piece * p + 1, 2 * piece * p - 5, 5 * piece * p + piece + 3):
@@ -134,10 +138,12 @@ def test_staged_windows_reused(ws, wire):
     world.close()
 
 
+@pytest.mark.parametrize("mode", [0, 3])
 @pytest.mark.parametrize("ws", [2, 5, 8])
-def test_rabenseifner_drops_lines(ws):
+def test_rabenseifner_drops_lines(ws, mode):
     # Long enough for slots whose lines are dropped as they are read; a ragged end, in place as well, two calls.
     world = ar.EmuWorld(ws)
+    world.set_direct_staging(mode)
     n = (52 << 20) // 4 // ws + 7
     for in_place in (False, True):
         for call in range(2):
@@ -150,9 +156,10 @@ def test_rabenseifner_drops_lines(ws):
     world.close()
 
 
+@pytest.mark.parametrize("mode", [0, 3])
 @pytest.mark.parametrize("ws", [2, 5, 7, 8])
-def test_rabenseifner_drops_lines_of_reused_slots(ws):
-    # Two slots per partner for many transfers: a slot is written again, by a peer, right after its lines were
+def test_rabenseifner_drops_lines_of_reused_slots(ws, mode):
+    # Two slots per partner for many transfers (two ranks that share buffers have none): a slot is written again, by a peer, right after its lines were
     # dropped.  Small whole numbers are summed, exactly, so a transfer that a late drop destroyed cannot come out right by chance.
     area = 4 << 20
     p = 1 << (ws.bit_length() - 1)
@@ -161,6 +168,7 @@ def test_rabenseifner_drops_lines_of_reused_slots(ws):
     largest_piece = area // (2 * regions) // 4
     assert n // largest_piece // 2 > 2 * 2  # half the message goes to the first partner
     world = ar.EmuWorld(ws, area // 2, area // 2)
+    world.set_direct_staging(mode)
     for in_place in (False, True):
         for call in range(3):
             ins = [values(n, torch.float32, r + call, 0) if call == 0 else torch.full((n,), float(1 + r + call), device="cuda") for r in range(ws)]
@@ -175,14 +183,16 @@ def test_rabenseifner_drops_lines_of_reused_slots(ws):
     world.close()
 
 
+@pytest.mark.parametrize("mode", [0, 3])
 @pytest.mark.parametrize("ws", [3, 5, 6, 7])
-def test_rabenseifner_blocks_longer_than_the_slots(ws):
-    # The message as one, in small pieces of which the slots hold a few: what the extra ranks contribute comes before
+def test_rabenseifner_blocks_longer_than_the_slots(ws, mode):
+    # The message as one, in small pieces of which the slots hold a few: what the extra ranks send (mode 3) comes before
     # all else then.  In place as well.
     lib = ar._native.lib()
     lib.ibcomm_set_tunable(b"IBCOMM_RABEN_PIECES", 64)
     try:
         world = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+        world.set_direct_staging(mode)
         for dtype in (torch.float32, torch.bfloat16):
             n = 64 * 16384 + 5
             for in_place in (False, True):
@@ -233,10 +243,12 @@ def test_longer_and_pinned_outputs():
     world.close()
 
 
+@pytest.mark.parametrize("mode", [2, 0])
 @pytest.mark.parametrize("pages", [6, 7, 8])
-def test_staged_in_the_smallest_staging(pages):
-    # Three windows of each kind is the least the kernel works with: six pages of staging.
+def test_staged_in_the_smallest_staging(pages, mode):
+    # Three windows of each kind is the least the staged kernel works with: six pages of staging.
     world = ar.EmuWorld(2, (pages - 1) * 4096, 4096)
+    world.set_direct_staging(mode)
     ins = [values(8 * 3001, torch.float32, r) for r in range(2)]
     outs = [torch.full_like(t, 7) for t in ins]
     world.allreduce(ins, outs, algo="direct", wire=torch.bfloat16)

@@ -18,6 +18,14 @@ def world(ws, pool=0, work=0):
     return _worlds[key]
 
 
+@pytest.fixture(params=[0, 3], ids=["shared", "own_gpu"])
+def mode(request):
+    # As ranks that share a GPU and its memory, and with the kernels and programs of ranks that have a GPU each.
+    yield request.param
+    for w in _worlds.values():
+        w.set_direct_staging(0)
+
+
 def make_inputs(ws, n, dtype, seed=0):
     g = torch.Generator(device="cuda")
     g.manual_seed(seed)
@@ -58,8 +66,9 @@ def test_native_library_is_loaded():
 
 @pytest.mark.parametrize("algo", ["ring", "rabenseifner"])
 @pytest.mark.parametrize("ws", [2, 3, 4, 5, 6, 7, 8])
-def test_program_algorithms_all_world_sizes(algo, ws):
+def test_program_algorithms_all_world_sizes(algo, ws, mode):
     w = world(ws)
+    w.set_direct_staging(mode)
     for n in (ws, 2 * ws, 2521, 65536 + 3, 1 << 20):
         ins = make_inputs(ws, n, torch.float32, seed=n)
         outs = [torch.full((n,), float("nan"), device="cuda") for _ in range(ws)]
@@ -69,9 +78,10 @@ def test_program_algorithms_all_world_sizes(algo, ws):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.int32, torch.int64, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("algo", ["ring", "rabenseifner", "oneshot"])
-def test_dtypes(algo, dtype):
+def test_dtypes(algo, dtype, mode):
     ws = 4
     w = world(ws)
+    w.set_direct_staging(mode)
     for n in (1000, 32768):
         ins = make_inputs(ws, n, dtype, seed=7)
         outs = [torch.zeros(n, device="cuda", dtype=dtype) for _ in range(ws)]
@@ -83,9 +93,10 @@ def test_dtypes(algo, dtype):
 
 
 @pytest.mark.parametrize("algo", ["ring", "rabenseifner", "oneshot"])
-def test_scale_and_in_place(algo):
+def test_scale_and_in_place(algo, mode):
     ws = 8
     w = world(ws)
+    w.set_direct_staging(mode)
     n = 40000
     ins = make_inputs(ws, n, torch.float32, seed=3)
     want = reference(ins, 1.0 / ws, torch.float32)
@@ -96,9 +107,10 @@ def test_scale_and_in_place(algo):
 
 @pytest.mark.parametrize("algo", ["ring", "rabenseifner"])
 @pytest.mark.parametrize("wire", [torch.bfloat16, torch.float16])
-def test_wire_compression(algo, wire):
+def test_wire_compression(algo, wire, mode):
     ws = 4
     w = world(ws)
+    w.set_direct_staging(mode)
     n = 1 << 18
     ins = make_inputs(ws, n, torch.float32, seed=11)
     outs = [torch.zeros(n, device="cuda") for _ in range(ws)]
@@ -110,13 +122,14 @@ def test_wire_compression(algo, wire):
 
 
 @pytest.mark.parametrize("algo", ["ring", "rabenseifner"])
-def test_small_staging_forces_slot_reuse(algo):
+def test_small_staging_forces_slot_reuse(algo, mode):
     # 1 MiB pool / work region with an 8 MiB message: chunks are cut to fit and
     # every staging slot is reused many times (credits).
     # Lengths that leave the last chunk shorter than the others: a slot then
     # holds chunks of different lengths over time.
     for ws in (4, 7):
         w = world(ws, 1 << 20, 1 << 20)
+        w.set_direct_staging(mode)
         for n in (2 << 20, (2 << 20) + 12345, 1000003):
             ins = make_inputs(ws, n, torch.float32, seed=5)
             outs = [torch.zeros(n, device="cuda") for _ in range(ws)]
@@ -128,11 +141,11 @@ def test_small_staging_forces_slot_reuse(algo):
 @pytest.mark.parametrize("ws", [2, 3, 4, 5, 8])
 def test_direct_two_shot(ws):
     # The two-shot kernel with peer loads/stores (the code path of the NVLS
-    # kernel minus multimem): in place on the ranks' buffers, and staged
-    # through pool windows (1 MiB pool = 512 KiB windows, so 4 MiB messages
+    # kernel minus multimem): in place on the ranks' buffers (by one kernel for all ranks, and by each rank's with
+    # barriers), and staged through pool windows (1 MiB pool = 512 KiB windows, so 4 MiB messages
     # take several windows; the odd lengths end in a short last window).
     w = world(ws, 1 << 20, 1 << 20)
-    for staged in (0, 1):
+    for staged in (0, 1, 3):
         w.set_direct_staging(staged)
         for n in (ws, 1000, 65536 + 3, 300001, 1 << 20, (1 << 20) + 12345):
             for dtype in (torch.float32, torch.bfloat16, torch.int32):
@@ -221,13 +234,14 @@ def test_pipelined_staged_groups_and_posters(ws, shape):
         w.set_direct_staging(0)
 
 
-@pytest.mark.parametrize("split", [1, 0])
+@pytest.mark.parametrize("staging,split", [(2, 1), (2, 0), (0, 0)])
 @pytest.mark.parametrize("wire", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("ws", [2, 4, 8])
-def test_two_shot_with_16_bit_wire(ws, wire, split):
+def test_two_shot_with_16_bit_wire(ws, wire, staging, split):
     # fp32 buffers, 16-bit values in the pool and on the wire, fp32 sums: the direct two-shot through the
-    # pipelined kernel.  Every rank must end up with the same bits.
+    # pipelined kernel, and rounded alike in place.  Every rank must end up with the same bits.
     w = world(ws, 1 << 20, 1 << 20)
+    w.set_direct_staging(staging)
     ar.utils.set_tunable("IBCOMM_STAGED_SPLIT", split)
     try:
         for n in (8 * ws, 65536, 300000, (1 << 20) + 8):
@@ -239,6 +253,7 @@ def test_two_shot_with_16_bit_wire(ws, wire, split):
                 assert torch.equal(o, outs[0])
     finally:
         ar.utils.set_tunable("IBCOMM_STAGED_SPLIT", -1)
+        w.set_direct_staging(0)
 
 
 @pytest.mark.parametrize("split", [1, 0])
@@ -267,9 +282,10 @@ def test_pipelined_staged_wait_runs_out(split):
         ar.utils.set_tunable("IBCOMM_STAGED_SPLIT", -1)
 
 
-def test_unaligned_buffers_take_the_scalar_path():
+def test_unaligned_buffers_take_the_scalar_path(mode):
     ws = 3
     w = world(ws)
+    w.set_direct_staging(mode)
     n = 5000
     base = make_inputs(ws, n + 1, torch.float32, seed=9)
     ins = [t[1:] for t in base]  # 4-byte aligned only
@@ -280,9 +296,10 @@ def test_unaligned_buffers_take_the_scalar_path():
         check(outs, reference(ins, 1.0, torch.float32), torch.float32, ws)
 
 
-def test_repeated_calls_mixed_algorithms():
+def test_repeated_calls_mixed_algorithms(mode):
     ws = 8
     w = world(ws)
+    w.set_direct_staging(mode)
     n = 50000
     ins = make_inputs(ws, n, torch.float32, seed=1)
     outs = [torch.zeros(n, device="cuda") for _ in range(ws)]
@@ -309,11 +326,12 @@ def test_error_codes():
     assert e.value.code == ar.NOT_SUPPORTED
 
 
-def test_bounded_wait_reports_timeout():
+def test_bounded_wait_reports_timeout(mode):
     # One rank does not take part: the others' waits run out after the limit,
     # the kernel returns, the status says who was missing, and the world stays usable.
     ws = 4
     w = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+    w.set_direct_staging(mode)
     w.set_timeout_ms(200)
     n = 4096
     ins = make_inputs(ws, n, torch.float32)
@@ -333,11 +351,11 @@ def test_bounded_wait_reports_timeout():
 @pytest.mark.parametrize("ws", [2, 3, 5, 8])
 def test_reduce_scatter_and_all_gather(ws):
     # The halves of the two-shot allreduce as collectives: in place on the
-    # ranks' buffers and through pool windows (1 MiB pool, so the larger
+    # ranks' buffers (by one kernel for all ranks, and with barriers) and through pool windows (1 MiB pool, so the larger
     # blocks take several windows, the last one short); blocks of whole
     # 16-byte vectors and ragged ones (element units); every element type.
     w = world(ws, 1 << 20, 1 << 20)
-    for staged in (0, 1):
+    for staged in (0, 1, 3):
         w.set_direct_staging(staged)
         for m in (1, 37, 4096, 100000 // ws * 4, 70001):
             for dtype in (torch.float32, torch.bfloat16, torch.int32, torch.float64):
@@ -368,12 +386,13 @@ def test_reduce_scatter_and_all_gather(ws):
     w.set_direct_staging(0)
 
 
-def test_executor_self_check_reports_bad_program():
+def test_executor_self_check_reports_bad_program(mode):
     # A rank whose ops do not fit the message it was given stops at the bounds
     # check of its first op (before any access), reports "bad program" and
     # tells the others to stop; the world stays usable.
     ws = 4
     w = ar.EmuWorld(ws, 1 << 20, 1 << 20)
+    w.set_direct_staging(mode)
     w.set_timeout_ms(2000)
     n = 8192
     ins = make_inputs(ws, n, torch.float32)
