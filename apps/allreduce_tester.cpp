@@ -15,7 +15,7 @@
 //                                         when every rank can have its own GPU)
 //                --dtype int|float|double element type (default int)
 //                --emulate N              run N ranks inside this one process
-//                                         on one GPU (single cooperative kernel)
+//                                         on one GPU (a single launch)
 //                --iters K                repeat the allreduce K times
 //                --ranks a,b,...          only the listed ranks of the job take
 //                                         part (the others exit with status 0);
@@ -220,7 +220,7 @@ int RunRanks(const Args& a) {
   if (a.emulate > 0 && a.op != "allreduce")
     IBCOMM_FAIL(NOT_SUPPORTED, "--emulate runs allreduce only.\n");
   if (a.emulate > 0) {
-    // All ranks in this process, one GPU, one cooperative kernel.
+    // All ranks in this process, one GPU, one launch.
     const int np = a.emulate;
     std::vector<std::vector<T>> ins(static_cast<size_t>(np), std::vector<T>(n)), outs = ins;
     for (int p = 0; p < np; ++p) {

@@ -316,9 +316,9 @@ def main() -> int:
             else:
                 per_algo["nccl_registered"] = {"error": note}
         else:
-            # One GPU: the same kernels with 8 emulated ranks in one cooperative
-            # launch (32 MiB per rank; local memory only, so this is a kernel
-            # check, not an NVLink number).
+            # One GPU: 8 ranks that share it and its memory (32 MiB per rank; the
+            # ring hands over as between GPUs, Rabenseifner uses the other ranks'
+            # buffers; local memory only, so this is no NVLink number).
             emu = ar.EmuWorld(8)
             m = 8 << 20
             ins = [torch.rand(m, device=dev) for _ in range(8)]
@@ -783,6 +783,7 @@ def kernel_case(args, comm, dev, time_steps) -> int:
         moved = None
     elif case in ("reduce_scatter_emu8", "all_gather_emu8"):
         emu = ar.EmuWorld(8)
+        emu.set_direct_staging(3)  # the kernel of ranks that have a GPU each
         m = 1 << 20  # elements per block: 32 MiB per rank in the full buffers
         full = [torch.rand(8 * m, device=dev) for _ in range(8)]
         shard = [torch.rand(m, device=dev) for _ in range(8)]
@@ -795,8 +796,9 @@ def kernel_case(args, comm, dev, time_steps) -> int:
         emu = ar.EmuWorld(8)
         algo = {"exec_ring_emu8": "ring", "exec_rabenseifner_emu8": "rabenseifner", "oneshot_emu8": "oneshot",
                 "direct_emu8": "direct", "staged_emu8": "direct"}[case]
-        if case == "staged_emu8":
-            emu.set_direct_staging(2)  # the pipelined staged kernel: copy in, peer reduce and copy out overlap
+        # The kernels of ranks that have a GPU each; 2: the pipelined staged kernel, where copy in, peer reduce and copy out
+        # overlap.
+        emu.set_direct_staging(2 if case == "staged_emu8" else 3)
         m = (16 << 10) if algo == "oneshot" else (8 << 20)  # elements per rank: 64 KiB or 32 MiB
         ins = [torch.rand(m, device=dev) for _ in range(8)]
         outs = [torch.empty(m, device=dev) for _ in range(8)]

@@ -104,7 +104,7 @@ int ibcomm_dump_trace(ibcomm_comm* c);
  * (8 x windows: pairs of nanoseconds from the first stamp; reducers, loader, storer, reducers' last store). */
 int ibcomm_staged_timeline(ibcomm_comm* c, uint64_t* out, size_t capacity_words, size_t* words);
 
-/* Several ranks emulated on one GPU (single cooperative launch per collective). */
+/* Several ranks emulated on one GPU (a single launch per collective). */
 int ibcomm_emu_create(int num_ranks, size_t pool_bytes, size_t work_bytes, ibcomm_emu** out);
 int ibcomm_emu_destroy(ibcomm_emu* w);
 int ibcomm_emu_allreduce(ibcomm_emu* w, int algo, int dtype, const void* const* sendbufs, void* const* recvbufs,

@@ -41,7 +41,7 @@
 // of them other ranks' buffers, and store into other ranks' recvbuf; a stage takes as many
 // packs as fit with that many sources.  5 ranks x 64 MiB Rabenseifner 271 -> 158 us, 7 x 64
 // MiB 458 -> 227, ring 2 x 64 MiB 71 -> 56.  The extra rank's work, the first step's sends
-// and the results' slots are gone: 64 block reads and writes a segment instead of 120.
+// and the results' slots are gone: of 5 ranks 60 block reads and writes a segment instead of 128.
 // Counterpart of the reference's host event loop around _reduce_inplace_cuda
 // (ibcomm/allreduce_cuda_impl.h:24-33, 103-299, 470-707).
 //
@@ -412,7 +412,7 @@ struct RingPos {
 };
 
 // The loader: turns the program into stages, in order, ahead of the data warps.
-// The lanes work out 32 ops at a time (an op is a 64-byte load and a division,
+// The lanes work out 32 ops at a time (an op is an 80-byte load and a division,
 // 1.5 us one after the other); lane 0 then only issues copies.  Returns after it
 // has handed out the exit stage (or could not, because the data warps gave up).
 template <typename T, typename W, bool kShared>

@@ -3,7 +3,8 @@
 // number of the call.  Whoever reads a line again and again until both numbers
 // are there has the data with the same access; a hand-over costs a store and a
 // load, no fence, no flag and no second trip for the data.  Twice the bytes, so it
-// is for messages that wait rather than stream.
+// is for messages that wait rather than stream.  (The idea is that of the low-latency
+// protocols of collective libraries; layout, numbering and code are this library's.)
 //
 // A half line is one 64-bit access, so its data and its number cannot be seen
 // apart; nothing depends on the order of the halves.  The memory is used for
