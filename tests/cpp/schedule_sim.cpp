@@ -137,6 +137,10 @@ MINI_TEST(RanksOnOneGpu) {
           CHECK_TRUE(RunCase<double>(Algo::kRing, ws, n, 0, 65536, nch, in_place, 0.5, 16384, 0, 0, true));
           CHECK_TRUE(RunCase<int>(Algo::kRabenseifner, ws, n, 0, size_t(1) << 22, nch, in_place, 1.0, 0, 1000, 0, true));
         }
+      for (size_t n : {size_t(2521), size_t(40007)}) {  // prescribed chunks and pieces
+        CHECK_TRUE(RunCase<int>(Algo::kRing, ws, n, 256, 65536, 2, in_place, 1.0, 16384, 0, 0, true));
+        CHECK_TRUE(RunCase<double>(Algo::kRabenseifner, ws, n, 512, 65536, 2, in_place, 0.5, 0, 64, 0, true));
+      }
       const size_t p = ws < 4 ? 2 : ws < 8 ? 4 : 8, regions = static_cast<size_t>(NumRegions(Algo::kRabenseifner, ws));
       for (size_t own : {size_t(1), size_t(3)})
         for (size_t n : {own * p * 256, 2 * own * p * 256 - 5, 20003 + 4 * own * p * 256})
