@@ -89,6 +89,7 @@ inline void IbcommWarning(const char* filename, int line, const char* format,
   do {                                                                        \
     cudaError_t e__ = (cmd);                                                  \
     if (e__ != cudaSuccess) {                                                 \
+      (void)cudaGetLastError(); /* reported here, not by the next launch */   \
       ::util::IbcommError(__FILE__, __LINE__,                                 \
                           ::util::IBCOMM_ERROR_CODE::CUDA_ERROR, "%s\n",      \
                           cudaGetErrorString(e__));                           \
