@@ -139,13 +139,15 @@ bool LinesPay(Algo algo, uint64_t bytes, uint64_t turns) {
 //           bf16 / fp64   .96  .96  1.00  1.06  1.12  1.08  1.08  1.11    /  .96  .94  .98  1.03
 //           bf16 wire     .96  .93   .95   .96  1.00  1.04  1.03  1.02
 //   8 ranks fp32          .98  .97  1.00  1.03  1.08  1.10  1.09  1.08
+//   around the bounds: 4 ranks x 20 MiB of bf16 1.01, of fp64 .98, in place .95 and .94, 24 MiB 1.06, 1.03, 1.00 and .98;
+//   5 ranks x 14 MiB of bf16 .98, of fp64 .96, 15 MiB 1.02 and .99; 6 ranks x 12 MiB .99 both, 15 MiB 1.05 and 1.04
 //   ragged ends 4 ranks 1.00 to 1.05, 5 ranks 1.10 to 1.15; slices off the boundary 3 ranks .86 to .97, 4 ranks 1.06 to 1.14
 //   in prescribed channels, bytes a channel:  256 KiB   512 KiB    1 MiB    2 MiB
 //   3 ranks fp32, 2 to 16 channels              .80       .90      1.01     1.00
 //   5 ranks fp32, 2 to 16 channels              .91       .92      1.05     1.16
 //   6 ranks fp32, one / two channels         1.01 .96  1.05 .96  1.07 1.07  1.21
 //   and beyond a block per SM, 4 ranks in 48 channels 8 MiB .93, 16 MiB 1.10; 5 ranks in 32 channels 4 MiB .95, 8 MiB 1.05
-bool SharingPays(Algo algo, int ws, size_t bytes, size_t wire_bytes, bool words, bool aligned, int channels) {
+bool SharingPays(Algo algo, int ws, size_t bytes, size_t wire_bytes, bool words, bool in_place, bool aligned, int channels) {
   if (algo == Algo::kRabenseifner) return true;
   if (!aligned || bytes % 16 != 0 || ws > 6) return false;
   if (ws == 2) return true;
@@ -155,8 +157,8 @@ bool SharingPays(Algo algo, int ws, size_t bytes, size_t wire_bytes, bool words,
     if (bytes > most) return false;
   }
   if (ws == 3) return true;
-  if (ws == 4) return words || wire_bytes <= (size_t(16) << 20);
-  return wire_bytes <= (size_t(words ? 16 : 12) << 20);
+  if (ws == 4) return words || wire_bytes <= (size_t(in_place ? 24 : 20) << 20);
+  return wire_bytes <= (size_t(words ? 16 : ws == 5 ? 14 : 12) << 20);
 }
 
 }  // namespace
@@ -257,7 +259,8 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
   local.len_elements = n;
   local.scale = scale;
 
-  bool all_aligned = true;
+  bool all_aligned = true, in_place = true;
+  for (int q = 0; q < m.ws; ++q) in_place = in_place && sendbufs[static_cast<size_t>(q)] == recvbufs[static_cast<size_t>(q)];
   for (int q = 0; q < m.ws; ++q)
     all_aligned = all_aligned && ((reinterpret_cast<uintptr_t>(sendbufs[static_cast<size_t>(q)]) | reinterpret_cast<uintptr_t>(recvbufs[static_cast<size_t>(q)])) & 15u) == 0;
   const size_t wsize = DTypeSize(wire);
@@ -410,7 +413,7 @@ void EmuWorld::Allreduce(Algo algo, DType dtype, const std::vector<const void*>&
     if (lines) {
       CUDACHECK(LaunchLineKernel(ps.data(), m.ws, ch, m.layout.lines_half_bytes, stream));
     } else {
-      bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, n * wsize, esize == 4 && wsize == 4, all_aligned, std::min(channels, m.exec_max_blocks / m.ws));
+      bool shared = m.direct_staging == 0 && SharingPays(algo, m.ws, bytes, n * wsize, esize == 4 && wsize == 4, in_place, all_aligned, std::min(channels, m.exec_max_blocks / m.ws));
       programs(shared ? ProgramForm::kShared : ProgramForm::kStaged);
       if (!hooked_has_ops) {
         // A rank that is to stay away, or to fail its self-check, needs ops of its own for that.
